@@ -196,7 +196,7 @@ int upload_tables(asr_op* op, const double* dmat, const double* block, int nsb, 
 }
 
 void free_op(asr_op* op) {
-  void* ptrs[] = {op->d_site, op->d_level, op->d_orb, op->d_lst, op->d_ncl, op->d_typ, op->d_start, op->d_frozen, op->d_sq,
+  void* ptrs[] = {op->d_site, op->d_level, op->d_orb, op->d_lst, op->d_ncl, op->d_typ, op->d_start, op->d_frozen, op->d_nflip, op->d_sq,
                   op->d_isq, op->d_flipr, op->d_hopr, op->d_stab_ptr, op->d_flipg, op->d_hopg, op->d_stab, op->d_nsc,
                   op->d_pi, op->d_sgm, op->d_blocks, op->d_blocks_f};
   for (void* p : ptrs) if (p) cudaFree(p);
@@ -373,6 +373,7 @@ static int op_build(asr_ctx* ctx, int nsite, const int* nbr_ptr, const int* nbr,
   op->mt.assign((size_t)nsm * nsm * nsm * ncls, 0.0);
   for (int k = 0; k < ncls; ++k) class_mt(conc + (size_t)ldspc * k, nsc[k], nsm, &op->mt[(size_t)nsm * nsm * nsm * k]);
   rc = upload_tables(op, dmat, block, nblock_slots, ntype_blocks, block0);
+  if (rc == ASR_OK) rc = count_flips(ctx, op);
   if (rc != ASR_OK) { free_op(op); return rc; }
   op->c.assign(9 * (size_t)nsp, 0.0); op->d = op->c; op->o = op->c; op->e = op->c;
   op->frozen_h.assign(op->nn, 0);

@@ -27,6 +27,7 @@
 
 #include "cf.cuh"
 #include "chain.cuh"
+#include "dmma.cuh"
 
 namespace asrb {
 
@@ -51,9 +52,51 @@ __device__ __forceinline__ void stv_cs(float2* p, double2 v) { __stcs(p, make_fl
 __device__ __forceinline__ double2 ld_cs(const double2* p) { return __ldcs(p); }
 __device__ __forceinline__ double2 ld_cs(const float2* p) { float2 v = __ldcs(p); return make_double2(v.x, v.y); }
 
-__device__ __forceinline__ size_t vix(int tile, int nn, int node, int l) {
-  return (((size_t)tile * nn + node) * 9 + l) * TL;
+// element of (tile, node, orbital l, lane): FP32 vectors keep orbital-major rows of 32 lanes, FP64 vectors the layout of the
+// tensor-core products (dmma.cuh)
+template <typename V>
+__host__ __device__ __forceinline__ size_t vx(int tile, int nn, int node, int l, int lane) {
+  const size_t at = ((size_t)tile * nn + node) * MNODE;
+  return sizeof(V) % 16 == 0 || std::is_same<V, double>::value ? at + mnode_at(l, lane) : at + l * TL + lane;
 }
+// the orbital and lane of element e of a node
+template <typename ST>
+__device__ __forceinline__ void node_elem(int e, int& l, int& lane) {
+  if (std::is_same<ST, double>::value && e < 256) {
+    l = 4 * (e >> 7) + (e & 3);
+    lane = (e & 127) >> 2;
+  } else {
+    l = e / TL;
+    lane = e % TL;
+  }
+}
+// the nine values of one lane of a node, in double: v the vector's element (tile, node, 0, lane)
+template <bool CS = false>
+__device__ __forceinline__ void ld9(const float2* v, double2 (&x)[9]) {
+#pragma unroll
+  for (int l = 0; l < 9; ++l) x[l] = CS ? ld_cs(v + l * TL) : ld(v + l * TL);
+}
+template <bool CS = false>
+__device__ __forceinline__ void ld9(const double2* v, int lane, double2 (&x)[9]) {   // v: element (tile, node, 0, 0)
+#pragma unroll
+  for (int l = 0; l < 8; l += 2) {
+    if (CS) ldg2_cs(v + mnode_at(l, lane), x[l], x[l + 1]);
+    else ldg2(v + mnode_at(l, lane), x[l], x[l + 1]);
+  }
+  x[8] = CS ? ld_cs(v + 256 + lane) : ld(v + 256 + lane);
+}
+template <bool CS = false>
+__device__ __forceinline__ void ld9(const float2* v, int lane, double2 (&x)[9]) { ld9<CS>(v + lane, x); }
+__device__ __forceinline__ void st9(double2* v, int lane, const double2 (&x)[9]) {
+#pragma unroll
+  for (int l = 0; l < 8; l += 2) stg2(v + mnode_at(l, lane), x[l], x[l + 1]);
+  v[256 + lane] = x[8];
+}
+__device__ __forceinline__ void st9(float2* v, int lane, const double2 (&x)[9]) {
+#pragma unroll
+  for (int l = 0; l < 9; ++l) stv(v + l * TL + lane, x[l]);
+}
+__device__ __forceinline__ size_t vnode(int tile, int nn, int node) { return ((size_t)tile * nn + node) * MNODE; }
 
 // complex weight W_p + z W_pz (pz < 0: none) of the diagonal term for (l, own, flip) of class kap; the edc route's
 // X(z) = z pa + pb enters as pz = PA
@@ -104,7 +147,7 @@ __device__ __forceinline__ void rand_term(const OpView& op, const GroupInfo& gi,
     uint32_t sgm = op.sgm[g];
     for (int l = 0; l < 9; ++l) {
       int pl = op.pi[g * 9 + l];
-      double2 x = ld(v + vix(tile, op.nn, r, pl) + lane);
+      double2 x = ld(v + vx<T2>(tile, op.nn, r, pl, lane));
       double sgn = (((sgm >> l) & 1u) ^ (neg ? 1u : 0u)) ? -1.0 : 1.0;
       out[l] = cadd(out[l], cmul(pweight(gb, GL, p, pz, z, nsm, kap, l0, k, l), cscale(x, sgn)));
     }
@@ -130,6 +173,21 @@ __device__ __forceinline__ void block_reduce_store(double2 v, double2* part, int
   __shared__ double2 red[WPB][TL];
   int w = threadIdx.x / TL, lane = threadIdx.x % TL;
   red[w][lane] = v;
+  __syncthreads();
+  if (w == 0) {
+    double2 s = red[0][lane];
+    for (int q = 1; q < WPB; ++q) s = cadd(s, red[q][lane]);
+    part[((size_t)tile * bpt + blockIdx.x % bpt) * TL + lane] = s;
+  }
+}
+
+// the same where a thread holds the value of lane `owner` (-1: none); a lane without an owner in a warp adds zero
+__device__ __forceinline__ void block_reduce_owned(double2 v, int owner, double2* part, int tile, int bpt) {
+  __shared__ double2 red[WPB][TL];
+  int w = threadIdx.x / TL, lane = threadIdx.x % TL;
+  red[w][lane] = make_double2(0.0, 0.0);
+  __syncwarp();
+  if (owner >= 0) red[w][owner] = v;
   __syncthreads();
   if (w == 0) {
     double2 s = red[0][lane];
@@ -212,6 +270,10 @@ __device__ __forceinline__ void reduce_a_lane(const BatchView& bv, double2 asum,
   else bv.lane_act[L] = 0;
 }
 
+// 1 / b, the scale of the next Lanczos vector.  One compiled copy for every caller: the forward and the adjoint's
+// recomputation of a level must scale with the same bits, which an inlined division does not promise.
+__device__ __noinline__ double2 chain_scale(double2 b) { return cdiv(make_double2(1.0, 0.0), b); }
+
 // b_k = sqrt(w . w) (wsum: the tile's partials summed by block_sum_rows); |b| < tol ends the chain; scales of the next
 // step (u <- w / b, up <- u).  One full warp per tile.
 __device__ __forceinline__ void reduce_b_lane(const BatchView& bv, double2 wsum, int k, double btol, int tile, int lane,
@@ -228,7 +290,7 @@ __device__ __forceinline__ void reduce_b_lane(const BatchView& bv, double2 wsum,
     else if (!ok && bv.lane_closed) bv.lane_closed[L] = 1;   // the Krylov space is exhausted
     if (ok) {
       bv.sup[L] = bv.su[L];
-      bv.su[L] = cdiv(make_double2(1.0, 0.0), b);
+      bv.su[L] = chain_scale(b);
       bv.bprev[L] = b;
       act = true;
     } else {
@@ -259,41 +321,12 @@ template <> struct Pair<float> { typedef float2 T; };
 
 constexpr int RW = 12;   // padded row of a shared-memory block (16-byte aligned pairs for FP64 and FP32)
 
-// Block products of the step kernel: acc_l += sum_lp B[l][lp] x[lp] over the nine rows of one shared-memory block, the
-// nine products of a row added in the order lp = 0 .. 8.  FP64: rows of RW doubles.  FP32: rows 2p and 2p + 1 (p < 4)
+// Block products of the FP32 step kernel: acc_l += sum_lp B[l][lp] x[lp] over the nine rows of one shared-memory block, the
+// nine products of a row added in the order lp = 0 .. 8 (the FP64 kernel's products: dmma.cuh).  Rows 2p and 2p + 1 (p < 4)
 // interleaved as {B[2p][lp], B[2p+1][lp]} pairs (18 floats, padded to 20), then row 8 alone (padded to 12); one paired
 // FMA (__ffma2_rn, each half rounded as a scalar FMA) updates one component of two rows, so the bits are those of the
 // scalar products with half their FMA instructions and no more shared-memory bytes.
 template <typename ST> struct BlockAcc;
-template <> struct BlockAcc<double> {
-  static constexpr int BLK = 9 * RW;   // elements per block
-  __device__ static void put(double* blk, int l, int lp, double v) { blk[l * RW + lp] = v; }
-  double2 a[9];
-  __device__ __forceinline__ void zero() {
-#pragma unroll
-    for (int l = 0; l < 9; ++l) a[l] = make_double2(0.0, 0.0);
-  }
-  __device__ __forceinline__ void mac(const double* __restrict__ blk, const double2* x) {
-#pragma unroll
-    for (int l = 0; l < 9; ++l) {
-      const double* row = blk + l * RW;
-#pragma unroll
-      for (int lp = 0; lp < 8; lp += 2) {
-        const double2 bb = *(const double2*)(row + lp);
-        a[l].x = fma(bb.x, x[lp].x, a[l].x);
-        a[l].y = fma(bb.x, x[lp].y, a[l].y);
-        a[l].x = fma(bb.y, x[lp + 1].x, a[l].x);
-        a[l].y = fma(bb.y, x[lp + 1].y, a[l].y);
-      }
-      a[l].x = fma(row[8], x[8].x, a[l].x);
-      a[l].y = fma(row[8], x[8].y, a[l].y);
-    }
-  }
-  __device__ __forceinline__ void out(double2* acc) const {
-#pragma unroll
-    for (int l = 0; l < 9; ++l) acc[l] = a[l];
-  }
-};
 template <> struct BlockAcc<float> {
   static constexpr int BLK = 4 * 20 + 12;
   __device__ static void put(float* blk, int l, int lp, double v) {
@@ -365,7 +398,7 @@ __device__ __forceinline__ void smul_node_out(const OpView& op, const BatchView&
                                               T2* __restrict__ out, const A2* acc, double2& dot) {
   if (!FINAL) {
 #pragma unroll
-    for (int l = 0; l < 9; ++l) stv(out + vix(tile, bv.nn, i, l) + lane, make_double2(acc[l].x, acc[l].y));
+    for (int l = 0; l < 9; ++l) stv(out + vx<ST>(tile, bv.nn, i, l, lane), make_double2(acc[l].x, acc[l].y));
   } else {
     // y_l = s (d_l t2_l + P_l(U)),  P = c + e + X(z) (src/asr_augblk.f90:219-250), orbital by orbital
     const double* gb = bv.gblob + (size_t)(grp >= 0 ? grp : 0) * bv.GL.stride;
@@ -379,7 +412,7 @@ __device__ __forceinline__ void smul_node_out(const OpView& op, const BatchView&
     if (EPI == 2) { ea = bv.adj.ca[L]; eb = bv.adj.cb[L]; ec = bv.adj.cc[L]; }
 #pragma unroll
     for (int l = 0; l < 9; ++l) {
-      double2 ui = ld(in + vix(tile, bv.nn, i, l) + lane);
+      double2 ui = ld(in + vx<ST>(tile, bv.nn, i, l, lane));
       double2 pt;
       if (fs > 0) {
         pt = cmul(praw(gb, bv.GL, PCEB, withx ? PA : -1, z, fs, l), ui);
@@ -391,12 +424,12 @@ __device__ __forceinline__ void smul_node_out(const OpView& op, const BatchView&
           if (r < 0) continue;
           const unsigned long long pw = piw[op.flipg[k + nsm * i]];
           int p = (int)((pw >> (4 * l)) & 15ull);
-          double2 xr = flip_if(ld(in + vix(tile, bv.nn, r, p) + lane), (uint32_t)((pw >> (40 + l)) & 1ull));
+          double2 xr = flip_if(ld(in + vx<ST>(tile, bv.nn, r, p, lane)), (uint32_t)((pw >> (40 + l)) & 1ull));
           pt = cadd(pt, cmul(pweight(gb, bv.GL, PCEB, withx ? PA : -1, z, nsm, kap, l0, k, l), xr));
         }
       }
       double2 y = cmul(s, cadd(make_double2(acc[l].x, acc[l].y), pt));
-      const size_t q = vix(tile, bv.nn, i, l) + lane;
+      const size_t q = vx<ST>(tile, bv.nn, i, l, lane);
       if (EPI != 2) stv_cs(out + q, y);
       if (EPI >= 1) {   // the blocks carry d on both sides: t2 = S (d o U) = acc / d_l
         const double il = 1.0 / bv.ginfo[grp >= 0 ? grp : 0].dd[l];
@@ -473,7 +506,7 @@ __global__ void __launch_bounds__(WPB * TL) k_smul(OpView op, BatchView bv, cons
     BlockAcc<ST> A;
     A.zero();
     {   // on-site block
-      const T2* src = in + vix(it.tile, bv.nn, i, 0) + lane;
+      const T2* src = in + vx<ST>(it.tile, bv.nn, i, 0, lane);
       T2 v[9];
       for (int l2 = 0; l2 < 9; ++l2) v[l2] = src[l2 * TL];
       A.mac(B, v);
@@ -494,7 +527,7 @@ __global__ void __launch_bounds__(WPB * TL) k_smul(OpView op, BatchView bv, cons
       }
       if (r < 0) continue;
       const unsigned long long pw = piw[gk];
-      const T2* src = in + vix(it.tile, bv.nn, r, 0) + lane;
+      const T2* src = in + vx<ST>(it.tile, bv.nn, r, 0, lane);
       T2 v[9];
       if (LINK_ID && pw == PW_IDENTITY) {                                        // warp-uniform: one node, one slot
         for (int lp = 0; lp < 9; ++lp) v[lp] = src[lp * TL];
@@ -522,190 +555,252 @@ __global__ void __launch_bounds__(WPB * TL) k_smul(OpView op, BatchView bv, cons
   }
 }
 
-// ------------------------------------------------------------------------------------------------ staged S application
-// The same product with the neighbour rows staged in shared memory by the bulk-copy engine: one node's nine rows of a
-// tile are contiguous (9 x 32 lanes), so lane 0 of each warp copies whole rows with cp.async.bulk into a ring of NST
-// stages per warp, completion counted on one mbarrier per stage, while the warp multiplies the previous rows out of
-// shared memory.  The gathers then cost no registers and no load latency in the FMA stream.  Every wait is bounded: on
-// timeout the warp records an error, stops computing, drains its copies (bounded) and still reaches the block barrier.
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* mb, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(mb)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_init_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* mb, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(mb)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* mb) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),
-               "l"(src), "r"(bytes), "r"(smem_addr(mb))
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* mb, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_addr(mb)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-constexpr int SMUL_NST = 2;            // stages per warp
-constexpr long SMUL_WAIT_LIMIT = 1L << 24;
-
-size_t smul_smem(const asr_op* op, size_t st_size);
-
-template <typename ST>
-size_t smul_bulk_smem(const asr_op* op) {
-  typedef typename St2<ST>::T T2;
-  size_t b = smul_smem(op, sizeof(ST));
-  b = (b + 127) & ~(size_t)127;
-  b += (size_t)WPB * SMUL_NST * 9 * TL * sizeof(T2);
-  b += (size_t)WPB * SMUL_NST * sizeof(uint64_t);
-  return b;
-}
-
-// acc += B x with x the staged rows (row pi(lp) for column lp, signs of pw)
-template <typename ST, typename T2>
-__device__ __forceinline__ void mac9_staged(const ST* __restrict__ Bk, const T2* __restrict__ rows, unsigned long long pw, T2* acc) {
-  typedef typename Pair<ST>::T P2;
-  T2 x[9];
-#pragma unroll
-  for (int lp = 0; lp < 9; ++lp)
-    x[lp] = flip_if(rows[(int)((pw >> (4 * lp)) & 15ull) * TL], (uint32_t)((pw >> (40 + lp)) & 1ull));
-#pragma unroll
-  for (int l = 0; l < 9; ++l) {
-    const ST* row = Bk + l * RW;
-#pragma unroll
-    for (int lp = 0; lp < 8; lp += 2) {
-      P2 bb = *(const P2*)(row + lp);
-      acc[l].x = fma_(bb.x, x[lp].x, acc[l].x);
-      acc[l].y = fma_(bb.x, x[lp].y, acc[l].y);
-      acc[l].x = fma_(bb.y, x[lp + 1].x, acc[l].x);
-      acc[l].y = fma_(bb.y, x[lp + 1].y, acc[l].y);
-    }
-    acc[l].x = fma_(row[8], x[8].x, acc[l].x);
-    acc[l].y = fma_(row[8], x[8].y, acc[l].y);
+// ------------------------------------------------------------------------------------------------ FP64 S application
+// The same operation in FP64 on the tensor cores (dmma.cuh): one warp per node, its own rows and its present neighbours,
+// the bond blocks transposed in shared memory, the diagonal terms in the fragment's own layout.  A tile computes only the
+// octets of lanes that hold a chain (with bv.by_act: a chain that still runs): the last tile of 48 energies has two of
+// four, a real chain one.  The epilogue's arithmetic has every rounding written out (zmul, zfma), so that the forward, the
+// adjoint's recomputation and every tile shape give a lane the same bits.
+// Bound by the FP64 tensor pipe and the latency of the row gathers together (62 % of the pipe's cycles, L1 data pipe 60 %,
+// 16 warps per SM at 128 registers).  fcc ternary, 20,969 nodes, 18 slots, 16 tiles: 2.44 ms per launch (27 TFLOP/s by
+// 6,156 flops per node and lane) with the loads one product step ahead, 2.60 ms without; plain FP64 FMAs (one lane per
+// thread, broadcast block reads) 4.06 ms, with fixed-offset link gathers 3.4 ms.
+struct MmaSm {   // shared memory of k_smul_mma: byte offsets
+  int opw, links, ldl, wtab, bytes;
+  __host__ __device__ MmaSm(const OpView& op) {
+    const int ns1 = op.nslot + 1;
+    ldl = (ns1 + 3) & ~3;                                                // links per warp
+    opw = (op.ntype * ns1 + 1) * MB * (int)sizeof(double);               // after the blocks and one of zeros
+    links = (opw + (op.nop + 1) * 9 * (int)sizeof(uint32_t) + 15) & ~15;
+    wtab = links + WPB * ldl * (int)sizeof(int2);
+    bytes = wtab + (op.ncls * op.nsmax + op.nsp) * 9 * (int)sizeof(double2);
   }
-}
+};
 
-template <typename ST, bool FUSE_D, bool FINAL>
-__global__ void __launch_bounds__(WPB * TL) k_smul_bulk(OpView op, BatchView bv, const ST* __restrict__ blocks,
-                                                        const typename St2<ST>::T* __restrict__ in,
-                                                        typename St2<ST>::T* __restrict__ out, double2* part, int npw, int* err) {
-  typedef typename St2<ST>::T T2;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  const int ns1 = op.nslot + 1;
-  ST* Bs = (ST*)smem_raw;                                                        // [ntype][ns1][9][RW]
-  const size_t bs_bytes = ((size_t)op.ntype * ns1 * 9 * RW * sizeof(ST) + 15) & ~(size_t)15;
-  unsigned long long* piw = (unsigned long long*)(smem_raw + bs_bytes);
-  const size_t stage_off = (bs_bytes + (size_t)op.nop * sizeof(unsigned long long) + 127) & ~(size_t)127;
-  T2* stages = (T2*)(smem_raw + stage_off);                                     // [WPB][NST][9][TL]
-  uint64_t* mbar = (uint64_t*)(smem_raw + stage_off + (size_t)WPB * SMUL_NST * 9 * TL * sizeof(T2));
-  NodeIter it;
-  int bpt;
-  bool live = node_iter(bv, npw, it, bpt);
-  const int grp = live ? bv.tile_group[it.tile] : -1;
-  unsigned long long chimask = 0ull;
-  int gflags = 0, gfrozen = 0;
-  if (grp >= 0) {
-    chimask = bv.ginfo[grp].chimask;
-    gflags = bv.ginfo[grp].flags;
-    gfrozen = bv.ginfo[grp].frozen_sp;
-  }
-  {
-    const double* dd = grp >= 0 ? bv.ginfo[grp].dd : nullptr;
-    const int nb = op.ntype * ns1 * 81;
-    for (int q = threadIdx.x; q < nb; q += blockDim.x) {
-      int lp = q % 9, l = (q / 9) % 9, tk = q / 81;
-      double v = (double)blocks[q];
-      if (FUSE_D && dd) v *= dd[lp];
-      if (FINAL && dd) v *= dd[l];
-      Bs[((size_t)tk * 9 + l) * RW + lp] = (ST)v;
-    }
-    for (int g = threadIdx.x; g < op.nop; g += blockDim.x) {
-      unsigned long long w = 0ull;
-      for (int l = 0; l < 9; ++l) w |= (unsigned long long)op.pi[g * 9 + l] << (4 * l);
-      uint32_t sg = op.sgm[g] ^ (((chimask >> g) & 1ull) ? 0x1FFu : 0u);
-      piw[g] = w | ((unsigned long long)sg << 40);
-    }
-    if (threadIdx.x < WPB * SMUL_NST) mbar_init(mbar + threadIdx.x, 1);
-    mbar_init_fence();
-  }
-  __syncthreads();
-  if (!live) return;
-  const int lane = threadIdx.x % TL, w = threadIdx.x / TL;
-  const int L = it.tile * TL + lane;
-  T2* stg = stages + (size_t)w * SMUL_NST * 9 * TL;
-  uint64_t* mb = mbar + w * SMUL_NST;
-  const uint32_t slab = 9 * TL * sizeof(T2);
-  double2 dot = make_double2(0.0, 0.0);
-  // slab stream of this warp: for each of its nodes, the own rows (slot -1) then every slot with a neighbour
-  auto node_of = [&](int qn) { return it.first + w + WPB * qn; };
-  auto valid_node = [&](int qn) { return qn < npw && node_of(qn) < bv.nn; };
-  auto next_slot = [&](int i, int k) {   // next slot after k with a neighbour, nslot if none
-    int kk = k + 1;
-    while (kk < op.nslot && op.hopr[kk + op.nslot * i] < 0) ++kk;
-    return kk;
+// two adjacent outputs (l0, l0 + 1; NL = 2) or one (NL = 1) of a lane of a node: acc the S application's values, wt the
+// diagonal weights {W, W_pa}
+template <bool FINAL, int EPI, int NL>
+__device__ __forceinline__ void mma_out(const OpView& op, const BatchView& bv, size_t q, int tile, int i, int l0, int lane,
+                                        const double2* acc, const double* gb, const double2* wt, bool withx, bool flips,
+                                        const uint32_t* opw, const double* il, const double2* __restrict__ in,
+                                        double2* __restrict__ out, double2& dot) {
+  auto get = [&](const double2* p, double2 (&v)[NL]) {
+    if constexpr (NL == 2) ldg2(p + q, v[0], v[1]);
+    else v[0] = p[q];
   };
-  int pq = 0, pk = -1;          // producer position
-  bool pdone = !valid_node(0);
-  auto issue = [&](int s) {     // lane 0: copy the producer's slab into stage s, then advance the producer
-    const int i = node_of(pq);
-    const int r = pk < 0 ? i : op.hopr[pk + op.nslot * i];
-    if (lane == 0) {
-      mbar_expect_tx(mb + s, slab);
-      bulk_g2s(stg + (size_t)s * 9 * TL, in + vix(it.tile, bv.nn, r, 0), slab, mb + s);
-    }
-    pk = next_slot(i, pk);
-    if (pk >= op.nslot) { ++pq; pk = -1; pdone = !valid_node(pq); }
+  auto put = [&](double2* p, const double2 (&v)[NL]) {
+    if constexpr (NL == 2) stg2(p + q, v[0], v[1]);
+    else p[q] = v[0];
   };
-  for (int s = 0; s < SMUL_NST && !pdone; ++s) issue(s);
-  bool ok = true;
-  long t = 0;
-  int cq = 0, ck = -1;
-  bool cdone = !valid_node(0);
-  T2 acc[9];
-  for (int l = 0; l < 9; ++l) { acc[l].x = 0; acc[l].y = 0; }
-  while (!cdone) {
-    const int s = (int)(t % SMUL_NST);
-    const uint32_t parity = (uint32_t)((t / SMUL_NST) & 1);
-    if (ok) {
-      long n = 0;
-      while (!mbar_try_wait(mb + s, parity)) {
-        if (++n > SMUL_WAIT_LIMIT) { ok = false; if (lane == 0) dev_fail(err, DERR_WAIT); break; }
+  double2 v[NL], ui[NL], t[NL], y[NL];
+  if (!FINAL) {
+#pragma unroll
+    for (int e = 0; e < NL; ++e) v[e] = acc[e];
+    put(out, v);
+    return;
+  }
+  get(in, ui);
+  const int L = tile * TL + lane;
+  const double2 z = bv.lane_z[L], s = bv.su[L];
+#pragma unroll
+  for (int e = 0; e < NL; ++e) t[e] = zfma(make_double2(fma(z.x, wt[e].y, wt[e].x), __dmul_rn(z.y, wt[e].y)), ui[e], acc[e]);
+  if (flips) {   // the flip links of the node (rare)
+    const int nsm = op.nsmax, kap = op.ncl[i], own = op.lst[i], nk = op.nsc[kap];
+    for (int k = 0; k < nk; ++k) {
+      if (k == own) continue;
+      const int r = op.flipr[k + nsm * i];
+      if (r < 0) continue;
+      const int g = op.flipg[k + nsm * i];
+#pragma unroll
+      for (int e = 0; e < NL; ++e) {
+        const int l = l0 + e, p = op.pi[g * 9 + l];
+        const double2 x = in[vx<double2>(tile, bv.nn, r, p, lane)];
+        const uint32_t sg = opw[g * 9 + p];
+        const int q2 = ((kap * nsm + own) * nsm + k) * 9 + l;
+        const double wf = __ldg(gb + bv.GL.w(PCEB) + q2), wx = withx ? __ldg(gb + bv.GL.w(PA) + q2) : 0.0;
+        t[e] = zfma(make_double2(fma(z.x, wx, wf), __dmul_rn(z.y, wx)), make_double2(xor_sign(x.x, sg), xor_sign(x.y, sg)), t[e]);
       }
     }
-    const int i = node_of(cq);
-    if (ok) {
-      const ST* B = Bs + (size_t)op.typ[i] * ns1 * 9 * RW;
-      const unsigned long long pw = ck < 0 ? PW_IDENTITY : piw[op.hopg[ck + op.nslot * i]];
-      mac9_staged<ST>(B + (size_t)(ck + 1) * 9 * RW, stg + (size_t)s * 9 * TL + lane, pw, acc);
+  }
+#pragma unroll
+  for (int e = 0; e < NL; ++e) y[e] = zmul(s, t[e]);
+  if (EPI != 2) {
+    if constexpr (NL == 2) stg2_cs(out + q, y[0], y[1]);
+    else __stcs(out + q, y[0]);
+  }
+  if (EPI >= 1) {   // the blocks carry d on both sides: t2 = S (d o U) = acc / d_l
+#pragma unroll
+    for (int e = 0; e < NL; ++e) v[e] = zscale(acc[e], il[e]);
+    put((double2*)bv.t2out, v);
+  }
+  if (EPI == 2) {
+    const double2 ca = bv.adj.ca[L], cb = zneg(bv.adj.cb[L]), cc = zneg(bv.adj.cc[L]);
+    get((const double2*)bv.adj.yk, v);
+#pragma unroll
+    for (int e = 0; e < NL; ++e) y[e] = zfma(cb, ui[e], zfma(ca, v[e], y[e]));
+    get((const double2*)bv.adj.wbn, v);
+#pragma unroll
+    for (int e = 0; e < NL; ++e) y[e] = zfma(cc, v[e], y[e]);
+    put((double2*)bv.adj.ubk, y);
+    get((const double2*)bv.adj.xk, v);
+#pragma unroll
+    for (int e = 0; e < NL; ++e) dot = zfma(y[e], v[e], dot);
+  } else {
+#pragma unroll
+    for (int e = 0; e < NL; ++e) dot = zfma(ui[e], t[e], dot);   // times s^2 and the orbit size below
+  }
+}
+
+// the nodes of one warp for a tile with NJ octets; oct: octet j in bits 2j, 2j + 1 (NJ = 4: j itself).  Returns the dot of
+// the lane this thread owns (row t / 4 of octet c; NJ < 4: where c < NJ).
+template <bool FINAL, int EPI, int NJ>
+__device__ __forceinline__ double2 mma_nodes(const OpView& op, const BatchView& bv, const NodeIter& it, const unsigned char* smem,
+                                             const MmaSm& sm, unsigned oct, int grp, const double2* __restrict__ in,
+                                             double2* __restrict__ out) {
+  const int t = threadIdx.x % TL, w = threadIdx.x / TL, c = t & 3, row = t >> 2;
+  const int ns1 = op.nslot + 1, zero_blk = op.ntype * ns1;
+  const char* Bs = (const char*)smem;
+  const uint32_t* opw = (const uint32_t*)(smem + sm.opw);
+  const double2* wtab = (const double2*)(smem + sm.wtab);
+  int2* links = (int2*)(smem + sm.links) + w * sm.ldl;
+  auto off = [&](int j) { return NJ == 4 ? j : (int)((oct >> (2 * j)) & 3u); };
+  const GroupInfo* gi = bv.ginfo + (grp >= 0 ? grp : 0);
+  const double* gb = bv.gblob + (size_t)(grp >= 0 ? grp : 0) * bv.GL.stride;
+  const bool withx = grp >= 0 && !(gi->flags & GF_X_ZERO);
+  const int gfrozen = grp >= 0 ? gi->frozen_sp : 0;
+  double2 own = make_double2(0.0, 0.0);
+  for (int qn = 0; qn < it.npw; ++qn) {
+    const int i = it.first + w + WPB * qn;
+    if (i >= bv.nn) break;
+    // links of the node: itself, then the present slots, {element of the node's first orbital, block | operation << 16}
+    const int tb = op.typ[i] * ns1;
+    int cnt = 1;
+    __syncwarp();
+    if (t == 0) links[0] = make_int2(i, tb | (op.nop << 16));
+    for (int k0 = 0; k0 < op.nslot; k0 += TL) {
+      const int k = k0 + t;
+      const int r = k < op.nslot ? op.hopr[k + op.nslot * i] : -1;
+      const unsigned m = __ballot_sync(0xffffffffu, r >= 0);
+      if (r >= 0) links[cnt + __popc(m & ((1u << t) - 1u))] = make_int2(r, (tb + k + 1) | ((int)op.hopg[k + op.nslot * i] << 16));
+      cnt += __popc(m);
     }
     __syncwarp();
-    if (ok && !pdone) {
-      if (lane == 0) fence_proxy_async_smem();
-      issue(s);
+    const int wrow0 = op.ncl[i] * op.nsmax + op.lst[i], fr = op.frozen[i], st = op.start[i], nfl = op.nflip[i];
+    const double sq = op.sq[i];
+    NodeAcc<NJ> A;
+    A.zero();
+    A.run(links, cnt, in + vnode(it.tile, bv.nn, 0), off, Bs, opw, zero_blk, t);
+    const double2 a8 = quad_own<NJ>(A.c8, c);
+    // diagonal weights of the node at this thread's orbitals, P = c + e + X(z) (src/asr_augblk.f90:219-250)
+    double2 wt[3];
+    double il[3] = {0.0, 0.0, 0.0};
+    bool flips = false;
+    if (FINAL) {
+      const int fs = (st && gfrozen > 0) ? gfrozen : fr;
+      const double2* wr = wtab + (fs > 0 ? op.ncls * op.nsmax + fs - 1 : wrow0) * 9;
+      wt[0] = wr[2 * c]; wt[1] = wr[2 * c + 1]; wt[2] = wr[8];
+      flips = fs == 0 && nfl > 0;
+      if (EPI >= 1) { il[0] = 1.0 / gi->dd[2 * c]; il[1] = 1.0 / gi->dd[2 * c + 1]; il[2] = 1.0 / gi->dd[8]; }
     }
-    ++t;
-    ck = next_slot(i, ck);
-    if (ck >= op.nslot) {   // the node is complete
-      if (ok) smul_node_out<ST, FINAL>(op, bv, it.tile, i, lane, L, grp, gflags, gfrozen, piw, in, out, acc, dot);
-      for (int l = 0; l < 9; ++l) { acc[l].x = 0; acc[l].y = 0; }
-      ++cq;
-      ck = -1;
-      cdone = !valid_node(cq);
+    const size_t q = vnode(it.tile, bv.nn, i);
+    double2 d[NJ];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      d[j] = make_double2(0.0, 0.0);
+      const int lane = row + 8 * off(j);
+      const double2 a[2] = {A.out(j, 0), A.out(j, 1)};
+      mma_out<FINAL, EPI, 2>(op, bv, q + mnode_at(2 * c, lane), it.tile, i, 2 * c, lane, a, gb, wt, withx, flips, opw, il, in, out,
+                             d[j]);
+    }
+    double2 dn = make_double2(0.0, 0.0);
+    if (FINAL) dn = quad_own<NJ>(d, c);
+    if (c < NJ) {
+      const int lane = row + 8 * off(c);
+      mma_out<FINAL, EPI, 1>(op, bv, q + 256 + lane, it.tile, i, 8, lane, &a8, gb, wt + 2, withx, flips, opw, il + 2, in, out, dn);
+    }
+    if (FINAL) {
+      const double norb = __dmul_rn(sq, sq);
+      own = make_double2(fma(norb, dn.x, own.x), fma(norb, dn.y, own.y));
     }
   }
-  if (!ok) {   // drain: the copies issued after the failed wait (bounded)
-    for (int s = 0; s < SMUL_NST; ++s) {
-      long n = 0;
-      while (!mbar_try_wait(mb + s, (uint32_t)(((t + s) / SMUL_NST) & 1)) && ++n < SMUL_WAIT_LIMIT) {}
+  return own;
+}
+
+// Template arguments as k_smul's (no link variants: the operation sits in the B fragment).
+template <bool FUSE_D, bool FINAL, int EPI = 0>
+__global__ void __launch_bounds__(WPB * TL, 2) k_smul_mma(OpView op, BatchView bv, const double* __restrict__ blocks,
+                                                          const double2* __restrict__ in, double2* __restrict__ out,
+                                                          double2* part, int npw) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int zero_blk = op.ntype * (op.nslot + 1);
+  const MmaSm sm(op);
+  NodeIter it;
+  int bpt;
+  if (!node_iter(bv, npw, it, bpt)) return;
+  const int grp = bv.tile_group[it.tile];
+  {
+    double* Bs = (double*)smem_raw;                               // [ntype][1 + nslot][l'][MB_ROW], then zeros
+    uint32_t* opw = (uint32_t*)(smem_raw + sm.opw);               // [nop + 1][9], the identity last
+    double2* wtab = (double2*)(smem_raw + sm.wtab);               // {W, W_pa} of (class, own state), then of frozen species
+    const GroupInfo* gi = grp >= 0 ? bv.ginfo + grp : nullptr;
+    const unsigned long long chimask = gi ? gi->chimask : 0ull;
+    for (int q = threadIdx.x; q < zero_blk * 81; q += blockDim.x) {
+      const int lp = q % 9, l = (q / 9) % 9, tk = q / 81;
+      double v = blocks[q];
+      if (FUSE_D && gi) v *= gi->dd[lp];
+      if (FINAL && gi) v *= gi->dd[l];
+      Bs[tk * MB + lp * MB_ROW + l] = v;
+    }
+    for (int q = threadIdx.x; q < MB; q += blockDim.x) Bs[zero_blk * MB + q] = 0.0;
+    for (int q = threadIdx.x; q < (op.nop + 1) * 9; q += blockDim.x) {
+      const int g = q / 9, l = q % 9;
+      if (g < op.nop) opw[g * 9 + op.pi[q]] = op_word(l, ((op.sgm[g] >> l) & 1u) ^ (uint32_t)((chimask >> g) & 1ull));
+      else opw[q] = op_word(l, 0u);
+    }
+    if (FINAL) {
+      const double* gb = bv.gblob + (size_t)(grp >= 0 ? grp : 0) * bv.GL.stride;
+      const bool withx = gi && !(gi->flags & GF_X_ZERO);
+      const int nsm = op.nsmax, nw = op.ncls * nsm;
+      for (int q = threadIdx.x; q < (nw + op.nsp) * 9; q += blockDim.x) {
+        const int r = q / 9, l = q % 9, kap = r / nsm, own = r % nsm;
+        const int at = r < nw ? ((kap * nsm + own) * nsm + own) * 9 + l : (r - nw) * 9 + l;
+        wtab[q] = make_double2(gb[(r < nw ? bv.GL.w(PCEB) : bv.GL.raw(PCEB)) + at],
+                               withx ? gb[(r < nw ? bv.GL.w(PA) : bv.GL.raw(PA)) + at] : 0.0);
+      }
     }
   }
-  if (FINAL) block_reduce_store(dot, part, it.tile, bpt);
+  __syncthreads();
+  // octets of the tile that hold a chain
+  const int t = threadIdx.x % TL, c = t & 3, row = t >> 2, Lt = it.tile * TL + t;
+  const unsigned live = __ballot_sync(0xffffffffu, bv.lane_group[Lt] >= 0 && (!bv.by_act || bv.lane_act[Lt]));
+  unsigned oct = 0;
+  int nj = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if ((live >> (8 * j)) & 0xffu) oct |= (unsigned)j << (2 * nj++);
+  double2 own = make_double2(0.0, 0.0);
+  int owner = -1;
+  if (nj > 2) {
+    own = mma_nodes<FINAL, EPI, 4>(op, bv, it, smem_raw, sm, oct, grp, in, out);
+    owner = row + 8 * c;
+  } else if (nj == 2) {
+    own = mma_nodes<FINAL, EPI, 2>(op, bv, it, smem_raw, sm, oct, grp, in, out);
+    if (c < 2) owner = row + 8 * (int)((oct >> (2 * c)) & 3u);
+  } else if (nj == 1) {
+    own = mma_nodes<FINAL, EPI, 1>(op, bv, it, smem_raw, sm, oct, grp, in, out);
+    if (c == 0) owner = row + 8 * (int)(oct & 3u);
+  }
+  if (FINAL) {
+    if (EPI != 2 && owner >= 0) {
+      const double2 s = bv.su[it.tile * TL + owner];
+      own = zmul(zmul(s, s), own);
+    }
+    block_reduce_owned(own, owner, part, it.tile, bpt);
+    if (bv.tick && last_block_of_tile(bv.tick, it.tile, bpt)) {
+      const double2 a = block_sum_rows(part + (size_t)it.tile * bpt * TL, bpt, TL);
+      if (threadIdx.x < TL) reduce_a_lane<false>(bv, a, bv.kstep, it.tile, threadIdx.x);
+    }
+  }
 }
 
 // ------------------------------------------------------------------------------------------------ random operators
@@ -726,9 +821,9 @@ __global__ void __launch_bounds__(WPB * TL) k_rand(OpView op, BatchView bv, int 
     int i = it.first + w + WPB * qn;
     if (i >= bv.nn) break;
     double2 xi[9], o[9];
-    for (int l = 0; l < 9; ++l) xi[l] = ld(in + vix(it.tile, bv.nn, i, l) + lane);
+    ld9(in + vnode(it.tile, bv.nn, i), lane, xi);
     rand_term(op, gi, gb, bv.GL, p, -1, make_double2(0, 0), in, it.tile, i, lane, o, xi);
-    for (int l = 0; l < 9; ++l) stv(out + vix(it.tile, bv.nn, i, l) + lane, o[l]);
+    st9(out + vnode(it.tile, bv.nn, i), lane, o);
   }
 }
 
@@ -759,34 +854,34 @@ __global__ void __launch_bounds__(WPB * TL) k_combine(OpView op, BatchView bv, c
         if (i >= bv.nn) break;
         double2 acc[9], tmp[9], xi[9];
         if (t2) {
-          for (int l = 0; l < 9; ++l) xi[l] = ld(t2 + vix(it.tile, bv.nn, i, l) + lane);
+          ld9(t2 + vnode(it.tile, bv.nn, i), lane, xi);
           if (gi.flags & GF_D_UNIFORM) for (int l = 0; l < 9; ++l) acc[l] = cscale(xi[l], gi.dd[l]);
           else rand_term(op, gi, gb, bv.GL, PD, -1, z, t2, it.tile, i, lane, acc, xi);
         } else {
           for (int l = 0; l < 9; ++l) acc[l] = make_double2(0, 0);
         }
         if (v1) {
-          for (int l = 0; l < 9; ++l) xi[l] = ld(v1 + vix(it.tile, bv.nn, i, l) + lane);
+          ld9(v1 + vnode(it.tile, bv.nn, i), lane, xi);
           rand_term(op, gi, gb, bv.GL, pB, bx ? PA : -1, z, v1, it.tile, i, lane, tmp, xi);
           for (int l = 0; l < 9; ++l) acc[l] = cadd(acc[l], tmp[l]);
         }
         for (int l = 0; l < 9; ++l) acc[l] = cscale(acc[l], sgnAB);
         double2 ui[9];
-        for (int l = 0; l < 9; ++l) ui[l] = ld(u + vix(it.tile, bv.nn, i, l) + lane);
+        ld9(u + vnode(it.tile, bv.nn, i), lane, ui);
         if (cterm) {
           rand_term(op, gi, gb, bv.GL, PEB, (gi.flags & GF_X_ZERO) ? -1 : PA, z, u, it.tile, i, lane, tmp, ui);
           for (int l = 0; l < 9; ++l) acc[l] = cadd(acc[l], tmp[l]);
         }
-        if (h1) for (int l = 0; l < 9; ++l) acc[l] = cadd(acc[l], ld(h1 + vix(it.tile, bv.nn, i, l) + lane));
+        if (h1) for (int l = 0; l < 9; ++l) acc[l] = cadd(acc[l], ld(h1 + vx<ST>(it.tile, bv.nn, i, l, lane)));
         if (final_) {
           const double norb = op.sq[i] * op.sq[i];
           for (int l = 0; l < 9; ++l) {
             double2 y = cmul(s, acc[l]);
-            stv(out + vix(it.tile, bv.nn, i, l) + lane, y);
+            stv(out + vx<ST>(it.tile, bv.nn, i, l, lane), y);
             dot = cadd(dot, cscale(cmul(cmul(s, ui[l]), y), norb));
           }
         } else {
-          for (int l = 0; l < 9; ++l) stv(out + vix(it.tile, bv.nn, i, l) + lane, acc[l]);
+          st9(out + vnode(it.tile, bv.nn, i), lane, acc);
         }
       }
     }
@@ -847,10 +942,13 @@ __global__ void __launch_bounds__(WPB * TL) k_lanczos_w(OpView op, BatchView bv,
     if (i >= bv.nn) break;
     double2 x[9];
     if (act) {
-      for (int l = 0; l < 9; ++l) {
-        size_t q = vix(it.tile, bv.nn, i, l) + lane;
-        x[l] = csub(csub(ld_cs(y + q), cmul(as, ld(u + q))), cmul(bs, ld_cs(up + q)));
-      }
+      const size_t q = vnode(it.tile, bv.nn, i);
+      double2 uu[9], pp[9];
+      ld9<true>(y + q, lane, x);
+      ld9(u + q, lane, uu);
+      ld9<true>(up + q, lane, pp);
+#pragma unroll
+      for (int l = 0; l < 9; ++l) x[l] = csub(csub(x[l], cmul(as, uu[l])), cmul(bs, pp[l]));
       if (bv.project) project_node(op, i, chim, x);
       double2 dn = make_double2(0, 0);
       for (int l = 0; l < 9; ++l) dn = cadd(dn, cmul(x[l], x[l]));
@@ -859,7 +957,7 @@ __global__ void __launch_bounds__(WPB * TL) k_lanczos_w(OpView op, BatchView bv,
       for (int l = 0; l < 9; ++l) x[l] = make_double2(0, 0);
     }
     typename St2<ST>::T* dst = wout ? wout : y;
-    for (int l = 0; l < 9; ++l) stv(dst + vix(it.tile, bv.nn, i, l) + lane, x[l]);
+    st9(dst + vnode(it.tile, bv.nn, i), lane, x);
   }
   block_reduce_store(dot, part, it.tile, bpt);
   if (bv.tick && last_block_of_tile(bv.tick, it.tile, bpt)) {
@@ -883,9 +981,9 @@ __global__ void __launch_bounds__(WPB * TL) k_project(OpView op, BatchView bv, t
     int i = it.first + w + WPB * qn;
     if (i >= bv.nn) break;
     double2 v[9];
-    for (int l = 0; l < 9; ++l) v[l] = ld(x + vix(it.tile, bv.nn, i, l) + lane);
+    ld9(x + vnode(it.tile, bv.nn, i), lane, v);
     project_node(op, i, chim, v);
-    for (int l = 0; l < 9; ++l) stv(x + vix(it.tile, bv.nn, i, l) + lane, v[l]);
+    st9(x + vnode(it.tile, bv.nn, i), lane, v);
   }
 }
 
@@ -959,7 +1057,7 @@ __global__ void k_proj_gather(OpView op, BatchView bv, const typename St2<ST>::T
       for (int l = 0; l < 9; ++l) {
         const int pl = op.pi[l + 9 * g];
         const double wgt = tw[l + 9 * ks] * chi * (((sgm >> l) & 1u) ? -1.0 : 1.0);
-        const double2 x = ld(u + vix(tile, bv.nn, r, pl) + lane);
+        const double2 x = ld(u + vx<ST>(tile, bv.nn, r, pl, lane));
         acc[l] = cadd(acc[l], cscale(x, wgt));
       }
     }
@@ -1003,10 +1101,9 @@ template <typename ST>
 __global__ void k_init(BatchView bv, typename St2<ST>::T* u, typename St2<ST>::T* up) {
   size_t n = (size_t)bv.ntile * bv.nn * 9 * TL;
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-    int lane = (int)(q % TL);
-    size_t rest = q / TL;
-    int l = (int)(rest % 9);
-    size_t nt = rest / 9;
+    int lane, l;
+    node_elem<ST>((int)(q % MNODE), l, lane);
+    size_t nt = q / MNODE;
     int node = (int)(nt % bv.nn);
     int tile = (int)(nt / bv.nn);
     int L = tile * TL + lane;
@@ -1024,49 +1121,16 @@ size_t smul_smem(const asr_op* op, size_t st_size) {
   return b;
 }
 
-// the staged (bulk-copy) S application when ASR_SMUL_BULK=1.  Measured on the fcc ternary workload it is slower than
-// the direct gathers (FP64 5.3 / 7.1 / 7.4 ms per 16-tile launch with 2 / 3 / 4 stages against 4.55 ms; FP32 1.72 ms
-// against 1.35 ms): the per-node rows are small copies, and the stage buffers cost the occupancy that hides the gathers
-bool smul_bulk_enabled() {
-  static int on = -1;
-  if (on < 0) {
-    const char* e = getenv("ASR_SMUL_BULK");
-    on = (e && atoi(e) == 1) ? 1 : 0;
-  }
-  return on == 1;
-}
-
 template <typename ST, bool FUSE_D, bool FINAL, int EPI = 0>
 void launch_smul(asr_op* op, const BatchView& bv, const ST* blk, const typename St2<ST>::T* in, typename St2<ST>::T* out,
                  double2* part, int npw, int grid, cudaStream_t s) {
-  OpView ov = op->view();
-  const int pix = std::is_same<ST, double>::value ? 0 : 1;
-  if (EPI) {   // the adjoint's fused steps: also t2 (bv.t2out); EPI 2, the reverse epilogue (bv.adj)
-    if (op->tuned_link[pix] == 1)
-      k_smul<ST, FUSE_D, FINAL, true, EPI><<<grid, WPB * TL, smul_smem(op, sizeof(ST)), s>>>(ov, bv, blk, in, out, part, npw);
-    else
-      k_smul<ST, FUSE_D, FINAL, false, EPI><<<grid, WPB * TL, smul_smem(op, sizeof(ST)), s>>>(ov, bv, blk, in, out, part, npw);
-    return;
-  }
-  if (smul_bulk_enabled())
-    k_smul_bulk<ST, FUSE_D, FINAL><<<grid, WPB * TL, smul_bulk_smem<ST>(op), s>>>(ov, bv, blk, in, out, part, npw, op->ctx->d_err);
-  else if (op->tuned_link[pix] == 1)
-    k_smul<ST, FUSE_D, FINAL, true><<<grid, WPB * TL, smul_smem(op, sizeof(ST)), s>>>(ov, bv, blk, in, out, part, npw);
+  OpView ov = op->view();   // EPI: the adjoint's fused steps, also t2 (bv.t2out); EPI 2, the reverse epilogue (bv.adj)
+  if constexpr (std::is_same<ST, double>::value)
+    k_smul_mma<FUSE_D, FINAL, EPI><<<grid, WPB * TL, MmaSm(ov).bytes, s>>>(ov, bv, blk, in, out, part, npw);
+  else if (op->tuned_link[1] == 1)
+    k_smul<ST, FUSE_D, FINAL, true, EPI><<<grid, WPB * TL, smul_smem(op, sizeof(ST)), s>>>(ov, bv, blk, in, out, part, npw);
   else
-    k_smul<ST, FUSE_D, FINAL, false><<<grid, WPB * TL, smul_smem(op, sizeof(ST)), s>>>(ov, bv, blk, in, out, part, npw);
-}
-
-// a bounded wait of the staged kernels that ran out (the device error word), as a status
-int check_wait_error(asr_ctx* ctx) {
-  int h = 0;
-  ASR_CUDA(cudaMemcpyAsync(&h, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  ASR_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (h == DERR_WAIT) {
-    cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream);
-    set_error("chains: a bulk copy of the staged operator did not complete in time");
-    return ASR_ESTATE;
-  }
-  return ASR_OK;
+    k_smul<ST, FUSE_D, FINAL, false, EPI><<<grid, WPB * TL, smul_smem(op, sizeof(ST)), s>>>(ov, bv, blk, in, out, part, npw);
 }
 
 // One chain step of the general operator on the batch; writes y into Y and the a-partials.
@@ -1257,6 +1321,7 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
     BatchView bv{nt, nn, op->nsmax, 0, opt.mode, opt.project, opt.tail, NLMAX, opt.depth_tol, d_gblob.p, GL, d_ginfo.p,
                  d_lgroup.p, d_tgroup.p, d_z.p, d_act.p, d_wact.p, d_m.p, d_a.p, d_b.p, d_gprev.p, d_acur.p, d_bprev.p, d_su.p,
                  d_sup.p, d_tact.p, d_nfall.p};
+    bv.by_act = 1;
     k_init<ST><<<std::min<size_t>(65535, ((size_t)nt * nn * 9 * TL + 255) / 256), 256, 0, s>>>(bv, V[1].p, V[0].p);
     ctx->launches += 2;
     const int gridb = nt * bpt;
@@ -1333,7 +1398,6 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
   int nf = 0;
   ASR_CUDA(cudaMemcpyAsync(&nf, d_nfall.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   ASR_CUDA(cudaStreamSynchronize(s));
-  ASR_TRY(check_wait_error(ctx));
   for (int L = 0; L < nlane; ++L) nsteps += hm_all[L];
   if (m_out) *m_out = hm_all;
   if (nfall_out) *nfall_out = nf;
@@ -1371,7 +1435,7 @@ __global__ void __launch_bounds__(WPB * TL) k_dot(OpView op, BatchView bv, const
     if (i >= bv.nn) break;
     double2 dn = make_double2(0, 0);
     for (int l = 0; l < 9; ++l) {
-      size_t q = vix(it.tile, bv.nn, i, l) + lane;
+      size_t q = vx<ST>(it.tile, bv.nn, i, l, lane);
       dn = cadd(dn, cmul(ld(a + q), ld(b + q)));
     }
     dot = cadd(dot, cscale(dn, op.sq[i] * op.sq[i]));
@@ -1398,18 +1462,21 @@ __global__ void __launch_bounds__(WPB * TL, 2) k_adj_w(OpView op, BatchView bv, 
     int i = it.first + w + WPB * qn;
     if (i >= bv.nn) break;
     double2 x[9];
-    for (int l = 0; l < 9; ++l) {
-      size_t q = vix(it.tile, bv.nn, i, l) + lane;
-      x[l] = cadd(cmul(a1, ld(ubn + q)), cmul(a2, ld(xn + q)));
-    }
+    const size_t q = vnode(it.tile, bv.nn, i);
+    double2 v[9];
+    ld9(ubn + q, lane, x);
+    ld9(xn + q, lane, v);
+#pragma unroll
+    for (int l = 0; l < 9; ++l) x[l] = cadd(cmul(a1, x[l]), cmul(a2, v[l]));
     if (bv.project) project_node(op, i, chim, x);
+    st9(wb + q, lane, x);
     double2 e1 = make_double2(0, 0), e2 = make_double2(0, 0);
-    for (int l = 0; l < 9; ++l) {
-      size_t q = vix(it.tile, bv.nn, i, l) + lane;
-      stv(wb + q, x[l]);
-      e1 = cadd(e1, cmul(x[l], ld(xk + q)));
-      e2 = cadd(e2, cmul(x[l], ld(xkm + q)));
-    }
+    ld9(xk + q, lane, v);
+#pragma unroll
+    for (int l = 0; l < 9; ++l) e1 = cadd(e1, cmul(x[l], v[l]));
+    ld9(xkm + q, lane, v);
+#pragma unroll
+    for (int l = 0; l < 9; ++l) e2 = cadd(e2, cmul(x[l], v[l]));
     double nb = op.sq[i] * op.sq[i];
     d1 = cadd(d1, cscale(e1, nb));
     d2 = cadd(d2, cscale(e2, nb));
@@ -1434,7 +1501,7 @@ __global__ void __launch_bounds__(WPB * TL) k_adj_y(OpView op, BatchView bv, con
     int i = it.first + w + WPB * qn;
     if (i >= bv.nn) break;
     for (int l = 0; l < 9; ++l) {
-      size_t q = vix(it.tile, bv.nn, i, l) + lane;
+      size_t q = vx<ST>(it.tile, bv.nn, i, l, lane);
       double2 wv = ld(wb + q);
       stv(yb + q, cadd(wv, cmul(a3, ld(xk + q))));
       if (ubp) stv(ubp + q, csub(ld(ubp + q), cmul(a4, wv)));
@@ -1457,7 +1524,7 @@ __global__ void __launch_bounds__(WPB * TL) k_adj_u(OpView op, BatchView bv, con
     int i = it.first + w + WPB * qn;
     if (i >= bv.nn) break;
     for (int l = 0; l < 9; ++l) {
-      size_t q = vix(it.tile, bv.nn, i, l) + lane;
+      size_t q = vx<ST>(it.tile, bv.nn, i, l, lane);
       double2 v = cadd(ld(ubk + q), ld(ay + q));
       v = cadd(v, cmul(a5, ld(yk + q)));
       v = csub(v, cmul(a6, ld(wb + q)));
@@ -1516,7 +1583,7 @@ __global__ void __launch_bounds__(GPW * TL) k_adj_grad(OpView op, BatchView bv, 
     z = bv.lane_z[L];
     const int i0 = blk * nodes_per_block, i1 = min(bv.nn, i0 + nodes_per_block);
     for (int i = i0; i < i1; ++i) {
-      size_t q = vix(tile, bv.nn, i, l) + lane;
+      size_t q = vx<ST>(tile, bv.nn, i, l, lane);
       double2 y = ld(yb + q), ty = ld(tb + q);
       if (WY) {   // the fused reverse step passes wbar and S D wbar: ybar = wbar + c3 X_k, S D ybar = S D wbar + c3 S D X_k
         y = cadd(y, cmul(c3, ld(xk + q)));
@@ -1537,7 +1604,7 @@ __global__ void __launch_bounds__(GPW * TL) k_adj_grad(OpView op, BatchView bv, 
           int g = op.flipg[kp + nsm * i];
           bool neg = (gi.chimask >> g) & 1ull;
           sgn = ((((uint32_t)op.sgm[g] >> l) & 1u) ^ (neg ? 1u : 0u)) ? -1.0 : 1.0;
-          qr = vix(tile, bv.nn, r, op.pi[g * 9 + l]) + lane;
+          qr = vx<ST>(tile, bv.nn, r, op.pi[g * 9 + l], lane);
         }
         const double2 x = cscale(cmul(s, ld(xk + qr)), sgn), t = cscale(cmul(s, ld(tk + qr)), sgn);
         double2 qe = cmul(y, x);                                          // G(yb, u)
@@ -1657,7 +1724,7 @@ __device__ __forceinline__ double2 scale_of(const AdjScal& S, int L, int k) {   
   if (k <= 1) return make_double2(k == 1 ? 1.0 : 0.0, 0.0);
   double2 b = S.b[(size_t)L * NLMAX + k - 2];
   if (cmag(b) == 0.0 || k > S.m[L]) return make_double2(0, 0);
-  return cdiv(make_double2(1.0, 0.0), b);
+  return chain_scale(b);
 }
 __global__ void k_adj_scal(AdjScal S, int nlane, const int* lane_group, int k, int phase, int* tile_act = nullptr) {
   int L = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2156,7 +2223,6 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
     const int fwd = fusedrev ? 2 : nap + 2, rev = fusedrev ? 9 : nap + 11;
     ctx->launches += 1 + (int64_t)kmax * (fwd + (keep ? 0 : nap + 2) + rev);
   }
-  ASR_TRY(check_wait_error(ctx));
   return ASR_OK;
 }
 
@@ -2188,13 +2254,13 @@ __global__ void __launch_bounds__(WPB * TL) k_ed3_t3(OpView op, BatchView bv, co
     if (i >= bv.nn) break;
     double2 xu[9], xt[9], o1[9], o2[9];
     for (int l = 0; l < 9; ++l) {
-      size_t q = vix(it.tile, bv.nn, i, l) + lane;
+      size_t q = vx<ST>(it.tile, bv.nn, i, l, lane);
       xu[l] = ld(U + q);
       xt[l] = ld(T1 + q);
     }
     rand_term(op, gi, gb, bv.GL, E3_UB, E3_UA, z, U, it.tile, i, lane, o1, xu);
     rand_term(op, gi, gb, bv.GL, E3_QB, E3_QA, z, T1, it.tile, i, lane, o2, xt);
-    for (int l = 0; l < 9; ++l) stv(T3 + vix(it.tile, bv.nn, i, l) + lane, csub(o1[l], o2[l]));
+    for (int l = 0; l < 9; ++l) stv(T3 + vx<ST>(it.tile, bv.nn, i, l, lane), csub(o1[l], o2[l]));
   }
 }
 
@@ -2223,7 +2289,7 @@ __global__ void __launch_bounds__(WPB * TL) k_ed3_w(OpView op, BatchView bv, con
       if (i >= bv.nn) break;
       double2 xu[9], xt1[9], xt3[9], r1[9], r2[9], r3[9], r4[9];
       for (int l = 0; l < 9; ++l) {
-        size_t q = vix(it.tile, bv.nn, i, l) + lane;
+        size_t q = vx<ST>(it.tile, bv.nn, i, l, lane);
         xu[l] = ld(U + q);
         xt1[l] = ld(T1 + q);
         xt3[l] = ld(T3 + q);
@@ -2232,16 +2298,16 @@ __global__ void __launch_bounds__(WPB * TL) k_ed3_w(OpView op, BatchView bv, con
       rand_term(op, gi, gb, bv.GL, E3_UB, E3_UA, z, T1, it.tile, i, lane, r2, xt1);   // u T1
       rand_term(op, gi, gb, bv.GL, E3_G, -1, z, T3, it.tile, i, lane, r3, xt3);       // g T3
       if (gi.flags & GF_D_UNIFORM) {
-        for (int l = 0; l < 9; ++l) r4[l] = cscale(ld(T3a + vix(it.tile, bv.nn, i, l) + lane), gi.dd[l]);
+        for (int l = 0; l < 9; ++l) r4[l] = cscale(ld(T3a + vx<ST>(it.tile, bv.nn, i, l, lane)), gi.dd[l]);
       } else {
         double2 xa[9];
-        for (int l = 0; l < 9; ++l) xa[l] = ld(T3a + vix(it.tile, bv.nn, i, l) + lane);
+        ld9(T3a + vnode(it.tile, bv.nn, i), lane, xa);
         rand_term(op, gi, gb, bv.GL, E3_D, -1, z, T3a, it.tile, i, lane, r4, xa);
       }
       const double norb = op.sq[i] * op.sq[i];
       double2 en = make_double2(0, 0), ec = make_double2(0, 0);
       for (int l = 0; l < 9; ++l) {
-        size_t q = vix(it.tile, bv.nn, i, l) + lane;
+        size_t q = vx<ST>(it.tile, bv.nn, i, l, lane);
         double2 kx = cadd(csub(r1[l], xt1[l]), cadd(r2[l], cadd(r3[l], r4[l])));
         double2 y = cmul(s, csub(cmul(z, xu[l]), kx));
         stv(Y + q, y);
@@ -2313,7 +2379,7 @@ __global__ void __launch_bounds__(WPB * TL) k_ed3_dots(OpView op, BatchView bv, 
       if (i >= bv.nn) break;
       double2 ev = make_double2(0, 0), ea = make_double2(0, 0);
       for (int l = 0; l < 9; ++l) {
-        double2 v = ld(VV + vix(it.tile, bv.nn, i, l) + lane);
+        double2 v = ld(VV + vx<ST>(it.tile, bv.nn, i, l, lane));
         double2 a = cscale(v, o);
         if (i == 0 && l == l0) a.x += 1.0;
         ev = cadd(ev, cmul(v, v));
@@ -2336,10 +2402,9 @@ __global__ void k_ed3_start(BatchView bv, const typename St2<ST>::T* __restrict_
                             typename St2<ST>::T* TV) {
   size_t n = (size_t)bv.ntile * bv.nn * 9 * TL;
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-    int lane = (int)(q % TL);
-    size_t rest = q / TL;
-    int l = (int)(rest % 9);
-    size_t nt = rest / 9;
+    int lane, l;
+    node_elem<ST>((int)(q % MNODE), l, lane);
+    size_t nt = q / MNODE;
     int node = (int)(nt % bv.nn);
     int tile = (int)(nt / bv.nn);
     int L = tile * TL + lane;
@@ -2559,7 +2624,6 @@ int run_ed3_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, con
   ASR_CUDA(cudaMemcpyAsync(&nf, d_nfall.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   ASR_CUDA(cudaStreamSynchronize(s));
   ASR_CUDA(cudaGetLastError());
-  ASR_TRY(check_wait_error(ctx));
   if (nfall_out) *nfall_out = nf;
   return ASR_OK;
 }
@@ -2575,10 +2639,9 @@ template <typename ST>
 __global__ void k_epi_init(BatchView bv, const double* v9, typename St2<ST>::T* u, typename St2<ST>::T* up) {
   size_t n = (size_t)bv.ntile * bv.nn * 9 * TL;
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-    int lane = (int)(q % TL);
-    size_t rest = q / TL;
-    int l = (int)(rest % 9);
-    size_t nt = rest / 9;
+    int lane, l;
+    node_elem<ST>((int)(q % MNODE), l, lane);
+    size_t nt = q / MNODE;
     int node = (int)(nt % bv.nn);
     int tile = (int)(nt / bv.nn);
     int grp = bv.lane_group[tile * TL + lane];
@@ -2595,7 +2658,8 @@ __global__ void k_epi_start(BatchView bv, const typename St2<ST>::T* __restrict_
                             typename St2<ST>::T* TV) {
   size_t n = (size_t)bv.ntile * bv.nn * 9 * TL;
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-    int lane = (int)(q % TL);
+    int lane, l;
+    node_elem<ST>((int)(q % MNODE), l, lane);
     int tile = (int)(q / ((size_t)bv.nn * 9 * TL));
     int L = tile * TL + lane;
     double2 u = make_double2(0, 0), t = make_double2(0, 0);
@@ -2772,45 +2836,35 @@ int run_epi_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, con
   ASR_CUDA(cudaMemcpyAsync(&nf, d_nfall.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   ASR_CUDA(cudaStreamSynchronize(s));
   ASR_CUDA(cudaGetLastError());
-  ASR_TRY(check_wait_error(ctx));
   if (nfall_out) *nfall_out = nf;
   return ASR_OK;
 }
 
 }  // namespace
 
-// the operator kernels stage up to 96 KB of bond blocks in shared memory (set once per device)
+// the operator kernels stage up to 96 KB of bond blocks in shared memory (set once per device); the FP64 kernel adds its
+// zero block, operation words, link lists and diagonal weights
+constexpr int MMA_SMEM = 200 * 1024;
 static void smem_attrs() {
   static bool done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || done[dev]) return;
-  cudaFuncSetAttribute(k_smul<double, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<double, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<double, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+  cudaFuncSetAttribute(k_smul_mma<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
+  cudaFuncSetAttribute(k_smul_mma<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
+  cudaFuncSetAttribute(k_smul_mma<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
+  cudaFuncSetAttribute(k_smul_mma<true, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
+  cudaFuncSetAttribute(k_smul_mma<true, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul<float, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   cudaFuncSetAttribute(k_smul<float, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   cudaFuncSetAttribute(k_smul<float, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<double, true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<double, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<double, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   cudaFuncSetAttribute(k_smul<float, true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   cudaFuncSetAttribute(k_smul<float, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   cudaFuncSetAttribute(k_smul<float, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<double, true, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<double, true, true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   cudaFuncSetAttribute(k_smul<float, true, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   cudaFuncSetAttribute(k_smul<float, true, true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<double, true, true, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<double, true, true, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   cudaFuncSetAttribute(k_smul<float, true, true, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   cudaFuncSetAttribute(k_smul<float, true, true, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul_bulk<double, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  cudaFuncSetAttribute(k_smul_bulk<double, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  cudaFuncSetAttribute(k_smul_bulk<double, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  cudaFuncSetAttribute(k_smul_bulk<float, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  cudaFuncSetAttribute(k_smul_bulk<float, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  cudaFuncSetAttribute(k_smul_bulk<float, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   done[dev] = true;
 }
 
@@ -2887,7 +2941,7 @@ int apply_vectors(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
       for (int l = 0; l < 9; ++l) {   // user vectors in the reference numbering, device rows in the device node order
         const int n = op->dev_node(i);
         size_t src = (size_t)v * 9 * nn + 9 * (size_t)i + l;
-        size_t dst = (((size_t)(v / TL) * nn + n) * 9 + l) * TL + v % TL;
+        size_t dst = vx<double2>(v / TL, nn, n, l, v % TL);
         double f = what == APPLY_PROJECT ? 1.0 : 1.0 / sqv[n];
         hx[dst] = complex_in ? make_double2(f * x_host[2 * src], f * x_host[2 * src + 1]) : make_double2(f * x_host[src], 0.0);
       }
@@ -2945,7 +2999,7 @@ int apply_vectors(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
       for (int l = 0; l < 9; ++l) {
         const int n = op->dev_node(i);
         size_t dst = (size_t)v * 9 * nn + 9 * (size_t)i + l;
-        double2 val = hy[(((size_t)(v / TL) * nn + n) * 9 + l) * TL + v % TL];
+        double2 val = hy[vx<double2>(v / TL, nn, n, l, v % TL)];
         if (what != APPLY_PROJECT) val = cscale(val, sqv[n]);
         if (complex_in || what != APPLY_H) { y_host[2 * dst] = val.x; y_host[2 * dst + 1] = val.y; }
         else y_host[dst] = val.x;

@@ -69,6 +69,7 @@ struct BatchView {
                            // epilogue of the tile's last block instead of separate reduction launches
   void* t2out;             // optional: the fused step kernel also stores t2 = S (d o U) (unscaled, the vector type of the
                            // batch) for the adjoint's parameter gradient
+  int by_act;              // 1: a lane whose lane_act is 0 has left its chain for good (its vectors are not needed any more)
   AdjEpi adj;              // the adjoint epilogue's vectors and coefficients (read only by that instantiation)
 };
 

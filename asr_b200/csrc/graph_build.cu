@@ -562,6 +562,21 @@ int reorder_nodes(asr_ctx* ctx, asr_op* op) {
   return ASR_OK;
 }
 
+// flip links of every node to other nodes (the states of its class that have one)
+__global__ void k_count_flips(OpView op, int8_t* nflip) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= op.nn) return;
+  int n = 0;
+  for (int k = 0; k < op.nsc[op.ncl[i]]; ++k) n += k != op.lst[i] && op.flipr[k + op.nsmax * i] >= 0;
+  nflip[i] = (int8_t)n;
+}
+int count_flips(asr_ctx* ctx, asr_op* op) {
+  ASR_CUDA(cudaMalloc(&op->d_nflip, op->nn));
+  k_count_flips<<<(op->nn + 255) / 256, 256, 0, ctx->stream>>>(op->view(), op->d_nflip);
+  ASR_CUDA(cudaGetLastError());
+  return ASR_OK;
+}
+
 int build_operator(asr_ctx* ctx, int nsite, const int* nbr_ptr, const int* nbr, int ncls, const int* nsc, const int* cls,
                    const int* perm, int nop, int start, int maxlevel, int maxrank, const int* flippable, const int* stype,
                    asr_op* op, const int* tsite, int ntarget, int* tnode, int* tgop) {

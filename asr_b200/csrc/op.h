@@ -75,6 +75,7 @@ struct OpView {
   const int8_t* frozen;   // (nn) operator-level frozen species (0: none)
   const double* sq;       // (nn) sqrt(orbit size)
   const double* isq;      // (nn) 1 / sqrt(orbit size)
+  const int8_t* nflip;    // (nn) flip links to other nodes
   const int* flipr;       // (nsmax, nn)
   const uint8_t* flipg;
   const int* hopr;        // (nslot, nn)
@@ -120,7 +121,7 @@ struct asr_op {
   int* d_site = nullptr;
   int* d_level = nullptr;
   int* d_orb = nullptr;
-  int8_t *d_lst = nullptr, *d_ncl = nullptr, *d_typ = nullptr, *d_start = nullptr, *d_frozen = nullptr;
+  int8_t *d_lst = nullptr, *d_ncl = nullptr, *d_typ = nullptr, *d_start = nullptr, *d_frozen = nullptr, *d_nflip = nullptr;
   double *d_sq = nullptr, *d_isq = nullptr;
   int *d_flipr = nullptr, *d_hopr = nullptr, *d_stab_ptr = nullptr;
   uint8_t *d_flipg = nullptr, *d_hopg = nullptr, *d_stab = nullptr;
@@ -131,7 +132,7 @@ struct asr_op {
   float* d_blocks_f = nullptr;
   asrb::OpView view() const {
     return asrb::OpView{nn, nslot, nsmax, nop, ncls, nsp, ntype, d_site, d_lst, d_ncl, d_typ, d_start, d_frozen,
-                        d_sq, d_isq, d_flipr, d_flipg, d_hopr, d_hopg, d_stab_ptr, d_stab, d_nsc, d_pi, d_sgm};
+                        d_sq, d_isq, d_nflip, d_flipr, d_flipg, d_hopr, d_hopg, d_stab_ptr, d_stab, d_nsc, d_pi, d_sgm};
   }
 };
 
@@ -140,6 +141,8 @@ namespace asrb {
 int build_operator(asr_ctx* ctx, int nsite, const int* nbr_ptr, const int* nbr, int ncls, const int* nsc, const int* cls,
                    const int* perm, int nop, int start, int maxlevel, int maxrank, const int* flippable, const int* stype,
                    asr_op* op, const int* tsite = nullptr, int ntarget = 0, int* tnode = nullptr, int* tgop = nullptr);
+// flip links of every node (graph_build.cu), from the tables and classes on the device
+int count_flips(asr_ctx* ctx, asr_op* op);
 // host helpers (capi.cu)
 void class_mt(const double* conc, int nsc, int nsm, double* mt);
 }  // namespace asrb
