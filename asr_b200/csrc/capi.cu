@@ -733,13 +733,11 @@ static int chains_common(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups
         ASR_CUDA(cudaMemcpyAsync(d_cb.p, cb.data(), cb.size() * sizeof(double2), cudaMemcpyHostToDevice, s));
         for (int q = 0; q < ngroup; ++q)
           ASR_CUDA(cudaMemcpyAsync(d_zz.p + (size_t)q * nz, d_z, nz * sizeof(double2), cudaMemcpyDeviceToDevice, s));
-        long nt = (long)nz * ngroup;
-        k_cf_eval<<<(unsigned)((nt + 127) / 128), 128, 0, s>>>(d_ca.p, d_cb.p, d_n.p, NLMAX, ngroup, d_zz.p, nz, tail, d_g, nullptr,
-                                                               d_nf.p);
+        cf_eval(s, d_ca.p, d_cb.p, d_n.p, NLMAX, ngroup, d_zz.p, nz, tail, d_g, nullptr, d_nf.p);
         ASR_CUDA(cudaGetLastError());
         ASR_CUDA(cudaStreamSynchronize(s));
       } else {
-        k_real_tail<<<(ngroup + 63) / 64, 64, 0, s>>>(d_a.p, d_b.p, d_n.p, NLMAX, ngroup, tail, d_ai.p, d_bi.p);
+        k_real_tail<<<ngroup, 32, 0, s>>>(d_a.p, d_b.p, d_n.p, NLMAX, tail, d_ai.p, d_bi.p);
         long nt = (long)nz * ngroup;
         k_real_green<<<(unsigned)((nt + 127) / 128), 128, 0, s>>>(d_a.p, d_b.p, d_n.p, NLMAX, ngroup, d_ai.p, d_bi.p, tail, d_z, nz,
                                                                    d_g);
@@ -1291,8 +1289,7 @@ int asr_cf_eval(asr_ctx* ctx, const double* a, const double* b, const int* m, in
   ASR_CUDA(cudaMemcpyAsync(d_z.p, z, nzz * sizeof(double2), cudaMemcpyHostToDevice, s));
   ASR_CUDA(cudaMemcpyAsync(d_m.p, m, nchain * sizeof(int), cudaMemcpyHostToDevice, s));
   ASR_CUDA(cudaMemsetAsync(d_nf.p, 0, sizeof(int), s));
-  k_cf_eval<<<(unsigned)((nzz + 127) / 128), 128, 0, s>>>(d_a.p, d_b.p, d_m.p, ld, nchain, d_z.p, nz, tail, d_g.p,
-                                                          edges ? d_e.p : nullptr, d_nf.p);
+  cf_eval(s, d_a.p, d_b.p, d_m.p, ld, nchain, d_z.p, nz, tail, d_g.p, edges ? d_e.p : nullptr, d_nf.p);
   int nf = 0;
   ASR_CUDA(cudaGetLastError());
   ctx->launches += 1;

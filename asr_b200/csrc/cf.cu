@@ -22,25 +22,63 @@ __global__ void k_cf_eval(const double2* a, const double2* b, const int* m, int 
   if (nf) atomicAdd(nfall, nf);
 }
 
-// real chains: (ainf, binf) per chain for the plain route.  method: ASR_TAIL_BP beer-pettifor, ASR_TAIL_AVG2
-// sqrt-avg2, ASR_TAIL_NONE no tail.
-__global__ void k_real_tail(const double* a, const double* b, const int* n, int ld, int nchain, int method, double* ainf,
-                            double* binf) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nchain) return;
+// the same, one block per chain: its first warp finds the tail, which does not depend on the energy, then every thread
+// evaluates energies
+__global__ void k_cf_eval_chain(const double2* a, const double2* b, const int* m, int ld, const double2* z, int nz, int tail, double2* g,
+                                double2* edges, int* nfall) {
+  __shared__ double2 sh[2];
+  const int c = blockIdx.x, mc = m[c];
+  const double2 *ac = a + (size_t)ld * c, *bc = b + (size_t)ld * c;
+  const bool ok = mc >= 1 && mc <= CF_NMAX;
+  if (threadIdx.x < 32) {
+    double2 wd[CF_NMAX], we[CF_NMAX], aa, bb;
+    int nf;
+    cf_tail_pair(ok && threadIdx.x < 2, ac, bc, mc, tail, wd, we, nf, aa, bb);
+    if (threadIdx.x == 0) {
+      sh[0] = aa;
+      sh[1] = bb;
+      if (nf) atomicAdd(nfall, nf * nz);   // a fallback counts for every energy
+    }
+  }
+  __syncthreads();
+  const double2 aa = sh[0], bb = sh[1];
+  for (int j = threadIdx.x; j < nz; j += blockDim.x) {
+    const size_t t = (size_t)c * nz + j;
+    g[t] = ok ? cf_green_dev(ac, bc, mc, z[t], aa, bb) : make_double2(0.0, 0.0);
+    if (edges && ok) { edges[2 * t] = aa; edges[2 * t + 1] = bb; }
+  }
+}
+
+// One eigenvalue problem per chain costs a block per chain, one per (energy, chain) a thread: from 8 energies on the
+// first is less work and fewer dependent steps; below, many chains fill the device better by threads.
+void cf_eval(cudaStream_t s, const double2* a, const double2* b, const int* m, int ld, int nchain, const double2* z, int nz, int tail,
+             double2* g, double2* edges, int* nfall) {
+  const long n = (long)nz * nchain;
+  if (nz >= 8) k_cf_eval_chain<<<nchain, 128, 0, s>>>(a, b, m, ld, z, nz, tail, g, edges, nfall);
+  else k_cf_eval<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(a, b, m, ld, nchain, z, nz, tail, g, edges, nfall);
+}
+
+// real chains: (ainf, binf) per chain for the plain route, one warp (block) per chain.  method: ASR_TAIL_BP
+// beer-pettifor, ASR_TAIL_AVG2 sqrt-avg2, ASR_TAIL_NONE no tail.
+// Bound by the latency of the Sturm counts: 9 chains of depth 12, 1.80 ms with one thread per chain bisecting by
+// quotients, 0.23 ms with a warp's sections and division-free counts.
+__global__ void k_real_tail(const double* a, const double* b, const int* n, int ld, int method, double* ainf, double* binf) {
+  __shared__ double d[CF_NMAX], e2[CF_NMAX];
+  const int c = blockIdx.x;
   const double* ac = a + (size_t)ld * c;
   const double* bc = b + (size_t)ld * c;
   int nc = n[c];
   double A = 0.0, B = 0.0;
   if (nc >= 2 && method == ASR_TAIL_BP) {
-    double wd[CF_NMAX];
-    bp_asymptote_dev(ac, bc, nc, wd, A, B);
+    bp_asymptote_warp(ac, bc, nc, d, e2, A, B);
   } else if (nc >= 2 && method == ASR_TAIL_AVG2) {
     A = 0.5 * (ac[nc - 1] + ac[nc - 2]);
     B = sqrt(0.5 * (bc[nc - 1] * bc[nc - 1] + bc[nc - 2] * bc[nc - 2]));
   }
-  ainf[c] = A;
-  binf[c] = B;
+  if (threadIdx.x == 0) {
+    ainf[c] = A;
+    binf[c] = B;
+  }
 }
 
 __global__ void k_real_green(const double* a, const double* b, const int* n, int ld, int nchain, const double* ainf,
@@ -130,7 +168,7 @@ extern "C" int asr_cf_eval_noalloc(asr_ctx* ctx, const double* a, const double* 
   ASR_CUDA(cudaMemcpyAsync(d_z, z, nzz * sizeof(double2), cudaMemcpyHostToDevice, s));
   ASR_CUDA(cudaMemcpyAsync(d_m, m, nchain * sizeof(int), cudaMemcpyHostToDevice, s));
   ASR_CUDA(cudaMemsetAsync(d_nf, 0, sizeof(int), s));
-  k_cf_eval<<<(unsigned)((nzz + 127) / 128), 128, 0, s>>>(d_a, d_b, d_m, ld, nchain, d_z, nz, tail, d_g, nullptr, d_nf);
+  cf_eval(s, d_a, d_b, d_m, ld, nchain, d_z, nz, tail, d_g, nullptr, d_nf);
   ASR_CUDA(cudaGetLastError());
   ctx->launches += 1;
   int nf = 0;

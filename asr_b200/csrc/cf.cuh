@@ -8,12 +8,40 @@
 // bisection for the extreme eigenvalue.
 #pragma once
 #include <cfloat>
+#include <cmath>
 
 #include "common.cuh"
 
 namespace asrb {
 
 constexpr int CF_NMAX = 128;   // longest chain the device fractions take
+
+__host__ __device__ inline double inv_sqrt(double x) {
+#ifdef __CUDA_ARCH__
+  return rsqrt(x);
+#else
+  return 1.0 / std::sqrt(x);
+#endif
+}
+// |re| + |im|: within a factor sqrt(2) of the modulus, for the tests that compare with DBL_EPSILON
+__host__ __device__ __forceinline__ double cabs1(double2 a) { return fabs(a.x) + fabs(a.y); }
+
+// r = sqrt(w) (principal, as csqrt_p) and ir = 1 / r from two reciprocal square roots: with 1/|w| = |w|^2 ^ -1/2,
+// sqrt(w) = (t, |w.y| / 2t) or its mirror for t = ((|w| + |w.x|) / 2)^1/2, and 1 / sqrt(w) = conj(sqrt(w)) / |w|.  The four
+// divisions, two square roots and a hypot of csqrt_p and two cdiv of a plane rotation are its whole latency, and one
+// rotation waits for the last.  Moduli whose square leaves the double range take csqrt_p and cdiv.
+__host__ __device__ __forceinline__ void csqrt_inv(double2 w, double2& r, double2& ir) {
+  const double q = w.x * w.x + w.y * w.y;
+  if (q > 1e-290 && q < 1e290) {
+    const double rq = inv_sqrt(q), t2 = 0.5 * (q * rq + fabs(w.x)), rt = inv_sqrt(t2);
+    const double t = t2 * rt, o = 0.5 * fabs(w.y) * rt;
+    r = w.x >= 0.0 ? make_double2(t, copysign(o, w.y)) : make_double2(o, copysign(t, w.y));
+    ir = make_double2(r.x * rq, -r.y * rq);
+  } else {
+    r = csqrt_p(w);
+    ir = cmag(r) == 0.0 ? make_double2(0.0, 0.0) : cdiv(make_double2(1.0, 0.0), r);
+  }
+}
 
 // eigenvalues of the complex symmetric tridiagonal (d[0..n-1], e[0..n-2]) in place in d; e is destroyed.  0 = converged.
 __host__ __device__ inline int cs_tridiag_eig(int n, double2* d, double2* e) {
@@ -23,36 +51,38 @@ __host__ __device__ inline int cs_tridiag_eig(int n, double2* d, double2* e) {
     int iter = 0;
     for (;;) {
       int m;
-      for (m = l; m < n - 1; ++m) {
-        double dd = cmag(d[m]) + cmag(d[m + 1]);
-        if (cmag(e[m]) <= DBL_EPSILON * dd || cmag(e[m]) == 0.0) break;
-      }
+      for (m = l; m < n - 1; ++m)
+        if (cabs1(e[m]) <= DBL_EPSILON * (cabs1(d[m]) + cabs1(d[m + 1]))) break;
       if (m == l) break;
       if (++iter > 60) return 1;
       double2 g = cdiv(csub(d[l + 1], d[l]), cscale(e[l], 2.0));
-      double2 r = csqrt_p(cadd(cmul(g, g), make_double2(1.0, 0.0)));
+      double2 r, ir;
+      r = csqrt_p(cadd(cmul(g, g), make_double2(1.0, 0.0)));
       double2 gp = cadd(g, r), gm = csub(g, r);
-      double2 den = cmag(gp) >= cmag(gm) ? gp : gm;
+      double2 den = cabs1(gp) >= cabs1(gm) ? gp : gm;
       g = cadd(csub(d[m], d[l]), cdiv(e[l], den));
       double2 s = make_double2(1.0, 0.0), c = make_double2(1.0, 0.0), p = make_double2(0.0, 0.0);
+      double2 dn = d[m];   // d[i + 1] of the next rotation
       bool early = false;
       for (int i = m - 1; i >= l; --i) {
-        double2 f = cmul(s, e[i]), b = cmul(c, e[i]);
-        r = csqrt_p(cadd(cmul(f, f), cmul(g, g)));
+        const double2 ei = e[i], di = d[i];
+        double2 f = cmul(s, ei), b = cmul(c, ei);
+        csqrt_inv(cadd(cmul(f, f), cmul(g, g)), r, ir);
         e[i + 1] = r;
-        if (cmag(r) == 0.0) {
-          d[i + 1] = csub(d[i + 1], p);
+        if (r.x == 0.0 && r.y == 0.0) {
+          d[i + 1] = csub(dn, p);
           e[m] = make_double2(0.0, 0.0);
           early = true;
           break;
         }
-        s = cdiv(f, r);
-        c = cdiv(g, r);
-        g = csub(d[i + 1], p);
-        r = cadd(cmul(csub(d[i], g), s), cscale(cmul(c, b), 2.0));
+        s = cmul(f, ir);
+        c = cmul(g, ir);
+        g = csub(dn, p);
+        r = cadd(cmul(csub(di, g), s), cscale(cmul(c, b), 2.0));
         p = cmul(s, r);
         d[i + 1] = cadd(g, p);
         g = csub(cmul(c, r), b);
+        dn = di;
       }
       if (early) continue;
       d[l] = csub(d[l], p);
@@ -119,6 +149,55 @@ __host__ __device__ inline void cf_tail_dev(const double2* a, const double2* b, 
   if (tail == 0) { aa = make_double2(0.0, 0.0); bb = make_double2(0.0, 0.0); }
 }
 
+#ifdef __CUDACC__
+// cf_tail_dev by pairs of threads (2 q, 2 q + 1) of a warp, which all call it: both get the tail of their chain (live:
+// there is one).  The two eigenvalue problems of a Beer-Pettifor iteration, T + bb and T - bb in the last diagonal entry,
+// run on the two threads; a chain that has converged waits for the warp's last.  nf: tail fallbacks (both threads).
+__device__ inline void cf_tail_pair(bool live, const double2* a, const double2* b, int m, int tail, double2* wd, double2* we, int& nf,
+                                    double2& aa, double2& bb) {
+  const int sub = threadIdx.x & 1;
+  nf = 0;
+  aa = bb = make_double2(0.0, 0.0);
+  if (tail != 2) {
+    if (live) cf_tail_dev(a, b, m, tail, wd, we, nullptr, aa, bb);
+    return;
+  }
+  double2 lo, hi, a0 = aa, b0 = bb;
+  const bool eig = live && m >= 2 && chain_extremes(a, b, m, a[m - 1], wd, we, lo, hi) == 0;
+  if (eig) {
+    aa = a0 = cscale(cadd(lo, hi), 0.5);
+    bb = b0 = cscale(csub(hi, lo), 0.25);
+  } else if (live) {   // the last coefficients
+    aa = a[m - 1];
+    bb = m > 1 ? b[m - 2] : make_double2(0.0, 0.0);
+  }
+  bool done = !eig;   // the same for both threads of a pair
+  for (int it = 0; it < 200 && __any_sync(0xffffffffu, !done); ++it) {
+    double2 edge = make_double2(0.0, 0.0);   // the upper edge of T + bb (sub 0), the lower of T - bb (sub 1)
+    int bad = 0;
+    if (!done) {
+      bad = chain_extremes(a, b, m, sub ? csub(a[m - 1], bb) : cadd(a[m - 1], bb), wd, we, lo, hi);
+      edge = sub ? lo : hi;
+    }
+    __syncwarp();
+    const double2 other = make_double2(__shfl_xor_sync(0xffffffffu, edge.x, 1), __shfl_xor_sync(0xffffffffu, edge.y, 1));
+    bad |= __shfl_xor_sync(0xffffffffu, bad, 1);
+    if (done) continue;
+    if (bad) { ++nf; done = true; continue; }   // an eigenvalue failure keeps the last iterate
+    const double2 h1 = sub ? other : edge, l2 = sub ? edge : other;
+    const double2 an = cscale(cadd(h1, l2), 0.5), bn = cscale(csub(h1, l2), 0.25);
+    done = cmag(csub(an, aa)) + cmag(csub(bn, bb)) < 1.0e-12 * (1.0 + cmag(bn));
+    aa = an;
+    bb = bn;
+  }
+  if (eig && !done) {   // no fixed point within 200 iterations: the hull
+    ++nf;
+    aa = a0;
+    bb = b0;
+  }
+}
+#endif
+
 // the square-root terminator of the tail (aa, bb) at z, on the branch with |bb g| minimal (src/asr_chain.f90:103-110)
 __host__ __device__ inline double2 cf_tail_term(double2 z, double2 aa, double2 bb) {
   double2 d = csub(z, aa), tl = make_double2(0.0, 0.0);
@@ -131,17 +210,22 @@ __host__ __device__ inline double2 cf_tail_term(double2 z, double2 aa, double2 b
   return tl;
 }
 
+// g11 of the chain (a, b) of depth m at z with the square-root tail (aa, bb)
+__host__ __device__ inline double2 cf_green_dev(const double2* a, const double2* b, int m, double2 z, double2 aa, double2 bb) {
+  double2 tl = cf_tail_term(z, aa, bb);
+  double2 one = make_double2(1.0, 0.0);
+  double2 gt = cdiv(one, csub(csub(z, a[m - 1]), tl));
+  for (int j = m - 2; j >= 0; --j) gt = cdiv(one, csub(csub(z, a[j]), cmul(cmul(b[j], b[j]), gt)));
+  return gt;
+}
+
 // cf_species: g11 of the chain (a, b) of depth m at z with the tail (0 none, 1 hull, 2 bp, 3 avg2).  wd, we: work (m).
 __host__ __device__ inline double2 cf_species_dev(const double2* a, const double2* b, int m, double2 z, int tail, double2* wd,
                                                   double2* we, int* nfall, double2* edges) {
   double2 aa, bb;
   cf_tail_dev(a, b, m, tail, wd, we, nfall, aa, bb);
   if (edges) { edges[0] = aa; edges[1] = bb; }
-  double2 tl = cf_tail_term(z, aa, bb);
-  double2 one = make_double2(1.0, 0.0);
-  double2 gt = cdiv(one, csub(csub(z, a[m - 1]), tl));
-  for (int j = m - 2; j >= 0; --j) gt = cdiv(one, csub(csub(z, a[j]), cmul(cmul(b[j], b[j]), gt)));
-  return gt;
+  return cf_green_dev(a, b, m, z, aa, bb);
 }
 
 // cf_species with the projection f = sum_k c_k prod_{j<k} (b_j gt_{j+1}) gt_1 (src/asr_chain.f90:111-122); closed: the exact
@@ -215,18 +299,75 @@ __host__ __device__ inline double tridiag_extreme(int n, const double* d, const 
   }
   return 0.5 * (lo + hi);
 }
-// bp_asymptote (src/reference/asr_terminator.f90:39-67); wd: work (n)
-__host__ __device__ inline void bp_asymptote_dev(const double* a, const double* b, int n, double* wd, double& ainf, double& binf) {
+#ifdef __CUDACC__
+// Number of eigenvalues below x of the real tridiagonal (d, e2 = e^2; last diagonal entry dl) from the signs of the leading
+// minors p_j = (d_j - x) p_{j-1} - e2_{j-1} p_{j-2}, rescaled before they leave the double range; a zero minor takes the
+// sign of its predecessor.  No division: the quotients of sturm_count are a chain of dependent divisions.
+__device__ inline int sturm_minors(int n, const double* d, const double* e2, double dl, double x) {
+  int cnt = 0;
+  double p0 = 1.0, p1 = (n > 1 ? d[0] : dl) - x;
+  bool neg = p1 < 0.0;
+  cnt += neg;
+  for (int i = 1; i < n; ++i) {
+    const double p2 = ((i < n - 1 ? d[i] : dl) - x) * p1 - e2[i - 1] * p0;
+    p0 = p1;
+    p1 = p2;
+    if (p1 != 0.0 && (p1 < 0.0) != neg) { ++cnt; neg = !neg; }
+    const double m = fabs(p1);
+    if (m > 1e150) { p0 *= 1e-150; p1 *= 1e-150; }
+    else if (m < 1e-150 && fabs(p0) < 1e-150) { p0 *= 1e150; p1 *= 1e150; }
+  }
+  return cnt;
+}
+// The extreme eigenvalue of the real tridiagonal with last diagonal entry dl, by the 16 threads of a half warp (thread h of
+// 16; mask: its half): every step cuts the bracket into 17 and keeps the section where the count passes the target, to the
+// resolution of a double.  (lo, hi): Gershgorin bounds.
+__device__ inline double tridiag_extreme_half(int n, const double* d, const double* e2, double dl, double lo, double hi, bool upper,
+                                              int h, unsigned mask) {
+  const int target = upper ? n : 1;
+  for (int it = 0; it < 64; ++it) {
+    const double w = hi - lo, x = lo + w * ((h + 1) * (1.0 / 17.0));
+    const double mid = 0.5 * (lo + hi);
+    if (mid <= lo || mid >= hi) break;
+    const unsigned ge = __ballot_sync(mask, sturm_minors(n, d, e2, dl, x) >= target) & mask;   // the sections at and above the edge
+    const unsigned g = ge >> (mask == 0xffff0000u ? 16 : 0);
+    const int k = g ? __ffs(g) - 1 : 16;   // the first such point
+    const double nlo = k == 0 ? lo : lo + w * (k * (1.0 / 17.0)), nhi = k == 16 ? hi : lo + w * ((k + 1) * (1.0 / 17.0));
+    if (nlo <= lo && nhi >= hi) break;
+    lo = nlo;
+    hi = nhi;
+  }
+  return 0.5 * (lo + hi);
+}
+// bp_asymptote (src/reference/asr_terminator.f90:39-67) by one warp: the upper edge of T + B on the lower half of the warp,
+// the lower edge of T - B on the upper half; d, e2: work (n) shared by the warp
+__device__ inline void bp_asymptote_warp(const double* a, const double* b, int n, double* d, double* e2, double& ainf, double& binf) {
+  const int t = threadIdx.x & 31, h = t & 15;
+  const bool upper = t < 16;
+  const unsigned mask = upper ? 0x0000ffffu : 0xffff0000u;
+  for (int i = t; i < n; i += 32) {
+    d[i] = a[i];
+    e2[i] = b[i] * b[i];
+  }
+  __syncwarp();
   double A = 0.5 * (a[n - 1] + a[n - 2]);
   double B = sqrt(0.5 * (b[n - 1] * b[n - 1] + b[n - 2] * b[n - 2]));
   for (int it = 0; it < 500; ++it) {
-    for (int i = 0; i < n; ++i) wd[i] = a[i];
-    wd[n - 1] = a[n - 1] + B;
-    double ep = tridiag_extreme(n, wd, b, true);
-    wd[n - 1] = a[n - 1] - B;
-    double em = tridiag_extreme(n, wd, b, false);
-    double an = 0.5 * (ep + em), bn = 0.25 * (ep - em);
-    bool conv = fabs(an - A) + fabs(bn - B) < 1.0e-13;
+    const double dl = upper ? a[n - 1] + B : a[n - 1] - B;
+    double lo = dl, hi = dl;   // Gershgorin bounds, widened as tridiag_extreme's
+    for (int i = 0; i < n; ++i) {
+      const double r = (i > 0 ? fabs(b[i - 1]) : 0.0) + (i < n - 1 ? fabs(b[i]) : 0.0), x = i < n - 1 ? d[i] : dl;
+      lo = fmin(lo, x - r);
+      hi = fmax(hi, x + r);
+    }
+    const double span = hi - lo;
+    lo -= 1e-12 * (span + 1.0);
+    hi += 1e-12 * (span + 1.0);
+    const double e = tridiag_extreme_half(n, d, e2, dl, lo, hi, upper, h, mask);
+    __syncwarp();
+    const double ep = __shfl_sync(0xffffffffu, e, 0), em = __shfl_sync(0xffffffffu, e, 16);
+    const double an = 0.5 * (ep + em), bn = 0.25 * (ep - em);
+    const bool conv = fabs(an - A) + fabs(bn - B) < 1.0e-13;
     A = an;
     B = bn;
     if (conv) break;
@@ -234,6 +375,7 @@ __host__ __device__ inline void bp_asymptote_dev(const double* a, const double* 
   ainf = A;
   binf = B;
 }
+#endif
 // sqrt_tail + cf_green (src/reference/asr_greens.f90:12-22, :80-90)
 __host__ __device__ inline double2 terminated_green_dev(const double* a, const double* b, int n, double2 z, double ainf, double binf,
                                                         bool has_tail) {
@@ -427,10 +569,9 @@ __host__ __device__ inline double2 cf_species_adjoint(const double2* a, const do
 }
 
 // kernels of cf.cu
-__global__ void k_cf_eval(const double2* a, const double2* b, const int* m, int ld, int nchain, const double2* z, int nz, int tail,
-                          double2* g, double2* edges, int* nfall);
-__global__ void k_real_tail(const double* a, const double* b, const int* n, int ld, int nchain, int method, double* ainf,
-                            double* binf);
+void cf_eval(cudaStream_t s, const double2* a, const double2* b, const int* m, int ld, int nchain, const double2* z, int nz, int tail,
+             double2* g, double2* edges, int* nfall);
+__global__ void k_real_tail(const double* a, const double* b, const int* n, int ld, int method, double* ainf, double* binf);
 __global__ void k_real_green(const double* a, const double* b, const int* n, int ld, int nchain, const double* ainf,
                              const double* binf, int method, const double2* z, int nz, double2* g);
 

@@ -240,9 +240,7 @@ __device__ __forceinline__ bool last_block_of_tile(int* tick, int tile, int bpt)
   return s_last != 0;
 }
 
-// a_k (asum: the tile's partials summed by block_sum_rows) for one lane of a tile; depth test every 4 levels from 8
-// (src/asr_edc.f90:121-127) when DEPTH (without it the caller guarantees that no depth test is due at level k)
-template <bool DEPTH>
+// a_k (asum: the tile's partials summed by block_sum_rows) for one lane of a tile
 __device__ __forceinline__ void reduce_a_lane(const BatchView& bv, double2 asum, int k, int tile, int lane) {
   int L = tile * TL + lane;
   int grp = bv.lane_group[L];
@@ -252,22 +250,29 @@ __device__ __forceinline__ void reduce_a_lane(const BatchView& bv, double2 asum,
   bv.acur[L] = a;
   bv.acoef[(size_t)L * NLMAX + k - 1] = a;
   bv.lane_m[L] = k;
-  int nlev = bv.ginfo[grp].nlev;
-  bool go = true;
-  if (k == nlev) {
-    go = false;   // edc exits before b_k (src/asr_edc.f90:120); the plain chain still forms b_n (asr_recursion.f90:50-57)
-    if (bv.mode == ASR_MODE_PLAIN) bv.lane_wact[L] = 1;
-  } else if (DEPTH && bv.depth_tol > 0.0 && k >= 8 && k % 4 == 0 && bv.mode == ASR_MODE_EDC) {
-    double2 wd[NLMAX], we[NLMAX];
-    int nf = 0;
-    double2 gtry = cf_species_dev(bv.acoef + (size_t)L * NLMAX, bv.bcoef + (size_t)L * NLMAX, k, bv.lane_z[L], bv.tail, wd, we,
-                                  &nf, nullptr);
-    if (nf) atomicAdd(bv.nfall, nf);
-    if (k > 8 && cmag(csub(gtry, bv.gprev[L])) <= bv.depth_tol * cmag(gtry)) go = false;   // :123-125
-    bv.gprev[L] = gtry;
+  // edc exits before b_k (src/asr_edc.f90:120); the plain chain still forms b_n (asr_recursion.f90:50-57)
+  const bool last = k == bv.ginfo[grp].nlev;
+  if (!last || bv.mode == ASR_MODE_PLAIN) bv.lane_wact[L] = 1;
+  if (last) bv.lane_act[L] = 0;
+}
+
+// the depth test of a level at which it is due (every 4 levels from 8, src/asr_edc.f90:121-127): the lanes that go on after
+// a_k evaluate their fraction, and those whose fraction has settled end here.  One lane per block: a lane is a chain of
+// dependent plane rotations, and lanes of one warp would wait for its longest (one warp per tile took 0.41 ms a test at
+// 616 chains of depth 8-24; 0.11 ms as blocks).
+__global__ void k_depth_test(BatchView bv, int k) {
+  const int L = blockIdx.x, grp = bv.lane_group[L];
+  if (grp < 0 || !bv.tile_act[L / TL] || !bv.lane_wact[L] || !bv.lane_act[L]) return;
+  double2 wd[NLMAX], we[NLMAX];
+  int nf = 0;
+  double2 gtry = cf_species_dev(bv.acoef + (size_t)L * NLMAX, bv.bcoef + (size_t)L * NLMAX, k, bv.lane_z[L], bv.tail, wd, we,
+                                &nf, nullptr);
+  if (nf) atomicAdd(bv.nfall, nf);
+  if (k > 8 && cmag(csub(gtry, bv.gprev[L])) <= bv.depth_tol * cmag(gtry)) {   // :123-125
+    bv.lane_wact[L] = 0;
+    bv.lane_act[L] = 0;
   }
-  if (go) bv.lane_wact[L] = 1;
-  else bv.lane_act[L] = 0;
+  bv.gprev[L] = gtry;
 }
 
 // 1 / b, the scale of the next Lanczos vector.  One compiled copy for every caller: the forward and the adjoint's
@@ -550,7 +555,7 @@ __global__ void __launch_bounds__(WPB * TL) k_smul(OpView op, BatchView bv, cons
     block_reduce_store(dot, part, it.tile, bpt);
     if (bv.tick && last_block_of_tile(bv.tick, it.tile, bpt)) {
       const double2 a = block_sum_rows(part + (size_t)it.tile * bpt * TL, bpt, TL);
-      if (threadIdx.x < TL) reduce_a_lane<false>(bv, a, bv.kstep, it.tile, threadIdx.x);
+      if (threadIdx.x < TL) reduce_a_lane(bv, a, bv.kstep, it.tile, threadIdx.x);
     }
   }
 }
@@ -798,7 +803,7 @@ __global__ void __launch_bounds__(WPB * TL, 2) k_smul_mma(OpView op, BatchView b
     block_reduce_owned(own, owner, part, it.tile, bpt);
     if (bv.tick && last_block_of_tile(bv.tick, it.tile, bpt)) {
       const double2 a = block_sum_rows(part + (size_t)it.tile * bpt * TL, bpt, TL);
-      if (threadIdx.x < TL) reduce_a_lane<false>(bv, a, bv.kstep, it.tile, threadIdx.x);
+      if (threadIdx.x < TL) reduce_a_lane(bv, a, bv.kstep, it.tile, threadIdx.x);
     }
   }
 }
@@ -994,7 +999,7 @@ __global__ void k_reduce_a(BatchView bv, const double2* part, int bpt, int k) {
   int tile = blockIdx.x;
   if (tile >= bv.ntile || !bv.tile_act[tile]) return;
   const double2 a = block_sum_rows(part + (size_t)tile * bpt * TL, bpt, TL);
-  if (threadIdx.x < TL) reduce_a_lane<true>(bv, a, k, tile, threadIdx.x);
+  if (threadIdx.x < TL) reduce_a_lane(bv, a, k, tile, threadIdx.x);
 }
 
 __global__ void k_reduce_b(BatchView bv, const double2* part, int bpt, int k, double btol) {
@@ -1005,19 +1010,23 @@ __global__ void k_reduce_b(BatchView bv, const double2* part, int bpt, int k, do
   if (threadIdx.x < TL) reduce_b_lane(bv, ww, k, btol, tile, threadIdx.x, live);
 }
 
-// final fraction of every lane: cf_species with the chosen tail (edc mode); lmap: batch lane -> output lane (-1: none)
+// final fraction of every lane: cf_species with the chosen tail (edc mode); lmap: batch lane -> output lane (-1: none).
+// Bound by the dependent plane rotations of one lane's eigenvalue problem, so a block is one lane: lanes of a warp would wait
+// for its longest.  Two threads share a Beer-Pettifor tail (cf_tail_pair).  A 16-level
+// hull takes 0.16 ms (0.69 ms with one thread per lane of a full warp, hypot, square roots and divisions in every rotation), a
+// batch of 16 tiles of Beer-Pettifor tails, depths 14-26, whose slowest lanes use all 200 iterations, 53 ms (455 ms before).
 __global__ void k_cf_final(BatchView bv, int nlane, const int* lmap, double2* g) {
-  int L = blockIdx.x * blockDim.x + threadIdx.x;
-  if (L >= nlane) return;
-  int dst = lmap[L];
-  if (bv.lane_group[L] < 0 || dst < 0) return;
-  int m = bv.lane_m[L];
-  double2 wd[NLMAX], we[NLMAX];
-  int nf = 0;
-  g[dst] = m > 0 ? cf_species_dev(bv.acoef + (size_t)L * NLMAX, bv.bcoef + (size_t)L * NLMAX, m, bv.lane_z[L], bv.tail, wd, we,
-                                  &nf, nullptr)
-                 : make_double2(0, 0);
-  if (nf) atomicAdd(bv.nfall, nf);
+  const int L = blockIdx.x;
+  if (lmap[L] < 0 || bv.lane_group[L] < 0) return;
+  const int m = bv.lane_m[L];
+  const double2 *a = bv.acoef + (size_t)L * NLMAX, *b = bv.bcoef + (size_t)L * NLMAX;
+  double2 wd[NLMAX], we[NLMAX], aa, bb;
+  int nf;
+  cf_tail_pair(m > 0 && threadIdx.x < 2, a, b, m, bv.tail, wd, we, nf, aa, bb);
+  if (threadIdx.x == 0) {
+    g[lmap[L]] = m > 0 ? cf_green_dev(a, b, m, bv.lane_z[L], aa, bb) : make_double2(0, 0);
+    if (nf) atomicAdd(bv.nfall, nf);
+  }
 }
 
 // depths of the batch lanes into the run's array, and the energies of the batch lanes from the run's array
@@ -1067,33 +1076,35 @@ __global__ void k_proj_gather(OpView op, BatchView bv, const typename St2<ST>::T
   for (int l = 0; l < 9; ++l) dst[(size_t)l * TL] = acc[l];
 }
 
-// gp(l, t) = sum_k cpr(k, l, t) pv_k with pv of cf_species at depth m, and gp4 the same at max(1, m - 4)
-// (src/asr_edc.f90:221-231); one thread per lane
-__global__ void k_proj_final(BatchView bv, int nlane, const int* lmap, ProjView P) {
-  int L = blockIdx.x * blockDim.x + threadIdx.x;
-  if (L >= nlane) return;
-  int dst = lmap[L];
-  if (bv.lane_group[L] < 0 || dst < 0) return;
-  const int tile = L / TL, lane = L % TL, m = bv.lane_m[L];
-  double2 pv[NLMAX], wd[NLMAX], we[NLMAX];
+// pv of cf_species at depth m (pass 0) and at max(1, m - 4) (pass 1) for every lane (src/asr_edc.f90:221-231), into
+// pv[(pass * nlane + lane) * NLMAX + k]; one lane and pass per block (as k_depth_test)
+__global__ void k_proj_pv(BatchView bv, int nlane, double2* pv) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x, pass = q / nlane, L = q % nlane;
+  if (pass > 1 || bv.lane_group[L] < 0 || bv.lane_m[L] < 1) return;
+  const int m = bv.lane_m[L], mm = pass == 0 ? m : (m - 4 > 1 ? m - 4 : 1);
+  double2 wd[NLMAX], we[NLMAX];
   int nf = 0;
-  for (int pass = 0; pass < 2; ++pass) {
-    double2* out = (pass == 0 ? P.gp : P.gp4) + (size_t)dst * P.nt * 9;
-    const int mm = pass == 0 ? m : (m - 4 > 1 ? m - 4 : 1);
-    if (m < 1) {
-      for (int q = 0; q < 9 * P.nt; ++q) out[q] = make_double2(0.0, 0.0);
-      continue;
-    }
-    cf_species_pv_dev(bv.acoef + (size_t)L * NLMAX, bv.bcoef + (size_t)L * NLMAX, mm, bv.lane_z[L], bv.tail, pv, wd, we,
-                      pass == 0 ? &nf : nullptr);
-    for (int q = 0; q < 9 * P.nt; ++q) {
-      double2 acc = make_double2(0.0, 0.0);
-      for (int kk = 0; kk < mm; ++kk)
-        acc = cadd(acc, cmul(P.cpr[(((size_t)tile * P.kcap + kk) * 9 * P.nt + q) * TL + lane], pv[kk]));
-      out[q] = acc;
-    }
-  }
+  cf_species_pv_dev(bv.acoef + (size_t)L * NLMAX, bv.bcoef + (size_t)L * NLMAX, mm, bv.lane_z[L], bv.tail,
+                    pv + (size_t)q * NLMAX, wd, we, pass == 0 ? &nf : nullptr);
   if (nf) atomicAdd(bv.nfall, nf);
+}
+// gp(l, t) = sum_k cpr(k, l, t) pv_k, and gp4 with the shorter chain's pv; one warp per (tile, l, t), one thread per lane
+__global__ void k_proj_final(BatchView bv, int nlane, const int* lmap, ProjView P, const double2* pv) {
+  const int lane = threadIdx.x % TL;
+  const long wq = ((long)blockIdx.x * blockDim.x + threadIdx.x) / TL;
+  const int tile = (int)(wq / (9 * P.nt)), q = (int)(wq % (9 * P.nt));
+  if (tile >= bv.ntile) return;
+  const int L = tile * TL + lane, dst = lmap[L];
+  if (bv.lane_group[L] < 0 || dst < 0) return;
+  const int m = bv.lane_m[L];
+  for (int pass = 0; pass < 2; ++pass) {
+    const int mm = pass == 0 ? m : (m - 4 > 1 ? m - 4 : 1);
+    const double2* pl = pv + ((size_t)pass * nlane + L) * NLMAX;
+    double2 acc = make_double2(0.0, 0.0);
+    if (m > 0)
+      for (int kk = 0; kk < mm; ++kk) acc = cadd(acc, cmul(P.cpr[(((size_t)tile * P.kcap + kk) * 9 * P.nt + q) * TL + lane], pl[kk]));
+    ((pass == 0 ? P.gp : P.gp4) + (size_t)dst * P.nt * 9)[q] = acc;
+  }
 }
 
 // start vectors: U = e_(node 0, l0) with scale 1, UP = 0
@@ -1260,10 +1271,11 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
   struct VecRef { T2* p; };
   VecRef V[7];
   for (int q = 0; q < nvec; ++q) V[q].p = vbase + (size_t)q * vlen;
-  Dev<double2> d_cpr;
+  Dev<double2> d_cpr, d_pv;
   ProjView PV{0, 1, nlevmax, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   if (proj) {
     ASR_TRY(d_cpr.alloc((size_t)tpb * nlevmax * 9 * proj->nt * TL));
+    ASR_TRY(d_pv.alloc((size_t)2 * nlp * NLMAX));
     PV = ProjView{proj->nt, proj->nsm, nlevmax, proj->tnode, proj->tgop, proj->tw, d_cpr.p, proj->gp, proj->gp4};
   }
   ASR_CUDA(cudaMemsetAsync(d_nfall.p, 0, sizeof(int), s));
@@ -1335,12 +1347,10 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
         k_proj_gather<ST><<<(unsigned)((nwarp * TL + 255) / 256), 256, 0, s>>>(op->view(), bv, U, PV, k);
         ctx->launches += 1;
       }
-      // the fused step reduces a_k in its epilogue (the tile's last block), except at the levels of the depth test, whose
-      // fraction evaluation runs in the separate reduction kernel; k_lanczos_w always reduces b_k in its epilogue
+      // the fused step reduces a_k in its epilogue (the tile's last block), k_lanczos_w b_k
       const bool depth_due = opt.depth_tol > 0.0 && opt.mode == ASR_MODE_EDC && k >= 8 && k % 4 == 0;
-      const bool a_in_step = fused && !depth_due;
       BatchView bvs = bv;
-      bvs.tick = a_in_step ? d_tick.p : nullptr;
+      bvs.tick = fused ? d_tick.p : nullptr;
       // timed regions (asr_ctx_profile): event pairs stay pending until the statistics are read (no synchronisation)
       int ps = ctx->prof_start(s);
       ASR_TRY(step_apply<ST>(ctx, op, bvs, fused, any_o, all_dunif, U, Y, nvec > 3 ? V[3].p : nullptr, nvec > 3 ? V[4].p : nullptr,
@@ -1350,23 +1360,25 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
         ctx->prof_stop(s, ps, ASR_KERNEL_STEP, (double)nt * nn * (2.0 * 9 * TL * sizeof(T2) + tab),
                        (double)nt * nn * TL * (op->nslot + 1) * 81.0 * 4.0);
       }
-      if (!a_in_step) k_reduce_a<<<nt, RED_THREADS, 0, s>>>(bv, d_part.p, bpt, k);
+      if (!fused) k_reduce_a<<<nt, RED_THREADS, 0, s>>>(bv, d_part.p, bpt, k);
+      if (depth_due) k_depth_test<<<nt * TL, 1, 0, s>>>(bv, k);
       BatchView bvw = bv;
       bvw.tick = d_tick.p;
       ps = ctx->prof_start(s);
       k_lanczos_w<ST><<<gridb, WPB * TL, 0, s>>>(op->view(), bvw, Y, U, UP, d_part.p, npw);
       // read y, u, u', write w per (node, lane); about 30 flops per complex element (scaled updates, projection, dot)
       ctx->prof_stop(s, ps, ASR_KERNEL_LANCZOS, (double)nt * nn * 4.0 * 9 * TL * sizeof(T2), (double)nt * nn * TL * 9 * 30.0);
-      ctx->launches += (a_in_step ? 1 : 2) + (fused ? 1 : (any_o ? 7 : (all_dunif ? 2 : 3)));
+      ctx->launches += (fused ? 1 : 2) + depth_due + (fused ? 1 : (any_o ? 7 : (all_dunif ? 2 : 3)));
     }
     ASR_CUDA(cudaGetLastError());
     if (opt.mode == ASR_MODE_EDC && d_g_out) {
-      k_cf_final<<<(nlp + 63) / 64, 64, 0, s>>>(bv, nlp, d_lmap.p, d_g_out);
+      k_cf_final<<<nlp, 32, 0, s>>>(bv, nlp, d_lmap.p, d_g_out);
       ctx->launches += 1;
     }
     if (proj && opt.mode == ASR_MODE_EDC) {
-      k_proj_final<<<(nlp + 63) / 64, 64, 0, s>>>(bv, nlp, d_lmap.p, PV);
-      ctx->launches += 1;
+      k_proj_pv<<<2 * nlp, 1, 0, s>>>(bv, nlp, d_pv.p);
+      k_proj_final<<<(unsigned)(((long)nt * 9 * proj->nt * TL + 255) / 256), 256, 0, s>>>(bv, nlp, d_lmap.p, PV, d_pv.p);
+      ctx->launches += 2;
     }
     k_scatter_m<<<(nlp + 127) / 128, 128, 0, s>>>(nlp, d_lmap.p, d_m.p, d_m_all.p);
     ctx->launches += 2;
@@ -1774,6 +1786,16 @@ __global__ void k_adj_scal(AdjScal S, int nlane, const int* lane_group, int k, i
   }
 }
 
+// G and the seeds abar, bbar (cleared) of every lane of depth m >= 1 from the adjoint of its fraction with the weight w; one
+// lane per block (as k_depth_test)
+__global__ void k_cf_adjoint(BatchView bv, int nlane, const double2* w, double2* abar, double2* bbar, double2* g) {
+  const int L = blockIdx.x * blockDim.x + threadIdx.x;
+  if (L >= nlane || bv.lane_group[L] < 0 || bv.lane_m[L] < 1) return;
+  const size_t o = (size_t)L * NLMAX;
+  double2 w1[NLMAX], w2[NLMAX], w3[NLMAX], w4[NLMAX], w5[NLMAX];
+  g[L] = cf_species_adjoint(bv.acoef + o, bv.bcoef + o, bv.lane_m[L], bv.lane_z[L], bv.tail, w[L], abar + o, bbar + o, w1, w2, w3, w4, w5);
+}
+
 // forward recompute of one level: acur = a_k, bprev = b_{k-1}, su = s_k, sup = s_{k-1}, wact = k < m
 __global__ void k_set_fwd(BatchView bv, AdjScal S, int nlane, int k) {
   int L = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1894,7 +1916,7 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
   ASR_CUDA(cudaMemcpyAsync(d_spc.p, op->spc.data(), op->spc.size() * sizeof(int), cudaMemcpyHostToDevice, s));
   Dev<int> d_lgroup, d_act, d_wact, d_m, d_tact, d_tact0, d_nfall, d_tgroup, d_tick;
   Dev<double2> d_a, d_b, d_abar, d_bbar, d_gprev, d_acur, d_bprev, d_su, d_sup, d_part, d_part2, d_z, d_gpart, d_gacc;
-  Dev<double2> d_sn, d_sk, d_sp, d_c[6], d_d1, d_d2, d_d3, d_one;
+  Dev<double2> d_sn, d_sk, d_sp, d_c[6], d_d1, d_d2, d_d3, d_one, d_w, d_g;
   ASR_TRY(d_lgroup.alloc(nlp)); ASR_TRY(d_act.alloc(nlp)); ASR_TRY(d_wact.alloc(nlp)); ASR_TRY(d_m.alloc(nlp));
   ASR_TRY(d_tact.alloc(tpb)); ASR_TRY(d_tact0.alloc(tpb)); ASR_TRY(d_nfall.alloc(1)); ASR_TRY(d_tgroup.alloc(tpb));
   ASR_TRY(d_tick.alloc(tpb));
@@ -1906,6 +1928,7 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
   ASR_TRY(d_sn.alloc(nlp)); ASR_TRY(d_sk.alloc(nlp)); ASR_TRY(d_sp.alloc(nlp));
   for (int q = 0; q < 6; ++q) ASR_TRY(d_c[q].alloc(nlp));
   ASR_TRY(d_d1.alloc(nlp)); ASR_TRY(d_d2.alloc(nlp)); ASR_TRY(d_d3.alloc(nlp)); ASR_TRY(d_one.alloc(nlp));
+  ASR_TRY(d_w.alloc(nlp)); ASR_TRY(d_g.alloc(nlp));
   // the vectors: one slab (the context's held one, or allocated here and freed on return)
   const size_t vlen = (size_t)tpb * nn * 9 * TL;
   Dev<unsigned char> own;
@@ -1940,7 +1963,7 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
   std::vector<double2> ones(nlp, make_double2(1.0, 0.0));
   ASR_CUDA(cudaMemcpyAsync(d_one.p, ones.data(), nlp * sizeof(double2), cudaMemcpyHostToDevice, s));
   std::vector<int> hgroup(nlp), lmap(nlp), hm(nlp);
-  std::vector<double2> hz(nlp), ha((size_t)nlp * NLMAX), hb((size_t)nlp * NLMAX), habar((size_t)nlp * NLMAX), hbbar((size_t)nlp * NLMAX);
+  std::vector<double2> hz(nlp), hw(nlp), hg(nlp);
   std::vector<double2> hgacc((size_t)tpb * ngd);
   OpView ov = op->view();
   const ST* blk = std::is_same<ST, double>::value ? (const ST*)op->d_blocks : (const ST*)op->d_blocks_f;
@@ -1956,6 +1979,7 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
       lmap[q] = L;
       hgroup[q] = L >= 0 ? lane_group[L] : -1;
       hz[q] = L >= 0 ? lane_z[L] : make_double2(0, 0);
+      hw[q] = L >= 0 ? lane_w[L] : make_double2(0, 0);
       if (L >= 0) { tact[bt] = 1; act[q] = 1; tgroup[bt] = hgroup[q]; }
     }
     ASR_CUDA(cudaMemcpyAsync(d_lgroup.p, hgroup.data(), nlp * sizeof(int), cudaMemcpyHostToDevice, s));
@@ -1965,6 +1989,7 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
     ASR_CUDA(cudaMemcpyAsync(d_tact0.p, d_tact.p, tpb * sizeof(int), cudaMemcpyDeviceToDevice, s));
     ASR_CUDA(cudaMemsetAsync(d_tick.p, 0, tpb * sizeof(int), s));
     ASR_CUDA(cudaMemcpyAsync(d_z.p, hz.data(), nlp * sizeof(double2), cudaMemcpyHostToDevice, s));
+    ASR_CUDA(cudaMemcpyAsync(d_w.p, hw.data(), nlp * sizeof(double2), cudaMemcpyHostToDevice, s));
     ASR_CUDA(cudaMemcpyAsync(d_su.p, ones.data(), nlp * sizeof(double2), cudaMemcpyHostToDevice, s));
     ASR_CUDA(cudaMemsetAsync(d_wact.p, 0, nlp * sizeof(int), s));
     ASR_CUDA(cudaMemsetAsync(d_m.p, 0, nlp * sizeof(int), s));
@@ -1984,9 +2009,8 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
     int kmax = 0;
     for (int q = 0; q < nlp; ++q) if (hgroup[q] >= 0) kmax = std::max(kmax, ginfo[hgroup[q]].nlev);
     // ---- forward with checkpoints (X_{k0-1}, X_{k0}) at k0 = 1 + j c, or keeping every level in the segment buffers.
-    // The Lanczos update reduces b_k in its epilogue (the tile's last block), the fused step a_k except at the levels of
-    // the depth test, whose fraction evaluation runs in the separate reduction kernel: the sums are those of the separate
-    // kernels, in the same order.
+    // The Lanczos update reduces b_k in its epilogue (the tile's last block), the fused step a_k: the sums are those of the
+    // separate kernels, in the same order.
     auto depth_due = [&](int k) { return depth_tol > 0.0 && k >= 8 && k % 4 == 0; };
     // algorithmic work of the forward's kernels (the step's vector streams: read U, write Y, and t2 where kept; the node
     // tables per tile), as the forward chains count them
@@ -2000,7 +2024,6 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
       k_init<ST><<<std::min<size_t>(65535, ((size_t)nt * nn * 9 * TL + 255) / 256), 256, 0, s>>>(bv, XS(1), XS(0));
       for (int k = 1; k <= kmax; ++k) {   // the recomputation's step, with the reductions of the forward
         const int q = k - 1;
-        const bool a_in_step = fusedrev && !depth_due(k);
         int ps = ctx->prof_start(s);
         if (gen) {
           apply_general_keep<ST>(op, bv, dunif, XS(q + 1), YS(q), TS(q), HS(q), RS(q), QS(q), TMP, d_part.p, npw, grid, s);
@@ -2008,7 +2031,7 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
           BatchView bvt = bv;
           bvt.kstep = k;
           bvt.t2out = TS(q);
-          bvt.tick = a_in_step ? d_tick.p : nullptr;
+          bvt.tick = fusedrev ? d_tick.p : nullptr;
           launch_smul<ST, true, true, 1>(op, bvt, blk, XS(q + 1), YS(q), d_part.p, npw, grid, s);
         } else {
           apply_SD<ST>(op, bv, dunif, XS(q + 1), TMP, TS(q), d_part.p, npw, grid, s);
@@ -2016,7 +2039,8 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
                                                   YS(q), d_part.p, npw);
         }
         ctx->prof_stop(s, ps, ASR_KERNEL_STEP, step_bytes(3), step_flops);
-        if (!a_in_step) k_reduce_a<<<nt, RED_THREADS, 0, s>>>(bv, d_part.p, bpt, k);
+        if (!fusedrev) k_reduce_a<<<nt, RED_THREADS, 0, s>>>(bv, d_part.p, bpt, k);
+        if (depth_due(k)) k_depth_test<<<nt * TL, 1, 0, s>>>(bv, k);
         BatchView bvw = bv;
         bvw.kstep = k;
         bvw.tick = d_tick.p;
@@ -2033,21 +2057,21 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
       T2* U = FW[k % 3];
       T2* UP = FW[(k + 2) % 3];
       T2* Y = FW[(k + 1) % 3];
-      const bool a_in_step = fusedrev && !depth_due(k);
       int ps = ctx->prof_start(s);
       if (gen) {
         apply_general_keep<ST>(op, bv, dunif, U, Y, AY, WB, YB, T2B, TMP, d_part.p, npw, grid, s);
       } else if (dunif) {   // the fused step of the forward chains (d folded into the blocks)
         BatchView bvt = bv;
         bvt.kstep = k;
-        bvt.tick = a_in_step ? d_tick.p : nullptr;
+        bvt.tick = fusedrev ? d_tick.p : nullptr;
         launch_smul<ST, true, true>(op, bvt, blk, U, Y, d_part.p, npw, grid, s);
       } else {
         apply_SD<ST>(op, bv, dunif, U, TMP, AY, d_part.p, npw, grid, s);
         k_combine<ST><<<grid, WPB * TL, 0, s>>>(ov, bv, AY, U, PCEB, true, U, false, nullptr, 1.0, true, Y, d_part.p, npw);
       }
       ctx->prof_stop(s, ps, ASR_KERNEL_STEP, step_bytes(2), step_flops);
-      if (!a_in_step) k_reduce_a<<<nt, RED_THREADS, 0, s>>>(bv, d_part.p, bpt, k);
+      if (!fusedrev) k_reduce_a<<<nt, RED_THREADS, 0, s>>>(bv, d_part.p, bpt, k);
+      if (depth_due(k)) k_depth_test<<<nt * TL, 1, 0, s>>>(bv, k);
       BatchView bvw = bv;
       bvw.kstep = k;
       bvw.tick = d_tick.p;
@@ -2063,27 +2087,11 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
     // the forward retired finished tiles; the recomputation visits every tile of the batch, the reverse step k the tiles
     // with a lane at least k deep (k_adj_scal)
     ASR_CUDA(cudaMemcpyAsync(d_tact.p, d_tact0.p, tpb * sizeof(int), cudaMemcpyDeviceToDevice, s));
-    phase.next("fraction adjoint (host)");
-    // ---- fraction adjoint on the host: G and the seeds abar, bbar
-    ASR_CUDA(cudaMemcpyAsync(hm.data(), d_m.p, nlp * sizeof(int), cudaMemcpyDeviceToHost, s));
-    ASR_CUDA(cudaMemcpyAsync(ha.data(), d_a.p, ha.size() * sizeof(double2), cudaMemcpyDeviceToHost, s));
-    ASR_CUDA(cudaMemcpyAsync(hb.data(), d_b.p, hb.size() * sizeof(double2), cudaMemcpyDeviceToHost, s));
-    ASR_CUDA(cudaStreamSynchronize(s));
-    std::fill(habar.begin(), habar.end(), make_double2(0, 0));
-    std::fill(hbbar.begin(), hbbar.end(), make_double2(0, 0));
-    {
-      std::vector<double2> w1(NLMAX), w2(NLMAX), w3(NLMAX), w4(NLMAX), w5(NLMAX);
-      for (int q = 0; q < nlp; ++q) {
-        int L = lmap[q];
-        if (L < 0 || hm[q] < 1) continue;
-        m_out[L] = hm[q];
-        g_out[L] = cf_species_adjoint(&ha[(size_t)q * NLMAX], &hb[(size_t)q * NLMAX], hm[q], lane_z[L], tail, lane_w[L],
-                                      &habar[(size_t)q * NLMAX], &hbbar[(size_t)q * NLMAX], w1.data(), w2.data(), w3.data(),
-                                      w4.data(), w5.data());
-      }
-    }
-    ASR_CUDA(cudaMemcpyAsync(d_abar.p, habar.data(), habar.size() * sizeof(double2), cudaMemcpyHostToDevice, s));
-    ASR_CUDA(cudaMemcpyAsync(d_bbar.p, hbbar.data(), hbbar.size() * sizeof(double2), cudaMemcpyHostToDevice, s));
+    phase.next("fraction adjoint");
+    // ---- fraction adjoint: G and the seeds abar, bbar
+    ASR_CUDA(cudaMemsetAsync(d_abar.p, 0, (size_t)nlp * NLMAX * sizeof(double2), s));
+    ASR_CUDA(cudaMemsetAsync(d_bbar.p, 0, (size_t)nlp * NLMAX * sizeof(double2), s));
+    k_cf_adjoint<<<nlp, 1, 0, s>>>(bv, nlp, d_w.p, d_abar.p, d_bbar.p, d_g.p);
     AdjScal S{d_a.p, d_b.p, d_m.p, d_abar.p, d_bbar.p, d_sn.p, d_sk.p, d_sp.p, d_c[0].p, d_c[1].p, d_c[2].p, d_c[3].p, d_c[4].p,
               d_c[5].p, d_d1.p, d_d2.p, d_d3.p};
     // adjoint BatchView: unit scales for applying A to ybar
@@ -2209,8 +2217,12 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
     }
     ASR_CUDA(cudaGetLastError());
     ASR_CUDA(cudaMemcpyAsync(hgacc.data(), d_gacc.p, (size_t)tpb * ngd * sizeof(double2), cudaMemcpyDeviceToHost, s));
+    ASR_CUDA(cudaMemcpyAsync(hm.data(), d_m.p, nlp * sizeof(int), cudaMemcpyDeviceToHost, s));
+    ASR_CUDA(cudaMemcpyAsync(hg.data(), d_g.p, nlp * sizeof(double2), cudaMemcpyDeviceToHost, s));
     ASR_CUDA(cudaStreamSynchronize(s));
     ASR_CUDA(cudaGetLastError());
+    for (int q = 0; q < nlp; ++q)
+      if (lmap[q] >= 0 && hm[q] >= 1) { m_out[lmap[q]] = hm[q]; g_out[lmap[q]] = hg[q]; }
     for (int bt = 0; bt < nt; ++bt) {
       int gq = tgroup[bt];
       if (gq < 0) continue;
