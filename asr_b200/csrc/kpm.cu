@@ -15,6 +15,8 @@
 #include <vector>
 
 #include "common.cuh"
+#include "dmma.cuh"
+#include "ffma2.cuh"
 #include "op.h"
 
 struct asr_supercell {
@@ -131,112 +133,199 @@ __global__ void __launch_bounds__(KSITES * KV) k_cheb(ScView S, const ST* __rest
   }
 }
 
-// acc += B[l][.] . x for one padded block row (12 entries, the last 3 zero): vector loads from shared memory.  The
-// loads are volatile so that they stay next to their use: hoisting all 27 rows of a block ahead of the multiplies
-// (what the compiler does otherwise) costs 80 registers a thread and halves the occupancy.
-__device__ __forceinline__ float4 lds_f4(const float* p) {
-  float4 r;
-  unsigned a = (unsigned)__cvta_generic_to_shared(p);
-  asm volatile("ld.volatile.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "r"(a));
-  return r;
-}
-__device__ __forceinline__ double2 lds_d2(const double* p) {
-  double2 r;
-  unsigned a = (unsigned)__cvta_generic_to_shared(p);
-  asm volatile("ld.volatile.shared.v2.f64 {%0, %1}, [%2];" : "=d"(r.x), "=d"(r.y) : "r"(a));
-  return r;
-}
-__device__ __forceinline__ float row9(const float* __restrict__ row, const float* x, float acc) {
-  float4 a = lds_f4(row), b = lds_f4(row + 4), c = lds_f4(row + 8);
-  acc = fmaf(a.x, x[0], acc); acc = fmaf(a.y, x[1], acc); acc = fmaf(a.z, x[2], acc); acc = fmaf(a.w, x[3], acc);
-  acc = fmaf(b.x, x[4], acc); acc = fmaf(b.y, x[5], acc); acc = fmaf(b.z, x[6], acc); acc = fmaf(b.w, x[7], acc);
-  return fmaf(c.x, x[8], acc);
-}
-__device__ __forceinline__ double row9(const double* __restrict__ row, const double* x, double acc) {
-#pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    double2 a = lds_d2(row + 2 * q);
-    acc = fma(a.x, x[2 * q], acc);
-    if (q < 4) acc = fma(a.y, x[2 * q + 1], acc);
-  }
-  return acc;
-}
-constexpr int KRW = 12;   // padded block row (16-byte aligned)
-
 // Chebyshev step for o = 0 on d-scaled vectors u = d o t (per site and orbital, d of the site's species): with
 // h t = c t + d S (d t), the recurrence t' = 2 (H t - cen t) / sc - t_old becomes
 //   u' = 2 ((c + e - cen) o u + d^2 o S u) / sc - u_old,
 // so the gathered neighbour rows need neither their species nor a scaling.  Partial dots of t (weights 1/d^2, 1/d):
-// part[blk][v] = (r . t', t' . t', t' . t).  The next slot's neighbour index and row are loaded while the current slot
-// is multiplied.
-struct UCoef {
-  const double* cc;   // (c + e - cen) per (orbital, species)
-  const double* d2;   // d^2
-  const double* w2;   // 1 / d^2
-  const double* w1;   // 1 / d
+// part[blk][v] = (r . t', t' . t', t' . t).  Both kernels take two vectors as one 2-component value, one site per warp:
+// FP32 (k_cheb_f) the orbital-major rows and paired FMAs of ffma2.cuh, FP64 (k_cheb_d) the layout and tensor-core products
+// of dmma.cuh.
+struct UCoef {   // tables per (orbital, species), 9 nsp each: c + e - cen | d^2 | 1 / d^2 | 1 / d
+  const double* p;
+  int np;
 };
+constexpr int KW = 8;            // warps (sites) per block
+constexpr int KP = KV / 2;       // vector pairs of a site
 
-template <typename ST, bool WANT_R>
-__global__ void __launch_bounds__(KSITES * KV, sizeof(ST) == 8 ? 3 : 0) k_cheb_u(ScView S, const ST* __restrict__ blocks, const double* __restrict__ coef,
-                                                        const ST* __restrict__ u, const ST* __restrict__ uold,
-                                                        ST* __restrict__ unew, double isc, bool first, uint64_t seed, int v0,
-                                                        double* part) {
-  extern __shared__ unsigned char sm_raw[];
+// u' of one (orbital, pair) from the S application's acc, and its shares of the dots
+template <bool WANT_R>
+struct ChebOut {
+  double2 rt, tt, tp;
+  __device__ __forceinline__ void zero() { rt = tt = tp = make_double2(0.0, 0.0); }
+  template <typename T2, typename A2>
+  __device__ __forceinline__ T2 step(const double* cs, int np, int q, T2 uo, A2 acc, double2 uold, double isc, bool first, uint64_t seed,
+                                     uint64_t v, uint64_t row) {
+    const double yx = cs[q] * (double)uo.x + cs[np + q] * (double)acc.x, yy = cs[q] * (double)uo.y + cs[np + q] * (double)acc.y;
+    T2 us;
+    us.x = first ? yx * isc : 2.0 * yx * isc - uold.x;
+    us.y = first ? yy * isc : 2.0 * yy * isc - uold.y;
+    const double ux = (double)us.x, uy = (double)us.y, w2 = cs[2 * np + q];
+    tt.x += w2 * ux * ux;
+    tt.y += w2 * uy * uy;
+    tp.x += w2 * ux * (double)uo.x;
+    tp.y += w2 * uy * (double)uo.y;
+    if (WANT_R) {
+      rt.x += rademacher(seed, v, row) * ux * cs[3 * np + q];
+      rt.y += rademacher(seed, v + 1, row) * uy * cs[3 * np + q];
+    }
+    return us;
+  }
+};
+// the block's sums of the pairs' dots (pair < 0: none) into part, in a fixed order
+__device__ __forceinline__ void cheb_reduce(double2 rt, double2 tt, double2 tp, int pair, double* part) {
+  __shared__ double2 red[KW][KP][3];
+  const int w = threadIdx.x / 32, t = threadIdx.x % 32;
+  for (int k = 0; k < 3; ++k) red[w][t][k] = make_double2(0.0, 0.0);
+  __syncwarp();
+  if (pair >= 0) { red[w][pair][0] = rt; red[w][pair][1] = tt; red[w][pair][2] = tp; }
+  __syncthreads();
+  if (threadIdx.x < 3 * KP) {
+    const int v = threadIdx.x / 3, k = threadIdx.x % 3;
+    double2 s = red[0][v][k];
+    for (int q = 1; q < KW; ++q) s = cadd(s, red[q][v][k]);
+    double* out = part + ((size_t)blockIdx.x * KV + 2 * v) * 3 + k;
+    out[0] = s.x;
+    out[3] = s.y;
+  }
+}
+
+// FP32: thread = pair.  The neighbour indices of a site are read once, one per thread.  Per output the FMAs run over the
+// on-site block, then the slots, nine source orbitals each; the rows of the next slot are in flight while a slot is
+// multiplied.  Bound by the shared-memory block reads (25 broadcasts per slot and site) and the gathers' latency.  256,000
+// sites x 64 vectors: 1.73 ms per step (29 TFLOP/s) at two blocks per SM; 2.11 ms without the prefetch, 1.90 / 2.24 ms at three
+// blocks (80 registers) without / with it; one vector per thread and scalar FMAs 2.49 ms.
+template <bool WANT_R>
+__global__ void __launch_bounds__(KW * 32, 2) k_cheb_f(ScView S, const float* __restrict__ blocks, const double* __restrict__ coef,
+                                                    const float2* __restrict__ u, const float2* __restrict__ uold,
+                                                    float2* __restrict__ unew, double isc, bool first, uint64_t seed, int v0,
+                                                    double* part) {
+  extern __shared__ __align__(16) unsigned char sm_raw[];
   const int np = 9 * S.nsp;
-  double* cs = (double*)sm_raw;                 // cc | d2 | w2 | w1
-  ST* Bs = (ST*)(cs + 4 * np);                  // [1 + ns][9][KRW]
+  double* cs = (double*)sm_raw;
+  float* Bs = (float*)(cs + 4 * np);   // (9 nsp doubles four times: a multiple of 16 bytes)
   for (int q = threadIdx.x; q < 4 * np; q += blockDim.x) cs[q] = coef[q];
-  for (int q = threadIdx.x; q < (S.ns + 1) * 9 * KRW; q += blockDim.x) {
-    int c = q % KRW, r = q / KRW;
-    Bs[q] = c < 9 ? blocks[r * 9 + c] : (ST)0;
-  }
+  for (int q = threadIdx.x; q < (S.ns + 1) * 81; q += blockDim.x)
+    BlockAcc<float>::put(Bs + (q / 81) * BlockAcc<float>::BLK, (q / 9) % 9, q % 9, (double)blocks[q]);
   __syncthreads();
-  const int v = threadIdx.x % KV, row = threadIdx.x / KV;
-  double rt = 0.0, tt = 0.0, tp = 0.0;
-  for (int i = blockIdx.x * KSITES + row; i < S.n; i += gridDim.x * KSITES) {
-    ST acc[9], xa[9], xb[9], uo[9];
-    for (int l = 0; l < 9; ++l) acc[l] = (ST)0;
-    const ST* ui = u + (size_t)i * 9 * KV + v;
-    for (int l = 0; l < 9; ++l) uo[l] = ui[l * KV];
-    const int* nb = S.nbr + (size_t)S.ns * i;
-    int jn = S.ns > 0 ? nb[0] : 0;
-    if (S.ns > 0) { const ST* src = u + (size_t)jn * 9 * KV + v; for (int l = 0; l < 9; ++l) xa[l] = src[l * KV]; }
-    // on-site block
-    for (int l = 0; l < 9; ++l) acc[l] = row9(Bs + l * KRW, uo, acc[l]);
+  const int t = threadIdx.x % 32, w = threadIdx.x / 32;
+  ChebOut<WANT_R> D;
+  D.zero();
+  for (int i = blockIdx.x * KW + w; i < S.n; i += gridDim.x * KW) {
+    BlockAcc<float> A;
+    A.zero();
+    const float2* ui = u + (size_t)i * MNODE + t;
+    const int nb = t < S.ns ? S.nbr[t + (size_t)S.ns * i] : 0;
+    float2 x[9];
+#pragma unroll
+    for (int l = 0; l < 9; ++l) x[l] = ui[l * KP];
+    A.mac(Bs, x);
+    float2 y[9];
+    auto fetch = [&](int k, float2 (&v)[9]) {
+      const int j = k < 32 ? __shfl_sync(0xffffffffu, nb, k) : S.nbr[k + (size_t)S.ns * i];
+      const float2* src = u + (size_t)j * MNODE + t;
+#pragma unroll
+      for (int l = 0; l < 9; ++l) v[l] = src[l * KP];
+    };
+    if (S.ns) fetch(0, x);
 #pragma unroll 1
-    for (int k = 0; k < S.ns; ++k) {
+    for (int k = 0; k < S.ns; k += 2) {
+      if (k + 1 < S.ns) fetch(k + 1, y);
+      A.mac(Bs + (k + 1) * BlockAcc<float>::BLK, x);
       if (k + 1 < S.ns) {
-        jn = nb[k + 1];
-        const ST* src = u + (size_t)jn * 9 * KV + v;
-        for (int l = 0; l < 9; ++l) xb[l] = src[l * KV];
+        if (k + 2 < S.ns) fetch(k + 2, x);
+        A.mac(Bs + (k + 2) * BlockAcc<float>::BLK, y);
       }
-      const ST* Bk = Bs + (size_t)(k + 1) * 9 * KRW;
-      for (int l = 0; l < 9; ++l) acc[l] = row9(Bk + l * KRW, xa, acc[l]);
-      for (int l = 0; l < 9; ++l) xa[l] = xb[l];
     }
+    float2 acc[9];
+    A.out(acc);
     const int si = S.spc[i];
-    ST* uni = unew + (size_t)i * 9 * KV + v;
-    const ST* uoi = first ? nullptr : uold + (size_t)i * 9 * KV + v;
+#pragma unroll
     for (int l = 0; l < 9; ++l) {
-      const int q = l + 9 * si;
-      double y = cs[q] * (double)uo[l] + cs[np + q] * (double)acc[l];
-      double un = first ? y * isc : 2.0 * y * isc - (double)uoi[l * KV];
-      ST us = (ST)un;
-      uni[l * KV] = us;
-      double ur = (double)us;
-      tt += cs[2 * np + q] * ur * ur;
-      tp += cs[2 * np + q] * ur * (double)uo[l];
-      if (WANT_R) rt += rademacher(seed, (uint64_t)(v0 + v), (uint64_t)i * 9 + l) * ur * cs[3 * np + q];
+      const float2 uo = ui[l * KP];
+      float2 ol = make_float2(0.f, 0.f);
+      if (!first) ol = uold[(size_t)i * MNODE + l * KP + t];
+      unew[(size_t)i * MNODE + l * KP + t] = D.step(cs, np, l + 9 * si, uo, acc[l], make_double2(ol.x, ol.y), isc, first, seed,
+                                                    (uint64_t)(v0 + 2 * t), (uint64_t)i * 9 + l);
     }
   }
-  __shared__ double red[KSITES][KV][3];
-  red[row][v][0] = rt; red[row][v][1] = tt; red[row][v][2] = tp;
+  cheb_reduce(D.rt, D.tt, D.tp, t, part);
+}
+
+// FP64: NJ octets of pairs (16 vectors each).  Bound by the FP64 tensor pipe and the gathers' latency, as the chain step.
+// 48,668 sites x 64 vectors: 0.40 ms per step (24 TFLOP/s); plain FP64 FMAs, one vector per thread, 1.31 ms.
+template <bool WANT_R, int NJ>
+__global__ void __launch_bounds__(KW * 32, 2) k_cheb_d(ScView S, const double* __restrict__ blocks, const double* __restrict__ coef,
+                                                       const double2* __restrict__ u, const double2* __restrict__ uold,
+                                                       double2* __restrict__ unew, double isc, bool first, uint64_t seed, int v0,
+                                                       double* part) {
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  const int np = 9 * S.nsp, ns1 = S.ns + 1, ldl = (ns1 + 3) & ~3;
+  double* cs = (double*)sm_raw;
+  double* Bs = cs + 4 * np;                                   // [1 + ns][l'][MB_ROW], then zeros
+  uint32_t* opw = (uint32_t*)(Bs + (ns1 + 1) * MB);           // the identity
+  int2* links = (int2*)(opw + 12) + (threadIdx.x / 32) * ldl;
+  for (int q = threadIdx.x; q < 4 * np; q += blockDim.x) cs[q] = coef[q];
+  for (int q = threadIdx.x; q < ns1 * 81; q += blockDim.x) Bs[(q / 81) * MB + (q % 9) * MB_ROW + (q / 9) % 9] = blocks[q];
+  for (int q = threadIdx.x; q < MB; q += blockDim.x) Bs[ns1 * MB + q] = 0.0;
+  if (threadIdx.x < 9) opw[threadIdx.x] = op_word(threadIdx.x, 0u);
   __syncthreads();
-  if (row == 0) {
-    for (int r = 1; r < KSITES; ++r) { rt += red[r][v][0]; tt += red[r][v][1]; tp += red[r][v][2]; }
-    double* out = part + ((size_t)blockIdx.x * KV + v) * 3;
-    out[0] = rt; out[1] = tt; out[2] = tp;
+  const int t = threadIdx.x % 32, w = threadIdx.x / 32, c = t & 3, n = t >> 2;
+  auto off = [](int j) { return j; };
+  ChebOut<WANT_R> D;   // of the pair this thread owns: row n of octet c (c < NJ)
+  D.zero();
+  for (int i = blockIdx.x * KW + w; i < S.n; i += gridDim.x * KW) {
+    __syncwarp();
+    for (int k = t; k < ns1; k += 32) links[k] = make_int2(k ? S.nbr[k - 1 + (size_t)S.ns * i] : i, k);
+    __syncwarp();
+    const int si = S.spc[i];
+    NodeAcc<NJ> A;
+    A.zero();
+    A.run(links, ns1, u, off, (const char*)Bs, opw, ns1, t);
+    const double2 a8 = quad_own<NJ>(A.c8, c);
+    const size_t q = (size_t)i * MNODE;
+    double2 rt[NJ], tt[NJ], tp[NJ];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const int pair = n + 8 * j;
+      const size_t at = q + mnode_at(2 * c, pair);
+      double2 uo[2], ol[2], un[2];
+      ldg2(u + at, uo[0], uo[1]);
+      ol[0] = ol[1] = make_double2(0.0, 0.0);
+      if (!first) ldg2_cs(uold + at, ol[0], ol[1]);
+      ChebOut<WANT_R> P;
+      P.zero();
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        un[e] = P.step(cs, np, 2 * c + e + 9 * si, uo[e], A.out(j, e), ol[e], isc, first, seed, (uint64_t)(v0 + 2 * pair),
+                       (uint64_t)i * 9 + 2 * c + e);
+      stg2(unew + at, un[0], un[1]);
+      rt[j] = P.rt; tt[j] = P.tt; tp[j] = P.tp;
+    }
+    const double2 otp = quad_own<NJ>(tp, c), ott = quad_own<NJ>(tt, c);
+    D.tp = cadd(D.tp, otp);
+    D.tt = cadd(D.tt, ott);
+    if (WANT_R) D.rt = cadd(D.rt, quad_own<NJ>(rt, c));
+    if (c < NJ) {
+      const size_t at = q + 256 + n + 8 * c;
+      double2 ol = make_double2(0.0, 0.0);
+      if (!first) ol = __ldcs(uold + at);
+      unew[at] = D.step(cs, np, 8 + 9 * si, u[at], a8, ol, isc, first, seed, (uint64_t)(v0 + 2 * (n + 8 * c)), (uint64_t)i * 9 + 8);
+    }
   }
+  cheb_reduce(D.rt, D.tt, D.tp, c < NJ ? n + 8 * c : -1, part);
+}
+
+// shared memory of the two kernels
+size_t cheb_f_smem(int nsp, int ns) { return (size_t)36 * nsp * sizeof(double) + (size_t)(ns + 1) * BlockAcc<float>::BLK * sizeof(float); }
+size_t cheb_d_smem(int nsp, int ns) {
+  return (size_t)36 * nsp * sizeof(double) + (size_t)(ns + 2) * MB * sizeof(double) + 12 * sizeof(uint32_t) +
+         (size_t)KW * ((ns + 4) & ~3) * sizeof(int2);
+}
+
+// element (site, orbital, vector) of the d-scaled vectors, as the kernels above keep them
+template <typename ST>
+__device__ __forceinline__ size_t cheb_at(size_t site, int l, int v) {
+  return std::is_same<ST, double>::value ? 2 * (site * MNODE + mnode_at(l, v >> 1)) + (v & 1) : (site * 9 + l) * KV + v;
 }
 
 // u_0 = d o r (d of each site's species)
@@ -248,7 +337,7 @@ __global__ void k_rademacher_init_scaled(ScView S, uint64_t seed, int v0, ST* t)
     size_t e = q / KV;   // site * 9 + l
     int site = (int)(e / 9), l = (int)(e % 9);
     double d = S.par[9 * S.nsp + l + 9 * S.spc[site]];
-    t[q] = (ST)(d * rademacher(seed, (uint64_t)(v0 + v), (uint64_t)e));
+    t[cheb_at<ST>(site, l, v)] = (ST)(d * rademacher(seed, (uint64_t)(v0 + v), (uint64_t)e));
   }
 }
 
@@ -314,16 +403,28 @@ __global__ void k_rademacher_init(int n, uint64_t seed, int v0, ST* t) {
   }
 }
 
-// sum of the block partials per vector in a fixed order: out[v][3]
+// sum of the block partials per vector in a fixed order: out[v][3].  32 of the 3 KV columns per block, the rows over its
+// warps with eight loads in flight (one thread per vector over all rows in turn took 0.11 ms a step, 4-9 % of a run).
 __global__ void k_kpm_reduce(const double* part, int nblk, double* out) {
-  int v = threadIdx.x;
-  if (v >= KV) return;
-  double a = 0, b = 0, c = 0;
-  for (int q = 0; q < nblk; ++q) {
-    const double* p = part + ((size_t)q * KV + v) * 3;
-    a += p[0]; b += p[1]; c += p[2];
+  __shared__ double sm[8][32];
+  const int t = threadIdx.x % 32, w = threadIdx.x / 32, col = blockIdx.x * 32 + t;
+  const double* p = part + col;
+  double s = 0.0;
+  int q = w;
+  for (; q + 56 < nblk; q += 64) {
+    double v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = p[(size_t)(q + 8 * j) * KV * 3];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s += v[j];
   }
-  out[v * 3 + 0] = a; out[v * 3 + 1] = b; out[v * 3 + 2] = c;
+  for (; q < nblk; q += 8) s += p[(size_t)q * KV * 3];
+  sm[w][t] = s;
+  __syncthreads();
+  if (w == 0) {
+    for (int j = 1; j < 8; ++j) s += sm[j][t];
+    out[col] = s;
+  }
 }
 
 template <typename T>
@@ -339,6 +440,25 @@ struct DevBuf {
   }
 };
 
+// blocks of the scaled steps: as many as run at once (each prepares its tables once and takes every grid-th group of sites)
+int cheb_grid(const asr_ctx* ctx) { return ctx->num_sms * 2; }
+
+// one scaled step on nv <= KV vectors
+void cheb_scaled(asr_ctx* ctx, const ScView& S, const float* blocks, const double* coef, const float* u, const float* uold, float* unew,
+                 double isc, bool first, bool want_r, int, uint64_t seed, int v0, double* part, int grid) {
+  auto k = want_r ? k_cheb_f<true> : k_cheb_f<false>;
+  k<<<grid, KW * 32, cheb_f_smem(S.nsp, S.ns), ctx->stream>>>(S, blocks, coef, (const float2*)u, (const float2*)uold, (float2*)unew, isc,
+                                                             first, seed, v0, part);
+}
+void cheb_scaled(asr_ctx* ctx, const ScView& S, const double* blocks, const double* coef, const double* u, const double* uold,
+                 double* unew, double isc, bool first, bool want_r, int nv, uint64_t seed, int v0, double* part, int grid) {
+  // octets of vector pairs in use: 16 vectors each; three run as four
+  auto k = nv <= 16 ? (want_r ? k_cheb_d<true, 1> : k_cheb_d<false, 1>)
+         : nv <= 32 ? (want_r ? k_cheb_d<true, 2> : k_cheb_d<false, 2>) : (want_r ? k_cheb_d<true, 4> : k_cheb_d<false, 4>);
+  k<<<grid, KW * 32, cheb_d_smem(S.nsp, S.ns), ctx->stream>>>(S, blocks, coef, (const double2*)u, (const double2*)uold, (double2*)unew, isc,
+                                                             first, seed, v0, part);
+}
+
 template <typename ST>
 int kpm_run(asr_ctx* ctx, asr_supercell* sc, double cen, double scl, int nmom, int v0, int nvec, uint64_t seed, bool doubling,
             double* mu) {
@@ -348,8 +468,8 @@ int kpm_run(asr_ctx* ctx, asr_supercell* sc, double cen, double scl, int nmom, i
   const ST* blocks = std::is_same<ST, double>::value ? (const ST*)sc->d_blocks : (const ST*)sc->d_blocks_f;
   const size_t nel = (size_t)n * 9 * KV;
   const size_t smem = 4 * 9 * sc->nsp * sizeof(double) + (size_t)(sc->ns + 1) * 81 * sizeof(ST);
-  const int grid = ctx->num_sms * 4;
   const bool general = !sc->o_zero;
+  const int grid = ctx->num_sms * 4;
   DevBuf<ST> T0, T1, T2, W1, W2, W3;
   ASR_TRY(T0.alloc(nel)); ASR_TRY(T1.alloc(nel)); ASR_TRY(T2.alloc(nel));
   if (general) { ASR_TRY(W1.alloc(nel)); ASR_TRY(W2.alloc(nel)); ASR_TRY(W3.alloc(nel)); }
@@ -364,7 +484,6 @@ int kpm_run(asr_ctx* ctx, asr_supercell* sc, double cen, double scl, int nmom, i
   std::vector<double> hred((size_t)nsteps * KV * 3);
   // coefficients of the d-scaled recurrence (o = 0): c + e - cen, d^2, 1/d^2, 1/d per (orbital, species)
   DevBuf<double> ucoef;
-  const size_t smem_u = 4 * 9 * sc->nsp * sizeof(double) + (size_t)(sc->ns + 1) * 9 * KRW * sizeof(ST);
   bool dpos = true;
   if (!general) {
     const int np = 9 * sc->nsp;
@@ -383,6 +502,14 @@ int kpm_run(asr_ctx* ctx, asr_supercell* sc, double cen, double scl, int nmom, i
     }
   }
   const bool scaled = !general && dpos;
+  if (scaled) {   // the scaled steps' static sums come on top of up to 48 KB of tables
+    if (std::is_same<ST, float>::value)
+      for (auto k : {k_cheb_f<true>, k_cheb_f<false>}) ASR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024));
+    else
+      for (auto k : {k_cheb_d<true, 1>, k_cheb_d<false, 1>, k_cheb_d<true, 2>, k_cheb_d<false, 2>, k_cheb_d<true, 4>, k_cheb_d<false, 4>})
+        ASR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024));
+  }
+  const int sgrid = std::min(cheb_grid(ctx), (n + KW - 1) / KW);
   for (int vb = 0; vb < nvec; vb += KV) {
     const int nv = std::min(KV, nvec - vb);
     if (scaled) k_rademacher_init_scaled<ST><<<ctx->num_sms * 8, 256, 0, s>>>(S, seed, v0 + vb, T0.p);
@@ -396,10 +523,7 @@ int kpm_run(asr_ctx* ctx, asr_supercell* sc, double cen, double scl, int nmom, i
       const int ps = ctx->prof_start(s);
       if (scaled) {
         // <r|t> is needed for every step without doubling, and for mu_1 (step 0) with it
-        if (!doubling || k == 0)
-          k_cheb_u<ST, true><<<grid, KSITES * KV, smem_u, s>>>(S, blocks, ucoef.p, tin, told, tout, isc, k == 0, seed, v0 + vb, part.p);
-        else
-          k_cheb_u<ST, false><<<grid, KSITES * KV, smem_u, s>>>(S, blocks, ucoef.p, tin, told, tout, isc, k == 0, seed, v0 + vb, part.p);
+        cheb_scaled(ctx, S, blocks, ucoef.p, tin, told, tout, isc, k == 0, !doubling || k == 0, nv, seed, v0 + vb, part.p, sgrid);
       } else if (!general) {
         k_cheb<ST><<<grid, KSITES * KV, smem, s>>>(S, blocks, tin, told, tout, cen, isc, k == 0, !sc->e_zero, seed, v0 + vb, part.p);
       } else {
@@ -415,7 +539,7 @@ int kpm_run(asr_ctx* ctx, asr_supercell* sc, double cen, double scl, int nmom, i
         ctx->prof_stop(s, ps, ASR_KERNEL_KPM, (double)n * (KV * streams * 9 * sizeof(ST) + 1.0),
                        sapp * (double)n * KV * 2.0 * 81.0 * (1 + sc->ns));
       }
-      k_kpm_reduce<<<1, KV, 0, s>>>(part.p, grid, red.p + (size_t)k * KV * 3);
+      k_kpm_reduce<<<KV * 3 / 32, 256, 0, s>>>(part.p, scaled ? sgrid : grid, red.p + (size_t)k * KV * 3);
       if (k > 0) { ST* t_ = ta; ta = tb; tb = tc; tc = t_; }
     }
     ASR_CUDA(cudaGetLastError());
