@@ -1213,12 +1213,12 @@ int asr_autotune(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, int ng
   const int tpbs[4] = {4, 8, 16, 32}, npws[4] = {1, 2, 4, 8};
   double tab[8];
   for (double& t : tab) t = -1.0;
-  double warm;
-  ASR_TRY(timed(4, 4, warm));
-  // a candidate replaces the built-in default (16 tiles in FP64, 8 in FP32, 4 nodes per warp) only when it is at least
+  // a candidate replaces the built-in default (16 tiles in FP64, 8 in FP32, default_npw nodes per warp) only when it is at least
   // 3 % faster: the timings carry a few per cent of noise, and the default is the measured best on the reference workload
-  const int def_t = precision == ASR_FP64 ? 16 : 8, def_n = 4;
+  const int def_t = precision == ASR_FP64 ? 16 : 8, def_n = default_npw(op->nn);
   const double margin = 0.97;
+  double warm;
+  ASR_TRY(timed(4, def_n, warm));
   for (int c = 0; c < 4; ++c) {
     if (tpbs[c] > ntile && tpbs[c] != def_t) continue;
     ASR_TRY(timed(tpbs[c], def_n, tab[c]));
@@ -1228,7 +1228,7 @@ int asr_autotune(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, int ng
   for (int c = 0; c < 4; ++c)
     if (tab[c] > 0 && tab[c] < margin * best) { best = tab[c]; best_t = tpbs[c]; }
   for (int c = 0; c < 4; ++c) ASR_TRY(timed(best_t, npws[c], tab[4 + c]));
-  best = tab[4 + 2];   // 4 nodes per warp
+  best = tab[4 + (def_n == 1 ? 0 : def_n == 2 ? 1 : 2)];
   for (int c = 0; c < 4; ++c)
     if (tab[4 + c] < margin * best) { best = tab[4 + c]; best_n = npws[c]; }
   op->tuned_tpb[pix] = best_t;

@@ -507,23 +507,25 @@ __global__ void __launch_bounds__(WPB * TL) k_smul(OpView op, BatchView bv, cons
 // 6,156 flops per node and lane) with the loads one product step ahead, 2.60 ms without; plain FP64 FMAs (one lane per
 // thread, broadcast block reads) 4.06 ms, with fixed-offset link gathers 3.4 ms.
 struct MmaSm {   // shared memory of k_smul_mma: byte offsets
-  int opw, links, ldl, wtab, bytes;
+  int opw, links, ldl, wtab, wtab2, ild, bytes;
   __host__ __device__ MmaSm(const OpView& op) {
     const int ns1 = op.nslot + 1;
     ldl = (ns1 + 3) & ~3;                                                // links per warp
     opw = (op.ntype * ns1 + 1) * MB * (int)sizeof(double);               // after the blocks and one of zeros
     links = (opw + (op.nop + 1) * 9 * (int)sizeof(uint32_t) + 15) & ~15;
     wtab = links + WPB * ldl * (int)sizeof(int2);
-    bytes = wtab + (op.ncls * op.nsmax + op.nsp) * 9 * (int)sizeof(double2);
+    wtab2 = wtab + (op.ncls * op.nsmax + op.nsp) * 9 * (int)sizeof(double2);
+    ild = wtab2 + (op.ncls * op.nsmax + op.nsp) * 9 * (int)sizeof(double);
+    bytes = ild + 9 * (int)sizeof(double);
   }
 };
 
 // two adjacent outputs (l0, l0 + 1; NL = 2) or one (NL = 1) of a lane of a node: acc the S application's values, wt the
-// diagonal weights {W, W_pa}
+// diagonal weights {W, W_pa}, wc those of c (EPI 4)
 template <bool FINAL, int EPI, int NL>
 __device__ __forceinline__ void mma_out(const OpView& op, const BatchView& bv, size_t q, int tile, int i, int l0, int lane,
-                                        const double2* acc, const double* gb, const double2* wt, bool withx, bool flips,
-                                        const uint32_t* opw, const double* il, const double2* __restrict__ in,
+                                        const double2* acc, const double* gb, const double2* wt, const double* wc, bool withx,
+                                        bool flips, const uint32_t* opw, const double* il, const double2* __restrict__ in,
                                         double2* __restrict__ out, double2& dot) {
   auto get = [&](const double2* p, double2 (&v)[NL]) {
     if constexpr (NL == 2) ldg2(p + q, v[0], v[1]);
@@ -540,12 +542,10 @@ __device__ __forceinline__ void mma_out(const OpView& op, const BatchView& bv, s
     put(out, v);
     return;
   }
-  get(in, ui);
   const int L = tile * TL + lane;
-  const double2 z = bv.lane_z[L], s = bv.su[L];
-#pragma unroll
-  for (int e = 0; e < NL; ++e) t[e] = zfma(make_double2(fma(z.x, wt[e].y, wt[e].x), __dmul_rn(z.y, wt[e].y)), ui[e], acc[e]);
-  if (flips) {   // the flip links of the node (rare)
+  const double2 z = EPI == 3 ? make_double2(0.0, 0.0) : bv.lane_z[L], s = EPI == 3 ? z : bv.su[L];
+  // t += sum over the flip links of the node (rare) of (W_p + z W_pa) x, x the link's row of `src`
+  auto add_flips = [&](const double2* src, int p, bool wx, double sign) {
     const int nsm = op.nsmax, kap = op.ncl[i], own = op.lst[i], nk = op.nsc[kap];
     for (int k = 0; k < nk; ++k) {
       if (k == own) continue;
@@ -554,25 +554,44 @@ __device__ __forceinline__ void mma_out(const OpView& op, const BatchView& bv, s
       const int g = op.flipg[k + nsm * i];
 #pragma unroll
       for (int e = 0; e < NL; ++e) {
-        const int l = l0 + e, p = op.pi[g * 9 + l];
-        const double2 x = in[vx<double2>(tile, bv.nn, r, p, lane)];
-        const uint32_t sg = opw[g * 9 + p];
+        const int l = l0 + e, pl = op.pi[g * 9 + l];
+        const double2 x = src[vx<double2>(tile, bv.nn, r, pl, lane)];
+        const uint32_t sg = opw[g * 9 + pl];
         const int q2 = ((kap * nsm + own) * nsm + k) * 9 + l;
-        const double wf = __ldg(gb + bv.GL.w(PCEB) + q2), wx = withx ? __ldg(gb + bv.GL.w(PA) + q2) : 0.0;
-        t[e] = zfma(make_double2(fma(z.x, wx, wf), __dmul_rn(z.y, wx)), make_double2(xor_sign(x.x, sg), xor_sign(x.y, sg)), t[e]);
+        const double wf = sign * __ldg(gb + bv.GL.w(p) + q2), wa = wx ? __ldg(gb + bv.GL.w(PA) + q2) : 0.0;
+        t[e] = zfma(make_double2(fma(z.x, wa, wf), __dmul_rn(z.y, wa)), make_double2(xor_sign(x.x, sg), xor_sign(x.y, sg)), t[e]);
       }
     }
+  };
+  get(in, ui);
+  if constexpr (EPI == 4) {   // t = h1 - (d S d r1 + C r1) + (E + X(z)) u, r1 the source
+    get((const double2*)bv.gen_h1, t);
+#pragma unroll
+    for (int e = 0; e < NL; ++e) t[e] = zadd(t[e], zneg(make_double2(fma(wc[e], ui[e].x, acc[e].x), fma(wc[e], ui[e].y, acc[e].y))));
+    if (flips) add_flips(in, PC, false, -1.0);
+    get((const double2*)bv.gen_u, ui);
+#pragma unroll
+    for (int e = 0; e < NL; ++e) t[e] = zfma(make_double2(fma(z.x, wt[e].y, wt[e].x), __dmul_rn(z.y, wt[e].y)), ui[e], t[e]);
+    if (flips) add_flips((const double2*)bv.gen_u, PEB, withx, 1.0);
+  } else {
+#pragma unroll
+    for (int e = 0; e < NL; ++e) t[e] = zfma(make_double2(fma(z.x, wt[e].y, wt[e].x), __dmul_rn(z.y, wt[e].y)), ui[e], acc[e]);
+    if (flips) add_flips(in, EPI == 3 ? PC : PCEB, EPI != 3 && withx, 1.0);
+  }
+  if (EPI == 1 || EPI == 2 || (EPI >= 3 && bv.t2out)) {   // the blocks carry d on both sides: t2 = S (d o U) = acc / d_l
+#pragma unroll
+    for (int e = 0; e < NL; ++e) v[e] = zscale(acc[e], il[e]);
+    put((double2*)bv.t2out, v);
+  }
+  if constexpr (EPI == 3) {
+    put(out, t);
+    return;
   }
 #pragma unroll
   for (int e = 0; e < NL; ++e) y[e] = zmul(s, t[e]);
   if (EPI != 2) {
     if constexpr (NL == 2) stg2_cs(out + q, y[0], y[1]);
     else __stcs(out + q, y[0]);
-  }
-  if (EPI >= 1) {   // the blocks carry d on both sides: t2 = S (d o U) = acc / d_l
-#pragma unroll
-    for (int e = 0; e < NL; ++e) v[e] = zscale(acc[e], il[e]);
-    put((double2*)bv.t2out, v);
   }
   if (EPI == 2) {
     const double2 ca = bv.adj.ca[L], cb = zneg(bv.adj.cb[L]), cc = zneg(bv.adj.cc[L]);
@@ -628,20 +647,38 @@ __device__ __forceinline__ double2 mma_nodes(const OpView& op, const BatchView& 
     __syncwarp();
     const int wrow0 = op.ncl[i] * op.nsmax + op.lst[i], fr = op.frozen[i], st = op.start[i], nfl = op.nflip[i];
     const double sq = op.sq[i];
+    // the epilogue's other streams come from memory: on their way into L2 while the node is multiplied
+    if (EPI == 2 || EPI == 4) {
+      const size_t o = vnode(it.tile, bv.nn, i);
+      auto warm = [&](const void* v) {   // 36 lines of 128 bytes
+        const char* p = (const char*)((const double2*)v + o);
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p + t * 128));
+        if (t < 4) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 4096 + t * 128));
+      };
+      if (EPI == 4) { warm(bv.gen_h1); warm(bv.gen_u); }
+      else { warm(bv.adj.yk); warm(bv.adj.wbn); warm(bv.adj.xk); }
+    }
     NodeAcc<NJ> A;
     A.zero();
     A.run(links, cnt, in + vnode(it.tile, bv.nn, 0), off, Bs, opw, zero_blk, t);
     const double2 a8 = quad_own<NJ>(A.c8, c);
     // diagonal weights of the node at this thread's orbitals, P = c + e + X(z) (src/asr_augblk.f90:219-250)
     double2 wt[3];
-    double il[3] = {0.0, 0.0, 0.0};
+    double il[3] = {0.0, 0.0, 0.0}, wc[3] = {0.0, 0.0, 0.0};
     bool flips = false;
     if (FINAL) {
       const int fs = (st && gfrozen > 0) ? gfrozen : fr;
       const double2* wr = wtab + (fs > 0 ? op.ncls * op.nsmax + fs - 1 : wrow0) * 9;
       wt[0] = wr[2 * c]; wt[1] = wr[2 * c + 1]; wt[2] = wr[8];
+      if (EPI == 4) {
+        const double* cr = (const double*)(smem + sm.wtab2) + (wr - wtab);
+        wc[0] = cr[2 * c]; wc[1] = cr[2 * c + 1]; wc[2] = cr[8];
+      }
       flips = fs == 0 && nfl > 0;
-      if (EPI >= 1) { il[0] = 1.0 / gi->dd[2 * c]; il[1] = 1.0 / gi->dd[2 * c + 1]; il[2] = 1.0 / gi->dd[8]; }
+      if (EPI >= 1) {
+        const double* ild = (const double*)(smem + sm.ild);
+        il[0] = ild[2 * c]; il[1] = ild[2 * c + 1]; il[2] = ild[8];
+      }
     }
     const size_t q = vnode(it.tile, bv.nn, i);
     double2 d[NJ];
@@ -650,16 +687,17 @@ __device__ __forceinline__ double2 mma_nodes(const OpView& op, const BatchView& 
       d[j] = make_double2(0.0, 0.0);
       const int lane = row + 8 * off(j);
       const double2 a[2] = {A.out(j, 0), A.out(j, 1)};
-      mma_out<FINAL, EPI, 2>(op, bv, q + mnode_at(2 * c, lane), it.tile, i, 2 * c, lane, a, gb, wt, withx, flips, opw, il, in, out,
-                             d[j]);
+      mma_out<FINAL, EPI, 2>(op, bv, q + mnode_at(2 * c, lane), it.tile, i, 2 * c, lane, a, gb, wt, wc, withx, flips, opw, il, in,
+                             out, d[j]);
     }
     double2 dn = make_double2(0.0, 0.0);
-    if (FINAL) dn = quad_own<NJ>(d, c);
+    if (FINAL && EPI != 3) dn = quad_own<NJ>(d, c);
     if (c < NJ) {
       const int lane = row + 8 * off(c);
-      mma_out<FINAL, EPI, 1>(op, bv, q + 256 + lane, it.tile, i, 8, lane, &a8, gb, wt + 2, withx, flips, opw, il + 2, in, out, dn);
+      mma_out<FINAL, EPI, 1>(op, bv, q + 256 + lane, it.tile, i, 8, lane, &a8, gb, wt + 2, wc + 2, withx, flips, opw, il + 2, in, out,
+                             dn);
     }
-    if (FINAL) {
+    if (FINAL && EPI != 3) {
       const double norb = __dmul_rn(sq, sq);
       own = make_double2(fma(norb, dn.x, own.x), fma(norb, dn.y, own.y));
     }
@@ -667,7 +705,11 @@ __device__ __forceinline__ double2 mma_nodes(const OpView& op, const BatchView& 
   return own;
 }
 
-// Template arguments as k_smul's (no link variants: the operation sits in the B fragment).
+// Template arguments as k_smul's (no link variants: the operation sits in the B fragment), with two more epilogues of the
+// general operator H = E + h - h O h + X(z) at uniform d: EPI 3, out = h U = d S d U + C U (unscaled; no dot), and EPI 4 on
+// r1 = O h U, y = s (h U - h r1 + (E + X(z)) U) with h U in bv.gen_h1 and U in bv.gen_u.  Both store t2 where bv.t2out is set.
+// As separate passes (the S application, then k_combine over its result) the two took 16 vector streams per level with the
+// random operators between them, 8 this way.
 template <bool FUSE_D, bool FINAL, int EPI = 0>
 __global__ void __launch_bounds__(WPB * TL, 2) k_smul_mma(OpView op, BatchView bv, const double* __restrict__ blocks,
                                                           const double2* __restrict__ in, double2* __restrict__ out,
@@ -693,6 +735,7 @@ __global__ void __launch_bounds__(WPB * TL, 2) k_smul_mma(OpView op, BatchView b
       Bs[tk * MB + lp * MB_ROW + l] = v;
     }
     for (int q = threadIdx.x; q < MB; q += blockDim.x) Bs[zero_blk * MB + q] = 0.0;
+    if (EPI >= 1 && gi && threadIdx.x < 9) ((double*)(smem_raw + sm.ild))[threadIdx.x] = 1.0 / gi->dd[threadIdx.x];
     for (int q = threadIdx.x; q < (op.nop + 1) * 9; q += blockDim.x) {
       const int g = q / 9, l = q % 9;
       if (g < op.nop) opw[g * 9 + op.pi[q]] = op_word(l, ((op.sgm[g] >> l) & 1u) ^ (uint32_t)((chimask >> g) & 1ull));
@@ -705,8 +748,10 @@ __global__ void __launch_bounds__(WPB * TL, 2) k_smul_mma(OpView op, BatchView b
       for (int q = threadIdx.x; q < (nw + op.nsp) * 9; q += blockDim.x) {
         const int r = q / 9, l = q % 9, kap = r / nsm, own = r % nsm;
         const int at = r < nw ? ((kap * nsm + own) * nsm + own) * 9 + l : (r - nw) * 9 + l;
-        wtab[q] = make_double2(gb[(r < nw ? bv.GL.w(PCEB) : bv.GL.raw(PCEB)) + at],
-                               withx ? gb[(r < nw ? bv.GL.w(PA) : bv.GL.raw(PA)) + at] : 0.0);
+        const int P = EPI == 3 ? PC : EPI == 4 ? PEB : PCEB;
+        wtab[q] = make_double2(gb[(r < nw ? bv.GL.w(P) : bv.GL.raw(P)) + at],
+                               withx && EPI != 3 ? gb[(r < nw ? bv.GL.w(PA) : bv.GL.raw(PA)) + at] : 0.0);
+        if (EPI == 4) ((double*)(smem_raw + sm.wtab2))[q] = gb[(r < nw ? bv.GL.w(PC) : bv.GL.raw(PC)) + at];
       }
     }
   }
@@ -731,7 +776,7 @@ __global__ void __launch_bounds__(WPB * TL, 2) k_smul_mma(OpView op, BatchView b
     own = mma_nodes<FINAL, EPI, 1>(op, bv, it, smem_raw, sm, oct, grp, in, out);
     if (c == 0) owner = row + 8 * (int)(oct & 3u);
   }
-  if (FINAL) {
+  if (FINAL && EPI != 3) {
     if (EPI != 2 && owner >= 0) {
       const double2 s = bv.su[it.tile * TL + owner];
       own = zmul(zmul(s, s), own);
@@ -878,6 +923,8 @@ __global__ void __launch_bounds__(WPB * TL) k_lanczos_w(OpView op, BatchView bv,
   const double2 a = bv.acur[L], b = bv.bprev[L], su = bv.su[L], sup = bv.sup[L];
   const double2 as = cmul(a, su), bs = cmul(b, sup);
   double2 dot = make_double2(0.0, 0.0);
+  // FP64 chains: an octet of lanes that have all left the chain is not read again (the step skips it), so nothing is written
+  const bool dead = std::is_same<ST, double>::value && bv.by_act && ((__ballot_sync(0xffffffffu, act) >> (lane & 24)) & 0xffu) == 0;
   for (int qn = 0; qn < npw; ++qn) {
     int i = it.first + w + WPB * qn;
     if (i >= bv.nn) break;
@@ -898,7 +945,7 @@ __global__ void __launch_bounds__(WPB * TL) k_lanczos_w(OpView op, BatchView bv,
       for (int l = 0; l < 9; ++l) x[l] = make_double2(0, 0);
     }
     typename St2<ST>::T* dst = wout ? wout : y;
-    st9(dst + vnode(it.tile, bv.nn, i), lane, x);
+    if (!dead) st9(dst + vnode(it.tile, bv.nn, i), lane, x);
   }
   block_reduce_store(dot, part, it.tile, bpt);
   if (bv.tick && last_block_of_tile(bv.tick, it.tile, bpt)) {
@@ -1080,6 +1127,21 @@ void launch_smul(asr_op* op, const BatchView& bv, const ST* blk, const typename 
     k_smul<ST, FUSE_D, FINAL, false, EPI><<<grid, WPB * TL, smul_smem(op, sizeof(ST)), s>>>(ov, bv, blk, in, out, part, npw);
 }
 
+// y = s (h U - h O h U + (E + X) U) in FP64 at uniform d: H1 = h U, R1 = O h U, Y and the dots; TA, TB (or null): S d U, S d R1
+void general_mma(asr_op* op, const BatchView& bv, const double2* U, double2* H1, double2* R1, double2* Y, double2* TA, double2* TB,
+                 double2* part, int npw, int grid, cudaStream_t s) {
+  BatchView b = bv;
+  b.t2out = TA;
+  b.tick = nullptr;
+  launch_smul<double, true, true, 3>(op, b, op->d_blocks, U, H1, part, npw, grid, s);
+  k_rand<double><<<grid, WPB * TL, 0, s>>>(op->view(), bv, PO, H1, R1, npw);
+  b = bv;
+  b.t2out = TB;
+  b.gen_h1 = H1;
+  b.gen_u = U;
+  launch_smul<double, true, true, 4>(op, b, op->d_blocks, R1, Y, part, npw, grid, s);
+}
+
 // One chain step of the general operator on the batch; writes y into Y and the a-partials.
 template <typename ST>
 int step_apply(asr_ctx* ctx, asr_op* op, const BatchView& bv, bool fused, bool any_o, bool all_dunif,
@@ -1093,6 +1155,12 @@ int step_apply(asr_ctx* ctx, asr_op* op, const BatchView& bv, bool fused, bool a
   if (fused) {
     launch_smul<ST, true, true>(op, bv, blk, U, Y, part, npw, grid, s);
     return ASR_OK;
+  }
+  if constexpr (std::is_same<ST, double>::value) {
+    if (all_dunif) {   // any_o: without it the step is fused
+      general_mma(op, bv, U, H1, R1, Y, nullptr, nullptr, part, npw, grid, s);
+      return ASR_OK;
+    }
   }
   // t1 = D x0, t2 = S t1
   if (all_dunif) {
@@ -1181,7 +1249,7 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
   const size_t proj_tile_bytes = proj ? (size_t)nlevmax * 9 * proj->nt * TL * sizeof(double2) : 0;
   while (tpb > 1 && (size_t)tpb * (nvec * vec_bytes + proj_tile_bytes) > freeb / 2) tpb /= 2;
   tpb = std::min(tpb, ntile_all);
-  int npw = opt.nodes_per_warp > 0 ? opt.nodes_per_warp : op->tuned_npw[prec_ix] > 0 ? op->tuned_npw[prec_ix] : 4;
+  int npw = opt.nodes_per_warp > 0 ? opt.nodes_per_warp : op->tuned_npw[prec_ix] > 0 ? op->tuned_npw[prec_ix] : default_npw(nn);
   if (const char* e = getenv("ASR_NODES_PER_WARP")) npw = std::max(1, atoi(e));
   const int npb = WPB * npw;
   const int bpt = (nn + npb - 1) / npb;
@@ -1283,10 +1351,11 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
         k_proj_gather<ST><<<(unsigned)((nwarp * TL + 255) / 256), 256, 0, s>>>(op->view(), bv, U, PV, k);
         ctx->launches += 1;
       }
-      // the fused step reduces a_k in its epilogue (the tile's last block), k_lanczos_w b_k
+      // the step reduces a_k in its epilogue (the tile's last block) where one kernel forms y, k_lanczos_w b_k
+      const bool a_in_step = fused || (all_dunif && std::is_same<ST, double>::value);
       const bool depth_due = opt.depth_tol > 0.0 && opt.mode == ASR_MODE_EDC && k >= 8 && k % 4 == 0;
       BatchView bvs = bv;
-      bvs.tick = fused ? d_tick.p : nullptr;
+      bvs.tick = a_in_step ? d_tick.p : nullptr;
       // timed regions (asr_ctx_profile): event pairs stay pending until the statistics are read (no synchronisation)
       int ps = ctx->prof_start(s);
       ASR_TRY(step_apply<ST>(ctx, op, bvs, fused, any_o, all_dunif, U, Y, nvec > 3 ? V[3].p : nullptr, nvec > 3 ? V[4].p : nullptr,
@@ -1296,7 +1365,7 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
         ctx->prof_stop(s, ps, ASR_KERNEL_STEP, (double)nt * nn * (2.0 * 9 * TL * sizeof(T2) + tab),
                        (double)nt * nn * TL * (op->nslot + 1) * 81.0 * 4.0);
       }
-      if (!fused) k_reduce_a<<<nt, RED_THREADS, 0, s>>>(bv, d_part.p, bpt, k);
+      if (!a_in_step) k_reduce_a<<<nt, RED_THREADS, 0, s>>>(bv, d_part.p, bpt, k);
       if (depth_due) k_depth_test<<<nt * TL, 1, 0, s>>>(bv, k);
       BatchView bvw = bv;
       bvw.tick = d_tick.p;
@@ -1304,7 +1373,7 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
       k_lanczos_w<ST><<<gridb, WPB * TL, 0, s>>>(op->view(), bvw, Y, U, UP, d_part.p, npw);
       // read y, u, u', write w per (node, lane); about 30 flops per complex element (scaled updates, projection, dot)
       ctx->prof_stop(s, ps, ASR_KERNEL_LANCZOS, (double)nt * nn * 4.0 * 9 * TL * sizeof(T2), (double)nt * nn * TL * 9 * 30.0);
-      ctx->launches += (fused ? 1 : 2) + depth_due + (fused ? 1 : (any_o ? 7 : (all_dunif ? 2 : 3)));
+      ctx->launches += (a_in_step ? 1 : 2) + depth_due + (fused ? 1 : a_in_step ? 3 : any_o ? 7 : all_dunif ? 2 : 3);
     }
     ASR_CUDA(cudaGetLastError());
     if (opt.mode == ASR_MODE_EDC && d_g_out) {
@@ -1481,7 +1550,7 @@ __global__ void __launch_bounds__(WPB * TL) k_adj_u(OpView op, BatchView bv, con
   }
 }
 
-// gradient partials of one reverse step: thread (orbital l = warp, lane); per block and kind the sums over its nodes and
+// gradient partials of one reverse step: thread = element (orbital l, lane) of a node; per block and kind the sums over its nodes and
 // the 32 lanes: gpart[((tile * gbpt + blk) * NGK + kind) * 9 * nsp + l * nsp + species], kinds 0 c, 1 d, 2 pa, 3 o, 4 e
 // (e and pb enter the same way).  With G_p(x, v) = x . (dR_p / dpar) v (x at the node, v through the flip links with the
 // class weights mt, or the node itself on a frozen site) and A = h - h O h + E + X(z), h = C + D S D:
@@ -1515,7 +1584,8 @@ __global__ void __launch_bounds__(GPW * TL) k_adj_grad(OpView op, BatchView bv, 
   const int gbpt = (bv.nn + nodes_per_block - 1) / nodes_per_block;
   const int tile = blockIdx.x / gbpt, blk = blockIdx.x % gbpt;
   if (tile >= bv.ntile || !bv.tile_act[tile]) return;
-  const int l = threadIdx.x / TL, lane = threadIdx.x % TL;
+  int l, lane;   // the thread's element of every node: whole lines in either layout
+  node_elem<ST>(threadIdx.x, l, lane);
   const int L = tile * TL + lane;
   const int grp = bv.tile_group[tile];
   const int nsp = op.nsp, nsm = op.nsmax;
@@ -1531,7 +1601,7 @@ __global__ void __launch_bounds__(GPW * TL) k_adj_grad(OpView op, BatchView bv, 
     z = bv.lane_z[L];
     const int i0 = blk * nodes_per_block, i1 = min(bv.nn, i0 + nodes_per_block);
     for (int i = i0; i < i1; ++i) {
-      size_t q = vx<ST>(tile, bv.nn, i, l, lane);
+      const size_t q = vnode(tile, bv.nn, i) + threadIdx.x;
       double2 y = ld(yb + q), ty = ld(tb + q);
       if (WY) {   // the fused reverse step passes wbar and S D wbar: ybar = wbar + c3 X_k, S D ybar = S D wbar + c3 S D X_k
         y = cadd(y, cmul(c3, ld(xk + q)));
@@ -1582,39 +1652,41 @@ __global__ void __launch_bounds__(GPW * TL) k_adj_grad(OpView op, BatchView bv, 
       }
     }
   }
-  // sum over the 32 lanes (one warp = one orbital), fixed order; pa = z e per lane before the sum
+  // sum over the 32 lanes, fixed order; pa = z e per lane before the sum.  FP32: one warp is one orbital.  FP64: warps 0-7 hold
+  // eight lanes of four orbitals each (thread t: orbital t % 4 of the quad w / 4), warp 8 orbital 8.
   double2 gpa[NS];
 #pragma unroll
   for (int q = 0; q < NS; ++q) {
     gpa[q] = cmul(z, ge[q]);
     if (!GEN) gc[q] = ge[q];   // o = 0: c enters as e does
   }
+  constexpr bool FRAG = std::is_same<ST, double>::value;
+  const int w = threadIdx.x / TL, t = threadIdx.x % TL, stop = FRAG && w < 8 ? 4 : 1;
+  double2* out = gpart + ((size_t)(tile * gbpt + blk) * NGK) * 9 * nsp;
+  __shared__ double2 quad[FRAG ? 8 : 1][FRAG ? 4 : 1][NGK * NS];
 #pragma unroll
   for (int q = 0; q < NS; ++q) {
     if (q >= nsp) break;
-    for (int off = 16; off > 0; off >>= 1) {
-      gc[q].x += __shfl_xor_sync(0xffffffffu, gc[q].x, off);
-      gc[q].y += __shfl_xor_sync(0xffffffffu, gc[q].y, off);
-      gd[q].x += __shfl_xor_sync(0xffffffffu, gd[q].x, off);
-      gd[q].y += __shfl_xor_sync(0xffffffffu, gd[q].y, off);
-      gpa[q].x += __shfl_xor_sync(0xffffffffu, gpa[q].x, off);
-      gpa[q].y += __shfl_xor_sync(0xffffffffu, gpa[q].y, off);
-      go[q].x += __shfl_xor_sync(0xffffffffu, go[q].x, off);
-      go[q].y += __shfl_xor_sync(0xffffffffu, go[q].y, off);
-      ge[q].x += __shfl_xor_sync(0xffffffffu, ge[q].x, off);
-      ge[q].y += __shfl_xor_sync(0xffffffffu, ge[q].y, off);
+    double2 v[NGK] = {gc[q], gd[q], gpa[q], go[q], ge[q]};
+    for (int off = 16; off >= stop; off >>= 1)
+#pragma unroll
+      for (int k = 0; k < NGK; ++k) v[k] = cadd(v[k], shfl_xor2(v[k], off));
+    if (FRAG && w < 8) {
+      if (t < 4)
+#pragma unroll
+        for (int k = 0; k < NGK; ++k) quad[w][t][k * NS + q] = v[k];
+    } else if (t == 0) {
+#pragma unroll
+      for (int k = 0; k < NGK; ++k) out[(k * 9 + l) * nsp + q] = v[k];
     }
   }
-  if (lane == 0) {
-    double2* out = gpart + ((size_t)(tile * gbpt + blk) * NGK) * 9 * nsp;
-#pragma unroll
-    for (int q = 0; q < NS; ++q) {
-      if (q >= nsp) break;
-      out[(0 * 9 + l) * nsp + q] = gc[q];
-      out[(1 * 9 + l) * nsp + q] = gd[q];
-      out[(2 * 9 + l) * nsp + q] = gpa[q];
-      out[(3 * 9 + l) * nsp + q] = go[q];
-      out[(4 * 9 + l) * nsp + q] = ge[q];
+  if (FRAG) {
+    __syncthreads();
+    for (int e = threadIdx.x; e < NGK * 8 * nsp; e += blockDim.x) {
+      const int q = e % nsp, lo = (e / nsp) % 8, k = e / (8 * nsp);
+      double2 v = quad[4 * (lo >> 2)][lo & 3][k * NS + q];
+      for (int j = 1; j < 4; ++j) v = cadd(v, quad[4 * (lo >> 2) + j][lo & 3][k * NS + q]);
+      out[(k * 9 + lo) * nsp + q] = v;
     }
   }
 }
@@ -1767,6 +1839,12 @@ void apply_general_keep(asr_op* op, const BatchView& bv, bool dunif, const typen
                         typename St2<ST>::T* TA, typename St2<ST>::T* H, typename St2<ST>::T* R, typename St2<ST>::T* TB,
                         typename St2<ST>::T* TMP, double2* part, int npw, int grid, cudaStream_t s) {
   OpView ov = op->view();
+  if constexpr (std::is_same<ST, double>::value) {
+    if (dunif) {
+      general_mma(op, bv, x, H, R, y, TA, TB, part, npw, grid, s);
+      return;
+    }
+  }
   apply_SD<ST>(op, bv, dunif, x, TMP, TA, part, npw, grid, s);
   k_combine<ST><<<grid, WPB * TL, 0, s>>>(ov, bv, TA, x, PC, false, x, false, nullptr, 1.0, false, H, part, npw);
   k_rand<ST><<<grid, WPB * TL, 0, s>>>(ov, bv, PO, H, R, npw);
@@ -1836,7 +1914,7 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
   while (tpb > 1 && (size_t)tpb * nvec * vec_bytes > freeb / 2) tpb /= 2;
   if ((size_t)nvec * vec_bytes > freeb) { set_error("adjoint: %d vectors of %zu bytes do not fit", nvec, vec_bytes); return ASR_ENOMEM; }
   tpb = std::min(tpb, ntile_all);
-  const int npw = 4, npb = WPB * npw, bpt = (nn + npb - 1) / npb;
+  const int npw = default_npw(nn), npb = WPB * npw, bpt = (nn + npb - 1) / npb;
   int gnpb = 64;   // nodes per block of the gradient kernel
   if (const char* e = getenv("ASR_ADJ_GRAD_NODES")) gnpb = std::max(1, atoi(e));
   const int gbpt = (nn + gnpb - 1) / gnpb, ngd = NGK * 9 * nsp;
@@ -2421,7 +2499,7 @@ int run_ed3_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, con
   while (tpb > 1 && (size_t)tpb * nvec * vec_bytes > freeb / 2) tpb /= 2;
   if ((size_t)nvec * vec_bytes > freeb) { set_error("ed3: %d vectors of %zu bytes do not fit", nvec, vec_bytes); return ASR_ENOMEM; }
   tpb = std::min(tpb, ntile_all);
-  const int npw = 4, npb = WPB * npw, bpt = (nn + npb - 1) / npb;
+  const int npw = default_npw(nn), npb = WPB * npw, bpt = (nn + npb - 1) / npb;
   const int nlp = tpb * TL;
   Dev<double> d_gblob, d_oc, d_na, d_nv, d_tn;
   Dev<GroupInfo> d_ginfo;
@@ -2666,7 +2744,7 @@ int run_epi_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, con
   while (tpb > 1 && (size_t)tpb * nvec * vec_bytes > freeb / 2) tpb /= 2;
   if ((size_t)nvec * vec_bytes > freeb) { set_error("epi_blocks: %d vectors of %zu bytes do not fit", nvec, vec_bytes); return ASR_ENOMEM; }
   tpb = std::min(tpb, ntile_all);
-  const int npw = 4, npb = WPB * npw, bpt = (nn + npb - 1) / npb;
+  const int npw = default_npw(nn), npb = WPB * npw, bpt = (nn + npb - 1) / npb;
   const int nlp = tpb * TL;
   Dev<double> d_gblob, d_v9, d_nv;
   Dev<GroupInfo> d_ginfo;
@@ -2802,6 +2880,8 @@ static void smem_attrs() {
   cudaFuncSetAttribute(k_smul_mma<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul_mma<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul_mma<true, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
+  cudaFuncSetAttribute(k_smul_mma<true, true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
+  cudaFuncSetAttribute(k_smul_mma<true, true, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul_mma<true, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul<float, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   cudaFuncSetAttribute(k_smul<float, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
@@ -2900,7 +2980,7 @@ int apply_vectors(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
   ASR_CUDA(cudaMemcpyAsync(d_gblob.p, gblob.data(), gblob.size() * sizeof(double), cudaMemcpyHostToDevice, s));
   ASR_CUDA(cudaMemcpyAsync(d_ginfo.p, ginfo.data(), ginfo.size() * sizeof(GroupInfo), cudaMemcpyHostToDevice, s));
   const int nlp = nt * TL;
-  const int npw = 4, npb = WPB * npw, bpt = (nn + npb - 1) / npb;
+  const int npw = default_npw(nn), npb = WPB * npw, bpt = (nn + npb - 1) / npb;
   std::vector<int> hgroup(nlp), ones(nlp, 1), tact(nt, 1), tgroup(nt, 0);
   for (int q = 0; q < nlp; ++q) hgroup[q] = q < nvec ? 0 : -1;
   std::vector<double2> hz(nlp, make_double2(0.0, what == APPLY_RAND_Z ? 1.0 : 0.0)), hsu(nlp, make_double2(1.0, 0.0));

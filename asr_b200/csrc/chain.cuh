@@ -69,9 +69,16 @@ struct BatchView {
                            // epilogue of the tile's last block instead of separate reduction launches
   void* t2out;             // optional: the fused step kernel also stores t2 = S (d o U) (unscaled, the vector type of the
                            // batch) for the adjoint's parameter gradient
+  const void* gen_h1;      // general operator: h U and U for the last pass (EPI 4)
+  const void* gen_u;
   int by_act;              // 1: a lane whose lane_act is 0 has left its chain for good (its vectors are not needed any more)
   AdjEpi adj;              // the adjoint epilogue's vectors and coefficients (read only by that instantiation)
 };
+
+// nodes per warp of the node kernels where the caller leaves it open: 4 amortise a block's tables; an operator too small to
+// give every SM two blocks of 32 nodes takes fewer (395 nodes: the step of one tile takes 48 us with 4, 21 us with 1; 994 and
+// 2,536 nodes are fastest with 2).  By the operator alone, so that a lane's sums do not depend on what else runs.
+inline int default_npw(int nn) { return nn < 148 * 4 ? 1 : nn < 148 * 64 ? 2 : 4; }
 
 struct RunOptions {
   int mode = ASR_MODE_EDC;

@@ -57,3 +57,23 @@ def test_more_neighbour_slots_than_lanes():
     for j in range(2):
         yo = oop.apply(x[:, j])
         assert np.max(np.abs(y[:, j] - yo)) <= 1e-12 * np.max(np.abs(yo))
+
+
+@pytest.mark.parametrize("nz", [5, 16, 20, 33])
+def test_general_operator_octets(pair, nz):
+    """H = E + h - h o h + X(z) at uniform d (two tensor-core passes with the random operator between them)."""
+    gop, oop, _ = pair
+    sp = S.draw_species(gop.nsp, 4)
+    ed = S.edc_params_o(sp, S.draw_o(gop.nsp, 4, 0.2), 1)
+    zs = np.linspace(-0.5, 0.3, nz) + 0.05j
+    for op in (gop, oop):
+        op.set_params(ed["c"], ed["d"], ed["o"], ed["e"])
+    try:
+        g, m, a, b = A.edc_green_blk(gop, ed, zs, 5, 10)
+        go, mo, ao, bo = oop.edc_green_blk(ed, zs, 5, 10)
+        assert np.array_equal(m, mo)
+        for x, y in ((g, go), (a, ao), (b, bo)):
+            assert np.max(np.abs(x - y)) <= 1e-9 * np.max(np.abs(y))
+    finally:
+        for op in (gop, oop):
+            op.set_params(*[pair[2][k] for k in ("c", "d", "o", "e")])
