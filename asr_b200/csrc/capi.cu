@@ -239,6 +239,20 @@ int asr_ctx_create(int device, asr_ctx** out) {
   }
   cudaMemset(c->d_err, 0, sizeof(int));
   c->stream = c->own_stream;
+  // an eighth of the device: holds the vectors of a 16-tile FP64 batch of the 20,969-node operator (5-8 GB), of a
+  // 256,000-site supercell (2-4 GB) and the adjoint's kept levels of three tiles (22 GB)
+  c->keep = prop.totalGlobalMem / 8;
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  if (cudaMemPoolCreate(&c->pool, &props) == cudaSuccess) {
+    uint64_t keep = asr_ctx::POOL_KEEP;
+    cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  } else {
+    c->pool = nullptr;   // no pools on this device: small arrays from the device
+    cudaGetLastError();
+  }
   *out = c;
   return ASR_OK;
 }
@@ -247,6 +261,11 @@ int asr_ctx_destroy(asr_ctx* ctx) {
   if (!ctx) return ASR_OK;
   DeviceGuard dg;
   dg.set(ctx->device);
+  ctx->mem_trim(0);
+  if (ctx->pool) {
+    cudaStreamSynchronize(ctx->own_stream);
+    cudaMemPoolDestroy(ctx->pool);
+  }
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   if (ctx->d_err) cudaFree(ctx->d_err);
   ctx->ws_release();
@@ -286,9 +305,10 @@ int asr_ctx_profile(asr_ctx* ctx, int on) {
 int asr_ctx_hold_workspace(asr_ctx* ctx, int on) {
   if (!ctx) { set_error("asr_ctx_hold_workspace: null context"); return ASR_EINVAL; }
   ASR_ON_DEVICE(ctx->device);
-  if (!on && ctx->ws) {
+  if (!on) {
     ASR_CUDA(cudaStreamSynchronize(ctx->stream));
     ctx->ws_release();
+    ctx->mem_trim(0);
   }
   ctx->ws_hold = on != 0;
   return ASR_OK;
@@ -598,7 +618,7 @@ static int op_group(asr_op* op, const GroupLayout& GL, const double* pa, const d
 
 int asr_op_apply(asr_op* op, const double* x, double* y, int nvec) {
   if (!op || !x || !y || nvec < 1) { set_error("augcls_apply: bad argument"); return ASR_EINVAL; }
-  ASR_ON_DEVICE(op->ctx->device);
+  ASR_ENTER(op->ctx);
   GroupLayout GL = layout(op);
   std::vector<double> blob;
   std::vector<GroupInfo> gi;
@@ -608,7 +628,7 @@ int asr_op_apply(asr_op* op, const double* x, double* y, int nvec) {
 
 int asr_op_hp_c(asr_op* op, const double* x, double* y, int nvec) {
   if (!op || !x || !y || nvec < 1) { set_error("augcls_hp_c: bad argument"); return ASR_EINVAL; }
-  ASR_ON_DEVICE(op->ctx->device);
+  ASR_ENTER(op->ctx);
   GroupLayout GL = layout(op);
   // h = c + D S D: the operator's c and d with o = e = 0 (H = E_nu + h - h o h reduces to h)
   std::vector<double> blob(GL.stride, 0.0), zero((size_t)9 * op->nsp, 0.0);
@@ -620,7 +640,7 @@ int asr_op_hp_c(asr_op* op, const double* x, double* y, int nvec) {
 
 int asr_op_rand_c(asr_op* op, const double* par, const double* x, double* w, int nvec) {
   if (!op || !par || !x || !w || nvec < 1) { set_error("augcls_rand_c: bad argument"); return ASR_EINVAL; }
-  ASR_ON_DEVICE(op->ctx->device);
+  ASR_ENTER(op->ctx);
   GroupLayout GL = layout(op);
   const int np = 9 * op->nsp;
   std::vector<double> pr(np), pim(np);
@@ -633,7 +653,7 @@ int asr_op_rand_c(asr_op* op, const double* par, const double* x, double* w, int
 
 int asr_op_project_c(asr_op* op, double* x, int nvec) {
   if (!op || !x || nvec < 1) { set_error("augcls_project_c: bad argument"); return ASR_EINVAL; }
-  ASR_ON_DEVICE(op->ctx->device);
+  ASR_ENTER(op->ctx);
   GroupLayout GL = layout(op);
   std::vector<double> blob;
   std::vector<GroupInfo> gi;
@@ -647,7 +667,7 @@ static int chains_common(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups
   if (!ctx || !op || !groups || ngroup < 1 || nz < 0) { set_error("asr_chains_run: bad argument"); return ASR_EINVAL; }
   if (mode != ASR_MODE_PLAIN && mode != ASR_MODE_EDC) { set_error("asr_chains_run: unknown mode"); return ASR_EINVAL; }
   if (tail < 0 || tail > 3) { set_error("asr_chains_run: unknown tail"); return ASR_EINVAL; }
-  ASR_ON_DEVICE(ctx->device);
+  ASR_ENTER(ctx);
   cudaStream_t s = ctx->stream;
   GroupLayout GL = layout(op);
   std::vector<double> blob((size_t)GL.stride * ngroup, 0.0);
@@ -760,7 +780,7 @@ int asr_epi_blocks(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, cons
                    const double* z, int nz, int tail, int precision, int project, double* x, int* mused) {
   if (!ctx || !op || !groups || !v9 || !chi || ngroup < 1 || nz < 1 || !z || !x) { set_error("asr_epi_blocks: bad argument"); return ASR_EINVAL; }
   if (tail < 0 || tail > 3) { set_error("asr_epi_blocks: unknown tail"); return ASR_EINVAL; }
-  ASR_ON_DEVICE(ctx->device);
+  ASR_ENTER(ctx);
   GroupLayout GL = layout(op);
   std::vector<double> blob((size_t)GL.stride * ngroup, 0.0), vv(9 * (size_t)ngroup);
   std::vector<GroupInfo> gi(ngroup);
@@ -812,7 +832,7 @@ int asr_ed3_blocks(asr_ctx* ctx, asr_op* op, const asr_ed3_group* groups, int ng
                    int tail, int precision, int project, double* bk, int* mused, double* a, double* b, double* c) {
   if (!ctx || !op || !groups || ngroup < 1 || nz < 1 || !z || !bk) { set_error("asr_ed3_blocks: bad argument"); return ASR_EINVAL; }
   if (tail < 0 || tail > 3) { set_error("asr_ed3_blocks: unknown tail"); return ASR_EINVAL; }
-  ASR_ON_DEVICE(ctx->device);
+  ASR_ENTER(ctx);
   const int nsp = op->nsp, np = 9 * nsp;
   GroupLayout GL = layout(op);
   std::vector<double> blob((size_t)GL.stride * ngroup, 0.0), oc(ngroup);
@@ -893,7 +913,7 @@ static int chains_adjoint_common(asr_ctx* ctx, asr_op* op, const asr_chain_group
   if (!ctx || !op || !groups || ngroup < 1 || nz < 1 || !z || !w || !grad) { set_error("%s: bad argument", who); return ASR_EINVAL; }
   if (tail < ASR_TAIL_NONE || tail > ASR_TAIL_AVG2) { set_error("%s: unknown tail", who); return ASR_EINVAL; }
   if (depth_tol < 0.0) { set_error("%s: depth_tol must be >= 0", who); return ASR_EINVAL; }
-  ASR_ON_DEVICE(ctx->device);
+  ASR_ENTER(ctx);
   GroupLayout GL = layout(op);
   std::vector<double> blob((size_t)GL.stride * ngroup, 0.0);
   std::vector<GroupInfo> gi(ngroup);
@@ -979,7 +999,7 @@ static int lanes_common(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups,
     if (lane_group[L] < 1 || lane_group[L] > ngroup) { set_error("asr_chains_run_lanes: lane %d has group %d", L + 1, lane_group[L]); return ASR_EINVAL; }
     lg[L] = lane_group[L] - 1;
   }
-  ASR_ON_DEVICE(ctx->device);
+  ASR_ENTER(ctx);
   GroupLayout GL = layout(op);
   std::vector<double> blob((size_t)GL.stride * ngroup, 0.0);
   std::vector<GroupInfo> gi(ngroup);
@@ -1010,7 +1030,7 @@ int asr_chains_run_lanes(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups
                          const double* lane_z, int nlane, double depth_tol, int tail, int precision, int project, double* g,
                          int* mused) {
   if (!ctx || !lane_z || !g || nlane < 1) { set_error("asr_chains_run_lanes: bad argument"); return ASR_EINVAL; }
-  ASR_ON_DEVICE(ctx->device);
+  ASR_ENTER(ctx);
   cudaStream_t s = ctx->stream;
   Dev<double2> d_z, d_g;
   ASR_TRY(d_z.alloc(nlane));
@@ -1039,7 +1059,7 @@ int asr_chains_run_dev(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, 
 int asr_chains_run(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, int ngroup, const double* z, int nz, int mode,
                    double depth_tol, int tail, int precision, int project, double* g, double* a, double* b, int* mused) {
   if (!ctx || !z || !g) { set_error("asr_chains_run: null argument"); return ASR_EINVAL; }
-  ASR_ON_DEVICE(ctx->device);
+  ASR_ENTER(ctx);
   if (nz < 0 || ngroup < 1) { set_error("asr_chains_run: bad argument"); return ASR_EINVAL; }
   cudaStream_t s = ctx->stream;
   const size_t ng = (size_t)nz * ngroup;
@@ -1106,7 +1126,7 @@ int asr_chains_proj(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, int
     tn[q] = tnode[q] > 0 ? op->dev_node(tnode[q] - 1) : -1;   // reference numbering -> the device's node order
     tg[q] = tnode[q] > 0 ? tgop[q] - 1 : 0;
   }
-  ASR_ON_DEVICE(ctx->device);
+  ASR_ENTER(ctx);
   cudaStream_t s = ctx->stream;
   GroupLayout GL = layout(op);
   std::vector<double> blob((size_t)GL.stride * ngroup, 0.0);
@@ -1165,7 +1185,7 @@ int asr_autotune(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, int ng
                  int levels, int* tpb_out, int* npw_out, double* times) {
   if (!ctx || !op || !groups || ngroup < 1 || !z || nz < 1 || levels < 1) { set_error("asr_autotune: bad argument"); return ASR_EINVAL; }
   if (precision != ASR_FP64 && precision != ASR_FP32) { set_error("asr_autotune: unknown precision"); return ASR_EINVAL; }
-  ASR_ON_DEVICE(ctx->device);
+  ASR_ENTER(ctx);
   GroupLayout GL = layout(op);
   std::vector<double> blob((size_t)GL.stride * ngroup, 0.0);
   std::vector<GroupInfo> gi(ngroup);
@@ -1183,7 +1203,7 @@ int asr_autotune(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, int ng
     for (int j = 0; j < nzt; ++j) { lg[(size_t)q * nzt + j] = q; lz[(size_t)q * nzt + j] = make_double2(z[2 * j], z[2 * j + 1]); }
   Dev<double2> d_lz, d_g;
   ASR_TRY(d_lz.alloc(nlane)); ASR_TRY(d_g.alloc(nlane));
-  ASR_CUDA(cudaMemcpy(d_lz.p, lz.data(), nlane * sizeof(double2), cudaMemcpyHostToDevice));
+  ASR_CUDA(cudaMemcpyAsync(d_lz.p, lz.data(), nlane * sizeof(double2), cudaMemcpyHostToDevice, ctx->stream));
   const int ntile = ngroup * ((nzt + TL - 1) / TL);
   const int pix = precision == ASR_FP64 ? 0 : 1;
   auto timed = [&](int tpb, int npw, double& ms) -> int {
@@ -1276,7 +1296,7 @@ int asr_cf_eval(asr_ctx* ctx, const double* a, const double* b, const int* m, in
   if (!ctx || !a || !b || !m || !z || !g || ld < 1 || nchain < 1 || nz < 1) { set_error("asr_cf_eval: bad argument"); return ASR_EINVAL; }
   for (int c = 0; c < nchain; ++c)
     if (m[c] < 1 || m[c] > ld || m[c] > CF_NMAX) { set_error("asr_cf_eval: depth of chain %d out of range", c + 1); return ASR_EINVAL; }
-  ASR_ON_DEVICE(ctx->device);
+  ASR_ENTER(ctx);
   cudaStream_t s = ctx->stream;
   size_t nab = (size_t)ld * nchain, nzz = (size_t)nz * nchain;
   Dev<double2> d_a, d_b, d_z, d_g, d_e;   // freed on every return path

@@ -1189,7 +1189,14 @@ int vector_slab(asr_ctx* ctx, size_t bytes, Dev<unsigned char>& own, void** base
   if (ctx->ws_hold) {
     if (ctx->ws_bytes < bytes) {
       ctx->ws_release();
-      if (cudaMalloc(&ctx->ws, bytes) != cudaSuccess) {
+      cudaError_t rc = cudaMalloc(&ctx->ws, bytes);
+      if (rc != cudaSuccess) {   // what the context holds unused back to the device, then once more
+        cudaGetLastError();
+        cudaStreamSynchronize(ctx->stream);
+        ctx->mem_trim(0);
+        rc = cudaMalloc(&ctx->ws, bytes);
+      }
+      if (rc != cudaSuccess) {
         ctx->ws = nullptr;
         set_error("chains: device allocation of %zu bytes failed", bytes);
         return ASR_ENOMEM;
@@ -1234,10 +1241,9 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
   if (op->nop > MAXOP) { set_error("chains: at most %d group operations", MAXOP); return ASR_EINVAL; }
   // batch size: tiles in flight, bounded by memory (3 vectors + temporaries per tile)
   const size_t vec_bytes = (size_t)nn * 9 * TL * sizeof(T2);
-  const int nvec = 3 + (fused ? 0 : (any_o ? 4 : 2));
-  size_t freeb = 0, totb = 0;
-  cudaMemGetInfo(&freeb, &totb);
-  freeb += ctx->ws_bytes;   // a held slab is this call's to reuse
+  // the general operator at uniform d in FP64 forms y from h U and O h U (general_mma); otherwise t1, t2, h1 and r1
+  const bool gen2 = std::is_same<ST, double>::value && all_dunif && any_o;
+  const int nvec = 3 + (fused ? 0 : gen2 ? 2 : any_o ? 4 : 2);
   // 32-lane tiles per batch: larger batches amortise the per-level reductions and launch gaps; the caller's shape, else
   // the operator's autotuned one, else the measured defaults of the fcc ternary workload (FP64 16 tiles, FP32 8, 4 nodes
   // per warp)
@@ -1247,12 +1253,13 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
   if (const char* e = getenv("ASR_TILES_PER_BATCH")) tpb = std::max(1, atoi(e));
   // projections: per tile nlevmax x 9 nt x 32 complex values
   const size_t proj_tile_bytes = proj ? (size_t)nlevmax * 9 * proj->nt * TL * sizeof(double2) : 0;
-  while (tpb > 1 && (size_t)tpb * (nvec * vec_bytes + proj_tile_bytes) > freeb / 2) tpb /= 2;
   tpb = std::min(tpb, ntile_all);
   int npw = opt.nodes_per_warp > 0 ? opt.nodes_per_warp : op->tuned_npw[prec_ix] > 0 ? op->tuned_npw[prec_ix] : default_npw(nn);
   if (const char* e = getenv("ASR_NODES_PER_WARP")) npw = std::max(1, atoi(e));
   const int npb = WPB * npw;
   const int bpt = (nn + npb - 1) / npb;
+  const size_t freeb = ctx->plan_bytes((size_t)tpb * (nvec * vec_bytes + proj_tile_bytes));
+  while (tpb > 1 && (size_t)tpb * (nvec * vec_bytes + proj_tile_bytes) > freeb / 2) tpb /= 2;
   // device state
   Dev<double> d_gblob;
   Dev<GroupInfo> d_ginfo;
@@ -1359,7 +1366,7 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
       // timed regions (asr_ctx_profile): event pairs stay pending until the statistics are read (no synchronisation)
       int ps = ctx->prof_start(s);
       ASR_TRY(step_apply<ST>(ctx, op, bvs, fused, any_o, all_dunif, U, Y, nvec > 3 ? V[3].p : nullptr, nvec > 3 ? V[4].p : nullptr,
-                             nvec > 5 ? V[5].p : nullptr, nvec > 5 ? V[6].p : nullptr, d_part.p, npw, gridb));
+                             gen2 ? V[3].p : nvec > 5 ? V[5].p : nullptr, gen2 ? V[4].p : nvec > 5 ? V[6].p : nullptr, d_part.p, npw, gridb));
       {   // algorithmic traffic of one operator pass: read U and write Y per (node, lane), plus the node tables per tile
         const double tab = (double)op->nslot * 5 + (double)op->nsmax * 5 + 8 + 8 + 4;
         ctx->prof_stop(s, ps, ASR_KERNEL_STEP, (double)nt * nn * (2.0 * 9 * TL * sizeof(T2) + tab),
@@ -1873,9 +1880,7 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
   // to the library and a batch of at least 4 tiles fits in half the free device memory; else checkpoints every c
   // levels (c = stride, or ceil(sqrt(depth))) with the segments recomputed.  Both give the same G and the same gradient
   // to rounding (bitwise on the operators of the stride tests).
-  size_t freeb0 = 0, totb0 = 0;
-  cudaMemGetInfo(&freeb0, &totb0);
-  freeb0 += ctx->ws_bytes;   // a held slab is this call's to reuse
+  const size_t freeb0 = ctx->plan_bytes();
   const size_t vbytes = (size_t)nn * 9 * TL * sizeof(T2);
   const bool keep = stride <= 0 && (size_t)4 * (3 * mmax + 15 + (gen ? 3 * mmax + 3 : 0)) * vbytes <= freeb0 / 2;
   const int c = keep ? std::max(1, mmax) : std::max(1, stride > 0 ? stride : (int)std::ceil(std::sqrt((double)mmax)));
@@ -1904,13 +1909,12 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
   // the general operator keeps h X, O h X, S D O h X per segment level and h ybar, O h ybar, S D O h ybar (3 c + 3 more)
   const size_t vec_bytes = (size_t)nn * 9 * TL * sizeof(T2);
   const int nvec = 3 + 2 * nseg + (c + 2) + 2 * c + 8 + (gen ? 3 * c + 3 : 0);
-  size_t freeb = 0, totb = 0;
-  cudaMemGetInfo(&freeb, &totb);
-  freeb += ctx->ws_bytes;
+  const size_t freeb = freeb0;
   // tiles per batch: as the forward's default (16), halved while the batch's vectors would take more than half the free
   // device memory (a 16-tile batch of the fcc ternary workload holds about 70 GB)
   int tpb = 16;
-  if (const char* e = getenv("ASR_TILES_PER_BATCH")) tpb = std::max(1, atoi(e));
+  const char* tile_env = getenv("ASR_TILES_PER_BATCH");
+  if (tile_env) tpb = std::max(1, atoi(tile_env));
   while (tpb > 1 && (size_t)tpb * nvec * vec_bytes > freeb / 2) tpb /= 2;
   if ((size_t)nvec * vec_bytes > freeb) { set_error("adjoint: %d vectors of %zu bytes do not fit", nvec, vec_bytes); return ASR_ENOMEM; }
   tpb = std::min(tpb, ntile_all);
@@ -2015,6 +2019,10 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
     ASR_CUDA(cudaMemsetAsync(d_nfall.p, 0, sizeof(int), s));
     ASR_CUDA(cudaMemsetAsync(d_gacc.p, 0, (size_t)tpb * ngd * sizeof(double2), s));
     // the forward stops each lane by the depth test of src/asr_edc.f90:121-127 when depth_tol > 0; the reverse sweep then
+  // and no more than the context keeps between calls, where that is two tiles or more and no slab is held: allocating and
+  // freeing 70 GB at every call took 50 ms to a second, the smaller batches of the fcc ternary workload (3 tiles) take 20 ms
+  if (!tile_env && !ctx->ws_hold && (size_t)nvec * vec_bytes <= ctx->keep / 2)
+    tpb = (int)std::min<size_t>(tpb, ctx->keep / ((size_t)nvec * vec_bytes));
     // differentiates the chain at the depth it stopped at
     BatchView bv{nt, nn, op->nsmax, 0, ASR_MODE_EDC, project, tail, NLMAX, depth_tol, d_gblob.p, GL, d_ginfo.p, d_lgroup.p,
                  d_tgroup.p, d_z.p, d_act.p, d_wact.p, d_m.p, d_a.p, d_b.p, d_gprev.p, d_acur.p, d_bprev.p, d_su.p, d_sup.p,
@@ -2493,8 +2501,7 @@ int run_ed3_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, con
   const int ntile_all = (int)tiles.size();
   const size_t vec_bytes = (size_t)nn * 9 * TL * sizeof(T2);
   const int nvec = 8;   // U, UP, Y (rotating), T1, T3, Sa (S d x), TMP (d x), TV
-  size_t freeb = 0, totb = 0;
-  cudaMemGetInfo(&freeb, &totb);
+  const size_t freeb = ctx->plan_bytes() - ctx->ws_bytes;   // its vectors are not the held slab's
   int tpb = std::is_same<ST, double>::value ? 16 : 8;
   while (tpb > 1 && (size_t)tpb * nvec * vec_bytes > freeb / 2) tpb /= 2;
   if ((size_t)nvec * vec_bytes > freeb) { set_error("ed3: %d vectors of %zu bytes do not fit", nvec, vec_bytes); return ASR_ENOMEM; }
@@ -2738,8 +2745,7 @@ int run_epi_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, con
   const int ntile_all = (int)tiles.size();
   const size_t vec_bytes = (size_t)nn * 9 * TL * sizeof(T2);
   const int nvec = 3 + 1 + 4 + 2;   // U, UP, Y (rotating), TV, four step temporaries, S d x and d x of h'
-  size_t freeb = 0, totb = 0;
-  cudaMemGetInfo(&freeb, &totb);
+  const size_t freeb = ctx->plan_bytes() - ctx->ws_bytes;   // its vectors are not the held slab's
   int tpb = std::is_same<ST, double>::value ? 16 : 8;
   while (tpb > 1 && (size_t)tpb * nvec * vec_bytes > freeb / 2) tpb /= 2;
   if ((size_t)nvec * vec_bytes > freeb) { set_error("epi_blocks: %d vectors of %zu bytes do not fit", nvec, vec_bytes); return ASR_ENOMEM; }

@@ -90,23 +90,25 @@ struct RunOptions {
   int nodes_per_warp = 0;    // 0: automatic (the operator's tuned value, else 4)
 };
 
-// owning device buffer (freed on scope exit)
+// owning device buffer of a call (freed on scope exit)
 template <typename T>
 struct Dev {
   T* p = nullptr;
   size_t n = 0;
+  DevMem mem;
   Dev() = default;
   Dev(const Dev&) = delete;
   Dev& operator=(const Dev&) = delete;
-  ~Dev() { if (p) cudaFree(p); }
+  ~Dev() { mem.put(); }
   int alloc(size_t m) {
     if (m <= n && p) return ASR_OK;
-    if (p) cudaFree(p);
+    mem.put();
     p = nullptr; n = 0;
-    if (cudaMalloc(&p, (m > 0 ? m : 1) * sizeof(T)) != cudaSuccess) {
+    if (!mem.get((m > 0 ? m : 1) * sizeof(T))) {
       set_error("chains: device allocation of %zu bytes failed", m * sizeof(T));
       return ASR_ENOMEM;
     }
+    p = (T*)mem.p;
     n = m;
     return ASR_OK;
   }

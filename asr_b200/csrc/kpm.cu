@@ -430,12 +430,17 @@ __global__ void k_kpm_reduce(const double* part, int nblk, double* out) {
 template <typename T>
 struct DevBuf {
   T* p = nullptr;
-  ~DevBuf() { if (p) cudaFree(p); }
+  DevMem mem;
+  DevBuf() = default;
+  DevBuf(const DevBuf&) = delete;
+  DevBuf& operator=(const DevBuf&) = delete;
+  ~DevBuf() { mem.put(); }
   int alloc(size_t n) {
-    if (cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) {
+    if (!mem.get(std::max<size_t>(n, 1) * sizeof(T))) {
       set_error("kpm: device allocation of %zu bytes failed", n * sizeof(T));
       return ASR_ENOMEM;
     }
+    p = (T*)mem.p;
     return ASR_OK;
   }
 };
@@ -470,6 +475,7 @@ int kpm_run(asr_ctx* ctx, asr_supercell* sc, double cen, double scl, int nmom, i
   const size_t smem = 4 * 9 * sc->nsp * sizeof(double) + (size_t)(sc->ns + 1) * 81 * sizeof(ST);
   const bool general = !sc->o_zero;
   const int grid = ctx->num_sms * 4;
+  ctx->plan_bytes();   // how much the pool may keep
   DevBuf<ST> T0, T1, T2, W1, W2, W3;
   ASR_TRY(T0.alloc(nel)); ASR_TRY(T1.alloc(nel)); ASR_TRY(T2.alloc(nel));
   if (general) { ASR_TRY(W1.alloc(nel)); ASR_TRY(W2.alloc(nel)); ASR_TRY(W3.alloc(nel)); }
@@ -644,7 +650,7 @@ int asr_supercell_free(asr_supercell* sc) {
 int asr_supercell_apply(asr_supercell* sc, const double* x, double* y, int nvec) {
   if (!sc || !x || !y || nvec < 1) { set_error("asr_supercell_apply: bad argument"); return ASR_EINVAL; }
   asr_ctx* ctx = sc->ctx;
-  ASR_ON_DEVICE(ctx->device);
+  ASR_ENTER(ctx);
   cudaStream_t s = ctx->stream;
   const int n = sc->n;
   const size_t nel = (size_t)n * 9 * KV;
@@ -686,7 +692,7 @@ int asr_supercell_apply(asr_supercell* sc, const double* x, double* y, int nvec)
 int asr_kpm_moments(asr_ctx* ctx, asr_supercell* sc, double cen, double scl, int nmom, int v0, int nvec, uint64_t seed,
                     int precision, int doubling, double* mu) {
   if (!ctx || !sc || !mu || nmom < 1 || nvec < 1 || !(scl > 0.0)) { set_error("kpm_moments: bad argument"); return ASR_EINVAL; }
-  ASR_ON_DEVICE(ctx->device);
+  ASR_ENTER(ctx);
   if (precision == ASR_FP32) return kpm_run<float>(ctx, sc, cen, scl, nmom, v0, nvec, seed, doubling != 0, mu);
   return kpm_run<double>(ctx, sc, cen, scl, nmom, v0, nvec, seed, doubling != 0, mu);
 }
