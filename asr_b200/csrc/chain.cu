@@ -36,9 +36,6 @@ namespace {
 
 constexpr int WPB = 8;   // warps per block
 
-__device__ __forceinline__ double fma_(double a, double b, double c) { return fma(a, b, c); }
-__device__ __forceinline__ float fma_(float a, float b, float c) { return fmaf(a, b, c); }
-
 template <typename ST> struct St2;
 template <> struct St2<double> { typedef double2 T; };
 template <> struct St2<float> { typedef float2 T; };
@@ -48,7 +45,6 @@ __device__ __forceinline__ double2 ld(const float2* p) { float2 v = *p; return m
 __device__ __forceinline__ void stv(double2* p, double2 v) { *p = v; }
 __device__ __forceinline__ void stv(float2* p, double2 v) { *p = make_float2((float)v.x, (float)v.y); }
 // evict-first store / last-use load: streams that are read once must not push the gathered vector out of L2
-__device__ __forceinline__ void stv_cs(double2* p, double2 v) { __stcs(p, v); }
 __device__ __forceinline__ void stv_cs(float2* p, double2 v) { __stcs(p, make_float2((float)v.x, (float)v.y)); }
 __device__ __forceinline__ double2 ld_cs(const double2* p) { return __ldcs(p); }
 __device__ __forceinline__ double2 ld_cs(const float2* p) { float2 v = __ldcs(p); return make_double2(v.x, v.y); }
@@ -489,9 +485,13 @@ __global__ void __launch_bounds__(WPB * TL) k_smul(OpView op, BatchView bv, cons
   }
   if (FINAL) {
     block_reduce_store(dot, part, it.tile, bpt);
-    if (bv.tick && last_block_of_tile(bv.tick, it.tile, bpt)) {
+    int* const tick = EPI == 2 ? bv.adj.tick : bv.tick;
+    if (tick && last_block_of_tile(tick, it.tile, bpt)) {
       const double2 a = block_sum_rows(part + (size_t)it.tile * bpt * TL, bpt, TL);
-      if (threadIdx.x < TL) reduce_a_lane(bv, a, bv.kstep, it.tile, threadIdx.x);
+      if (threadIdx.x < TL) {
+        if (EPI == 2) bv.adj.d1[it.tile * TL + threadIdx.x] = a;
+        else reduce_a_lane(bv, a, bv.kstep, it.tile, threadIdx.x);
+      }
     }
   }
 }
@@ -782,9 +782,13 @@ __global__ void __launch_bounds__(WPB * TL, 2) k_smul_mma(OpView op, BatchView b
       own = zmul(zmul(s, s), own);
     }
     block_reduce_owned(own, owner, part, it.tile, bpt);
-    if (bv.tick && last_block_of_tile(bv.tick, it.tile, bpt)) {
+    int* const tick = EPI == 2 ? bv.adj.tick : bv.tick;
+    if (tick && last_block_of_tile(tick, it.tile, bpt)) {
       const double2 a = block_sum_rows(part + (size_t)it.tile * bpt * TL, bpt, TL);
-      if (threadIdx.x < TL) reduce_a_lane(bv, a, bv.kstep, it.tile, threadIdx.x);
+      if (threadIdx.x < TL) {
+        if (EPI == 2) bv.adj.d1[it.tile * TL + threadIdx.x] = a;
+        else reduce_a_lane(bv, a, bv.kstep, it.tile, threadIdx.x);
+      }
     }
   }
 }
@@ -1254,12 +1258,12 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
   // projections: per tile nlevmax x 9 nt x 32 complex values
   const size_t proj_tile_bytes = proj ? (size_t)nlevmax * 9 * proj->nt * TL * sizeof(double2) : 0;
   tpb = std::min(tpb, ntile_all);
+  const size_t freeb = ctx->plan_bytes((size_t)tpb * (nvec * vec_bytes + proj_tile_bytes));
+  while (tpb > 1 && (size_t)tpb * (nvec * vec_bytes + proj_tile_bytes) > freeb / 2) tpb /= 2;
   int npw = opt.nodes_per_warp > 0 ? opt.nodes_per_warp : op->tuned_npw[prec_ix] > 0 ? op->tuned_npw[prec_ix] : default_npw(nn);
   if (const char* e = getenv("ASR_NODES_PER_WARP")) npw = std::max(1, atoi(e));
   const int npb = WPB * npw;
   const int bpt = (nn + npb - 1) / npb;
-  const size_t freeb = ctx->plan_bytes((size_t)tpb * (nvec * vec_bytes + proj_tile_bytes));
-  while (tpb > 1 && (size_t)tpb * (nvec * vec_bytes + proj_tile_bytes) > freeb / 2) tpb /= 2;
   // device state
   Dev<double> d_gblob;
   Dev<GroupInfo> d_ginfo;
@@ -1467,12 +1471,80 @@ __global__ void __launch_bounds__(WPB * TL) k_dot(OpView op, BatchView bv, const
   block_reduce_store(dot, part, it.tile, bpt);
 }
 
-// wbar = P (c1 ubar_next + c2 X_next); partial dots wbar . X_k and wbar . X_{k-1}
+// scalars of reverse step k for every lane (state arrays indexed [lane][NLMAX], k 1-based):
+//   phase 0: coefficients of wbar from d1 = ubar_{k+1} . X_{k+1} (raw); with tile_act, a tile takes part in step k
+//            when one of its lanes is at least k deep (a warp of the launch is a tile)
+//   phase 1: abar', bbar_{k-1} update from d2 = wbar . X_k, d3 = wbar . X_{k-1} (raw), the coefficients of ybar and of
+//            ubar_k += A ybar + abar y_k - a_k wbar, ubar_{k-1} -= b_{k-1} wbar
+//   phase 2: phase 1 for the fused reverse step, where A ybar = A wbar + abar y_k and ubar_k is written whole:
+//            ubar_k = A wbar + 2 abar y_k - a_k wbar - b_k wbar_{k+1} (c5 = 2 abar, c6 = a_k, c4 = b_k below the lane's
+//            last level, else 0)
+struct AdjScal {
+  const double2* a;       // forward a_k
+  const double2* b;       // forward b_k
+  const int* m;           // depth per lane
+  double2* abar;
+  double2* bbar;
+  double2 *s_next, *s_k, *s_prev;   // scales of X_{k+1}, X_k, X_{k-1}
+  double2 *c1, *c2, *c3, *c4, *c5, *c6;
+  const double2* d1;
+};
+__device__ __forceinline__ double2 scale_of(const AdjScal& S, int L, int k) {   // s_k: u_k = s_k X_k
+  if (k <= 1) return make_double2(k == 1 ? 1.0 : 0.0, 0.0);
+  double2 b = S.b[(size_t)L * NLMAX + k - 2];
+  if (cmag(b) == 0.0 || k > S.m[L]) return make_double2(0, 0);
+  return chain_scale(b);
+}
+__device__ __forceinline__ void adj_scal_lane(const AdjScal& S, bool in, int L, int k, int phase, double2 d2, double2 d3) {
+  const double2 zero = make_double2(0, 0);
+  if (!in) {
+    if (phase == 0) { S.c1[L] = zero; S.c2[L] = zero; S.s_next[L] = zero; S.s_k[L] = zero; S.s_prev[L] = zero; }
+    else { S.c3[L] = zero; S.c4[L] = zero; S.c5[L] = zero; S.c6[L] = zero; }
+    return;
+  }
+  const size_t o = (size_t)L * NLMAX;
+  if (phase == 0) {
+    double2 sn = k < S.m[L] ? scale_of(S, L, k + 1) : zero;
+    S.s_next[L] = sn;
+    S.s_k[L] = scale_of(S, L, k);
+    S.s_prev[L] = scale_of(S, L, k - 1);
+    if (k < S.m[L]) {
+      double2 bk = S.b[o + k - 1];
+      double2 ib = cdiv(make_double2(1.0, 0.0), bk);
+      double2 d1 = cmul(sn, S.d1[L]);                           // ubar_{k+1} . u_{k+1}
+      double2 bb = csub(S.bbar[o + k - 1], cmul(d1, ib));
+      S.bbar[o + k - 1] = bb;
+      S.c1[L] = ib;                                              // wbar' = ubar_{k+1} / b_k + bbar_k u_{k+1}
+      S.c2[L] = cmul(bb, sn);
+    } else {
+      S.c1[L] = zero;
+      S.c2[L] = zero;
+    }
+  } else {
+    double2 sk = S.s_k[L], sp = S.s_prev[L];
+    double2 ab = csub(S.abar[o + k - 1], cmul(sk, d2));         // abar_k -= wbar . u_k
+    S.abar[o + k - 1] = ab;
+    if (k > 1) S.bbar[o + k - 2] = csub(S.bbar[o + k - 2], cmul(sp, d3));   // bbar_{k-1} -= wbar . u_{k-1}
+    S.c3[L] = cmul(ab, sk);                                      // ybar = wbar + abar u_k
+    if (phase == 2) {
+      S.c4[L] = k < S.m[L] ? S.b[o + k - 1] : zero;
+      S.c5[L] = cscale(ab, 2.0);
+    } else {
+      S.c4[L] = k > 1 ? S.b[o + k - 2] : zero;                   // ubar_{k-1} -= b_{k-1} wbar
+      S.c5[L] = ab;                                              // ubar_k += A ybar + abar y_k - a_k wbar
+    }
+    S.c6[L] = S.a[o + k - 1];
+  }
+}
+
+// wbar = P (c1 ubar_next + c2 X_next) and the dots wbar . X_k and wbar . X_{k-1}; the tile's last block sums the dots and runs
+// the scalars' phase 1 or 2 (as launches of their own the two sums and the scalars took 36 us a level, whatever the batch)
 template <typename ST>
 __global__ void __launch_bounds__(WPB * TL, 2) k_adj_w(OpView op, BatchView bv, const typename St2<ST>::T* __restrict__ ubn,
                                                     const typename St2<ST>::T* __restrict__ xn, const typename St2<ST>::T* __restrict__ xk,
-                                                    const typename St2<ST>::T* __restrict__ xkm, const double2* c1, const double2* c2,
-                                                    typename St2<ST>::T* __restrict__ wb, double2* part1, double2* part2, int npw) {
+                                                    const typename St2<ST>::T* __restrict__ xkm, AdjScal S, int k, int phase,
+                                                    typename St2<ST>::T* __restrict__ wb, double2* part1, double2* part2, int npw,
+                                                    int* tick) {
   NodeIter it;
   int bpt;
   if (!node_iter(bv, npw, it, bpt)) return;
@@ -1480,7 +1552,7 @@ __global__ void __launch_bounds__(WPB * TL, 2) k_adj_w(OpView op, BatchView bv, 
   const int L = it.tile * TL + lane;
   const int grp = bv.lane_group[L];
   const unsigned long long chim = grp >= 0 ? bv.ginfo[grp].chimask : 0ull;
-  const double2 a1 = c1[L], a2 = c2[L];
+  const double2 a1 = S.c1[L], a2 = S.c2[L];
   double2 d1 = make_double2(0, 0), d2 = make_double2(0, 0);
   for (int qn = 0; qn < npw; ++qn) {
     int i = it.first + w + WPB * qn;
@@ -1508,6 +1580,11 @@ __global__ void __launch_bounds__(WPB * TL, 2) k_adj_w(OpView op, BatchView bv, 
   block_reduce_store(d1, part1, it.tile, bpt);
   __syncthreads();
   block_reduce_store(d2, part2, it.tile, bpt);
+  if (last_block_of_tile(tick, it.tile, bpt)) {
+    const double2 s1 = block_sum_rows(part1 + (size_t)it.tile * bpt * TL, bpt, TL);
+    const double2 s2 = block_sum_rows(part2 + (size_t)it.tile * bpt * TL, bpt, TL);
+    if (threadIdx.x < TL) adj_scal_lane(S, grp >= 0 && k <= S.m[L], L, k, phase, s1, s2);
+  }
 }
 
 // ybar = wbar + c3 X_k;  ubar_{k-1} -= c4 wbar
@@ -1558,7 +1635,7 @@ __global__ void __launch_bounds__(WPB * TL) k_adj_u(OpView op, BatchView bv, con
 }
 
 // gradient partials of one reverse step: thread = element (orbital l, lane) of a node; per block and kind the sums over its nodes and
-// the 32 lanes: gpart[((tile * gbpt + blk) * NGK + kind) * 9 * nsp + l * nsp + species], kinds 0 c, 1 d, 2 pa, 3 o, 4 e
+// the 32 lanes, added to those of the levels above: gpart[((tile * gbpt + blk) * NGK + kind) * 9 * nsp + l * nsp + species], kinds 0 c, 1 d, 2 pa, 3 o, 4 e
 // (e and pb enter the same way).  With G_p(x, v) = x . (dR_p / dpar) v (x at the node, v through the flip links with the
 // class weights mt, or the node itself on a frozen site) and A = h - h O h + E + X(z), h = C + D S D:
 //   c: G(yb, u) - G(yb, O h u) - G(O h yb, u)
@@ -1571,20 +1648,49 @@ struct AdjVecs {   // per level: node side (yb: ybar; tb = S D ybar; hb = h ybar
   const void *yb, *tb, *hb, *rb, *qb;
   const void *xk, *tk, *hk, *rk, *qk;
 };
-// a[sp] += v with sp known only at run time: an unrolled select over the NS accumulators keeps them in registers (an
-// indexed array would live in local memory); the accumulator sees the same additions in the same order
-template <int NS>
-__device__ __forceinline__ void add_sp(double2 (&a)[NS], int sp, double2 v) {
-#pragma unroll
-  for (int q = 0; q < NS; ++q)
-    if (q == sp) a[q] = cadd(a[q], v);
+// the register accumulators' species count for an operator of nsp species
+inline int grad_ns(int nsp) { return nsp <= 3 ? 3 : nsp <= 5 ? 5 : MAXSP; }
+// Weights of a link by species, dense: row (class, own state, link state) has NS weights (zero where the class lacks the
+// species), the rows after those are the frozen species' unit weights.  A row's mask has the species of nonzero weight.
+inline void grad_rows(const asr_op* op, int NS, std::vector<double>& wt, std::vector<unsigned char>& mask) {
+  const int nsm = op->nsmax, nrow = op->ncls * nsm * nsm + op->nsp;
+  wt.assign((size_t)nrow * NS, 0.0);
+  mask.assign(nrow, 0);
+  for (int kap = 0; kap < op->ncls; ++kap)
+    for (int own = 0; own < nsm; ++own)
+      for (int kp = 0; kp < nsm; ++kp) {
+        const int row = (kap * nsm + own) * nsm + kp;
+        for (int q = 0; q < op->nsc[kap]; ++q) {
+          const int sp = op->spc[q + (size_t)op->ldspc * kap] - 1;
+          wt[(size_t)row * NS + sp] += op->mt[own + nsm * (kp + nsm * (q + (size_t)nsm * kap))];
+        }
+        for (int sp = 0; sp < op->nsp; ++sp)
+          if (wt[(size_t)row * NS + sp] != 0.0) mask[row] |= 1u << sp;
+      }
+  for (int sp = 0; sp < op->nsp; ++sp) {
+    wt[(size_t)(nrow - op->nsp + sp) * NS + sp] = 1.0;
+    mask[nrow - op->nsp + sp] = 1u << sp;
+  }
 }
+struct GradRows {
+  const double* wt;
+  const unsigned char* mask;
+};
 
+// What bounds it: the streams of w-bar, S D w-bar, X_k and S D X_k (the floor at 16 tiles of 20,969 nodes is 0.88 ms) and,
+// before the sums were regrouped, the FP64 pipe: scaling each link value and adding its products species by species with
+// run-time selects took some 70 operations per link.  Now a link's products are formed once (12 operations), go to every
+// species with the row's dense weights (4 each), and what is common comes out of the sum: the orbit size into the node's
+// own side, the link's sign as a bit of the products, the lane's scale to the end.  The links of 64 nodes are looked up once
+// per block, so that the node loop holds no chain of dependent table reads, and all loads of a node and its first links are on
+// their way before the first product.  The fcc ternary adjoint's 60 launches of 16 tiles: 56 -> 27 ms, 3.9 TB/s of streams (two
+// blocks per SM by their registers; three, or the next node's values read ahead, spilled: 28 and 32 ms).
 // NS: a compile-time bound on the operator's species count (nsp <= NS), which sizes the register accumulators
+constexpr int GRN = 64, GRL = 512;   // nodes whose links a block looks up at once (fewer where GRL links would not do)
 template <typename ST, bool GEN, bool WY = false, int NS = MAXSP>
-__global__ void __launch_bounds__(GPW * TL) k_adj_grad(OpView op, BatchView bv, const double* mt, const int* spc, int ldspc,
-                                                       AdjVecs V, const double2* sk, int nodes_per_block, double2* gpart,
-                                                       const double2* cy = nullptr) {
+__global__ void __launch_bounds__(GPW * TL, GEN || NS > 5 ? 1 : 2) k_adj_grad(OpView op, BatchView bv, GradRows R, AdjVecs V, const double2* sk,
+                                                                    int nodes_per_block, double2* gpart,
+                                                                    const double2* cy = nullptr) {
   typedef typename St2<ST>::T T2;
   const T2 *yb = (const T2*)V.yb, *tb = (const T2*)V.tb, *hb = (const T2*)V.hb, *rb = (const T2*)V.rb, *qb = (const T2*)V.qb;
   const T2 *xk = (const T2*)V.xk, *tk = (const T2*)V.tk, *hk = (const T2*)V.hk, *rk = (const T2*)V.rk, *qk = (const T2*)V.qk;
@@ -1599,65 +1705,125 @@ __global__ void __launch_bounds__(GPW * TL) k_adj_grad(OpView op, BatchView bv, 
   double2 gc[NS], gd[NS], ge[NS], go[NS];   // pa = z e-kind
 #pragma unroll
   for (int q = 0; q < NS; ++q) { gc[q] = make_double2(0, 0); gd[q] = gc[q]; ge[q] = gc[q]; go[q] = gc[q]; }
+  // per node: the number of links to other nodes and the own link's row and species mask, the orbit size; per link (nsmax a
+  // node): the node, the row, the operation with the sign (bit 8), the species mask
+  __shared__ int4 s_own[GRN];
+  __shared__ double s_nb[GRN];
+  __shared__ int4 s_link[GRL];
+  const int cn = max(1, min(GRN, GRL / nsm));
   const bool live = bv.lane_group[L] >= 0 && grp >= 0;
-  double2 z = make_double2(0, 0);
-  if (live) {
-    const GroupInfo gi = bv.ginfo[grp];
-    const double2 s = sk[L];
-    const double2 c3 = WY ? cy[L] : make_double2(0, 0);
-    z = bv.lane_z[L];
-    const int i0 = blk * nodes_per_block, i1 = min(bv.nn, i0 + nodes_per_block);
-    for (int i = i0; i < i1; ++i) {
-      const size_t q = vnode(tile, bv.nn, i) + threadIdx.x;
-      double2 y = ld(yb + q), ty = ld(tb + q);
-      if (WY) {   // the fused reverse step passes wbar and S D wbar: ybar = wbar + c3 X_k, S D ybar = S D wbar + c3 S D X_k
-        y = cadd(y, cmul(c3, ld(xk + q)));
-        ty = cadd(ty, cmul(c3, ld(tk + q)));
-      }
-      double2 hy = make_double2(0, 0), ry = hy, qy = hy;
-      if (GEN) { hy = ld(hb + q); ry = ld(rb + q); qy = ld(qb + q); }
-      const double nb = op.sq[i] * op.sq[i];
-      const int fs = frozen_of(op, gi, i);
-      const int kap = op.ncl[i], own = op.lst[i], nk = op.nsc[kap];
-      const int nlink = fs > 0 ? 1 : nk;
-      for (int kp = 0; kp < nlink; ++kp) {
-        size_t qr = q;
-        double sgn = 1.0;
-        if (fs == 0 && kp != own) {
-          int r = op.flipr[kp + nsm * i];
+  const double2 z = live ? bv.lane_z[L] : make_double2(0, 0), s = live ? sk[L] : make_double2(0, 0);
+  const double2 c3 = WY && live ? cy[L] : make_double2(0, 0);
+  const int i0 = blk * nodes_per_block, i1 = min(bv.nn, i0 + nodes_per_block);
+  for (int c0 = i0; c0 < i1 && grp >= 0; c0 += cn) {
+    const int nc = min(cn, i1 - c0);
+    __syncthreads();
+    if (threadIdx.x < nc) {
+      const GroupInfo gi = bv.ginfo[grp];
+      const int i = c0 + threadIdx.x, fs = frozen_of(op, gi, i), kap = op.ncl[i], own = op.lst[i], nk = op.nsc[kap];
+      const int wrow = (kap * nsm + own) * nsm, row = fs > 0 ? op.ncls * nsm * nsm + fs - 1 : wrow + own;
+      int n = 0;
+      if (fs <= 0)
+        for (int kp = 0; kp < nk; ++kp) {
+          const int r = kp == own ? -1 : op.flipr[kp + nsm * i];
           if (r < 0) continue;
-          int g = op.flipg[kp + nsm * i];
-          bool neg = (gi.chimask >> g) & 1ull;
-          sgn = ((((uint32_t)op.sgm[g] >> l) & 1u) ^ (neg ? 1u : 0u)) ? -1.0 : 1.0;
-          qr = vx<ST>(tile, bv.nn, r, op.pi[g * 9 + l], lane);
+          const int g = op.flipg[kp + nsm * i];
+          s_link[threadIdx.x * nsm + n++] = make_int4(r, wrow + kp, g | (int)((gi.chimask >> g) & 1ull) << 8, R.mask[wrow + kp]);
         }
-        const double2 x = cscale(cmul(s, ld(xk + qr)), sgn), t = cscale(cmul(s, ld(tk + qr)), sgn);
-        double2 qe = cmul(y, x);                                          // G(yb, u)
-        double2 qc = qe, qd = cadd(cmul(y, t), cmul(ty, x)), qo = make_double2(0, 0);
-        if (GEN) {
-          const double2 hx = cscale(cmul(s, ld(hk + qr)), sgn), rx = cscale(cmul(s, ld(rk + qr)), sgn);
-          const double2 qx = cscale(cmul(s, ld(qk + qr)), sgn);
-          qc = csub(csub(qe, cmul(y, rx)), cmul(ry, x));
-          qd = csub(csub(qd, cadd(cmul(y, qx), cmul(ty, rx))), cadd(cmul(ry, t), cmul(qy, x)));
-          qo = csub(make_double2(0, 0), cmul(hy, hx));
+      s_nb[threadIdx.x] = op.sq[i] * op.sq[i];
+      s_own[threadIdx.x] = make_int4(n, row, 0, R.mask[row]);
+    }
+    __syncthreads();
+    if (!live) continue;
+    struct Side { double2 y, ty, hy, ry, qy; };
+    auto own_side = [&](int j, Side& a) {
+      const size_t q = vnode(tile, bv.nn, c0 + j) + threadIdx.x;
+      a.y = ld(yb + q);
+      a.ty = ld(tb + q);
+      if (GEN) { a.hy = ld(hb + q); a.ry = ld(rb + q); a.qy = ld(qb + q); }
+    };
+    // one link's products, with its sign
+    struct Link { double2 x, t, hx, rx, qx; int row, mask; bool neg; };
+    auto link_side = [&](size_t q, Link& k) {
+      k.x = ld(xk + q);
+      k.t = ld(tk + q);
+      if (GEN) { k.hx = ld(hk + q); k.rx = ld(rk + q); k.qx = ld(qk + q); }
+    };
+    auto link = [&](const Side& a, const Link& k) {
+      const double2 x = k.x, t = k.t;
+      double2 pe = zmul(a.y, x), pd = zfma(a.ty, x, zmul(a.y, t)), pc = pe, po = make_double2(0, 0);
+      if (GEN) {
+        const double2 n = make_double2(-k.rx.x, -k.rx.y), m = make_double2(-x.x, -x.y), p = make_double2(-a.y.x, -a.y.y);
+        pc = zfma(a.ry, m, zfma(a.y, n, pe));
+        pd = zfma(a.qy, m, zfma(a.ty, n, zfma(p, k.qx, zfma(make_double2(-a.ry.x, -a.ry.y), t, pd))));
+        po = zmul(a.hy, k.hx);
+        po = k.neg ? po : make_double2(-po.x, -po.y);
+      }
+      if (k.neg) {
+        pe = make_double2(-pe.x, -pe.y);
+        pd = make_double2(-pd.x, -pd.y);
+        if (GEN) pc = make_double2(-pc.x, -pc.y);
+      }
+      const double* wt = R.wt + (size_t)k.row * NS;
+#pragma unroll
+      for (int sp = 0; sp < NS; ++sp)
+        if (k.mask >> sp & 1) {
+          const double m = __ldg(wt + sp);
+          ge[sp] = make_double2(fma(m, pe.x, ge[sp].x), fma(m, pe.y, ge[sp].y));
+          gd[sp] = make_double2(fma(m, pd.x, gd[sp].x), fma(m, pd.y, gd[sp].y));
+          if (GEN) {
+            gc[sp] = make_double2(fma(m, pc.x, gc[sp].x), fma(m, pc.y, gc[sp].y));
+            go[sp] = make_double2(fma(m, po.x, go[sp].x), fma(m, po.y, go[sp].y));
+          }
         }
-        qe = cscale(qe, nb); qc = cscale(qc, nb); qd = cscale(qd, nb); qo = cscale(qo, nb);
-        if (fs > 0) {
-          add_sp<NS>(ge, fs - 1, qe);
-          add_sp<NS>(gd, fs - 1, qd);
-          if (GEN) { add_sp<NS>(gc, fs - 1, qc); add_sp<NS>(go, fs - 1, qo); }
-          continue;
-        }
-        for (int sidx = 0; sidx < nk; ++sidx) {
-          double m = mt[own + nsm * (kp + nsm * (sidx + (size_t)nsm * kap))];
-          if (m == 0.0) continue;
-          int sp = spc[sidx + ldspc * kap] - 1;
-          add_sp<NS>(ge, sp, cscale(qe, m));
-          add_sp<NS>(gd, sp, cscale(qd, m));
-          if (GEN) { add_sp<NS>(gc, sp, cscale(qc, m)); add_sp<NS>(go, sp, cscale(qo, m)); }
-        }
+    };
+    Side a;
+    for (int j = 0; j < nc; ++j) {
+      const size_t q0 = vnode(tile, bv.nn, c0 + j) + threadIdx.x;
+      const int cnt = s_own[j].x;
+      // the values of the first links and the node's own, all on their way before the first product
+      constexpr int NF = GEN ? 1 : 2;
+      Link k[NF], own;
+      auto fetch = [&](int e, Link& k) {
+        const int4 lk = s_link[j * nsm + e];
+        const int g = lk.z & 255;
+        k.row = lk.y;
+        k.mask = lk.w;
+        k.neg = ((((uint32_t)__ldg(op.sgm + g) >> l) ^ (lk.z >> 8)) & 1u) != 0;
+        link_side(vx<ST>(tile, bv.nn, lk.x, __ldg(op.pi + g * 9 + l), lane), k);
+      };
+#pragma unroll
+      for (int e = 0; e < NF; ++e)
+        if (cnt > e) fetch(e, k[e]);
+      own_side(j, a);
+      link_side(q0, own);
+      own.row = s_own[j].y;
+      own.mask = s_own[j].w;
+      own.neg = false;
+      const double nb = s_nb[j];
+      if (WY) {   // the fused reverse step passes wbar and S D wbar: ybar = wbar + c3 X_k, S D ybar = S D wbar + c3 S D X_k
+        a.y = zfma(c3, own.x, a.y);
+        a.ty = zfma(c3, own.t, a.ty);
+      }
+      a.y = zscale(a.y, nb);
+      a.ty = zscale(a.ty, nb);
+      if (GEN) { a.hy = zscale(a.hy, nb); a.ry = zscale(a.ry, nb); a.qy = zscale(a.qy, nb); }
+      link(a, own);
+#pragma unroll
+      for (int e = 0; e < NF; ++e)
+        if (cnt > e) link(a, k[e]);
+      for (int e = NF; e < cnt; ++e) {
+        fetch(e, own);
+        link(a, own);
       }
     }
+  }
+#pragma unroll
+  for (int q = 0; q < NS; ++q) {   // the link side is s X_k
+    ge[q] = zmul(s, ge[q]);
+    gd[q] = zmul(s, gd[q]);
+    // h ybar and O h ybar are linear in ybar: one factor s in every product
+    if (GEN) { gc[q] = zmul(s, gc[q]); go[q] = zmul(s, go[q]); }
   }
   // sum over the 32 lanes, fixed order; pa = z e per lane before the sum.  FP32: one warp is one orbital.  FP64: warps 0-7 hold
   // eight lanes of four orbitals each (thread t: orbital t % 4 of the quad w / 4), warp 8 orbital 8.
@@ -1684,7 +1850,7 @@ __global__ void __launch_bounds__(GPW * TL) k_adj_grad(OpView op, BatchView bv, 
         for (int k = 0; k < NGK; ++k) quad[w][t][k * NS + q] = v[k];
     } else if (t == 0) {
 #pragma unroll
-      for (int k = 0; k < NGK; ++k) out[(k * 9 + l) * nsp + q] = v[k];
+      for (int k = 0; k < NGK; ++k) out[(k * 9 + l) * nsp + q] = cadd(out[(k * 9 + l) * nsp + q], v[k]);
     }
   }
   if (FRAG) {
@@ -1693,32 +1859,32 @@ __global__ void __launch_bounds__(GPW * TL) k_adj_grad(OpView op, BatchView bv, 
       const int q = e % nsp, lo = (e / nsp) % 8, k = e / (8 * nsp);
       double2 v = quad[4 * (lo >> 2)][lo & 3][k * NS + q];
       for (int j = 1; j < 4; ++j) v = cadd(v, quad[4 * (lo >> 2) + j][lo & 3][k * NS + q]);
-      out[(k * 9 + lo) * nsp + q] = v;
+      out[(k * 9 + lo) * nsp + q] = cadd(out[(k * 9 + lo) * nsp + q], v);
     }
   }
 }
 
 // k_adj_grad with the register accumulators sized for the operator's species count
 template <typename ST, bool GEN, bool WY = false>
-void launch_adj_grad(int nsp, unsigned grid, cudaStream_t s, const OpView& ov, const BatchView& bv, const double* mt,
-                     const int* spc, int ldspc, const AdjVecs& av, const double2* sk, int gnpb, double2* gpart,
-                     const double2* cy = nullptr) {
-  if (nsp <= 3)
-    k_adj_grad<ST, GEN, WY, 3><<<grid, GPW * TL, 0, s>>>(ov, bv, mt, spc, ldspc, av, sk, gnpb, gpart, cy);
-  else if (nsp <= 5)
-    k_adj_grad<ST, GEN, WY, 5><<<grid, GPW * TL, 0, s>>>(ov, bv, mt, spc, ldspc, av, sk, gnpb, gpart, cy);
+void launch_adj_grad(int nsp, unsigned grid, cudaStream_t s, const OpView& ov, const BatchView& bv, const GradRows& R,
+                     const AdjVecs& av, const double2* sk, int gnpb, double2* gpart, const double2* cy = nullptr) {
+  const int ns = grad_ns(nsp);
+  if (ns == 3)
+    k_adj_grad<ST, GEN, WY, 3><<<grid, GPW * TL, 0, s>>>(ov, bv, R, av, sk, gnpb, gpart, cy);
+  else if (ns == 5)
+    k_adj_grad<ST, GEN, WY, 5><<<grid, GPW * TL, 0, s>>>(ov, bv, R, av, sk, gnpb, gpart, cy);
   else
-    k_adj_grad<ST, GEN, WY, MAXSP><<<grid, GPW * TL, 0, s>>>(ov, bv, mt, spc, ldspc, av, sk, gnpb, gpart, cy);
+    k_adj_grad<ST, GEN, WY, MAXSP><<<grid, GPW * TL, 0, s>>>(ov, bv, R, av, sk, gnpb, gpart, cy);
 }
 
-// gacc[tile][NGK][9][nsp] += sum over the blocks of the step's partials (fixed order)
+// gacc[tile][NGK][9][nsp] = sum over the blocks of their partials (fixed order), which hold every level's
 // grid (ntile, ceil(ng / 32)), RED_THREADS per block: lane j of the block's warps sums entry 32 blockIdx.y + j
 __global__ void k_adj_gsum(int ntile, int gbpt, int ng, const int* tile_act, const double2* gpart, double2* gacc) {
   const int tile = blockIdx.x;
   if (tile >= ntile || !tile_act[tile]) return;
   const int e0 = blockIdx.y * TL, e = e0 + threadIdx.x % TL;
   const double2 sum = block_sum_rows(gpart + (size_t)tile * gbpt * ng + e0, gbpt, ng, e < ng);
-  if (threadIdx.x < TL && e < ng) gacc[(size_t)tile * ng + e] = cadd(gacc[(size_t)tile * ng + e], sum);
+  if (threadIdx.x < TL && e < ng) gacc[(size_t)tile * ng + e] = sum;
 }
 
 // per-lane sum of partials: out[L] = sum_q part[(tile * bpt + q) * TL + lane]
@@ -1729,76 +1895,13 @@ __global__ void k_lane_sum(int ntile, int bpt, const int* tile_act, const double
   if (threadIdx.x < TL) out[tile * TL + threadIdx.x] = sum;
 }
 
-// scalars of reverse step k for every lane (state arrays indexed [lane][NLMAX], k 1-based):
-//   phase 0: coefficients of wbar from d1 = ubar_{k+1} . X_{k+1} (raw); with tile_act, a tile takes part in step k
-//            when one of its lanes is at least k deep (a warp of the launch is a tile)
-//   phase 1: abar', bbar_{k-1} update from d2 = wbar . X_k, d3 = wbar . X_{k-1} (raw), the coefficients of ybar and of
-//            ubar_k += A ybar + abar y_k - a_k wbar, ubar_{k-1} -= b_{k-1} wbar
-//   phase 2: phase 1 for the fused reverse step, where A ybar = A wbar + abar y_k and ubar_k is written whole:
-//            ubar_k = A wbar + 2 abar y_k - a_k wbar - b_k wbar_{k+1} (c5 = 2 abar, c6 = a_k, c4 = b_k below the lane's
-//            last level, else 0)
-struct AdjScal {
-  const double2* a;       // forward a_k
-  const double2* b;       // forward b_k
-  const int* m;           // depth per lane
-  double2* abar;
-  double2* bbar;
-  double2 *s_next, *s_k, *s_prev;   // scales of X_{k+1}, X_k, X_{k-1}
-  double2 *c1, *c2, *c3, *c4, *c5, *c6;
-  const double2 *d1, *d2, *d3;
-};
-__device__ __forceinline__ double2 scale_of(const AdjScal& S, int L, int k) {   // s_k: u_k = s_k X_k
-  if (k <= 1) return make_double2(k == 1 ? 1.0 : 0.0, 0.0);
-  double2 b = S.b[(size_t)L * NLMAX + k - 2];
-  if (cmag(b) == 0.0 || k > S.m[L]) return make_double2(0, 0);
-  return chain_scale(b);
-}
-__global__ void k_adj_scal(AdjScal S, int nlane, const int* lane_group, int k, int phase, int* tile_act = nullptr) {
+__global__ void k_adj_scal(AdjScal S, int nlane, const int* lane_group, int k, int* tile_act) {
   int L = blockIdx.x * blockDim.x + threadIdx.x;
   if (L >= nlane) return;   // nlane is a multiple of TL: whole warps leave
-  if (tile_act) {
-    const unsigned any = __ballot_sync(0xffffffffu, lane_group[L] >= 0 && k <= S.m[L]);
-    if (L % TL == 0) tile_act[L / TL] = any != 0;
-  }
-  const double2 zero = make_double2(0, 0);
-  if (lane_group[L] < 0 || k > S.m[L]) {
-    if (phase == 0) { S.c1[L] = zero; S.c2[L] = zero; S.s_next[L] = zero; S.s_k[L] = zero; S.s_prev[L] = zero; }
-    else { S.c3[L] = zero; S.c4[L] = zero; S.c5[L] = zero; S.c6[L] = zero; }
-    return;
-  }
-  const size_t o = (size_t)L * NLMAX;
-  if (phase == 0) {
-    double2 sn = k < S.m[L] ? scale_of(S, L, k + 1) : zero;
-    S.s_next[L] = sn;
-    S.s_k[L] = scale_of(S, L, k);
-    S.s_prev[L] = scale_of(S, L, k - 1);
-    if (k < S.m[L]) {
-      double2 bk = S.b[o + k - 1];
-      double2 ib = cdiv(make_double2(1.0, 0.0), bk);
-      double2 d1 = cmul(sn, S.d1[L]);                           // ubar_{k+1} . u_{k+1}
-      double2 bb = csub(S.bbar[o + k - 1], cmul(d1, ib));
-      S.bbar[o + k - 1] = bb;
-      S.c1[L] = ib;                                              // wbar' = ubar_{k+1} / b_k + bbar_k u_{k+1}
-      S.c2[L] = cmul(bb, sn);
-    } else {
-      S.c1[L] = zero;
-      S.c2[L] = zero;
-    }
-  } else {
-    double2 sk = S.s_k[L], sp = S.s_prev[L];
-    double2 ab = csub(S.abar[o + k - 1], cmul(sk, S.d2[L]));   // abar_k -= wbar . u_k
-    S.abar[o + k - 1] = ab;
-    if (k > 1) S.bbar[o + k - 2] = csub(S.bbar[o + k - 2], cmul(sp, S.d3[L]));   // bbar_{k-1} -= wbar . u_{k-1}
-    S.c3[L] = cmul(ab, sk);                                      // ybar = wbar + abar u_k
-    if (phase == 2) {
-      S.c4[L] = k < S.m[L] ? S.b[o + k - 1] : zero;
-      S.c5[L] = cscale(ab, 2.0);
-    } else {
-      S.c4[L] = k > 1 ? S.b[o + k - 2] : zero;                   // ubar_{k-1} -= b_{k-1} wbar
-      S.c5[L] = ab;                                              // ubar_k += A ybar + abar y_k - a_k wbar
-    }
-    S.c6[L] = S.a[o + k - 1];
-  }
+  const bool in = lane_group[L] >= 0 && k <= S.m[L];
+  const unsigned any = __ballot_sync(0xffffffffu, in);
+  if (L % TL == 0) tile_act[L / TL] = any != 0;
+  adj_scal_lane(S, in, L, k, 0, make_double2(0, 0), make_double2(0, 0));
 }
 
 // G and the seeds abar, bbar (cleared) of every lane of depth m >= 1 from the adjoint of its fraction with the weight w; one
@@ -1916,25 +2019,33 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
   const char* tile_env = getenv("ASR_TILES_PER_BATCH");
   if (tile_env) tpb = std::max(1, atoi(tile_env));
   while (tpb > 1 && (size_t)tpb * nvec * vec_bytes > freeb / 2) tpb /= 2;
+  // and no more than the context keeps between calls, where that is two tiles or more and no slab is held: allocating and
+  // freeing 70 GB at every call took 50 ms to a second, the smaller batches of the fcc ternary workload (3 tiles) take 20 ms
+  if (!tile_env && !ctx->ws_hold && (size_t)nvec * vec_bytes <= ctx->keep / 2)
+    tpb = (int)std::min<size_t>(tpb, ctx->keep / ((size_t)nvec * vec_bytes));
   if ((size_t)nvec * vec_bytes > freeb) { set_error("adjoint: %d vectors of %zu bytes do not fit", nvec, vec_bytes); return ASR_ENOMEM; }
   tpb = std::min(tpb, ntile_all);
   const int npw = default_npw(nn), npb = WPB * npw, bpt = (nn + npb - 1) / npb;
-  int gnpb = 64;   // nodes per block of the gradient kernel
+  int gnpb = 64;   // nodes per block of the gradient kernel (16 on the 994-node operator: 155 us a level for 116, the block sums)
   if (const char* e = getenv("ASR_ADJ_GRAD_NODES")) gnpb = std::max(1, atoi(e));
   const int gbpt = (nn + gnpb - 1) / gnpb, ngd = NGK * 9 * nsp;
   const int nlp = tpb * TL;
-  Dev<double> d_gblob, d_mt;
+  Dev<double> d_gblob, d_wt;
   Dev<GroupInfo> d_ginfo;
-  Dev<int> d_spc;
+  Dev<unsigned char> d_mask;
+  std::vector<double> wt;
+  std::vector<unsigned char> wmask;
+  grad_rows(op, grad_ns(nsp), wt, wmask);
   ASR_TRY(d_gblob.alloc(gblob.size())); ASR_TRY(d_ginfo.alloc(ginfo.size()));
-  ASR_TRY(d_mt.alloc(op->mt.size())); ASR_TRY(d_spc.alloc(op->spc.size()));
+  ASR_TRY(d_wt.alloc(wt.size())); ASR_TRY(d_mask.alloc(wmask.size()));
+  const GradRows gr{d_wt.p, d_mask.p};
   ASR_CUDA(cudaMemcpyAsync(d_gblob.p, gblob.data(), gblob.size() * sizeof(double), cudaMemcpyHostToDevice, s));
   ASR_CUDA(cudaMemcpyAsync(d_ginfo.p, ginfo.data(), ginfo.size() * sizeof(GroupInfo), cudaMemcpyHostToDevice, s));
-  ASR_CUDA(cudaMemcpyAsync(d_mt.p, op->mt.data(), op->mt.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-  ASR_CUDA(cudaMemcpyAsync(d_spc.p, op->spc.data(), op->spc.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+  ASR_CUDA(cudaMemcpyAsync(d_wt.p, wt.data(), wt.size() * sizeof(double), cudaMemcpyHostToDevice, s));
+  ASR_CUDA(cudaMemcpyAsync(d_mask.p, wmask.data(), wmask.size(), cudaMemcpyHostToDevice, s));
   Dev<int> d_lgroup, d_act, d_wact, d_m, d_tact, d_tact0, d_nfall, d_tgroup, d_tick;
   Dev<double2> d_a, d_b, d_abar, d_bbar, d_gprev, d_acur, d_bprev, d_su, d_sup, d_part, d_part2, d_z, d_gpart, d_gacc;
-  Dev<double2> d_sn, d_sk, d_sp, d_c[6], d_d1, d_d2, d_d3, d_one, d_w, d_g;
+  Dev<double2> d_sn, d_sk, d_sp, d_c[6], d_d1, d_one, d_w, d_g;
   ASR_TRY(d_lgroup.alloc(nlp)); ASR_TRY(d_act.alloc(nlp)); ASR_TRY(d_wact.alloc(nlp)); ASR_TRY(d_m.alloc(nlp));
   ASR_TRY(d_tact.alloc(tpb)); ASR_TRY(d_tact0.alloc(tpb)); ASR_TRY(d_nfall.alloc(1)); ASR_TRY(d_tgroup.alloc(tpb));
   ASR_TRY(d_tick.alloc(tpb));
@@ -1945,7 +2056,7 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
   ASR_TRY(d_z.alloc(nlp)); ASR_TRY(d_gpart.alloc((size_t)tpb * gbpt * ngd)); ASR_TRY(d_gacc.alloc((size_t)tpb * ngd));
   ASR_TRY(d_sn.alloc(nlp)); ASR_TRY(d_sk.alloc(nlp)); ASR_TRY(d_sp.alloc(nlp));
   for (int q = 0; q < 6; ++q) ASR_TRY(d_c[q].alloc(nlp));
-  ASR_TRY(d_d1.alloc(nlp)); ASR_TRY(d_d2.alloc(nlp)); ASR_TRY(d_d3.alloc(nlp)); ASR_TRY(d_one.alloc(nlp));
+  ASR_TRY(d_d1.alloc(nlp)); ASR_TRY(d_one.alloc(nlp));
   ASR_TRY(d_w.alloc(nlp)); ASR_TRY(d_g.alloc(nlp));
   // the vectors: one slab (the context's held one, or allocated here and freed on return)
   const size_t vlen = (size_t)tpb * nn * 9 * TL;
@@ -2017,12 +2128,8 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
     ASR_CUDA(cudaMemsetAsync(d_bprev.p, 0, nlp * sizeof(double2), s));
     ASR_CUDA(cudaMemsetAsync(d_sup.p, 0, nlp * sizeof(double2), s));
     ASR_CUDA(cudaMemsetAsync(d_nfall.p, 0, sizeof(int), s));
-    ASR_CUDA(cudaMemsetAsync(d_gacc.p, 0, (size_t)tpb * ngd * sizeof(double2), s));
+    ASR_CUDA(cudaMemsetAsync(d_gpart.p, 0, (size_t)tpb * gbpt * ngd * sizeof(double2), s));
     // the forward stops each lane by the depth test of src/asr_edc.f90:121-127 when depth_tol > 0; the reverse sweep then
-  // and no more than the context keeps between calls, where that is two tiles or more and no slab is held: allocating and
-  // freeing 70 GB at every call took 50 ms to a second, the smaller batches of the fcc ternary workload (3 tiles) take 20 ms
-  if (!tile_env && !ctx->ws_hold && (size_t)nvec * vec_bytes <= ctx->keep / 2)
-    tpb = (int)std::min<size_t>(tpb, ctx->keep / ((size_t)nvec * vec_bytes));
     // differentiates the chain at the depth it stopped at
     BatchView bv{nt, nn, op->nsmax, 0, ASR_MODE_EDC, project, tail, NLMAX, depth_tol, d_gblob.p, GL, d_ginfo.p, d_lgroup.p,
                  d_tgroup.p, d_z.p, d_act.p, d_wact.p, d_m.p, d_a.p, d_b.p, d_gprev.p, d_acur.p, d_bprev.p, d_su.p, d_sup.p,
@@ -2115,7 +2222,7 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
     ASR_CUDA(cudaMemsetAsync(d_bbar.p, 0, (size_t)nlp * NLMAX * sizeof(double2), s));
     k_cf_adjoint<<<nlp, 1, 0, s>>>(bv, nlp, d_w.p, d_abar.p, d_bbar.p, d_g.p);
     AdjScal S{d_a.p, d_b.p, d_m.p, d_abar.p, d_bbar.p, d_sn.p, d_sk.p, d_sp.p, d_c[0].p, d_c[1].p, d_c[2].p, d_c[3].p, d_c[4].p,
-              d_c[5].p, d_d1.p, d_d2.p, d_d3.p};
+              d_c[5].p, d_d1.p};
     // adjoint BatchView: unit scales for applying A to ybar
     BatchView bva = bv;
     bva.su = d_one.p;
@@ -2167,31 +2274,22 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
         T2* ubn = UB[(k + 1) % 2];
         const int ps = ctx->prof_start(s);
         int pp = ctx->prof_start(s);
-        k_adj_scal<<<(nlp + 127) / 128, 128, 0, s>>>(S, nlp, d_lgroup.p, k, 0, d_tact.p);
+        k_adj_scal<<<(nlp + 127) / 128, 128, 0, s>>>(S, nlp, d_lgroup.p, k, d_tact.p);
         ctx->prof_stop(s, pp, ASR_KERNEL_ADJ_SCAL, 0.0, 0.0);
         pp = ctx->prof_start(s);
-        k_adj_w<ST><<<grid, WPB * TL, 0, s>>>(ov, bva, ubn, XS(q + 2), XS(q + 1), XS(q), d_c[0].p, d_c[1].p, wk, d_part.p, d_part2.p,
-                                              npw);
+        k_adj_w<ST><<<grid, WPB * TL, 0, s>>>(ov, bva, ubn, XS(q + 2), XS(q + 1), XS(q), S, k, 2, wk, d_part.p, d_part2.p, npw,
+                                              d_tick.p);
         ctx->prof_stop(s, pp, ASR_KERNEL_ADJ_VEC, vstream * 5.0, 0.0);
-        pp = ctx->prof_start(s);
-        k_lane_sum<<<nt, RED_THREADS, 0, s>>>(nt, bpt, d_tact.p, d_part.p, d_d2.p);
-        k_lane_sum<<<nt, RED_THREADS, 0, s>>>(nt, bpt, d_tact.p, d_part2.p, d_d3.p);
-        k_adj_scal<<<(nlp + 127) / 128, 128, 0, s>>>(S, nlp, d_lgroup.p, k, 2);
-        ctx->prof_stop(s, pp, ASR_KERNEL_ADJ_SCAL, 0.0, 0.0);
         BatchView bvt = bva;
         bvt.t2out = T2B;
-        bvt.adj = AdjEpi{YS(q), wn, XS(q + 1), ubk, d_c[4].p, d_c[5].p, d_c[3].p};
+        bvt.adj = AdjEpi{YS(q), wn, XS(q + 1), ubk, d_c[4].p, d_c[5].p, d_c[3].p, d_d1.p, d_tick.p};
         pp = ctx->prof_start(s);
         launch_smul<ST, true, true, 2>(op, bvt, blk, wk, nullptr, d_part.p, npw, grid, s);
         ctx->prof_stop(s, pp, ASR_KERNEL_ADJ_STEP, vstream * 6.0, sflops);
-        pp = ctx->prof_start(s);
-        k_lane_sum<<<nt, RED_THREADS, 0, s>>>(nt, bpt, d_tact.p, d_part.p, d_d1.p);
-        ctx->prof_stop(s, pp, ASR_KERNEL_ADJ_SCAL, 0.0, 0.0);
         AdjVecs av{wk, T2B, nullptr, nullptr, nullptr, XS(q + 1), TS(q), nullptr, nullptr, nullptr};
         pp = ctx->prof_start(s);
-        launch_adj_grad<ST, false, true>(nsp, nt * gbpt, s, ov, bva, d_mt.p, d_spc.p, op->ldspc, av, d_sk.p, gnpb, d_gpart.p,
+        launch_adj_grad<ST, false, true>(nsp, nt * gbpt, s, ov, bva, gr, av, d_sk.p, gnpb, d_gpart.p,
                                          d_c[2].p);
-        k_adj_gsum<<<dim3(nt, (ngd + TL - 1) / TL), RED_THREADS, 0, s>>>(nt, gbpt, ngd, d_tact.p, d_gpart.p, d_gacc.p);
         ctx->prof_stop(s, pp, ASR_KERNEL_ADJ_GRAD, vstream * 4.0, 0.0);
         // one fused reverse level: 15 vector streams per (node, lane) (w-bar 5, step 6, parameter gradient 4); flops of its
         // one S application
@@ -2205,12 +2303,9 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
         const int ps = ctx->prof_start(s);
         k_dot<ST><<<grid, WPB * TL, 0, s>>>(ov, bva, ubn, XS(q + 2), d_part.p, npw);
         k_lane_sum<<<nt, RED_THREADS, 0, s>>>(nt, bpt, d_tact.p, d_part.p, d_d1.p);
-        k_adj_scal<<<(nlp + 127) / 128, 128, 0, s>>>(S, nlp, d_lgroup.p, k, 0, d_tact.p);
-        k_adj_w<ST><<<grid, WPB * TL, 0, s>>>(ov, bva, ubn, XS(q + 2), XS(q + 1), XS(q), d_c[0].p, d_c[1].p, WB, d_part.p, d_part2.p,
-                                              npw);
-        k_lane_sum<<<nt, RED_THREADS, 0, s>>>(nt, bpt, d_tact.p, d_part.p, d_d2.p);
-        k_lane_sum<<<nt, RED_THREADS, 0, s>>>(nt, bpt, d_tact.p, d_part2.p, d_d3.p);
-        k_adj_scal<<<(nlp + 127) / 128, 128, 0, s>>>(S, nlp, d_lgroup.p, k, 1);
+        k_adj_scal<<<(nlp + 127) / 128, 128, 0, s>>>(S, nlp, d_lgroup.p, k, d_tact.p);
+        k_adj_w<ST><<<grid, WPB * TL, 0, s>>>(ov, bva, ubn, XS(q + 2), XS(q + 1), XS(q), S, k, 1, WB, d_part.p, d_part2.p, npw,
+                                              d_tick.p);
         k_adj_y<ST><<<grid, WPB * TL, 0, s>>>(ov, bva, WB, XS(q + 1), d_c[2].p, d_c[3].p, YB, k > 1 ? ubp : nullptr, npw);
         // A ybar (unit scale) and t2bar = S R_d ybar (the general operator: also h ybar, O h ybar, S D O h ybar)
         if (gen) {
@@ -2226,10 +2321,9 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
         k_adj_u<ST><<<grid, WPB * TL, 0, s>>>(ov, bva, AY, YS(q), WB, d_c[4].p, d_c[5].p, ubk, npw);
         AdjVecs av{YB, T2B, HB, RB, QB, XS(q + 1), TS(q), HS(q), RS(q), QS(q)};
         if (gen)
-          launch_adj_grad<ST, true>(nsp, nt * gbpt, s, ov, bva, d_mt.p, d_spc.p, op->ldspc, av, d_sk.p, gnpb, d_gpart.p);
+          launch_adj_grad<ST, true>(nsp, nt * gbpt, s, ov, bva, gr, av, d_sk.p, gnpb, d_gpart.p);
         else
-          launch_adj_grad<ST, false>(nsp, nt * gbpt, s, ov, bva, d_mt.p, d_spc.p, op->ldspc, av, d_sk.p, gnpb, d_gpart.p);
-        k_adj_gsum<<<dim3(nt, (ngd + TL - 1) / TL), RED_THREADS, 0, s>>>(nt, gbpt, ngd, d_tact.p, d_gpart.p, d_gacc.p);
+          launch_adj_grad<ST, false>(nsp, nt * gbpt, s, ov, bva, gr, av, d_sk.p, gnpb, d_gpart.p);
         ASR_CUDA(cudaMemsetAsync(ubn, 0, cpy, s));   // becomes ubar_{k-2}
         // one reverse level: 26 vector streams per (node, lane) over its kernels (dot 2, w-bar 5, y-bar 4, S application
         // 2, combine 3, u-bar 5, parameter gradient 4, clear 1); flops of its one S application
@@ -2237,6 +2331,7 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
                        (double)nt * nn * TL * (op->nslot + 1) * 81.0 * 4.0);
       }
     }
+    k_adj_gsum<<<dim3(nt, (ngd + TL - 1) / TL), RED_THREADS, 0, s>>>(nt, gbpt, ngd, d_tact0.p, d_gpart.p, d_gacc.p);
     ASR_CUDA(cudaGetLastError());
     ASR_CUDA(cudaMemcpyAsync(hgacc.data(), d_gacc.p, (size_t)tpb * ngd * sizeof(double2), cudaMemcpyDeviceToHost, s));
     ASR_CUDA(cudaMemcpyAsync(hm.data(), d_m.p, nlp * sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -2251,11 +2346,11 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
       for (int e = 0; e < ngd; ++e) grad_out[(size_t)gq * ngd + e] = cadd(grad_out[(size_t)gq * ngd + e], hgacc[(size_t)bt * ngd + e]);
     }
     // launches per level: forward (operator, a reduction unless in the step, Lanczos update), recomputation (scalars,
-    // operator, update), reverse (fused: 9; else 11 and the operator); the depth test's separate reductions not counted
+    // operator, update), reverse (fused: 4; else 7 and the operator); the depth test's separate reductions not counted
     const int nsd = dunif ? 1 : 2;                                       // one S application
     const int nap = gen ? 2 * nsd + 3 : (dunif ? 1 : nsd + 1);           // one operator application
-    const int fwd = fusedrev ? 2 : nap + 2, rev = fusedrev ? 9 : nap + 11;
-    ctx->launches += 1 + (int64_t)kmax * (fwd + (keep ? 0 : nap + 2) + rev);
+    const int fwd = fusedrev ? 2 : nap + 2, rev = fusedrev ? 4 : nap + 7;
+    ctx->launches += 2 + (int64_t)kmax * (fwd + (keep ? 0 : nap + 2) + rev);
   }
   return ASR_OK;
 }

@@ -40,6 +40,8 @@ struct AdjEpi {
   const double2* ca;       // per lane: 2 abar_k
   const double2* cb;       // a_k
   const double2* cc;       // b_k (0 at the lane's last level)
+  double2* d1;             // per lane ubar_k . X_k, summed by the tile's last block
+  int* tick;
 };
 
 // One batch: ntile tiles x TL lanes.  Lane L = tile * TL + j.
