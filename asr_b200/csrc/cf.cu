@@ -27,13 +27,14 @@ __global__ void k_cf_eval(const double2* a, const double2* b, const int* m, int 
 __global__ void k_cf_eval_chain(const double2* a, const double2* b, const int* m, int ld, const double2* z, int nz, int tail, double2* g,
                                 double2* edges, int* nfall) {
   __shared__ double2 sh[2];
+  __shared__ BpRoots R;
   const int c = blockIdx.x, mc = m[c];
   const double2 *ac = a + (size_t)ld * c, *bc = b + (size_t)ld * c;
   const bool ok = mc >= 1 && mc <= CF_NMAX;
   if (threadIdx.x < 32) {
     double2 wd[CF_NMAX], we[CF_NMAX], aa, bb;
     int nf;
-    cf_tail_pair(ok && threadIdx.x < 2, ac, bc, mc, tail, wd, we, nf, aa, bb);
+    cf_tail_warp(ok, ac, bc, mc, tail, R, wd, we, nf, aa, bb);
     if (threadIdx.x == 0) {
       sh[0] = aa;
       sh[1] = bb;

@@ -150,51 +150,198 @@ __host__ __device__ inline void cf_tail_dev(const double2* a, const double2* b, 
 }
 
 #ifdef __CUDACC__
-// cf_tail_dev by pairs of threads (2 q, 2 q + 1) of a warp, which all call it: both get the tail of their chain (live:
-// there is one).  The two eigenvalue problems of a Beer-Pettifor iteration, T + bb and T - bb in the last diagonal entry,
-// run on the two threads; a chain that has converged waits for the warp's last.  nf: tail fallbacks (both threads).
-__device__ inline void cf_tail_pair(bool live, const double2* a, const double2* b, int m, int tail, double2* wd, double2* we, int& nf,
-                                    double2& aa, double2& bb) {
-  const int sub = threadIdx.x & 1;
+// The roots of one chain's two Beer-Pettifor problems, T with +bb and with -bb in the last diagonal entry, for one warp.
+struct BpRoots {
+  double2 a[CF_NMAX], b2[CF_NMAX];        // diagonal and squared off-diagonal, scaled to entries of order one
+  double2 lam[2][2][CF_NMAX];             // [buffer][+bb, -bb][root]
+};
+// one Ehrlich-Aberth sweep over the m roots of both problems, from buffer `cur` into the other one (all roots at once; a thread
+// takes the roots t, t + 32, ..): with N = p / p' of the characteristic polynomial (its three-term recurrence) a root moves by
+// N / (1 - N sum_j 1 / (x - x_j)).  al: the last diagonal entries.  True when every root moved less than 1e-11: the sweep's
+// convergence is cubic, so what is left is below the rounding of the entries.
+__device__ inline bool bp_sweep(BpRoots& R, int m, int cur, const double2 (&al)[2]) {
+  bool settled = true;
+  for (int i = threadIdx.x & 31; i < m; i += 32) {
+    double2 x[2], p0[2], pm[2], q0[2], qm[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      x[u] = R.lam[cur][u][i];
+      p0[u] = make_double2(1.0, 0.0);
+      pm[u] = q0[u] = qm[u] = make_double2(0.0, 0.0);
+    }
+    for (int k = 0; k < m; ++k) {
+      const double2 ak = R.a[k], c = k > 0 ? R.b2[k - 1] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const double2 t = csub(x[u], k == m - 1 ? al[u] : ak);
+        const double2 q1 = cadd(csub(cmul(t, q0[u]), cmul(c, qm[u])), p0[u]), p1 = csub(cmul(t, p0[u]), cmul(c, pm[u]));
+        pm[u] = p0[u];
+        p0[u] = p1;
+        qm[u] = q0[u];
+        q0[u] = q1;
+      }
+    }
+    // sum_j 1 / (x - x_j) as a fraction num / den: one division a root, none in the loop
+    double2 num[2], den[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      num[u] = make_double2(0.0, 0.0);
+      den[u] = make_double2(1.0, 0.0);
+    }
+    for (int j = 0; j < m; ++j) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const double2 d = csub(x[u], R.lam[cur][u][j]);
+        const bool other = d.x != 0.0 || d.y != 0.0;   // not itself
+        const double2 n1 = cadd(cmul(num[u], d), den[u]), d1 = cmul(den[u], d);
+        num[u] = other ? n1 : num[u];
+        den[u] = other ? d1 : den[u];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {   // p / p' / (1 - p / p' num / den)
+      double2 step = make_double2(0.0, 0.0);
+      if (p0[u].x != 0.0 || p0[u].y != 0.0)
+        step = cdiv(cmul(p0[u], den[u]), csub(cmul(q0[u], den[u]), cmul(p0[u], num[u])));
+      if (!(cabs1(step) <= 1.0e-11)) settled = false;
+      R.lam[cur ^ 1][u][i] = csub(x[u], step);
+    }
+  }
+  __syncwarp();
+  return __all_sync(0xffffffffu, settled);
+}
+// the warp's sums of N values a thread
+template <int N>
+__device__ __forceinline__ void warp_sums(double (&v)[N]) {
+  for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], off);
+}
+// the roots of both problems from those in buffer `cur`: settled within 24 sweeps, and complete (sum and sum of squares of the
+// roots against the traces of T and T^2, tr and tr2 without the last entry)
+__device__ inline bool bp_roots(BpRoots& R, int m, int& cur, const double2 (&al)[2], double2 tr, double2 tr2) {
+  int left = 24;
+  for (bool ok = false; !ok; cur ^= 1) {
+    if (left-- == 0) return false;
+    ok = bp_sweep(R, m, cur, al);
+  }
+  double v[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  for (int i = threadIdx.x & 31; i < m; i += 32)
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const double2 x = R.lam[cur][u][i], q = cmul(x, x);
+      v[4 * u] += x.x;
+      v[4 * u + 1] += x.y;
+      v[4 * u + 2] += q.x;
+      v[4 * u + 3] += q.y;
+    }
+  warp_sums(v);
+  bool good = true;
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const double2 e1 = csub(make_double2(v[4 * u], v[4 * u + 1]), cadd(tr, al[u]));
+    const double2 e2 = csub(make_double2(v[4 * u + 2], v[4 * u + 3]), cadd(tr2, cmul(al[u], al[u])));
+    good = good && cabs1(e1) <= 1.0e-11 * m && cabs1(e2) <= 1.0e-10 * m;
+  }
+  return good;
+}
+// the root of problem u with the largest (sgn = 1) or smallest (-1) real part
+__device__ inline double2 bp_edge(const BpRoots& R, int m, int cur, int u, double sgn) {
+  double best = -1.0 / 0.0;
+  int at = 0;
+  for (int i = threadIdx.x & 31; i < m; i += 32)
+    if (sgn * R.lam[cur][u][i].x > best) { best = sgn * R.lam[cur][u][i].x; at = i; }
+  for (int off = 16; off > 0; off >>= 1) {
+    const double v = __shfl_xor_sync(0xffffffffu, best, off);
+    const int w = __shfl_xor_sync(0xffffffffu, at, off);
+    if (v > best || (v == best && w < at)) { best = v; at = w; }
+  }
+  return R.lam[cur][u][at];
+}
+
+// cf_tail_dev by one warp (live: there is a chain, the same for the whole warp); every thread gets the tail.  nf: tail fallbacks.
+// Only the Beer-Pettifor tail uses more than one thread: its map bb -> (edge of T + bb, edge of T - bb) is iterated as
+// written there, up to 200 times, but after the hull's eigenvalue problem (plane rotations, one thread) the spectra are
+// followed from one iteration to the next by bp_roots, all roots at once, some three sweeps an iteration (17 us with its checks at 20 levels;
+// the rotations, a serial chain, took 265 us).  Roots that do not settle or are not complete, near-defective chains, are
+// left to the rotations, for good after the third time.
+__device__ inline void cf_tail_warp(bool live, const double2* a, const double2* b, int m, int tail, BpRoots& R, double2* wd, double2* we,
+                                    int& nf, double2& aa, double2& bb) {
+  const int t = threadIdx.x & 31;
   nf = 0;
   aa = bb = make_double2(0.0, 0.0);
-  if (tail != 2) {
-    if (live) cf_tail_dev(a, b, m, tail, wd, we, nullptr, aa, bb);
-    return;
-  }
-  double2 lo, hi, a0 = aa, b0 = bb;
-  const bool eig = live && m >= 2 && chain_extremes(a, b, m, a[m - 1], wd, we, lo, hi) == 0;
-  if (eig) {
-    aa = a0 = cscale(cadd(lo, hi), 0.5);
-    bb = b0 = cscale(csub(hi, lo), 0.25);
-  } else if (live) {   // the last coefficients
-    aa = a[m - 1];
-    bb = m > 1 ? b[m - 2] : make_double2(0.0, 0.0);
-  }
-  bool done = !eig;   // the same for both threads of a pair
-  for (int it = 0; it < 200 && __any_sync(0xffffffffu, !done); ++it) {
-    double2 edge = make_double2(0.0, 0.0);   // the upper edge of T + bb (sub 0), the lower of T - bb (sub 1)
-    int bad = 0;
-    if (!done) {
-      bad = chain_extremes(a, b, m, sub ? csub(a[m - 1], bb) : cadd(a[m - 1], bb), wd, we, lo, hi);
-      edge = sub ? lo : hi;
+  if (!live) return;
+  double2 lo, hi;
+  int eig = 0;
+  if (t == 0) {
+    if (tail != 2) cf_tail_dev(a, b, m, tail, wd, we, nullptr, aa, bb);
+    else if (m >= 2 && chain_extremes(a, b, m, a[m - 1], wd, we, lo, hi) == 0) {
+      eig = 1;
+      aa = cscale(cadd(lo, hi), 0.5);
+      bb = cscale(csub(hi, lo), 0.25);
+    } else {   // the last coefficients
+      aa = a[m - 1];
+      bb = m > 1 ? b[m - 2] : make_double2(0.0, 0.0);
     }
-    __syncwarp();
-    const double2 other = make_double2(__shfl_xor_sync(0xffffffffu, edge.x, 1), __shfl_xor_sync(0xffffffffu, edge.y, 1));
-    bad |= __shfl_xor_sync(0xffffffffu, bad, 1);
-    if (done) continue;
-    if (bad) { ++nf; done = true; continue; }   // an eigenvalue failure keeps the last iterate
-    const double2 h1 = sub ? other : edge, l2 = sub ? edge : other;
+  }
+  __syncwarp();
+  auto bcast = [](double2 v) { return make_double2(__shfl_sync(0xffffffffu, v.x, 0), __shfl_sync(0xffffffffu, v.y, 0)); };
+  aa = bcast(aa);
+  bb = bcast(bb);
+  if (!__shfl_sync(0xffffffffu, eig, 0)) return;
+  const double2 a0 = aa, b0 = bb;
+  // a power of two that brings the largest entry to order one
+  double big = 0.0;
+  for (int k = t; k < m; k += 32) big = fmax(big, fmax(cabs1(a[k]), k < m - 1 ? cabs1(b[k]) : 0.0));
+  for (int off = 16; off > 0; off >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, off));
+  const int ex = big > 0.0 && big < 1e300 ? ilogb(big) : 0;
+  const double sc = scalbn(1.0, -ex), us = scalbn(1.0, ex);
+  double2 tr = make_double2(0.0, 0.0), tr2 = tr;
+  for (int k = t; k < m; k += 32) {
+    const double2 ak = cscale(a[k], sc), bk = k < m - 1 ? cscale(b[k], sc) : make_double2(0.0, 0.0), c = cmul(bk, bk);
+    R.a[k] = ak;
+    R.b2[k] = c;
+    if (k < m - 1) { tr = cadd(tr, ak); tr2 = cadd(tr2, cadd(cmul(ak, ak), cscale(c, 2.0))); }
+  }
+  double trs[4] = {tr.x, tr.y, tr2.x, tr2.y};
+  warp_sums(trs);
+  tr = make_double2(trs[0], trs[1]);
+  tr2 = make_double2(trs[2], trs[3]);
+  if (t == 0)
+    for (int k = 0; k < m; ++k) R.lam[0][0][k] = R.lam[0][1][k] = cscale(wd[k], sc);
+  __syncwarp();
+  int cur = 0, lost = 0;
+  for (int it = 0; it < 200; ++it) {
+    const double2 ap = cadd(a[m - 1], bb), am = csub(a[m - 1], bb);
+    const double2 al[2] = {cscale(ap, sc), cscale(am, sc)};
+    double2 h1, l2;
+    if (lost < 3 && bp_roots(R, m, cur, al, tr, tr2)) {
+      h1 = cscale(bp_edge(R, m, cur, 0, 1.0), us);
+      l2 = cscale(bp_edge(R, m, cur, 1, -1.0), us);
+    } else {
+      ++lost;
+      int bad = 0;
+      double2 edge = make_double2(0.0, 0.0);
+      if (t < 2) {
+        bad = chain_extremes(a, b, m, t ? am : ap, wd, we, lo, hi);
+        edge = t ? lo : hi;
+        if (!bad)
+          for (int k = 0; k < m; ++k) R.lam[cur][t][k] = cscale(wd[k], sc);
+      }
+      __syncwarp();
+      if (__any_sync(0xffffffffu, bad)) { ++nf; return; }   // an eigenvalue failure keeps the last iterate
+      h1 = bcast(edge);
+      l2 = make_double2(__shfl_sync(0xffffffffu, edge.x, 1), __shfl_sync(0xffffffffu, edge.y, 1));
+    }
     const double2 an = cscale(cadd(h1, l2), 0.5), bn = cscale(csub(h1, l2), 0.25);
-    done = cmag(csub(an, aa)) + cmag(csub(bn, bb)) < 1.0e-12 * (1.0 + cmag(bn));
+    const bool done = cmag(csub(an, aa)) + cmag(csub(bn, bb)) < 1.0e-12 * (1.0 + cmag(bn));
     aa = an;
     bb = bn;
+    if (__shfl_sync(0xffffffffu, (int)done, 0)) return;
   }
-  if (eig && !done) {   // no fixed point within 200 iterations: the hull
-    ++nf;
-    aa = a0;
-    bb = b0;
-  }
+  ++nf;   // no fixed point within 200 iterations: the hull
+  aa = a0;
+  bb = b0;
 }
 #endif
 
@@ -252,10 +399,8 @@ __host__ __device__ inline double2 cf_species_f_dev(const double2* a, const doub
 
 // cf_species with the factors pv_k = [g]_{k1} = gt_1 prod_{j<k} (b_j gt_{j+1}) of the projections f = sum_k c_k pv_k
 // (src/asr_chain.f90:111-122, the pv output used by edc_green_proj); pv (m) receives them, the return value is g11.
-__host__ __device__ inline double2 cf_species_pv_dev(const double2* a, const double2* b, int m, double2 z, int tail, double2* pv,
-                                                     double2* wd, double2* we, int* nfall) {
-  double2 aa, bb;
-  cf_tail_dev(a, b, m, tail, wd, we, nfall, aa, bb);
+__host__ __device__ inline double2 cf_species_pv_dev(const double2* a, const double2* b, int m, double2 z, double2 aa, double2 bb,
+                                                     double2* pv) {
   double2 tl = cf_tail_term(z, aa, bb);
   double2 one = make_double2(1.0, 0.0);
   pv[m - 1] = cdiv(one, csub(csub(z, a[m - 1]), tl));   // gt in place, then turned into the products

@@ -260,10 +260,13 @@ __device__ __forceinline__ void reduce_a_lane(const BatchView& bv, double2 asum,
 __global__ void k_depth_test(BatchView bv, int k) {
   const int L = blockIdx.x, grp = bv.lane_group[L];
   if (grp < 0 || !bv.tile_act[L / TL] || !bv.lane_wact[L] || !bv.lane_act[L]) return;
-  double2 wd[NLMAX], we[NLMAX];
-  int nf = 0;
-  double2 gtry = cf_species_dev(bv.acoef + (size_t)L * NLMAX, bv.bcoef + (size_t)L * NLMAX, k, bv.lane_z[L], bv.tail, wd, we,
-                                &nf, nullptr);
+  __shared__ BpRoots R;
+  const double2 *a = bv.acoef + (size_t)L * NLMAX, *b = bv.bcoef + (size_t)L * NLMAX;
+  double2 wd[NLMAX], we[NLMAX], aa, bb;
+  int nf;
+  cf_tail_warp(true, a, b, k, bv.tail, R, wd, we, nf, aa, bb);
+  if (threadIdx.x != 0) return;
+  const double2 gtry = cf_green_dev(a, b, k, bv.lane_z[L], aa, bb);
   if (nf) atomicAdd(bv.nfall, nf);
   if (k > 8 && cmag(csub(gtry, bv.gprev[L])) <= bv.depth_tol * cmag(gtry)) {   // :123-125
     bv.lane_wact[L] = 0;
@@ -999,17 +1002,19 @@ __global__ void k_reduce_b(BatchView bv, const double2* part, int bpt, int k, do
 
 // final fraction of every lane: cf_species with the chosen tail (edc mode); lmap: batch lane -> output lane (-1: none).
 // Bound by the dependent plane rotations of one lane's eigenvalue problem, so a block is one lane: lanes of a warp would wait
-// for its longest.  Two threads share a Beer-Pettifor tail (cf_tail_pair).  A 16-level
+// for its longest; the block's warp shares a Beer-Pettifor tail (cf_tail_warp).  A 16-level
 // hull takes 0.16 ms (0.69 ms with one thread per lane of a full warp, hypot, square roots and divisions in every rotation), a
-// batch of 16 tiles of Beer-Pettifor tails, depths 14-26, whose slowest lanes use all 200 iterations, 53 ms (455 ms before).
+// batch of 16 tiles of Beer-Pettifor tails, depths 14-26, whose slowest lanes use all 200 iterations, 3.4 ms (53 ms where every
+// iteration solved its two eigenvalue problems from the start, on two threads).
 __global__ void k_cf_final(BatchView bv, int nlane, const int* lmap, double2* g) {
   const int L = blockIdx.x;
   if (lmap[L] < 0 || bv.lane_group[L] < 0) return;
   const int m = bv.lane_m[L];
   const double2 *a = bv.acoef + (size_t)L * NLMAX, *b = bv.bcoef + (size_t)L * NLMAX;
+  __shared__ BpRoots R;
   double2 wd[NLMAX], we[NLMAX], aa, bb;
   int nf;
-  cf_tail_pair(m > 0 && threadIdx.x < 2, a, b, m, bv.tail, wd, we, nf, aa, bb);
+  cf_tail_warp(m > 0, a, b, m, bv.tail, R, wd, we, nf, aa, bb);
   if (threadIdx.x == 0) {
     g[lmap[L]] = m > 0 ? cf_green_dev(a, b, m, bv.lane_z[L], aa, bb) : make_double2(0, 0);
     if (nf) atomicAdd(bv.nfall, nf);
@@ -1066,14 +1071,17 @@ __global__ void k_proj_gather(OpView op, BatchView bv, const typename St2<ST>::T
 // pv of cf_species at depth m (pass 0) and at max(1, m - 4) (pass 1) for every lane (src/asr_edc.f90:221-231), into
 // pv[(pass * nlane + lane) * NLMAX + k]; one lane and pass per block (as k_depth_test)
 __global__ void k_proj_pv(BatchView bv, int nlane, double2* pv) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x, pass = q / nlane, L = q % nlane;
+  const int q = blockIdx.x, pass = q / nlane, L = q % nlane;
   if (pass > 1 || bv.lane_group[L] < 0 || bv.lane_m[L] < 1) return;
+  __shared__ BpRoots R;
   const int m = bv.lane_m[L], mm = pass == 0 ? m : (m - 4 > 1 ? m - 4 : 1);
-  double2 wd[NLMAX], we[NLMAX];
-  int nf = 0;
-  cf_species_pv_dev(bv.acoef + (size_t)L * NLMAX, bv.bcoef + (size_t)L * NLMAX, mm, bv.lane_z[L], bv.tail,
-                    pv + (size_t)q * NLMAX, wd, we, pass == 0 ? &nf : nullptr);
-  if (nf) atomicAdd(bv.nfall, nf);
+  const double2 *a = bv.acoef + (size_t)L * NLMAX, *b = bv.bcoef + (size_t)L * NLMAX;
+  double2 wd[NLMAX], we[NLMAX], aa, bb;
+  int nf;
+  cf_tail_warp(true, a, b, mm, bv.tail, R, wd, we, nf, aa, bb);
+  if (threadIdx.x != 0) return;
+  cf_species_pv_dev(a, b, mm, bv.lane_z[L], aa, bb, pv + (size_t)q * NLMAX);
+  if (nf && pass == 0) atomicAdd(bv.nfall, nf);
 }
 // gp(l, t) = sum_k cpr(k, l, t) pv_k, and gp4 with the shorter chain's pv; one warp per (tile, l, t), one thread per lane
 __global__ void k_proj_final(BatchView bv, int nlane, const int* lmap, ProjView P, const double2* pv) {
@@ -1377,7 +1385,7 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
                        (double)nt * nn * TL * (op->nslot + 1) * 81.0 * 4.0);
       }
       if (!a_in_step) k_reduce_a<<<nt, RED_THREADS, 0, s>>>(bv, d_part.p, bpt, k);
-      if (depth_due) k_depth_test<<<nt * TL, 1, 0, s>>>(bv, k);
+      if (depth_due) k_depth_test<<<nt * TL, 32, 0, s>>>(bv, k);
       BatchView bvw = bv;
       bvw.tick = d_tick.p;
       ps = ctx->prof_start(s);
@@ -1392,7 +1400,7 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
       ctx->launches += 1;
     }
     if (proj && opt.mode == ASR_MODE_EDC) {
-      k_proj_pv<<<2 * nlp, 1, 0, s>>>(bv, nlp, d_pv.p);
+      k_proj_pv<<<2 * nlp, 32, 0, s>>>(bv, nlp, d_pv.p);
       k_proj_final<<<(unsigned)(((long)nt * 9 * proj->nt * TL + 255) / 256), 256, 0, s>>>(bv, nlp, d_lmap.p, PV, d_pv.p);
       ctx->launches += 2;
     }
@@ -2169,7 +2177,7 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
         }
         ctx->prof_stop(s, ps, ASR_KERNEL_STEP, step_bytes(3), step_flops);
         if (!fusedrev) k_reduce_a<<<nt, RED_THREADS, 0, s>>>(bv, d_part.p, bpt, k);
-        if (depth_due(k)) k_depth_test<<<nt * TL, 1, 0, s>>>(bv, k);
+        if (depth_due(k)) k_depth_test<<<nt * TL, 32, 0, s>>>(bv, k);
         BatchView bvw = bv;
         bvw.kstep = k;
         bvw.tick = d_tick.p;
@@ -2200,7 +2208,7 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
       }
       ctx->prof_stop(s, ps, ASR_KERNEL_STEP, step_bytes(2), step_flops);
       if (!fusedrev) k_reduce_a<<<nt, RED_THREADS, 0, s>>>(bv, d_part.p, bpt, k);
-      if (depth_due(k)) k_depth_test<<<nt * TL, 1, 0, s>>>(bv, k);
+      if (depth_due(k)) k_depth_test<<<nt * TL, 32, 0, s>>>(bv, k);
       BatchView bvw = bv;
       bvw.kstep = k;
       bvw.tick = d_tick.p;
