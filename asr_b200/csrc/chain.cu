@@ -316,17 +316,12 @@ __device__ __forceinline__ double2 flip_if(double2 x, uint32_t bit) {
   unsigned long long m = (unsigned long long)bit << 63;
   return make_double2(__longlong_as_double(__double_as_longlong(x.x) ^ m), __longlong_as_double(__double_as_longlong(x.y) ^ m));
 }
-__device__ __forceinline__ float2 flip_if(float2 x, uint32_t bit) {
-  unsigned m = bit << 31;
-  return make_float2(__uint_as_float(__float_as_uint(x.x) ^ m), __uint_as_float(__float_as_uint(x.y) ^ m));
+// An orbital operation in shared memory, twelve words: word l has the sign of row l (bit 31) and the place of its orbital in a
+// node, pi(l) TL (bits 0..15); word 9 is 1 where no orbital moves (the identity and the sign changes of diagonal groups).
+constexpr int OPW = 12;
+__device__ __forceinline__ float2 flip_by(float2 x, uint32_t word) {
+  return make_float2(__uint_as_float(__float_as_uint(x.x) ^ (word & 0x80000000u)), __uint_as_float(__float_as_uint(x.y) ^ (word & 0x80000000u)));
 }
-template <typename ST> struct Pair;
-template <> struct Pair<double> { typedef double2 T; };
-template <> struct Pair<float> { typedef float2 T; };
-
-// packed orbital operation of the identity: permutation pi(l) = l in bits 4l..4l+3, no signs (bits 40..48)
-constexpr unsigned long long PW_IDENTITY = 0x876543210ull;
-constexpr unsigned long long PW_PERM_MASK = 0xFFFFFFFFFull;   // the nine 4-bit orbital indices
 
 // the output of one node of the S application: t2 (unscaled), or with FINAL y = s (d t2 + (c + e + X(z)) U) and the
 // node's share of the dot sum norb (s U) . y.  EPI 1: also t2 = S (d o U) into bv.t2out.  EPI 2 (the adjoint, U = wbar_k,
@@ -334,7 +329,7 @@ constexpr unsigned long long PW_PERM_MASK = 0xFFFFFFFFFull;   // the nine 4-bit 
 // being sum norb ubar_k . X_k (raw)
 template <typename ST, bool FINAL, int EPI = 0, typename T2, typename A2>
 __device__ __forceinline__ void smul_node_out(const OpView& op, const BatchView& bv, int tile, int i, int lane, int L, int grp,
-                                              int gflags, int gfrozen, const unsigned long long* piw, const T2* __restrict__ in,
+                                              int gflags, int gfrozen, const uint32_t* opw, const T2* __restrict__ in,
                                               T2* __restrict__ out, const A2* acc, double2& dot) {
   if (!FINAL) {
 #pragma unroll
@@ -350,6 +345,22 @@ __device__ __forceinline__ void smul_node_out(const OpView& op, const BatchView&
     const int nsm = op.nsmax, kap = op.ncl[i], l0 = op.lst[i], nk = op.nsc[kap];
     double2 ea = make_double2(0, 0), eb = ea, ec = ea;
     if (EPI == 2) { ea = bv.adj.ca[L]; eb = bv.adj.cb[L]; ec = bv.adj.cc[L]; }
+    // the first two flip links (all there are up to three species) are looked up once, not orbital by orbital
+    int fr[2] = {-1, -1}, fk[2] = {0, 0}, k2 = nk;
+    const uint32_t* fw[2] = {opw, opw};
+    if (fs <= 0) {
+      int n = 0;
+      for (int k = 0; k < nk; ++k) {
+        if (k == l0) continue;
+        const int r = op.flipr[k + nsm * i];
+        if (r < 0) continue;
+        if (n == 2) { k2 = k; break; }
+        const uint32_t* w = opw + OPW * op.flipg[k + nsm * i];
+        if (n == 0) { fr[0] = r; fk[0] = k; fw[0] = w; }
+        else { fr[1] = r; fk[1] = k; fw[1] = w; }
+        ++n;
+      }
+    }
 #pragma unroll
     for (int l = 0; l < 9; ++l) {
       double2 ui = ld(in + vx<ST>(tile, bv.nn, i, l, lane));
@@ -358,14 +369,16 @@ __device__ __forceinline__ void smul_node_out(const OpView& op, const BatchView&
         pt = cmul(praw(gb, bv.GL, PCEB, withx ? PA : -1, z, fs, l), ui);
       } else {
         pt = cmul(pweight(gb, bv.GL, PCEB, withx ? PA : -1, z, nsm, kap, l0, l0, l), ui);
-        for (int k = 0; k < nk; ++k) {
+        auto flip_link = [&](int r, int k, uint32_t w) {
+          const double2 xr = ld(in + vx<ST>(tile, bv.nn, r, 0, lane) + (w & 0xffffu));
+          pt = cadd(pt, cmul(pweight(gb, bv.GL, PCEB, withx ? PA : -1, z, nsm, kap, l0, k, l), flip_if(xr, w >> 31)));
+        };
+        if (fr[0] >= 0) flip_link(fr[0], fk[0], fw[0][l]);
+        if (fr[1] >= 0) flip_link(fr[1], fk[1], fw[1][l]);
+        for (int k = k2; k < nk; ++k) {
           if (k == l0) continue;
-          int r = op.flipr[k + nsm * i];
-          if (r < 0) continue;
-          const unsigned long long pw = piw[op.flipg[k + nsm * i]];
-          int p = (int)((pw >> (4 * l)) & 15ull);
-          double2 xr = flip_if(ld(in + vx<ST>(tile, bv.nn, r, p, lane)), (uint32_t)((pw >> (40 + l)) & 1ull));
-          pt = cadd(pt, cmul(pweight(gb, bv.GL, PCEB, withx ? PA : -1, z, nsm, kap, l0, k, l), xr));
+          const int r = op.flipr[k + nsm * i];
+          if (r >= 0) flip_link(r, k, opw[OPW * op.flipg[k + nsm * i] + l]);
         }
       }
       double2 y = cmul(s, cadd(make_double2(acc[l].x, acc[l].y), pt));
@@ -393,19 +406,20 @@ __device__ __forceinline__ void smul_node_out(const OpView& op, const BatchView&
 // FUSE_D: t1 = d o U is folded into the shared-memory blocks (the tile's d per orbital; d is invariant under the orbital
 // permutations of the group).  FINAL (needs FUSE_D, o = 0): y = s (d o S d o U + (c + e + X(z)) U) and the partial dot
 // sum_i norb_i (s U_i) . y_i (normalised-coordinate bilinear form).  Group data are per tile (single-group tiles).
-// LINK_ID: links whose orbital operation keeps the orbital order (the identity, and the pure sign changes of diagonal
-// groups such as D2h) gather their nine rows at fixed offsets, without the per-orbital index and sign decoding; the
-// products and their order are those of the general path, so both instantiations give the same bits.
-template <typename ST, bool FUSE_D, bool FINAL, bool LINK_ID, int EPI = 0>
-__global__ void __launch_bounds__(WPB * TL) k_smul(OpView op, BatchView bv, const ST* __restrict__ blocks,
+// Links whose operation moves no orbital (all of a diagonal group such as D2h) gather their nine rows at fixed offsets; the
+// others at the offsets of the operation's words.  Products and their order are the same.  FP32 only (FP64: k_smul_mma).
+// Bound by the instructions issued: a link is 90 paired or single FMAs, 25 shared-memory reads of the block, nine row reads and
+// the signs.  With the operation as a packed 64-bit word, decoded orbital by orbital, it was some 315 instructions in all and
+// 1.19 ms at 8 tiles of 20,969 nodes; with the words 1.01 ms (three blocks per SM; two 1.12, four, with spills, 1.06).
+template <typename ST, bool FUSE_D, bool FINAL, int EPI = 0>
+__global__ void __launch_bounds__(WPB * TL, 3) k_smul(OpView op, BatchView bv, const ST* __restrict__ blocks,
                                                    const typename St2<ST>::T* __restrict__ in,
                                                    typename St2<ST>::T* __restrict__ out, double2* part, int npw) {
   typedef typename St2<ST>::T T2;
-  typedef typename Pair<ST>::T P2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ns1 = op.nslot + 1;
   ST* Bs = (ST*)smem_raw;                                                        // [ntype][ns1][9][RW]
-  unsigned long long* piw = (unsigned long long*)(smem_raw + (((size_t)op.ntype * ns1 * BlockAcc<ST>::BLK * sizeof(ST) + 15) & ~(size_t)15));
+  uint32_t* opw = (uint32_t*)(smem_raw + (((size_t)op.ntype * ns1 * BlockAcc<ST>::BLK * sizeof(ST) + 15) & ~(size_t)15));   // [nop][OPW]
   NodeIter it;
   int bpt;
   bool live = node_iter(bv, npw, it, bpt);
@@ -428,10 +442,13 @@ __global__ void __launch_bounds__(WPB * TL) k_smul(OpView op, BatchView bv, cons
       BlockAcc<ST>::put(Bs + (size_t)tk * BlockAcc<ST>::BLK, l, lp, v);
     }
     for (int g = threadIdx.x; g < op.nop; g += blockDim.x) {
-      unsigned long long w = 0ull;
-      for (int l = 0; l < 9; ++l) w |= (unsigned long long)op.pi[g * 9 + l] << (4 * l);
-      uint32_t sg = op.sgm[g] ^ (((chimask >> g) & 1ull) ? 0x1FFu : 0u);
-      piw[g] = w | ((unsigned long long)sg << 40);
+      uint32_t fixed = 1u;
+      for (int l = 0; l < 9; ++l) {
+        const uint32_t p = op.pi[g * 9 + l];
+        fixed &= p == (uint32_t)l;
+        opw[g * OPW + l] = p * TL | (((op.sgm[g] >> l) ^ (uint32_t)((chimask >> g) & 1ull)) & 1u) << 31;
+      }
+      opw[g * OPW + 9] = fixed;
     }
   }
   __syncthreads();
@@ -466,25 +483,23 @@ __global__ void __launch_bounds__(WPB * TL) k_smul(OpView op, BatchView bv, cons
         gk = op.hopg[k + op.nslot * i];
       }
       if (r < 0) continue;
-      const unsigned long long pw = piw[gk];
+      uint32_t wd[OPW];
+#pragma unroll
+      for (int q = 0; q < OPW; q += 4) *(uint4*)(wd + q) = *(const uint4*)(opw + gk * OPW + q);
       const T2* src = in + vx<ST>(it.tile, bv.nn, r, 0, lane);
       T2 v[9];
-      if (LINK_ID && pw == PW_IDENTITY) {                                        // warp-uniform: one node, one slot
-        for (int lp = 0; lp < 9; ++lp) v[lp] = src[lp * TL];
-      } else if (LINK_ID && (pw & PW_PERM_MASK) == PW_IDENTITY) {               // signs only
-        const uint32_t sg = (uint32_t)(pw >> 40);
-        for (int lp = 0; lp < 9; ++lp) v[lp] = flip_if(src[lp * TL], (sg >> lp) & 1u);
+      if (wd[9]) {   // warp-uniform: one node, one slot
+#pragma unroll
+        for (int lp = 0; lp < 9; ++lp) v[lp] = flip_by(src[lp * TL], wd[lp]);
       } else {
-        for (int lp = 0; lp < 9; ++lp) {
-          int p = (int)((pw >> (4 * lp)) & 15ull);
-          v[lp] = flip_if(src[p * TL], (uint32_t)((pw >> (40 + lp)) & 1ull));
-        }
+#pragma unroll
+        for (int lp = 0; lp < 9; ++lp) v[lp] = flip_by(src[wd[lp] & 0xffffu], wd[lp]);
       }
       A.mac(B + (size_t)(k + 1) * BlockAcc<ST>::BLK, v);
     }
     T2 acc[9];
     A.out(acc);
-    smul_node_out<ST, FINAL, EPI>(op, bv, it.tile, i, lane, L, grp, gflags, gfrozen, piw, in, out, acc, dot);
+    smul_node_out<ST, FINAL, EPI>(op, bv, it.tile, i, lane, L, grp, gflags, gfrozen, opw, in, out, acc, dot);
   }
   if (FINAL) {
     block_reduce_store(dot, part, it.tile, bpt);
@@ -1123,7 +1138,7 @@ __global__ void k_init(BatchView bv, typename St2<ST>::T* u, typename St2<ST>::T
 size_t smul_smem(const asr_op* op, size_t st_size) {
   size_t b = (size_t)op->ntype * (op->nslot + 1) * 9 * RW * st_size;
   b = (b + 15) & ~(size_t)15;
-  b += (size_t)op->nop * sizeof(unsigned long long);
+  b += (size_t)op->nop * (st_size == sizeof(float) ? OPW * sizeof(uint32_t) : sizeof(unsigned long long));
   return b;
 }
 
@@ -1133,10 +1148,8 @@ void launch_smul(asr_op* op, const BatchView& bv, const ST* blk, const typename 
   OpView ov = op->view();   // EPI: the adjoint's fused steps, also t2 (bv.t2out); EPI 2, the reverse epilogue (bv.adj)
   if constexpr (std::is_same<ST, double>::value)
     k_smul_mma<FUSE_D, FINAL, EPI><<<grid, WPB * TL, MmaSm(ov).bytes, s>>>(ov, bv, blk, in, out, part, npw);
-  else if (op->tuned_link[1] == 1)
-    k_smul<ST, FUSE_D, FINAL, true, EPI><<<grid, WPB * TL, smul_smem(op, sizeof(ST)), s>>>(ov, bv, blk, in, out, part, npw);
   else
-    k_smul<ST, FUSE_D, FINAL, false, EPI><<<grid, WPB * TL, smul_smem(op, sizeof(ST)), s>>>(ov, bv, blk, in, out, part, npw);
+    k_smul<ST, FUSE_D, FINAL, EPI><<<grid, WPB * TL, smul_smem(op, sizeof(ST)), s>>>(ov, bv, blk, in, out, part, npw);
 }
 
 // y = s (h U - h O h U + (E + X) U) in FP64 at uniform d: H1 = h U, R1 = O h U, Y and the dots; TA, TB (or null): S d U, S d R1
@@ -2992,16 +3005,11 @@ static void smem_attrs() {
   cudaFuncSetAttribute(k_smul_mma<true, true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul_mma<true, true, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul_mma<true, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
-  cudaFuncSetAttribute(k_smul<float, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<float, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<float, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<float, true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<float, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<float, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<float, true, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<float, true, true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<float, true, true, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  cudaFuncSetAttribute(k_smul<float, true, true, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+  cudaFuncSetAttribute(k_smul<float, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+  cudaFuncSetAttribute(k_smul<float, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+  cudaFuncSetAttribute(k_smul<float, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+  cudaFuncSetAttribute(k_smul<float, true, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+  cudaFuncSetAttribute(k_smul<float, true, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   done[dev] = true;
 }
 
