@@ -360,7 +360,7 @@ static int op_build(asr_ctx* ctx, int nsite, const int* nbr_ptr, const int* nbr,
   }
   *out = nullptr;
   if (nsite < 1 || ncls < 1 || nop < 1 || nsp < 1 || ldspc < 1) { set_error("asr_op_build: empty input"); return ASR_EINVAL; }
-  ASR_ON_DEVICE(ctx->device);
+  ASR_ENTER(ctx);
   for (int k = 0; k < ncls; ++k) {
     if (nsc[k] < 1 || nsc[k] > ldspc) { set_error("asr_op_build: species count of class %d", k + 1); return ASR_EINVAL; }
     double sum = 0.0;

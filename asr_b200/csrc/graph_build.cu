@@ -357,35 +357,52 @@ __global__ void k_targets(BuildView B, int nt, const int* tsite, const int* nkey
 }
 
 // ---------------------------------------------------------------------------------------------------- host side
-template <typename T>
+// an array of the build: the operator's own tables (KEEP, handed over by release) from the device, the rest from the context
+template <typename T, bool KEEP = false>
 struct DBuf {
   T* p = nullptr;
   size_t n = 0;
-  ~DBuf() { if (p) cudaFree(p); }
-  int alloc(size_t m) {
-    if (m <= n && p) return ASR_OK;
-    if (p) cudaFree(p);
-    p = nullptr; n = 0;
-    if (cudaMalloc(&p, std::max<size_t>(m, 1) * sizeof(T)) != cudaSuccess) {
-      set_error("graph build: device allocation of %zu bytes failed", m * sizeof(T));
-      return ASR_ENOMEM;
+  DevMem m;
+  ~DBuf() { drop(); }
+  bool get(size_t k, T*& q, DevMem& d) {
+    const size_t bytes = std::max<size_t>(k, 1) * sizeof(T);
+    if (KEEP) {
+      if (cudaMalloc(&q, bytes) == cudaSuccess) return true;
+      cudaGetLastError();
+      if (pool_ctx()) pool_ctx()->mem_trim(0);
+      if (cudaMalloc(&q, bytes) == cudaSuccess) return true;
+    } else if (d.get(bytes)) {
+      q = (T*)d.p;
+      return true;
     }
-    n = m;
+    set_error("graph build: device allocation of %zu bytes failed", bytes);
+    return false;
+  }
+  void drop() {
+    if (KEEP) { if (p) cudaFree(p); }
+    else m.put();
+    p = nullptr;
+    n = 0;
+  }
+  int alloc(size_t k) {
+    if (k <= n && p) return ASR_OK;
+    drop();
+    if (!get(k, p, m)) return ASR_ENOMEM;
+    n = k;
     return ASR_OK;
   }
-  int grow_keep(size_t m, cudaStream_t s) {   // grow, keeping contents
-    if (m <= n && p) return ASR_OK;
-    size_t nm = std::max(m, 2 * n);
+  int grow_keep(size_t k, cudaStream_t s) {   // grow, keeping contents
+    if (k <= n && p) return ASR_OK;
+    const size_t nk = std::max(k, 2 * n), had = n;
     T* q = nullptr;
-    if (cudaMalloc(&q, nm * sizeof(T)) != cudaSuccess) {
-      set_error("graph build: device allocation of %zu bytes failed", nm * sizeof(T));
-      return ASR_ENOMEM;
-    }
-    if (p) { cudaMemcpyAsync(q, p, n * sizeof(T), cudaMemcpyDeviceToDevice, s); cudaStreamSynchronize(s); cudaFree(p); }
-    p = q; n = nm;
+    DevMem d;
+    if (!get(nk, q, d)) return ASR_ENOMEM;
+    if (p) { cudaMemcpyAsync(q, p, had * sizeof(T), cudaMemcpyDeviceToDevice, s); cudaStreamSynchronize(s); }
+    drop();
+    p = q; n = nk; m = d;
     return ASR_OK;
   }
-  T* release() { T* q = p; p = nullptr; n = 0; return q; }
+  T* release() { T* q = p; p = nullptr; n = 0; return q; }   // KEEP
 };
 
 int check_err(asr_ctx* ctx, const char* where) {
@@ -434,21 +451,14 @@ __global__ void k_perm_rows(int nn, int w, const int* old_of_new, const int* new
 }
 
 template <typename T>
-int permute_rows(cudaStream_t s, int nn, int w, const int* d_oon, const int* d_noo, T*& p, bool remap) {
+int permute_rows(cudaStream_t s, int nn, int w, const int* d_oon, const int* d_noo, T* p, DBuf<double>& tmp, bool remap) {
   if (!p || w == 0) return ASR_OK;
-  T* q = nullptr;
-  ASR_CUDA(cudaMalloc(&q, std::max<size_t>((size_t)nn * w, 1) * sizeof(T)));
+  const size_t bytes = (size_t)nn * w * sizeof(T);
+  ASR_TRY(tmp.alloc((bytes + 7) / 8));
   long n = (long)nn * w;
-  k_perm_rows<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(nn, w, d_oon, d_noo, p, q, remap);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) {
-    cudaFree(q);
-    set_error("permute_rows: %s", cudaGetErrorString(e));
-    return ASR_ECUDA;
-  }
-  cudaFree(p);
-  p = q;
+  k_perm_rows<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(nn, w, d_oon, d_noo, p, (T*)tmp.p, remap);
+  ASR_CUDA(cudaGetLastError());
+  ASR_CUDA(cudaMemcpyAsync(p, tmp.p, bytes, cudaMemcpyDeviceToDevice, s));
   return ASR_OK;
 }
 
@@ -518,33 +528,29 @@ int reorder_nodes(asr_ctx* ctx, asr_op* op) {
   ASR_CUDA(cudaStreamSynchronize(s));
   std::vector<int> oon = rcm_order(nn, ns, hr), noo(nn);
   for (int n = 0; n < nn; ++n) noo[oon[n]] = n;
-  int *d_oon = nullptr, *d_noo = nullptr;
-  if (cudaMalloc(&d_oon, nn * sizeof(int)) != cudaSuccess || cudaMalloc(&d_noo, nn * sizeof(int)) != cudaSuccess ||
-      cudaMemcpyAsync(d_oon, oon.data(), nn * sizeof(int), cudaMemcpyHostToDevice, s) != cudaSuccess ||
-      cudaMemcpyAsync(d_noo, noo.data(), nn * sizeof(int), cudaMemcpyHostToDevice, s) != cudaSuccess) {
-    cudaFree(d_oon);
-    cudaFree(d_noo);
-    set_error("reorder_nodes: device allocation or copy of the node order failed");
-    return ASR_ENOMEM;
-  }
+  DBuf<int> b_oon, b_noo;
+  DBuf<double> tmp;
+  ASR_TRY(b_oon.alloc(nn)); ASR_TRY(b_noo.alloc(nn));
+  ASR_TRY(tmp.alloc(((size_t)nn * std::max(std::max(ns, nsm), 2) * sizeof(int) + 7) / 8));   // the largest table
+  const int *d_oon = b_oon.p, *d_noo = b_noo.p;
+  ASR_CUDA(cudaMemcpyAsync(b_oon.p, oon.data(), nn * sizeof(int), cudaMemcpyHostToDevice, s));
+  ASR_CUDA(cudaMemcpyAsync(b_noo.p, noo.data(), nn * sizeof(int), cudaMemcpyHostToDevice, s));
   int rc = ASR_OK;
   auto run = [&](int r) { if (rc == ASR_OK) rc = r; };
-  run(permute_rows<int>(s, nn, 1, d_oon, d_noo, op->d_site, false));
-  run(permute_rows<int>(s, nn, 1, d_oon, d_noo, op->d_level, false));
-  run(permute_rows<int>(s, nn, 1, d_oon, d_noo, op->d_orb, false));
-  run(permute_rows<int8_t>(s, nn, 1, d_oon, d_noo, op->d_lst, false));
-  run(permute_rows<int8_t>(s, nn, 1, d_oon, d_noo, op->d_ncl, false));
-  run(permute_rows<int8_t>(s, nn, 1, d_oon, d_noo, op->d_typ, false));
-  run(permute_rows<int8_t>(s, nn, 1, d_oon, d_noo, op->d_start, false));
-  run(permute_rows<int8_t>(s, nn, 1, d_oon, d_noo, op->d_frozen, false));
-  run(permute_rows<double>(s, nn, 1, d_oon, d_noo, op->d_sq, false));
-  run(permute_rows<double>(s, nn, 1, d_oon, d_noo, op->d_isq, false));
-  run(permute_rows<int>(s, nn, nsm, d_oon, d_noo, op->d_flipr, true));
-  run(permute_rows<uint8_t>(s, nn, nsm, d_oon, d_noo, op->d_flipg, false));
-  run(permute_rows<int>(s, nn, ns, d_oon, d_noo, op->d_hopr, true));
-  run(permute_rows<uint8_t>(s, nn, ns, d_oon, d_noo, op->d_hopg, false));
-  cudaFree(d_oon);
-  cudaFree(d_noo);
+  run(permute_rows<int>(s, nn, 1, d_oon, d_noo, op->d_site, tmp, false));
+  run(permute_rows<int>(s, nn, 1, d_oon, d_noo, op->d_level, tmp, false));
+  run(permute_rows<int>(s, nn, 1, d_oon, d_noo, op->d_orb, tmp, false));
+  run(permute_rows<int8_t>(s, nn, 1, d_oon, d_noo, op->d_lst, tmp, false));
+  run(permute_rows<int8_t>(s, nn, 1, d_oon, d_noo, op->d_ncl, tmp, false));
+  run(permute_rows<int8_t>(s, nn, 1, d_oon, d_noo, op->d_typ, tmp, false));
+  run(permute_rows<int8_t>(s, nn, 1, d_oon, d_noo, op->d_start, tmp, false));
+  run(permute_rows<int8_t>(s, nn, 1, d_oon, d_noo, op->d_frozen, tmp, false));
+  run(permute_rows<double>(s, nn, 1, d_oon, d_noo, op->d_sq, tmp, false));
+  run(permute_rows<double>(s, nn, 1, d_oon, d_noo, op->d_isq, tmp, false));
+  run(permute_rows<int>(s, nn, nsm, d_oon, d_noo, op->d_flipr, tmp, true));
+  run(permute_rows<uint8_t>(s, nn, nsm, d_oon, d_noo, op->d_flipg, tmp, false));
+  run(permute_rows<int>(s, nn, ns, d_oon, d_noo, op->d_hopr, tmp, true));
+  run(permute_rows<uint8_t>(s, nn, ns, d_oon, d_noo, op->d_hopg, tmp, false));
   if (rc != ASR_OK) return rc;
   // stabiliser lists (ragged): rebuilt on the host in the new order
   std::vector<int> sp2(nn + 1, 0);
@@ -635,7 +641,8 @@ int build_operator(asr_ctx* ctx, int nsite, const int* nbr_ptr, const int* nbr, 
   // ---- start node: the start site with the reference configuration (its orbit must be 1)
   for (int g = 0; g < nop; ++g) if (perm[(size_t)g * nsite + start - 1] != start) { set_error("build_augcls_operator: start site is not invariant under the group"); return ASR_EINVAL; }
   size_t cap = 1 << 16;
-  DBuf<int> nkey, nlevel, norb;
+  DBuf<int> nkey;
+  DBuf<int, true> nlevel, norb;
   ASR_TRY(nkey.alloc(cap * W)); ASR_TRY(nlevel.alloc(cap)); ASR_TRY(norb.alloc(cap));
   {
     std::vector<int> k0(W, INT_MAX);
@@ -716,7 +723,8 @@ int build_operator(asr_ctx* ctx, int nsite, const int* nbr_ptr, const int* nbr, 
   ASR_TRY(check_err(ctx, "closure"));
   // ---- node tables
   int nslot = maxdeg;
-  DBuf<int> scnt, sptr;
+  DBuf<int> scnt;
+  DBuf<int, true> sptr;
   ASR_TRY(scnt.alloc(nn + 1)); ASR_TRY(sptr.alloc(nn + 1));
   k_stab_count<<<blocks(nn, 128), 128, 0, s>>>(B, nn, nkey.p, norb.p, scnt.p, ctx->d_err);
   ASR_CUDA(cudaMemsetAsync(scnt.p + nn, 0, sizeof(int), s));
@@ -724,10 +732,10 @@ int build_operator(asr_ctx* ctx, int nsite, const int* nbr_ptr, const int* nbr, 
   int nstab = 0;
   ASR_CUDA(cudaMemcpyAsync(&nstab, sptr.p + nn, sizeof(int), cudaMemcpyDeviceToHost, s));
   ASR_TRY(check_err(ctx, "stabilisers"));
-  DBuf<int> site, flipr, hopr;
-  DBuf<int8_t> lst, ncl, typ, stt, frz;
-  DBuf<double> sq, isq;
-  DBuf<uint8_t> flipg, hopg, stab;
+  DBuf<int, true> site, flipr, hopr;
+  DBuf<int8_t, true> lst, ncl, typ, stt, frz;
+  DBuf<double, true> sq, isq;
+  DBuf<uint8_t, true> flipg, hopg, stab;
   ASR_TRY(site.alloc(nn)); ASR_TRY(lst.alloc(nn)); ASR_TRY(ncl.alloc(nn)); ASR_TRY(typ.alloc(nn)); ASR_TRY(stt.alloc(nn));
   ASR_TRY(frz.alloc(nn)); ASR_TRY(sq.alloc(nn)); ASR_TRY(isq.alloc(nn));
   ASR_TRY(flipr.alloc((size_t)nsm * nn)); ASR_TRY(flipg.alloc((size_t)nsm * nn));
