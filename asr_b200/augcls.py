@@ -66,7 +66,7 @@ class Context:
 
     def hold_workspace(self, on: bool):
         """Keep the device vector memory of the chain runs and the adjoint in this context between calls (on) or free it
-        (off, the default)."""
+        and what the context keeps of its calls' temporaries (off, the default)."""
         check(lib().asr_ctx_hold_workspace(self.h, int(bool(on))))
 
     def profile(self, on: bool):

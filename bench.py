@@ -25,19 +25,14 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 NZ_SLICE = 192
-# DRAM bytes (read + write) per launch of the step kernel from one ncu capture (64-energy slice of this workload), the
-# algorithmic bytes of that launch and what was captured, per (precision, link-gather variant); traffic is scaled to the
-# bench's mean launch
+# DRAM bytes (read + write) per launch of the step kernel from one ncu capture (4 groups x 128 energies of this operator), the
+# algorithmic bytes of that launch and what was captured, per (precision, link-gather choice; one kernel for both); traffic is
+# scaled to the bench's mean launch
 _TAB = 18 * 5 + 3 * 5 + 20
-NCU_STEP_TRAFFIC = {
-    ("fp64", "fixed-offset"): (3.171e9, 16 * 20969 * (2 * 4608.0 + _TAB),
-                               "ncu capture of k_smul<double,1,1,1> (fixed-offset link gathers, a_k epilogue) at 16 tiles"),
-    ("fp32", "fixed-offset"): (0.762e9, 8 * 20969 * (2 * 2304.0 + _TAB),
-                               "ncu capture of k_smul<float,1,1,1> (fixed-offset link gathers, a_k epilogue, paired FMAs) at "
-                               "8 tiles"),
-    ("fp64", "general"): (3.30e9, 16 * 20969 * (2 * 4608.0 + _TAB),
-                          "ncu capture of the general-link k_smul<double,1,1,0> at 16 tiles (before the a_k epilogue)"),
-}
+_FP64 = (3.18e9, 16 * 20969 * (2 * 4608.0 + _TAB), "ncu capture of k_smul_mma<1,1,0> at 16 tiles")
+_FP32 = (0.771e9, 8 * 20969 * (2 * 2304.0 + _TAB), "ncu capture of k_smul<float,1,1,0> at 8 tiles")
+NCU_STEP_TRAFFIC = {("fp64", "fixed-offset"): _FP64, ("fp64", "general"): _FP64,
+                    ("fp32", "fixed-offset"): _FP32, ("fp32", "general"): _FP32}
 
 
 def roof(st, hbm_peak, pipe_peak=None):
@@ -934,7 +929,7 @@ def main():
             "e2e": {"value": e2e, "unit": "chain-steps/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
                          "traffic": traffic, "traffic_source": traffic_source,
-                         "kernel": "chain step operator (k_smul, fused S + diagonal + dot; %s link gathers)" % tune["link_gather"],
+                         "kernel": "chain step operator (%s, fused S + diagonal + dot)" % ("k_smul_mma" if args.precision == "fp64" else "k_smul"),
                          "per_launch_ms": per_launch_ms, "launches": ks["launches"], "fp64_tflops": tflops,
                          "share_of_step": ks["ms"] / ms, "peak_source": peak_source,
                          "fp64_frac": (tflops / legs["fp64_peak_tflops"]) if legs else None,

@@ -72,8 +72,9 @@ int asr_ctx_profile(asr_ctx* ctx, int on);
 /* on = 1: the batched chain runs (asr_chains_run and its lane and device forms) and the adjoint (asr_chains_adjoint,
  * asr_chains_adjoint_ext) keep their device vector memory (one slab, at most half of the device memory free when it is
  * first needed, grown when a later call needs more) in the context after they return and reuse it on the next call,
- * instead of allocating and freeing it per call; on = 0 (the default) frees it.  For loops that run many chain sets or
- * gradients on one operator.  No counterpart in the reference (whose arrays are allocated per call). */
+ * instead of allocating and freeing it per call; on = 0 (the default) frees it, and with it what the context keeps anyway:
+ * the temporaries of its calls, up to an eighth of the device's memory (nothing after a call that found less than a quarter
+ * of it free).  For loops whose batches are larger than that.  No counterpart in the reference (whose arrays are allocated per call). */
 int asr_ctx_hold_workspace(asr_ctx* ctx, int on);
 int asr_ctx_kernel_stats(asr_ctx* ctx, double* ms, int64_t* launches, double* bytes, double* flops);
 int asr_ctx_kernel_stats_kind(asr_ctx* ctx, int kind, double* ms, int64_t* launches, double* bytes, double* flops);
@@ -206,18 +207,17 @@ int asr_epi_blocks(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, cons
 /* Batch-shape autotuner (no counterpart in the reference, which has no device): times the chains of the given groups
  * (depth capped at `levels`, at most 64 of the energies) over tiles per batch {4, 8, 16, 32} and nodes per warp
  * {1, 2, 4, 8} and keeps the fastest shape (a candidate must beat the built-in default, 16 tiles in FP64 and 8 in FP32
- * at 4 nodes per warp, by 3 %) on the operator for this precision; later calls that leave the shape
+ * at 1, 2 or 4 nodes per warp by the operator's size, by 3 %) on the operator for this precision; later calls that leave the shape
  * automatic use it.  The shape does not change results beyond the order of the per-block partial sums (rounding).
  * Each candidate is timed on the device (CUDA events around its batches, allocations excluded, best of two runs).
- * At the chosen shape it then times the step kernel with fixed-offset link gathers (links whose orbital operation keeps
- * the orbital order read their nine rows without index decoding; the same bits) against the general one and keeps it
- * when it is 3 % faster.
+ * At the chosen shape it then times the run with the fixed-offset link choice against the general one and keeps it when it
+ * is 3 % faster; the step kernels of both precisions read such links at fixed offsets under either choice.
  * tpb, npw: the chosen shape; times(8) the device times in ms (-1: skipped) or NULL. */
 int asr_autotune(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, int ngroup, const double* z, int nz, int precision,
                  int levels, int* tpb, int* npw, double* times);
 
 /* The operator's tuned state for a precision: tpb, npw (0: never tuned, the built-in defaults apply), link = 1 when the
- * fixed-offset link gathers are in use, ms(2) the device times of the general and the fixed-offset step at the tuned shape
+ * fixed-offset link gathers are chosen, ms(2) the device times of the general and the fixed-offset step at the tuned shape
  * (-1: not timed).  Any pointer may be NULL.  No counterpart in the reference. */
 int asr_op_tuning(const asr_op* op, int precision, int* tpb, int* npw, int* link, double* ms);
 /* Set the tuned state for a precision (a shape saved from an earlier asr_autotune, or a pinned one): tpb in {4, 8, 16, 32}
