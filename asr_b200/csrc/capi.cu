@@ -124,7 +124,10 @@ int make_group_slots(const asr_op* op, const GroupLayout& GL, const double* cons
   if (all_zero(P[PO], np)) gi.flags |= GF_O_ZERO;
   if (all_zero(P[PE], np)) gi.flags |= GF_E_ZERO;
   if (all_zero(P[PA], np) && all_zero(P[PB], np)) gi.flags |= GF_X_ZERO;
-  for (int l = 0; l < 9; ++l) gi.dd[l] = P[PD][l];
+  for (int l = 0; l < 9; ++l) {
+    gi.dd[l] = P[PD][l];
+    if (!(std::fabs(gi.dd[l]) >= D_ROW)) gi.flags |= GF_D_SMALL;
+  }
   if (frozen_sp < 0 || frozen_sp > op->nsp) { set_error("chain group: frozen species out of range"); return ASR_EINVAL; }
   gi.frozen_sp = frozen_sp;
   if (l0 < 1 || l0 > 9) { set_error("chain group: start orbital out of range"); return ASR_EINVAL; }

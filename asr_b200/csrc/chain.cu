@@ -335,7 +335,7 @@ __device__ __forceinline__ float2 flip_by(float2 x, uint32_t word) {
 // node's share of the dot sum norb (s U) . y.  EPI 1: also t2 = S (d o U) into bv.t2out.  EPI 2 (the adjoint, U = wbar_k,
 // unit scales): t2 into bv.t2out and, in place of y, ubar_k = y + ca Y_k - cb U - cc wbar_{k+1} into bv.adj.ubk, the dot
 // being sum norb ubar_k . X_k (raw)
-template <typename ST, bool FINAL, int EPI = 0, typename T2, typename A2>
+template <typename ST, bool FINAL, int EPI = 0, bool SMALL = false, typename T2, typename A2>
 __device__ __forceinline__ void smul_node_out(const OpView& op, const BatchView& bv, int tile, int i, int lane, int L, int grp,
                                               int gflags, int gfrozen, const uint32_t* opw, const T2* __restrict__ in,
                                               T2* __restrict__ out, const A2* acc, double2& dot) {
@@ -389,11 +389,14 @@ __device__ __forceinline__ void smul_node_out(const OpView& op, const BatchView&
           if (r >= 0) flip_link(r, k, opw[OPW * op.flipg[k + nsm * i] + l]);
         }
       }
-      double2 y = cmul(s, cadd(make_double2(acc[l].x, acc[l].y), pt));
+      const double d = EPI >= 1 ? bv.ginfo[grp >= 0 ? grp : 0].dd[l] : 1.0;
+      double2 sd = make_double2(acc[l].x, acc[l].y);
+      if (SMALL && row_d(d) != d) sd = cscale(sd, d);
+      double2 y = cmul(s, cadd(sd, pt));
       const size_t q = vx<ST>(tile, bv.nn, i, l, lane);
       if (EPI != 2) stv_cs(out + q, y);
       if (EPI >= 1) {   // the blocks carry d on both sides: t2 = S (d o U) = acc / d_l
-        const double il = 1.0 / bv.ginfo[grp >= 0 ? grp : 0].dd[l];
+        const double il = 1.0 / (SMALL ? row_d(d) : d);
         stv((T2*)bv.t2out + q, make_double2(acc[l].x * il, acc[l].y * il));
       }
       if (EPI == 2) {
@@ -419,7 +422,7 @@ __device__ __forceinline__ void smul_node_out(const OpView& op, const BatchView&
 // Bound by the instructions issued: a link is 90 paired or single FMAs, 25 shared-memory reads of the block, nine row reads and
 // the signs.  With the operation as a packed 64-bit word, decoded orbital by orbital, it was some 315 instructions in all and
 // 1.19 ms at 8 tiles of 20,969 nodes; with the words 1.01 ms (three blocks per SM; two 1.12, four, with spills, 1.06).
-template <typename ST, bool FUSE_D, bool FINAL, int EPI = 0>
+template <typename ST, bool FUSE_D, bool FINAL, int EPI = 0, bool SMALL = false>
 __global__ void __launch_bounds__(WPB * TL, 3) k_smul(OpView op, BatchView bv, const ST* __restrict__ blocks,
                                                    const typename St2<ST>::T* __restrict__ in,
                                                    typename St2<ST>::T* __restrict__ out, double2* part, int npw) {
@@ -446,7 +449,7 @@ __global__ void __launch_bounds__(WPB * TL, 3) k_smul(OpView op, BatchView bv, c
       int lp = q % 9, l = (q / 9) % 9, tk = q / 81;
       double v = (double)blocks[q];
       if (FUSE_D && dd) v *= dd[lp];
-      if (FINAL && dd) v *= dd[l];
+      if (FINAL && dd) v *= SMALL ? row_d(dd[l]) : dd[l];
       BlockAcc<ST>::put(Bs + (size_t)tk * BlockAcc<ST>::BLK, l, lp, v);
     }
     for (int g = threadIdx.x; g < op.nop; g += blockDim.x) {
@@ -507,7 +510,7 @@ __global__ void __launch_bounds__(WPB * TL, 3) k_smul(OpView op, BatchView bv, c
     }
     T2 acc[9];
     A.out(acc);
-    smul_node_out<ST, FINAL, EPI>(op, bv, it.tile, i, lane, L, grp, gflags, gfrozen, opw, in, out, acc, dot);
+    smul_node_out<ST, FINAL, EPI, SMALL>(op, bv, it.tile, i, lane, L, grp, gflags, gfrozen, opw, in, out, acc, dot);
   }
   if (FINAL) {
     block_reduce_store(dot, part, it.tile, bpt);
@@ -547,12 +550,12 @@ struct MmaSm {   // shared memory of k_smul_mma: byte offsets
 };
 
 // two adjacent outputs (l0, l0 + 1; NL = 2) or one (NL = 1) of a lane of a node: acc the S application's values, wt the
-// diagonal weights {W, W_pa}, wc those of c (EPI 4)
-template <bool FINAL, int EPI, int NL>
+// diagonal weights {W, W_pa}, wc those of c (EPI 4), dd (SMALL) the group's d at l0
+template <bool FINAL, int EPI, bool SMALL, int NL>
 __device__ __forceinline__ void mma_out(const OpView& op, const BatchView& bv, size_t q, int tile, int i, int l0, int lane,
                                         const double2* acc, const double* gb, const double2* wt, const double* wc, bool withx,
-                                        bool flips, const uint32_t* opw, const double* il, const double2* __restrict__ in,
-                                        double2* __restrict__ out, double2& dot) {
+                                        bool flips, const uint32_t* opw, const double* il, const double* dd,
+                                        const double2* __restrict__ in, double2* __restrict__ out, double2& dot) {
   auto get = [&](const double2* p, double2 (&v)[NL]) {
     if constexpr (NL == 2) ldg2(p + q, v[0], v[1]);
     else v[0] = p[q];
@@ -589,11 +592,16 @@ __device__ __forceinline__ void mma_out(const OpView& op, const BatchView& bv, s
       }
     }
   };
+  auto sds = [&](int e) {   // d S (d o U)
+    if constexpr (SMALL)
+      if (row_d(dd[e]) != dd[e]) return zscale(acc[e], dd[e]);
+    return acc[e];
+  };
   get(in, ui);
   if constexpr (EPI == 4) {   // t = h1 - (d S d r1 + C r1) + (E + X(z)) u, r1 the source
     get((const double2*)bv.gen_h1, t);
 #pragma unroll
-    for (int e = 0; e < NL; ++e) t[e] = zadd(t[e], zneg(make_double2(fma(wc[e], ui[e].x, acc[e].x), fma(wc[e], ui[e].y, acc[e].y))));
+    for (int e = 0; e < NL; ++e) t[e] = zadd(t[e], zneg(make_double2(fma(wc[e], ui[e].x, sds(e).x), fma(wc[e], ui[e].y, sds(e).y))));
     if (flips) add_flips(in, PC, false, -1.0);
     get((const double2*)bv.gen_u, ui);
 #pragma unroll
@@ -601,7 +609,7 @@ __device__ __forceinline__ void mma_out(const OpView& op, const BatchView& bv, s
     if (flips) add_flips((const double2*)bv.gen_u, PEB, withx, 1.0);
   } else {
 #pragma unroll
-    for (int e = 0; e < NL; ++e) t[e] = zfma(make_double2(fma(z.x, wt[e].y, wt[e].x), __dmul_rn(z.y, wt[e].y)), ui[e], acc[e]);
+    for (int e = 0; e < NL; ++e) t[e] = zfma(make_double2(fma(z.x, wt[e].y, wt[e].x), __dmul_rn(z.y, wt[e].y)), ui[e], sds(e));
     if (flips) add_flips(in, EPI == 3 ? PC : PCEB, EPI != 3 && withx, 1.0);
   }
   if (EPI == 1 || EPI == 2 || (EPI >= 3 && bv.t2out)) {   // the blocks carry d on both sides: t2 = S (d o U) = acc / d_l
@@ -639,7 +647,7 @@ __device__ __forceinline__ void mma_out(const OpView& op, const BatchView& bv, s
 
 // the nodes of one warp for a tile with NJ octets; oct: octet j in bits 2j, 2j + 1 (NJ = 4: j itself).  Returns the dot of
 // the lane this thread owns (row t / 4 of octet c; NJ < 4: where c < NJ).
-template <bool FINAL, int EPI, int NJ>
+template <bool FINAL, int EPI, bool SMALL, int NJ>
 __device__ __forceinline__ double2 mma_nodes(const OpView& op, const BatchView& bv, const NodeIter& it, const unsigned char* smem,
                                              const MmaSm& sm, unsigned oct, int grp, const double2* __restrict__ in,
                                              double2* __restrict__ out) {
@@ -715,15 +723,15 @@ __device__ __forceinline__ double2 mma_nodes(const OpView& op, const BatchView& 
       d[j] = make_double2(0.0, 0.0);
       const int lane = row + 8 * off(j);
       const double2 a[2] = {A.out(j, 0), A.out(j, 1)};
-      mma_out<FINAL, EPI, 2>(op, bv, q + mnode_at(2 * c, lane), it.tile, i, 2 * c, lane, a, gb, wt, wc, withx, flips, opw, il, in,
-                             out, d[j]);
+      mma_out<FINAL, EPI, SMALL, 2>(op, bv, q + mnode_at(2 * c, lane), it.tile, i, 2 * c, lane, a, gb, wt, wc, withx, flips, opw, il,
+                                    gi->dd + 2 * c, in, out, d[j]);
     }
     double2 dn = make_double2(0.0, 0.0);
     if (FINAL && EPI != 3) dn = quad_own<NJ>(d, c);
     if (c < NJ) {
       const int lane = row + 8 * off(c);
-      mma_out<FINAL, EPI, 1>(op, bv, q + 256 + lane, it.tile, i, 8, lane, &a8, gb, wt + 2, wc + 2, withx, flips, opw, il + 2, in, out,
-                             dn);
+      mma_out<FINAL, EPI, SMALL, 1>(op, bv, q + 256 + lane, it.tile, i, 8, lane, &a8, gb, wt + 2, wc + 2, withx, flips, opw, il + 2,
+                                    gi->dd + 8, in, out, dn);
     }
     if (FINAL && EPI != 3) {
       const double norb = __dmul_rn(sq, sq);
@@ -738,7 +746,7 @@ __device__ __forceinline__ double2 mma_nodes(const OpView& op, const BatchView& 
 // r1 = O h U, y = s (h U - h r1 + (E + X(z)) U) with h U in bv.gen_h1 and U in bv.gen_u.  Both store t2 where bv.t2out is set.
 // As separate passes (the S application, then k_combine over its result) the two took 16 vector streams per level with the
 // random operators between them, 8 this way.
-template <bool FUSE_D, bool FINAL, int EPI = 0>
+template <bool FUSE_D, bool FINAL, int EPI = 0, bool SMALL = false>
 __global__ void __launch_bounds__(WPB * TL, 2) k_smul_mma(OpView op, BatchView bv, const double* __restrict__ blocks,
                                                           const double2* __restrict__ in, double2* __restrict__ out,
                                                           double2* part, int npw) {
@@ -759,11 +767,11 @@ __global__ void __launch_bounds__(WPB * TL, 2) k_smul_mma(OpView op, BatchView b
       const int lp = q % 9, l = (q / 9) % 9, tk = q / 81;
       double v = blocks[q];
       if (FUSE_D && gi) v *= gi->dd[lp];
-      if (FINAL && gi) v *= gi->dd[l];
+      if (FINAL && gi) v *= SMALL ? row_d(gi->dd[l]) : gi->dd[l];
       Bs[tk * MB + lp * MB_ROW + l] = v;
     }
     for (int q = threadIdx.x; q < MB; q += blockDim.x) Bs[zero_blk * MB + q] = 0.0;
-    if (EPI >= 1 && gi && threadIdx.x < 9) ((double*)(smem_raw + sm.ild))[threadIdx.x] = 1.0 / gi->dd[threadIdx.x];
+    if (EPI >= 1 && gi && threadIdx.x < 9) ((double*)(smem_raw + sm.ild))[threadIdx.x] = 1.0 / (SMALL ? row_d(gi->dd[threadIdx.x]) : gi->dd[threadIdx.x]);
     for (int q = threadIdx.x; q < (op.nop + 1) * 9; q += blockDim.x) {
       const int g = q / 9, l = q % 9;
       if (g < op.nop) opw[g * 9 + op.pi[q]] = op_word(l, ((op.sgm[g] >> l) & 1u) ^ (uint32_t)((chimask >> g) & 1ull));
@@ -795,13 +803,13 @@ __global__ void __launch_bounds__(WPB * TL, 2) k_smul_mma(OpView op, BatchView b
   double2 own = make_double2(0.0, 0.0);
   int owner = -1;
   if (nj > 2) {
-    own = mma_nodes<FINAL, EPI, 4>(op, bv, it, smem_raw, sm, oct, grp, in, out);
+    own = mma_nodes<FINAL, EPI, SMALL, 4>(op, bv, it, smem_raw, sm, oct, grp, in, out);
     owner = row + 8 * c;
   } else if (nj == 2) {
-    own = mma_nodes<FINAL, EPI, 2>(op, bv, it, smem_raw, sm, oct, grp, in, out);
+    own = mma_nodes<FINAL, EPI, SMALL, 2>(op, bv, it, smem_raw, sm, oct, grp, in, out);
     if (c < 2) owner = row + 8 * (int)((oct >> (2 * c)) & 3u);
   } else if (nj == 1) {
-    own = mma_nodes<FINAL, EPI, 1>(op, bv, it, smem_raw, sm, oct, grp, in, out);
+    own = mma_nodes<FINAL, EPI, SMALL, 1>(op, bv, it, smem_raw, sm, oct, grp, in, out);
     if (c == 0) owner = row + 8 * (int)(oct & 3u);
   }
   if (FINAL && EPI != 3) {
@@ -1197,10 +1205,23 @@ template <typename ST, bool FUSE_D, bool FINAL, int EPI = 0>
 void launch_smul(asr_op* op, const BatchView& bv, const ST* blk, const typename St2<ST>::T* in, typename St2<ST>::T* out,
                  double2* part, int npw, int grid, cudaStream_t s) {
   OpView ov = op->view();   // EPI: the adjoint's fused steps, also t2 (bv.t2out); EPI 2, the reverse epilogue (bv.adj)
-  if constexpr (std::is_same<ST, double>::value)
-    k_smul_mma<FUSE_D, FINAL, EPI><<<grid, WPB * TL, MmaSm(ov).bytes, s>>>(ov, bv, blk, in, out, part, npw);
-  else
-    k_smul<ST, FUSE_D, FINAL, EPI><<<grid, WPB * TL, smul_smem(op, sizeof(ST)), s>>>(ov, bv, blk, in, out, part, npw);
+  if constexpr (std::is_same<ST, double>::value) {
+    const int sm = MmaSm(ov).bytes;
+    if constexpr (EPI >= 1)
+      if (bv.small_d && bv.t2out) {
+        k_smul_mma<FUSE_D, FINAL, EPI, true><<<grid, WPB * TL, sm, s>>>(ov, bv, blk, in, out, part, npw);
+        return;
+      }
+    k_smul_mma<FUSE_D, FINAL, EPI><<<grid, WPB * TL, sm, s>>>(ov, bv, blk, in, out, part, npw);
+  } else {
+    const size_t sm = smul_smem(op, sizeof(ST));
+    if constexpr (EPI >= 1)
+      if (bv.small_d && bv.t2out) {
+        k_smul<ST, FUSE_D, FINAL, EPI, true><<<grid, WPB * TL, sm, s>>>(ov, bv, blk, in, out, part, npw);
+        return;
+      }
+    k_smul<ST, FUSE_D, FINAL, EPI><<<grid, WPB * TL, sm, s>>>(ov, bv, blk, in, out, part, npw);
+  }
 }
 
 // y = s (h U - h O h U + (E + X) U) in FP64 at uniform d: H1 = h U, R1 = O h U, Y and the dots; TA, TB (or null): S d U, S d R1
@@ -2044,9 +2065,10 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
   cudaStream_t s = ctx->stream;
   const int nn = op->nn, nsp = op->nsp, nlane = (int)lane_group.size();
   if (nsp > MAXSP) { set_error("adjoint: at most %d species", MAXSP); return ASR_EINVAL; }
-  bool dunif = true, gen = false;
+  bool dunif = true, gen = false, small_d = false;
   int mmax = 0;
   for (auto& g : ginfo) {
+    if (g.flags & GF_D_SMALL) small_d = true;
     if (!(g.flags & GF_O_ZERO)) gen = true;   // H = E_nu + h - h o h: the general operator and its intermediates
     if (!(g.flags & GF_D_UNIFORM)) dunif = false;
     mmax = std::max(mmax, g.nlev);
@@ -2207,6 +2229,7 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
     BatchView bv{nt, nn, op->nsmax, 0, ASR_MODE_EDC, project, tail, NLMAX, depth_tol, d_gblob.p, GL, d_ginfo.p, d_lgroup.p,
                  d_tgroup.p, d_z.p, d_act.p, d_wact.p, d_m.p, d_a.p, d_b.p, d_gprev.p, d_acur.p, d_bprev.p, d_su.p, d_sup.p,
                  d_tact.p, d_nfall.p};
+    bv.small_d = small_d;
     const int grid = nt * bpt;
     int kmax = 0;
     for (int q = 0; q < nlp; ++q) if (hgroup[q] >= 0) kmax = std::max(kmax, ginfo[hgroup[q]].nlev);
@@ -3053,14 +3076,20 @@ static void smem_attrs() {
   cudaFuncSetAttribute(k_smul_mma<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul_mma<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul_mma<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
+  cudaFuncSetAttribute(k_smul_mma<true, true, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul_mma<true, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
+  cudaFuncSetAttribute(k_smul_mma<true, true, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul_mma<true, true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
+  cudaFuncSetAttribute(k_smul_mma<true, true, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul_mma<true, true, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
+  cudaFuncSetAttribute(k_smul_mma<true, true, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul_mma<true, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul<float, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   cudaFuncSetAttribute(k_smul<float, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   cudaFuncSetAttribute(k_smul<float, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+  cudaFuncSetAttribute(k_smul<float, true, true, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   cudaFuncSetAttribute(k_smul<float, true, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+  cudaFuncSetAttribute(k_smul<float, true, true, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   cudaFuncSetAttribute(k_smul<float, true, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   done[dev] = true;
 }
