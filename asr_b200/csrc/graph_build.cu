@@ -580,6 +580,7 @@ int count_flips(asr_ctx* ctx, asr_op* op) {
   ASR_CUDA(cudaMalloc(&op->d_nflip, op->nn));
   k_count_flips<<<(op->nn + 255) / 256, 256, 0, ctx->stream>>>(op->view(), op->d_nflip);
   ASR_CUDA(cudaGetLastError());
+  ASR_CUDA(cudaStreamSynchronize(ctx->stream));   // the operator may be used next on another stream or context
   return ASR_OK;
 }
 
