@@ -335,7 +335,7 @@ __device__ __forceinline__ float2 flip_by(float2 x, uint32_t word) {
 // node's share of the dot sum norb (s U) . y.  EPI 1: also t2 = S (d o U) into bv.t2out.  EPI 2 (the adjoint, U = wbar_k,
 // unit scales): t2 into bv.t2out and, in place of y, ubar_k = y + ca Y_k - cb U - cc wbar_{k+1} into bv.adj.ubk, the dot
 // being sum norb ubar_k . X_k (raw)
-template <typename ST, bool FINAL, int EPI = 0, bool SMALL = false, typename T2, typename A2>
+template <typename ST, bool FINAL, int EPI = 0, bool RARE = false, typename T2, typename A2>
 __device__ __forceinline__ void smul_node_out(const OpView& op, const BatchView& bv, int tile, int i, int lane, int L, int grp,
                                               int gflags, int gfrozen, const uint32_t* opw, const T2* __restrict__ in,
                                               T2* __restrict__ out, const A2* acc, double2& dot) {
@@ -391,12 +391,12 @@ __device__ __forceinline__ void smul_node_out(const OpView& op, const BatchView&
       }
       const double d = EPI >= 1 ? bv.ginfo[grp >= 0 ? grp : 0].dd[l] : 1.0;
       double2 sd = make_double2(acc[l].x, acc[l].y);
-      if (SMALL && row_d(d) != d) sd = cscale(sd, d);
+      if (RARE && row_d(d) != d) sd = cscale(sd, d);
       double2 y = cmul(s, cadd(sd, pt));
       const size_t q = vx<ST>(tile, bv.nn, i, l, lane);
       if (EPI != 2) stv_cs(out + q, y);
       if (EPI >= 1) {   // the blocks carry d on both sides: t2 = S (d o U) = acc / d_l
-        const double il = 1.0 / (SMALL ? row_d(d) : d);
+        const double il = 1.0 / (RARE ? row_d(d) : d);
         stv((T2*)bv.t2out + q, make_double2(acc[l].x * il, acc[l].y * il));
       }
       if (EPI == 2) {
@@ -422,7 +422,7 @@ __device__ __forceinline__ void smul_node_out(const OpView& op, const BatchView&
 // Bound by the instructions issued: a link is 90 paired or single FMAs, 25 shared-memory reads of the block, nine row reads and
 // the signs.  With the operation as a packed 64-bit word, decoded orbital by orbital, it was some 315 instructions in all and
 // 1.19 ms at 8 tiles of 20,969 nodes; with the words 1.01 ms (three blocks per SM; two 1.12, four, with spills, 1.06).
-template <typename ST, bool FUSE_D, bool FINAL, int EPI = 0, bool SMALL = false>
+template <typename ST, bool FUSE_D, bool FINAL, int EPI = 0, bool RARE = false>
 __global__ void __launch_bounds__(WPB * TL, 3) k_smul(OpView op, BatchView bv, const ST* __restrict__ blocks,
                                                    const typename St2<ST>::T* __restrict__ in,
                                                    typename St2<ST>::T* __restrict__ out, double2* part, int npw) {
@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(WPB * TL, 3) k_smul(OpView op, BatchView bv, c
       int lp = q % 9, l = (q / 9) % 9, tk = q / 81;
       double v = (double)blocks[q];
       if (FUSE_D && dd) v *= dd[lp];
-      if (FINAL && dd) v *= SMALL ? row_d(dd[l]) : dd[l];
+      if (FINAL && dd) v *= RARE ? row_d(dd[l]) : dd[l];
       BlockAcc<ST>::put(Bs + (size_t)tk * BlockAcc<ST>::BLK, l, lp, v);
     }
     for (int g = threadIdx.x; g < op.nop; g += blockDim.x) {
@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(WPB * TL, 3) k_smul(OpView op, BatchView bv, c
     }
     T2 acc[9];
     A.out(acc);
-    smul_node_out<ST, FINAL, EPI, SMALL>(op, bv, it.tile, i, lane, L, grp, gflags, gfrozen, opw, in, out, acc, dot);
+    smul_node_out<ST, FINAL, EPI, RARE>(op, bv, it.tile, i, lane, L, grp, gflags, gfrozen, opw, in, out, acc, dot);
   }
   if (FINAL) {
     block_reduce_store(dot, part, it.tile, bpt);
@@ -535,23 +535,31 @@ __global__ void __launch_bounds__(WPB * TL, 3) k_smul(OpView op, BatchView bv, c
 // 16 warps per SM at 128 registers).  fcc ternary, 20,969 nodes, 18 slots, 16 tiles: 2.44 ms per launch (27 TFLOP/s by
 // 6,156 flops per node and lane) with the loads one product step ahead, 2.60 ms without; plain FP64 FMAs (one lane per
 // thread, broadcast block reads) 4.06 ms, with fixed-offset link gathers 3.4 ms.
-struct MmaSm {   // shared memory of k_smul_mma: byte offsets
+// The diagonal weights of an operator with many classes do not fit beside the bond blocks: the RARE instantiations read them
+// from global memory.
+struct MmaSm {   // shared memory of k_smul_mma: byte offsets; tables: with the diagonal weights
   int opw, links, ldl, wtab, wtab2, ild, bytes;
-  __host__ __device__ MmaSm(const OpView& op) {
-    const int ns1 = op.nslot + 1;
+  __host__ __device__ MmaSm(const OpView& op, bool tables) {
+    const int ns1 = op.nslot + 1, nrow = tables ? (op.ncls * op.nsmax + op.nsp) * 9 : 0;
     ldl = (ns1 + 3) & ~3;                                                // links per warp
     opw = (op.ntype * ns1 + 1) * MB * (int)sizeof(double);               // after the blocks and one of zeros
     links = (opw + (op.nop + 1) * 9 * (int)sizeof(uint32_t) + 15) & ~15;
     wtab = links + WPB * ldl * (int)sizeof(int2);
-    wtab2 = wtab + (op.ncls * op.nsmax + op.nsp) * 9 * (int)sizeof(double2);
-    ild = wtab2 + (op.ncls * op.nsmax + op.nsp) * 9 * (int)sizeof(double);
+    wtab2 = wtab + nrow * (int)sizeof(double2);
+    ild = wtab2 + nrow * (int)sizeof(double);
     bytes = ild + 9 * (int)sizeof(double);
   }
 };
 
+// where weight l of row r lies in slot p of a group's blob: a (class, own state), then the frozen species
+__device__ __forceinline__ int diag_at(const OpView& op, const GroupLayout& GL, int p, int r, int l) {
+  const int nsm = op.nsmax, nw = op.ncls * nsm;
+  return r < nw ? GL.w(p) + (r * nsm + r % nsm) * 9 + l : GL.raw(p) + (r - nw) * 9 + l;
+}
+
 // two adjacent outputs (l0, l0 + 1; NL = 2) or one (NL = 1) of a lane of a node: acc the S application's values, wt the
-// diagonal weights {W, W_pa}, wc those of c (EPI 4), dd (SMALL) the group's d at l0
-template <bool FINAL, int EPI, bool SMALL, int NL>
+// diagonal weights {W, W_pa}, wc those of c (EPI 4), dd (RARE) the group's d at l0
+template <bool FINAL, int EPI, bool RARE, int NL>
 __device__ __forceinline__ void mma_out(const OpView& op, const BatchView& bv, size_t q, int tile, int i, int l0, int lane,
                                         const double2* acc, const double* gb, const double2* wt, const double* wc, bool withx,
                                         bool flips, const uint32_t* opw, const double* il, const double* dd,
@@ -593,7 +601,7 @@ __device__ __forceinline__ void mma_out(const OpView& op, const BatchView& bv, s
     }
   };
   auto sds = [&](int e) {   // d S (d o U)
-    if constexpr (SMALL)
+    if constexpr (RARE)
       if (row_d(dd[e]) != dd[e]) return zscale(acc[e], dd[e]);
     return acc[e];
   };
@@ -647,7 +655,7 @@ __device__ __forceinline__ void mma_out(const OpView& op, const BatchView& bv, s
 
 // the nodes of one warp for a tile with NJ octets; oct: octet j in bits 2j, 2j + 1 (NJ = 4: j itself).  Returns the dot of
 // the lane this thread owns (row t / 4 of octet c; NJ < 4: where c < NJ).
-template <bool FINAL, int EPI, bool SMALL, int NJ>
+template <bool FINAL, int EPI, bool RARE, int NJ>
 __device__ __forceinline__ double2 mma_nodes(const OpView& op, const BatchView& bv, const NodeIter& it, const unsigned char* smem,
                                              const MmaSm& sm, unsigned oct, int grp, const double2* __restrict__ in,
                                              double2* __restrict__ out) {
@@ -704,11 +712,21 @@ __device__ __forceinline__ double2 mma_nodes(const OpView& op, const BatchView& 
     bool flips = false;
     if (FINAL) {
       const int fs = (st && gfrozen > 0) ? gfrozen : fr;
-      const double2* wr = wtab + (fs > 0 ? op.ncls * op.nsmax + fs - 1 : wrow0) * 9;
-      wt[0] = wr[2 * c]; wt[1] = wr[2 * c + 1]; wt[2] = wr[8];
-      if (EPI == 4) {
-        const double* cr = (const double*)(smem + sm.wtab2) + (wr - wtab);
-        wc[0] = cr[2 * c]; wc[1] = cr[2 * c + 1]; wc[2] = cr[8];
+      if constexpr (RARE) {
+        constexpr int P = EPI == 3 ? PC : EPI == 4 ? PEB : PCEB;
+        const int wrow = fs > 0 ? op.ncls * op.nsmax + fs - 1 : wrow0;
+        for (int e = 0; e < 3; ++e) {
+          const int l = e < 2 ? 2 * c + e : 8;
+          wt[e] = make_double2(gb[diag_at(op, bv.GL, P, wrow, l)], withx && EPI != 3 ? gb[diag_at(op, bv.GL, PA, wrow, l)] : 0.0);
+          if (EPI == 4) wc[e] = gb[diag_at(op, bv.GL, PC, wrow, l)];
+        }
+      } else {
+        const double2* wr = wtab + (fs > 0 ? op.ncls * op.nsmax + fs - 1 : wrow0) * 9;
+        wt[0] = wr[2 * c]; wt[1] = wr[2 * c + 1]; wt[2] = wr[8];
+        if (EPI == 4) {
+          const double* cr = (const double*)(smem + sm.wtab2) + (wr - wtab);
+          wc[0] = cr[2 * c]; wc[1] = cr[2 * c + 1]; wc[2] = cr[8];
+        }
       }
       flips = fs == 0 && nfl > 0;
       if (EPI >= 1) {
@@ -723,14 +741,14 @@ __device__ __forceinline__ double2 mma_nodes(const OpView& op, const BatchView& 
       d[j] = make_double2(0.0, 0.0);
       const int lane = row + 8 * off(j);
       const double2 a[2] = {A.out(j, 0), A.out(j, 1)};
-      mma_out<FINAL, EPI, SMALL, 2>(op, bv, q + mnode_at(2 * c, lane), it.tile, i, 2 * c, lane, a, gb, wt, wc, withx, flips, opw, il,
+      mma_out<FINAL, EPI, RARE, 2>(op, bv, q + mnode_at(2 * c, lane), it.tile, i, 2 * c, lane, a, gb, wt, wc, withx, flips, opw, il,
                                     gi->dd + 2 * c, in, out, d[j]);
     }
     double2 dn = make_double2(0.0, 0.0);
     if (FINAL && EPI != 3) dn = quad_own<NJ>(d, c);
     if (c < NJ) {
       const int lane = row + 8 * off(c);
-      mma_out<FINAL, EPI, SMALL, 1>(op, bv, q + 256 + lane, it.tile, i, 8, lane, &a8, gb, wt + 2, wc + 2, withx, flips, opw, il + 2,
+      mma_out<FINAL, EPI, RARE, 1>(op, bv, q + 256 + lane, it.tile, i, 8, lane, &a8, gb, wt + 2, wc + 2, withx, flips, opw, il + 2,
                                     gi->dd + 8, in, out, dn);
     }
     if (FINAL && EPI != 3) {
@@ -746,13 +764,13 @@ __device__ __forceinline__ double2 mma_nodes(const OpView& op, const BatchView& 
 // r1 = O h U, y = s (h U - h r1 + (E + X(z)) U) with h U in bv.gen_h1 and U in bv.gen_u.  Both store t2 where bv.t2out is set.
 // As separate passes (the S application, then k_combine over its result) the two took 16 vector streams per level with the
 // random operators between them, 8 this way.
-template <bool FUSE_D, bool FINAL, int EPI = 0, bool SMALL = false>
+template <bool FUSE_D, bool FINAL, int EPI = 0, bool RARE = false>
 __global__ void __launch_bounds__(WPB * TL, 2) k_smul_mma(OpView op, BatchView bv, const double* __restrict__ blocks,
                                                           const double2* __restrict__ in, double2* __restrict__ out,
                                                           double2* part, int npw) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int zero_blk = op.ntype * (op.nslot + 1);
-  const MmaSm sm(op);
+  const MmaSm sm(op, FINAL && !RARE);
   NodeIter it;
   int bpt;
   if (!node_iter(bv, npw, it, bpt)) return;
@@ -767,17 +785,17 @@ __global__ void __launch_bounds__(WPB * TL, 2) k_smul_mma(OpView op, BatchView b
       const int lp = q % 9, l = (q / 9) % 9, tk = q / 81;
       double v = blocks[q];
       if (FUSE_D && gi) v *= gi->dd[lp];
-      if (FINAL && gi) v *= SMALL ? row_d(gi->dd[l]) : gi->dd[l];
+      if (FINAL && gi) v *= RARE ? row_d(gi->dd[l]) : gi->dd[l];
       Bs[tk * MB + lp * MB_ROW + l] = v;
     }
     for (int q = threadIdx.x; q < MB; q += blockDim.x) Bs[zero_blk * MB + q] = 0.0;
-    if (EPI >= 1 && gi && threadIdx.x < 9) ((double*)(smem_raw + sm.ild))[threadIdx.x] = 1.0 / (SMALL ? row_d(gi->dd[threadIdx.x]) : gi->dd[threadIdx.x]);
+    if (EPI >= 1 && gi && threadIdx.x < 9) ((double*)(smem_raw + sm.ild))[threadIdx.x] = 1.0 / (RARE ? row_d(gi->dd[threadIdx.x]) : gi->dd[threadIdx.x]);
     for (int q = threadIdx.x; q < (op.nop + 1) * 9; q += blockDim.x) {
       const int g = q / 9, l = q % 9;
       if (g < op.nop) opw[g * 9 + op.pi[q]] = op_word(l, ((op.sgm[g] >> l) & 1u) ^ (uint32_t)((chimask >> g) & 1ull));
       else opw[q] = op_word(l, 0u);
     }
-    if (FINAL) {
+    if (FINAL && !RARE) {
       const double* gb = bv.gblob + (size_t)(grp >= 0 ? grp : 0) * bv.GL.stride;
       const bool withx = gi && !(gi->flags & GF_X_ZERO);
       const int nsm = op.nsmax, nw = op.ncls * nsm;
@@ -803,13 +821,13 @@ __global__ void __launch_bounds__(WPB * TL, 2) k_smul_mma(OpView op, BatchView b
   double2 own = make_double2(0.0, 0.0);
   int owner = -1;
   if (nj > 2) {
-    own = mma_nodes<FINAL, EPI, SMALL, 4>(op, bv, it, smem_raw, sm, oct, grp, in, out);
+    own = mma_nodes<FINAL, EPI, RARE, 4>(op, bv, it, smem_raw, sm, oct, grp, in, out);
     owner = row + 8 * c;
   } else if (nj == 2) {
-    own = mma_nodes<FINAL, EPI, SMALL, 2>(op, bv, it, smem_raw, sm, oct, grp, in, out);
+    own = mma_nodes<FINAL, EPI, RARE, 2>(op, bv, it, smem_raw, sm, oct, grp, in, out);
     if (c < 2) owner = row + 8 * (int)((oct >> (2 * c)) & 3u);
   } else if (nj == 1) {
-    own = mma_nodes<FINAL, EPI, SMALL, 1>(op, bv, it, smem_raw, sm, oct, grp, in, out);
+    own = mma_nodes<FINAL, EPI, RARE, 1>(op, bv, it, smem_raw, sm, oct, grp, in, out);
     if (c == 0) owner = row + 8 * (int)(oct & 3u);
   }
   if (FINAL && EPI != 3) {
@@ -1201,15 +1219,20 @@ size_t smul_smem(const asr_op* op, size_t st_size) {
   return b;
 }
 
+// The FP64 step's dynamic shared memory: without weight tables at most 96 KB of blocks (checked in the host driver), one more
+// of zeros, the operation words and the links (up to 112 slots there).  With tables as long as two blocks fit an SM: at 127
+// classes of 5 species (40,673 nodes, 512 chains of 16 levels) the tables leave room for one, 158 ms against 109 ms without.
+constexpr int MMA_SMEM = 108 * 1024, MMA_TABLES = 104 * 1024;
+
 template <typename ST, bool FUSE_D, bool FINAL, int EPI = 0>
 void launch_smul(asr_op* op, const BatchView& bv, const ST* blk, const typename St2<ST>::T* in, typename St2<ST>::T* out,
                  double2* part, int npw, int grid, cudaStream_t s) {
   OpView ov = op->view();   // EPI: the adjoint's fused steps, also t2 (bv.t2out); EPI 2, the reverse epilogue (bv.adj)
   if constexpr (std::is_same<ST, double>::value) {
-    const int sm = MmaSm(ov).bytes;
-    if constexpr (EPI >= 1)
-      if (bv.small_d && bv.t2out) {
-        k_smul_mma<FUSE_D, FINAL, EPI, true><<<grid, WPB * TL, sm, s>>>(ov, bv, blk, in, out, part, npw);
+    const int sm = MmaSm(ov, FINAL).bytes;
+    if constexpr (FINAL)
+      if ((EPI >= 1 && bv.small_d && bv.t2out) || sm > MMA_TABLES) {
+        k_smul_mma<FUSE_D, FINAL, EPI, true><<<grid, WPB * TL, MmaSm(ov, false).bytes, s>>>(ov, bv, blk, in, out, part, npw);
         return;
       }
     k_smul_mma<FUSE_D, FINAL, EPI><<<grid, WPB * TL, sm, s>>>(ov, bv, blk, in, out, part, npw);
@@ -3065,14 +3088,13 @@ int run_epi_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, con
 
 }  // namespace
 
-// the operator kernels stage up to 96 KB of bond blocks in shared memory (set once per device); the FP64 kernel adds its
-// zero block, operation words, link lists and diagonal weights
-constexpr int MMA_SMEM = 200 * 1024;
+// the operator kernels stage up to 96 KB of bond blocks in shared memory (set once per device)
 static void smem_attrs() {
   static bool done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || done[dev]) return;
+  cudaFuncSetAttribute(k_smul_mma<true, true, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul_mma<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul_mma<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
   cudaFuncSetAttribute(k_smul_mma<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
@@ -3153,6 +3175,7 @@ int run_lanes(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, con
 int apply_vectors(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, const std::vector<double>& gblob,
                   const GroupLayout& GL, int nvec, const double* x_host, bool complex_in, double* y_host, int what) {
   smem_attrs();
+  if (what == APPLY_H && smul_smem(op, sizeof(double)) > 96 * 1024) { set_error("apply: bond tables above 96 KB of shared memory"); return ASR_EINVAL; }
   cudaStream_t s = ctx->stream;
   const int nn = op->nn;
   const int nt = (nvec + TL - 1) / TL;

@@ -23,7 +23,7 @@ enum { GF_D_UNIFORM = 1, GF_O_ZERO = 2, GF_E_ZERO = 4, GF_X_ZERO = 8, GF_D_SMALL
 
 // The adjoint's step kernels fold d into the block rows and columns and get S (d o U) back by dividing the rows' d_l out
 // again.  A d_l that cannot be divided out (zero), or whose products leave the range of FP32, stays out of its row: there the
-// row carries 1, and the epilogue multiplies by d_l (the SMALL instantiations: the test in every epilogue made the others,
+// row carries 1, and the epilogue multiplies by d_l (the RARE instantiations: the test in every epilogue made the others,
 // which have no registers to spare, 2-7 % slower).
 constexpr double D_ROW = 1e-8;
 __host__ __device__ __forceinline__ double row_d(double d) { return fabs(d) >= D_ROW ? d : 1.0; }
@@ -81,7 +81,7 @@ struct BatchView {
   const void* gen_h1;      // general operator: h U and U for the last pass (EPI 4)
   const void* gen_u;
   int by_act;              // 1: a lane whose lane_act is 0 has left its chain for good (its vectors are not needed any more)
-  int small_d;             // 1: a group has GF_D_SMALL (host: the kernels that store t2 are the SMALL ones)
+  int small_d;             // 1: a group has GF_D_SMALL (host: the kernels that store t2 are the RARE ones)
   AdjEpi adj;              // the adjoint epilogue's vectors and coefficients (read only by that instantiation)
 };
 
