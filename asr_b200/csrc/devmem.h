@@ -1,0 +1,223 @@
+// Device memory of a call's temporaries, kept between calls.  Host code on the CUDA runtime's calls alone, so that its rules
+// can be tested without a device.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <atomic>
+#include <cstddef>
+#include <cstdint>
+#include <mutex>
+
+namespace asrb {
+
+// The memory of a call's temporaries (DevMem) stays with the context, so that a call neither maps nor unmaps device memory
+// (cudaMalloc and cudaFree of a chain batch's vectors took 10-50 ms a call, a second when the device's other processes did
+// the same).  Arrays of BIG bytes or more are blocks of the device's allocator, at most `keep` bytes of them held between
+// calls (the least recently used go first); smaller ones come from a stream-ordered pool that holds at most POOL_KEEP.  (The
+// pool for all sizes: mapping a 20 GB array that it had given back took a second.)  All of it goes back with the context,
+// when hold_workspace is switched off, when an allocation would fail, and at the end of a call that found less than a quarter
+// of the device free or this store's (MemScope).  A call finds out when it takes new memory, and every LOOK-th that plans.
+struct DevStore {
+  static constexpr size_t BIG = (size_t)32 << 20, POOL_KEEP = (size_t)256 << 20;
+  static constexpr int MOST = 64;   // held blocks
+  static constexpr int LOOK = 64;   // 0.1 to 1 ms a question: at most some 15 us a call (4 % of a 0.9 ms call at 8)
+  struct Block {
+    void* p;
+    size_t bytes;
+    cudaEvent_t done;   // after the last use
+    uint64_t used;
+  };
+  std::mutex lock;
+  Block blocks[MOST];   // held, not in use
+  int n = 0;
+  uint64_t uses = 0;
+  size_t keep = 0, out = 0;   // out: bytes of the blocks in use
+  int plans = 0;              // served without asking the device, since it was asked last
+  std::atomic<bool> scarce{false};
+  cudaMemPool_t pool = nullptr;
+
+  void open(int device, size_t total) {
+    keep = total / 8;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    if (cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
+      uint64_t most = POOL_KEEP;
+      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &most);
+    } else {
+      pool = nullptr;   // no pools on this device: small arrays from the device
+      cudaGetLastError();
+    }
+  }
+  void close(cudaStream_t s) {
+    trim();
+    if (pool) {
+      cudaStreamSynchronize(s);
+      cudaMemPoolDestroy(pool);
+    }
+    pool = nullptr;
+  }
+  // a block of at least `bytes` for work on stream s: the smallest held one of up to twice that (a larger one is wanted by a
+  // larger array of the same call), else a new one (false: out of memory)
+  bool get(size_t bytes, cudaStream_t s, Block& b) {
+    {
+      std::lock_guard<std::mutex> g(lock);
+      int at = -1;
+      for (int q = 0; q < n; ++q)
+        if (blocks[q].bytes >= bytes && blocks[q].bytes / 2 <= bytes && (at < 0 || blocks[q].bytes < blocks[at].bytes)) at = q;
+      if (at >= 0) {
+        if (cudaStreamWaitEvent(s, blocks[at].done, 0) != cudaSuccess) {
+          cudaGetLastError();
+          return false;
+        }
+        b = blocks[at];
+        blocks[at] = blocks[--n];
+        out += b.bytes;
+        return true;
+      }
+    }
+    b = Block{nullptr, bytes, nullptr, 0};
+    if (cudaMalloc(&b.p, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      trim();
+      if (cudaMalloc(&b.p, bytes) != cudaSuccess) return false;
+    }
+    if (cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming) != cudaSuccess) {
+      cudaFree(b.p);
+      return false;
+    }
+    {
+      std::lock_guard<std::mutex> g(lock);
+      out += bytes;
+    }
+    look();
+    return true;
+  }
+  // back from a call whose work on stream s still uses it
+  void put(Block b, cudaStream_t s) {
+    std::lock_guard<std::mutex> g(lock);
+    out -= b.bytes;
+    if (scarce || b.bytes > keep || cudaEventRecord(b.done, s) != cudaSuccess) {
+      cudaGetLastError();
+      cudaFree(b.p);   // waits for the work
+      cudaEventDestroy(b.done);
+      return;
+    }
+    drop(keep - b.bytes, MOST - 1);
+    b.used = ++uses;
+    blocks[n++] = b;
+  }
+  // what is held unused back to the device
+  void trim() {
+    if (pool) cudaMemPoolTrimTo(pool, 0);
+    std::lock_guard<std::mutex> g(lock);
+    drop(0, 0);
+  }
+  // asks the device; bytes free there or held unused here
+  size_t look() {
+    size_t freeb = pool_unused(), devb = 0, totb = 0;
+    cudaMemGetInfo(&devb, &totb);
+    std::lock_guard<std::mutex> g(lock);
+    for (int q = 0; q < n; ++q) freeb += blocks[q].bytes;
+    freeb += devb;
+    scarce = freeb + out < totb / 4;
+    plans = 0;
+    return freeb;
+  }
+  // Bytes a call may plan with: free device memory and what is held unused.  A call that needs at most `need` bytes for its
+  // largest batch plans the same with any figure of twice that or more, so the device (0.1 to 1 ms) is not asked every time
+  // where what is held will do.
+  size_t plan(size_t need) {
+    {
+      std::lock_guard<std::mutex> g(lock);
+      bool fits = pool_unused() / 2 >= need;
+      for (int q = 0; q < n; ++q) fits = fits || (blocks[q].bytes >= need && blocks[q].bytes / 2 <= need);
+      if (fits && ++plans < LOOK) return 2 * need;
+    }
+    return look();
+  }
+
+ private:
+  size_t pool_unused() const {
+    uint64_t held = 0, used = 0;
+    if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess || held <= used)
+      return 0;
+    return (size_t)(held - used);
+  }
+  // held blocks down to `most` bytes and `count` (under the lock)
+  void drop(size_t most, int count) {
+    size_t sum = 0;
+    for (int q = 0; q < n; ++q) sum += blocks[q].bytes;
+    while (sum > most || n > count) {
+      int old = 0;
+      for (int q = 1; q < n; ++q)
+        if (blocks[q].used < blocks[old].used) old = q;
+      sum -= blocks[old].bytes;
+      cudaFree(blocks[old].p);
+      cudaEventDestroy(blocks[old].done);
+      blocks[old] = blocks[--n];
+    }
+  }
+};
+
+// the store and stream that the calling thread's temporaries come from (set for the length of an entry point)
+struct CallMem {
+  DevStore* store = nullptr;
+  cudaStream_t stream = nullptr;
+};
+inline CallMem& call_mem() {
+  static thread_local CallMem c;
+  return c;
+}
+struct MemScope {
+  CallMem prev;
+  MemScope(DevStore* store, cudaStream_t s) : prev(call_mem()) { call_mem() = CallMem{store, s}; }
+  ~MemScope() {
+    DevStore* st = call_mem().store;
+    if (st && st != prev.store && st->scarce) {   // the call's own arrays have gone back before
+      cudaStreamSynchronize(call_mem().stream);
+      st->trim();
+    }
+    call_mem() = prev;
+  }
+  MemScope(const MemScope&) = delete;
+  MemScope& operator=(const MemScope&) = delete;
+};
+
+// one device allocation of a call, from the call's store (in the order of its stream, and given back to it), else from the
+// device
+struct DevMem {
+  void* p = nullptr;
+  CallMem c;
+  DevStore::Block b{};
+  bool get(size_t bytes) {
+    c = call_mem();
+    b = DevStore::Block{};
+    if (c.store && bytes >= DevStore::BIG) {
+      if (c.store->get(bytes, c.stream, b)) { p = b.p; return true; }
+    } else if (c.store && c.store->pool) {
+      if (cudaMallocFromPoolAsync(&p, bytes, c.store->pool, c.stream) == cudaSuccess) return true;
+      cudaGetLastError();
+      cudaStreamSynchronize(c.stream);   // what is held unused back to the device, then once more
+      c.store->trim();
+      if (cudaMallocFromPoolAsync(&p, bytes, c.store->pool, c.stream) == cudaSuccess) return true;
+    } else {
+      c.store = nullptr;
+      if (cudaMalloc(&p, bytes) == cudaSuccess) return true;
+    }
+    cudaGetLastError();
+    p = nullptr;
+    return false;
+  }
+  void put() {
+    if (!p) return;
+    if (!c.store) cudaFree(p);
+    else if (b.p) c.store->put(b, c.stream);
+    else cudaFreeAsync(p, c.stream);
+    p = nullptr;
+  }
+};
+
+}  // namespace asrb

@@ -369,7 +369,7 @@ struct DBuf {
     if (KEEP) {
       if (cudaMalloc(&q, bytes) == cudaSuccess) return true;
       cudaGetLastError();
-      if (pool_ctx()) pool_ctx()->mem_trim(0);
+      if (call_mem().store) call_mem().store->trim();
       if (cudaMalloc(&q, bytes) == cudaSuccess) return true;
     } else if (d.get(bytes)) {
       q = (T*)d.p;

@@ -3,10 +3,10 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <mutex>
 #include <vector>
 
 #include "common.cuh"
+#include "devmem.h"
 
 struct asr_ctx {
   int device = 0;
@@ -54,106 +54,9 @@ struct asr_ctx {
   int ws_hold = 0;
   void* ws = nullptr;
   size_t ws_bytes = 0;
-  // The memory of a call's temporaries (DevMem) stays with the context, so that a call neither maps nor unmaps device memory
-  // (cudaMalloc and cudaFree of a chain batch's vectors took 10-50 ms a call, a second when the device's other processes did
-  // the same).  Arrays of BIG bytes or more are blocks of the device's allocator, at most `keep` bytes of them held between
-  // calls (the least recently used go first); smaller ones come from a stream-ordered pool that holds at most POOL_KEEP.  (The
-  // pool for all sizes: mapping a 20 GB array that it had given back took a second.)  All of it goes back with the context,
-  // when hold_workspace is switched off, when an allocation would fail, and after a call that found less than a quarter of
-  // the device free.
-  static constexpr size_t BIG = (size_t)32 << 20, POOL_KEEP = (size_t)256 << 20;
-  struct Block {
-    void* p;
-    size_t bytes;
-    cudaEvent_t done;   // after the last use
-    uint64_t used;
-  };
-  std::mutex mem_lock;
-  std::vector<Block> blocks;   // held, not in use
-  uint64_t uses = 0;
-  size_t keep = 0;
-  bool scarce = false;
-  cudaMemPool_t pool = nullptr;
-  // a block of at least `bytes` for work on stream s: the smallest held one of up to twice that (a larger one is wanted by a
-  // larger array of the same call), else a new one (false: out of memory)
-  bool block_get(size_t bytes, cudaStream_t s, Block& b) {
-    {
-      std::lock_guard<std::mutex> g(mem_lock);
-      int at = -1;
-      for (int q = 0; q < (int)blocks.size(); ++q)
-        if (blocks[q].bytes >= bytes && blocks[q].bytes / 2 <= bytes && (at < 0 || blocks[q].bytes < blocks[at].bytes)) at = q;
-      if (at >= 0) {
-        b = blocks[at];
-        blocks.erase(blocks.begin() + at);
-        if (cudaStreamWaitEvent(s, b.done, 0) == cudaSuccess) return true;
-        cudaGetLastError();
-        blocks.push_back(b);
-        return false;
-      }
-    }
-    b = Block{nullptr, bytes, nullptr, 0};
-    if (cudaMalloc(&b.p, bytes) != cudaSuccess) {
-      cudaGetLastError();
-      mem_trim(0);
-      if (cudaMalloc(&b.p, bytes) != cudaSuccess) return false;
-    }
-    if (cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming) == cudaSuccess) return true;
-    cudaFree(b.p);
-    return false;
-  }
-  // back from a call whose work on stream s still uses it
-  void block_put(Block b, cudaStream_t s) {
-    const size_t most = scarce ? 0 : keep;
-    if (b.bytes > most || cudaEventRecord(b.done, s) != cudaSuccess) {
-      cudaGetLastError();
-      cudaFree(b.p);   // waits for the work
-      cudaEventDestroy(b.done);
-      return;
-    }
-    mem_trim(most - b.bytes, false);
-    std::lock_guard<std::mutex> g(mem_lock);
-    b.used = ++uses;
-    blocks.push_back(b);
-  }
-  // held memory down to `most` bytes of blocks
-  void mem_trim(size_t most, bool with_pool = true) {
-    if (with_pool && pool) cudaMemPoolTrimTo(pool, 0);
-    std::lock_guard<std::mutex> g(mem_lock);
-    size_t sum = 0;
-    for (const Block& b : blocks) sum += b.bytes;
-    while (sum > most) {
-      size_t old = 0;
-      for (size_t q = 1; q < blocks.size(); ++q)
-        if (blocks[q].used < blocks[old].used) old = q;
-      sum -= blocks[old].bytes;
-      cudaFree(blocks[old].p);
-      cudaEventDestroy(blocks[old].done);
-      blocks.erase(blocks.begin() + old);
-    }
-  }
-  // Bytes a call may plan with: free device memory and what the context holds unused, the held slab with it.  A call that
-  // needs at most `need` bytes for its largest batch plans the same with any figure of twice that or more, so the device (0.1
-  // to 1 ms) is asked only where what is held would not do.
-  size_t plan_bytes(size_t need = SIZE_MAX / 2) {
-    size_t freeb = 0, devb = 0, totb = 0;
-    {
-      std::lock_guard<std::mutex> g(mem_lock);
-      for (const Block& b : blocks) {
-        freeb += b.bytes;
-        if (b.bytes >= need && b.bytes / 2 <= need) return 2 * need;
-      }
-    }
-    uint64_t held = 0, used = 0;
-    if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && held > used) {
-      if ((size_t)(held - used) / 2 >= need) return 2 * need;
-      freeb += (size_t)(held - used);
-    }
-    cudaMemGetInfo(&devb, &totb);
-    freeb += devb;
-    scarce = freeb < totb / 4;
-    return freeb + ws_bytes;
-  }
+  asrb::DevStore mem;   // memory of the calls' temporaries
+  // bytes a call may plan with (DevStore::plan), the held slab with it
+  size_t plan_bytes(size_t need = SIZE_MAX / 2) { return mem.plan(need) + ws_bytes; }
   void ws_release() {
     if (ws) cudaFree(ws);
     ws = nullptr;
@@ -163,56 +66,9 @@ struct asr_ctx {
 
 namespace asrb {
 
-// the context whose pool the calling thread's temporaries come from (set for the length of an entry point)
-inline asr_ctx*& pool_ctx() {
-  static thread_local asr_ctx* c = nullptr;
-  return c;
-}
-struct PoolScope {
-  asr_ctx* prev;
-  explicit PoolScope(asr_ctx* c) : prev(pool_ctx()) { pool_ctx() = c; }
-  ~PoolScope() { pool_ctx() = prev; }
-  PoolScope(const PoolScope&) = delete;
-  PoolScope& operator=(const PoolScope&) = delete;
-};
 #define ASR_ENTER(ctx_)          \
   ASR_ON_DEVICE((ctx_)->device); \
-  ::asrb::PoolScope pool_call_(ctx_)
-
-// one device allocation of a call, from the context (in the order of its stream, and given back to it), else from the device
-struct DevMem {
-  void* p = nullptr;
-  cudaStream_t s = nullptr;
-  asr_ctx* c = nullptr;
-  asr_ctx::Block b{};
-  bool get(size_t bytes) {
-    c = pool_ctx();
-    b = asr_ctx::Block{};
-    s = c ? c->stream : nullptr;
-    if (c && bytes >= asr_ctx::BIG) {
-      if (c->block_get(bytes, s, b)) { p = b.p; return true; }
-    } else if (c && c->pool) {
-      if (cudaMallocFromPoolAsync(&p, bytes, c->pool, s) == cudaSuccess) return true;
-      cudaGetLastError();
-      cudaStreamSynchronize(s);   // what the context holds unused back to the device, then once more
-      c->mem_trim(0);
-      if (cudaMallocFromPoolAsync(&p, bytes, c->pool, s) == cudaSuccess) return true;
-    } else {
-      c = nullptr;
-      if (cudaMalloc(&p, bytes) == cudaSuccess) return true;
-    }
-    cudaGetLastError();
-    p = nullptr;
-    return false;
-  }
-  void put() {
-    if (!p) return;
-    if (!c) cudaFree(p);
-    else if (b.p) c->block_put(b, s);
-    else cudaFreeAsync(p, s);
-    p = nullptr;
-  }
-};
+  ::asrb::MemScope mem_call_(&(ctx_)->mem, (ctx_)->stream)
 
 // Device view of the node tables, passed by value to the kernels.  Node indices are 0-based, -1 = absent link;
 // operation indices 0-based.  Layouts follow the reference: flipr/flipg (nsmax, nn) and hopr/hopg (nslot, nn) with the

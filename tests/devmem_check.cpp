@@ -1,0 +1,91 @@
+// What asr_b200/csrc/devmem.h promises, on the made-up device of fake_cuda: one case per name on the command line.
+#include <cstdio>
+#include <cstring>
+#include <string>
+
+#include "../asr_b200/csrc/devmem.h"
+
+using namespace asrb;
+
+static const size_t MB = (size_t)1 << 20, GB = (size_t)1 << 30;
+static int bad = 0;
+#define CHECK(c) do { if (!(c)) { std::printf("line %d: %s\n", __LINE__, #c); bad = 1; } } while (0)
+
+// a call that plans with its largest array and takes arrays of the given sizes
+static bool call(DevStore& st, std::initializer_list<size_t> sizes) {
+  MemScope scope(&st, nullptr);
+  size_t most = 0;
+  for (size_t s : sizes) most = s > most ? s : most;
+  st.plan(most);
+  DevMem m[8];
+  int k = 0;
+  bool ok = true;
+  for (size_t s : sizes) ok = ok && m[k++].get(s);
+  while (k) m[--k].put();
+  return ok;
+}
+
+// memory that a call took stays for the next one: no allocation, and no question to the device
+static void reuse() {
+  DevStore st;
+  st.open(0, fake().total);
+  CHECK(call(st, {4 * GB, 100 * MB, MB}));
+  const int had = fake().mallocs, asked = fake().asked;
+  for (int q = 0; q < 4; ++q) CHECK(call(st, {4 * GB, 100 * MB, MB}));
+  CHECK(fake().mallocs == had && fake().asked == asked);
+  CHECK(fake().used <= fake().total / 8 + DevStore::POOL_KEEP);
+  CHECK(call(st, {20 * GB, 15 * GB, 10 * GB}));   // more than an eighth: the least recently used go
+  CHECK(fake().used <= fake().total / 8 + DevStore::POOL_KEEP);
+  st.close(nullptr);
+  CHECK(fake().used == 0 && fake().events == 0);
+}
+// more blocks than the store holds places for
+static void many() {
+  DevStore st;
+  st.open(0, fake().total);
+  for (int q = 0; q < 3 * DevStore::MOST; ++q) CHECK(call(st, {(33 + 70 * (size_t)q) * MB, 40 * MB}));
+  CHECK(st.n <= DevStore::MOST && fake().used <= fake().total / 8 + DevStore::POOL_KEEP);
+  st.close(nullptr);
+  CHECK(fake().used == 0 && fake().events == 0);
+}
+// nothing stays after a call that found less than a quarter of the device free: neither the blocks of earlier calls nor the
+// pool, and also when the call's own arrays are small
+static void scarce() {
+  for (int small = 0; small < 2; ++small) {
+    DevStore st;
+    st.open(0, fake().total);
+    CHECK(call(st, {4 * GB, 2 * GB, 200 * MB, MB}));
+    CHECK(fake().used > 6 * GB);
+    fake().others = fake().total - 30 * GB;
+    CHECK(call(st, {small ? 3 * MB : 9 * GB}));
+    if (small) call(st, {300 * MB});   // (a size that is not held)
+    CHECK(fake().used == 0);
+    fake().others = 0;
+    st.close(nullptr);
+  }
+}
+// a program whose calls are served by what is held finds out within some calls that the device has become scarce
+static void scarce_later() {
+  DevStore st;
+  st.open(0, fake().total);
+  CHECK(call(st, {4 * GB, MB}));
+  fake().others = fake().total - 10 * GB;
+  for (int q = 0; q < DevStore::LOOK; ++q) CHECK(call(st, {4 * GB, MB}));
+  CHECK(fake().used == 0);
+  fake().others = 0;
+  for (int q = 0; q < 2; ++q) CHECK(call(st, {4 * GB, MB}));
+  CHECK(fake().used >= 4 * GB);   // and the other way
+  st.close(nullptr);
+}
+
+int main(int argc, char** argv) {
+  for (int k = 1; k < argc; ++k) {
+    const std::string s = argv[k];
+    if (s == "reuse") reuse();
+    else if (s == "many") many();
+    else if (s == "scarce") scarce();
+    else if (s == "scarce_later") scarce_later();
+    else { std::printf("no case %s\n", argv[k]); bad = 1; }
+  }
+  return bad;
+}
