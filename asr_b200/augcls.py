@@ -65,8 +65,11 @@ class Context:
                     "adj_scal": 7}
 
     def hold_workspace(self, on: bool):
-        """Keep the device vector memory of the chain runs and the adjoint in this context between calls (on) or free it
-        and what the context keeps of its calls' temporaries (off, the default)."""
+        """On: keep the device vector memory of the chain runs and the adjoint in this context between calls, whatever its
+        size.  Off (the state of a new context): free it, and with it the memory of the calls' temporaries that stays
+        allocated between calls in any case, up to an eighth of the device for all its contexts together (nothing after a
+        call that found less than a quarter of the device free).  A program that needs that memory itself calls this
+        with False."""
         check(lib().asr_ctx_hold_workspace(self.h, int(bool(on))))
 
     def profile(self, on: bool):

@@ -244,7 +244,8 @@ int asr_ctx_create(int device, asr_ctx** out) {
   c->stream = c->own_stream;
   // an eighth of the device: holds the vectors of a 16-tile FP64 batch of the 20,969-node operator (5-8 GB), of a
   // 256,000-site supercell (2-4 GB) and the adjoint's kept levels of three tiles (22 GB)
-  c->mem.open(device, prop.totalGlobalMem);
+  c->mem = dev_store(device);
+  c->mem->open(device, prop.totalGlobalMem);
   *out = c;
   return ASR_OK;
 }
@@ -253,7 +254,7 @@ int asr_ctx_destroy(asr_ctx* ctx) {
   if (!ctx) return ASR_OK;
   DeviceGuard dg;
   dg.set(ctx->device);
-  ctx->mem.close(ctx->own_stream);
+  ctx->mem->close(ctx->own_stream, ctx);
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   if (ctx->d_err) cudaFree(ctx->d_err);
   ctx->ws_release();
@@ -296,7 +297,7 @@ int asr_ctx_hold_workspace(asr_ctx* ctx, int on) {
   if (!on) {
     ASR_CUDA(cudaStreamSynchronize(ctx->stream));
     ctx->ws_release();
-    ctx->mem.trim();
+    ctx->mem->trim();
   }
   ctx->ws_hold = on != 0;
   return ASR_OK;

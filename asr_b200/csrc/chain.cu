@@ -1313,7 +1313,7 @@ int vector_slab(asr_ctx* ctx, size_t bytes, Dev<unsigned char>& own, void** base
       if (rc != cudaSuccess) {   // what the context holds unused back to the device, then once more
         cudaGetLastError();
         cudaStreamSynchronize(ctx->stream);
-        ctx->mem.trim();
+        ctx->mem->trim();
         rc = cudaMalloc(&ctx->ws, bytes);
       }
       if (rc != cudaSuccess) {
@@ -2139,8 +2139,8 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
   while (tpb > 1 && (size_t)tpb * nvec * vec_bytes > freeb / 2) tpb /= 2;
   // and no more than the context keeps between calls, where that is two tiles or more and no slab is held: allocating and
   // freeing 70 GB at every call took 50 ms to a second, the smaller batches of the fcc ternary workload (3 tiles) take 20 ms
-  if (!tile_env && !ctx->ws_hold && (size_t)nvec * vec_bytes <= ctx->mem.keep / 2)
-    tpb = (int)std::min<size_t>(tpb, ctx->mem.keep / ((size_t)nvec * vec_bytes));
+  if (!tile_env && !ctx->ws_hold && (size_t)nvec * vec_bytes <= ctx->mem->keep / 2)
+    tpb = (int)std::min<size_t>(tpb, ctx->mem->keep / ((size_t)nvec * vec_bytes));
   if ((size_t)nvec * vec_bytes > freeb) { set_error("adjoint: %d vectors of %zu bytes do not fit", nvec, vec_bytes); return ASR_ENOMEM; }
   tpb = std::min(tpb, ntile_all);
   const int npw = default_npw(nn), npb = WPB * npw, bpt = (nn + npb - 1) / npb;

@@ -10,13 +10,15 @@
 
 namespace asrb {
 
-// The memory of a call's temporaries (DevMem) stays with the context, so that a call neither maps nor unmaps device memory
+// The memory of a call's temporaries (DevMem) stays with the library, so that a call neither maps nor unmaps device memory
 // (cudaMalloc and cudaFree of a chain batch's vectors took 10-50 ms a call, a second when the device's other processes did
 // the same).  Arrays of BIG bytes or more are blocks of the device's allocator, at most `keep` bytes of them held between
 // calls (the least recently used go first); smaller ones come from a stream-ordered pool that holds at most POOL_KEEP.  (The
-// pool for all sizes: mapping a 20 GB array that it had given back took a second.)  All of it goes back with the context,
-// when hold_workspace is switched off, when an allocation would fail, and at the end of a call that found less than a quarter
-// of the device free or this store's (MemScope).  A call finds out when it takes new memory, and every LOOK-th that plans.
+// pool for all sizes: mapping a 20 GB array that it had given back took a second.)  One store serves all contexts of a
+// device, so that several hold no more than one and an allocation of one that would fail gets what another has left.  What a
+// context's calls left goes back with the context, and everything when a context's hold_workspace is switched off, when an
+// allocation would fail, and at the end of a call that found less than a quarter of the device free or this store's
+// (MemScope).  A call finds out when it takes new memory, and every LOOK-th that plans.
 struct DevStore {
   static constexpr size_t BIG = (size_t)32 << 20, POOL_KEEP = (size_t)256 << 20;
   static constexpr int MOST = 64;   // held blocks
@@ -26,8 +28,10 @@ struct DevStore {
     size_t bytes;
     cudaEvent_t done;   // after the last use
     uint64_t used;
+    const void* owner;   // context of the last use
   };
   std::mutex lock;
+  int users = 0;        // contexts
   Block blocks[MOST];   // held, not in use
   int n = 0;
   uint64_t uses = 0;
@@ -36,7 +40,10 @@ struct DevStore {
   std::atomic<bool> scarce{false};
   cudaMemPool_t pool = nullptr;
 
+  // the first and every further context of the device
   void open(int device, size_t total) {
+    std::lock_guard<std::mutex> g(lock);
+    if (users++) return;
     keep = total / 8;
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
@@ -50,12 +57,15 @@ struct DevStore {
       cudaGetLastError();
     }
   }
-  void close(cudaStream_t s) {
-    trim();
-    if (pool) {
-      cudaStreamSynchronize(s);
-      cudaMemPoolDestroy(pool);
-    }
+  // a context goes, with what its calls left
+  void close(cudaStream_t s, const void* owner) {
+    cudaStreamSynchronize(s);
+    std::lock_guard<std::mutex> g(lock);
+    for (int q = n - 1; q >= 0; --q)
+      if (blocks[q].owner == owner) release(q);
+    if (pool) cudaMemPoolTrimTo(pool, 0);
+    if (--users) return;
+    if (pool) cudaMemPoolDestroy(pool);
     pool = nullptr;
   }
   // a block of at least `bytes` for work on stream s: the smallest held one of up to twice that (a larger one is wanted by a
@@ -77,7 +87,7 @@ struct DevStore {
         return true;
       }
     }
-    b = Block{nullptr, bytes, nullptr, 0};
+    b = Block{nullptr, bytes, nullptr, 0, nullptr};
     if (cudaMalloc(&b.p, bytes) != cudaSuccess) {
       cudaGetLastError();
       trim();
@@ -95,7 +105,7 @@ struct DevStore {
     return true;
   }
   // back from a call whose work on stream s still uses it
-  void put(Block b, cudaStream_t s) {
+  void put(Block b, cudaStream_t s, const void* owner) {
     std::lock_guard<std::mutex> g(lock);
     out -= b.bytes;
     if (scarce || b.bytes > keep || cudaEventRecord(b.done, s) != cudaSuccess) {
@@ -106,6 +116,7 @@ struct DevStore {
     }
     drop(keep - b.bytes, MOST - 1);
     b.used = ++uses;
+    b.owner = owner;
     blocks[n++] = b;
   }
   // what is held unused back to the device
@@ -155,17 +166,27 @@ struct DevStore {
       for (int q = 1; q < n; ++q)
         if (blocks[q].used < blocks[old].used) old = q;
       sum -= blocks[old].bytes;
-      cudaFree(blocks[old].p);
-      cudaEventDestroy(blocks[old].done);
-      blocks[old] = blocks[--n];
+      release(old);
     }
+  }
+  void release(int q) {
+    cudaFree(blocks[q].p);
+    cudaEventDestroy(blocks[q].done);
+    blocks[q] = blocks[--n];
   }
 };
 
-// the store and stream that the calling thread's temporaries come from (set for the length of an entry point)
+// the store of a device (up to 64 in a machine); never destroyed
+inline DevStore* dev_store(int device) {
+  static DevStore* st = new DevStore[64];
+  return st + (device & 63);
+}
+
+// the store, stream and context that the calling thread's temporaries belong to (set for the length of an entry point)
 struct CallMem {
   DevStore* store = nullptr;
   cudaStream_t stream = nullptr;
+  const void* owner = nullptr;
 };
 inline CallMem& call_mem() {
   static thread_local CallMem c;
@@ -173,7 +194,7 @@ inline CallMem& call_mem() {
 }
 struct MemScope {
   CallMem prev;
-  MemScope(DevStore* store, cudaStream_t s) : prev(call_mem()) { call_mem() = CallMem{store, s}; }
+  MemScope(DevStore* store, cudaStream_t s, const void* owner) : prev(call_mem()) { call_mem() = CallMem{store, s, owner}; }
   ~MemScope() {
     DevStore* st = call_mem().store;
     if (st && st != prev.store && st->scarce) {   // the call's own arrays have gone back before
@@ -214,7 +235,7 @@ struct DevMem {
   void put() {
     if (!p) return;
     if (!c.store) cudaFree(p);
-    else if (b.p) c.store->put(b, c.stream);
+    else if (b.p) c.store->put(b, c.stream, c.owner);
     else cudaFreeAsync(p, c.stream);
     p = nullptr;
   }

@@ -54,9 +54,9 @@ struct asr_ctx {
   int ws_hold = 0;
   void* ws = nullptr;
   size_t ws_bytes = 0;
-  asrb::DevStore mem;   // memory of the calls' temporaries
+  asrb::DevStore* mem = nullptr;   // the device's, of the calls' temporaries
   // bytes a call may plan with (DevStore::plan), the held slab with it
-  size_t plan_bytes(size_t need = SIZE_MAX / 2) { return mem.plan(need) + ws_bytes; }
+  size_t plan_bytes(size_t need = SIZE_MAX / 2) { return mem->plan(need) + ws_bytes; }
   void ws_release() {
     if (ws) cudaFree(ws);
     ws = nullptr;
@@ -68,7 +68,7 @@ namespace asrb {
 
 #define ASR_ENTER(ctx_)          \
   ASR_ON_DEVICE((ctx_)->device); \
-  ::asrb::MemScope mem_call_(&(ctx_)->mem, (ctx_)->stream)
+  ::asrb::MemScope mem_call_((ctx_)->mem, (ctx_)->stream, (ctx_))
 
 // Device view of the node tables, passed by value to the kernels.  Node indices are 0-based, -1 = absent link;
 // operation indices 0-based.  Layouts follow the reference: flipr/flipg (nsmax, nn) and hopr/hopg (nslot, nn) with the

@@ -72,9 +72,11 @@ int asr_ctx_profile(asr_ctx* ctx, int on);
 /* on = 1: the batched chain runs (asr_chains_run and its lane and device forms) and the adjoint (asr_chains_adjoint,
  * asr_chains_adjoint_ext) keep their device vector memory (one slab, at most half of the device memory free when it is
  * first needed, grown when a later call needs more) in the context after they return and reuse it on the next call,
- * instead of allocating and freeing it per call; on = 0 (the default) frees it, and with it what the context keeps anyway:
- * the temporaries of its calls, up to an eighth of the device's memory (nothing after a call that found less than a quarter
- * of it free).  For loops whose batches are larger than that.  No counterpart in the reference (whose arrays are allocated per call). */
+ * instead of allocating and freeing it per call.  on = 0 (the state of a new context): no slab.  Without a slab, too, the
+ * memory of the calls' temporaries stays allocated between calls, for all contexts of a device together up to an eighth of
+ * its memory (nothing after a call that found less than a quarter of it free); calling this with on = 0 frees the slab and
+ * all of that at once, for a program that needs the memory itself.  on = 1 is for loops whose batches are larger than an
+ * eighth.  No counterpart in the reference (whose arrays are allocated per call). */
 int asr_ctx_hold_workspace(asr_ctx* ctx, int on);
 int asr_ctx_kernel_stats(asr_ctx* ctx, double* ms, int64_t* launches, double* bytes, double* flops);
 int asr_ctx_kernel_stats_kind(asr_ctx* ctx, int kind, double* ms, int64_t* launches, double* bytes, double* flops);

@@ -12,8 +12,8 @@ static int bad = 0;
 #define CHECK(c) do { if (!(c)) { std::printf("line %d: %s\n", __LINE__, #c); bad = 1; } } while (0)
 
 // a call that plans with its largest array and takes arrays of the given sizes
-static bool call(DevStore& st, std::initializer_list<size_t> sizes) {
-  MemScope scope(&st, nullptr);
+static bool call(DevStore& st, std::initializer_list<size_t> sizes, const void* ctx = nullptr) {
+  MemScope scope(&st, nullptr, ctx);
   size_t most = 0;
   for (size_t s : sizes) most = s > most ? s : most;
   st.plan(most);
@@ -36,7 +36,7 @@ static void reuse() {
   CHECK(fake().used <= fake().total / 8 + DevStore::POOL_KEEP);
   CHECK(call(st, {20 * GB, 15 * GB, 10 * GB}));   // more than an eighth: the least recently used go
   CHECK(fake().used <= fake().total / 8 + DevStore::POOL_KEEP);
-  st.close(nullptr);
+  st.close(nullptr, nullptr);
   CHECK(fake().used == 0 && fake().events == 0);
 }
 // more blocks than the store holds places for
@@ -45,7 +45,7 @@ static void many() {
   st.open(0, fake().total);
   for (int q = 0; q < 3 * DevStore::MOST; ++q) CHECK(call(st, {(33 + 70 * (size_t)q) * MB, 40 * MB}));
   CHECK(st.n <= DevStore::MOST && fake().used <= fake().total / 8 + DevStore::POOL_KEEP);
-  st.close(nullptr);
+  st.close(nullptr, nullptr);
   CHECK(fake().used == 0 && fake().events == 0);
 }
 // nothing stays after a call that found less than a quarter of the device free: neither the blocks of earlier calls nor the
@@ -61,7 +61,7 @@ static void scarce() {
     if (small) call(st, {300 * MB});   // (a size that is not held)
     CHECK(fake().used == 0);
     fake().others = 0;
-    st.close(nullptr);
+    st.close(nullptr, nullptr);
   }
 }
 // a program whose calls are served by what is held finds out within some calls that the device has become scarce
@@ -75,7 +75,29 @@ static void scarce_later() {
   fake().others = 0;
   for (int q = 0; q < 2; ++q) CHECK(call(st, {4 * GB, MB}));
   CHECK(fake().used >= 4 * GB);   // and the other way
-  st.close(nullptr);
+  st.close(nullptr, nullptr);
+}
+
+// several contexts of a device: together no more than one may hold; what one has left serves an allocation of another that
+// would fail, and counts when another plans; it goes with its context alone
+static void contexts() {
+  DevStore& st = *dev_store(3);
+  int a, b, c;
+  for (int q = 0; q < 3; ++q) st.open(3, fake().total);
+  CHECK(call(st, {12 * GB, MB}, &a) && call(st, {9 * GB, MB}, &b) && call(st, {11 * GB, MB}, &c));
+  CHECK(fake().used <= fake().total / 8 + DevStore::POOL_KEEP);
+  st.close(nullptr, &c);
+  CHECK(call(st, {8 * GB}, &a) && call(st, {33 * MB, MB}, &b));
+  fake().others = fake().total - 60 * GB;
+  CHECK(st.plan(SIZE_MAX / 2) == 60 * GB);
+  CHECK(call(st, {59 * GB}, &b));
+  fake().others = 0;
+  st.trim();
+  CHECK(call(st, {8 * GB}, &a) && call(st, {700 * MB}, &b));
+  st.close(nullptr, &a);
+  CHECK(fake().used == 700 * MB);
+  st.close(nullptr, &b);
+  CHECK(fake().used == 0 && fake().events == 0);
 }
 
 int main(int argc, char** argv) {
@@ -85,6 +107,7 @@ int main(int argc, char** argv) {
     else if (s == "many") many();
     else if (s == "scarce") scarce();
     else if (s == "scarce_later") scarce_later();
+    else if (s == "contexts") contexts();
     else { std::printf("no case %s\n", argv[k]); bad = 1; }
   }
   return bad;
