@@ -184,11 +184,13 @@ int upload_tables(asr_op* op, const double* dmat, const double* block, int nsb, 
   std::vector<float> Bf(B.begin(), B.end());
   std::vector<int8_t> nsc8(op->ncls);
   for (int k = 0; k < op->ncls; ++k) nsc8[k] = (int8_t)op->nsc[k];
-  ASR_CUDA(cudaMalloc(&op->d_blocks, B.size() * sizeof(double)));
-  ASR_CUDA(cudaMalloc(&op->d_blocks_f, B.size() * sizeof(float)));
-  ASR_CUDA(cudaMalloc(&op->d_pi, pi0.size()));
-  ASR_CUDA(cudaMalloc(&op->d_sgm, sgm.size() * sizeof(uint16_t)));
-  ASR_CUDA(cudaMalloc(&op->d_nsc, nsc8.size()));
+  DevStore* st = op->ctx->mem;
+  if (!dev_alloc(st, s, &op->d_blocks, B.size() * sizeof(double)) || !dev_alloc(st, s, &op->d_blocks_f, B.size() * sizeof(float)) ||
+      !dev_alloc(st, s, &op->d_pi, pi0.size()) || !dev_alloc(st, s, &op->d_sgm, sgm.size() * sizeof(uint16_t)) ||
+      !dev_alloc(st, s, &op->d_nsc, nsc8.size())) {   // the caller frees the operator
+    set_error("build_augcls_operator: device allocation of the bond tables failed");
+    return ASR_ENOMEM;
+  }
   ASR_CUDA(cudaMemcpyAsync(op->d_blocks, B.data(), B.size() * sizeof(double), cudaMemcpyHostToDevice, s));
   ASR_CUDA(cudaMemcpyAsync(op->d_blocks_f, Bf.data(), Bf.size() * sizeof(float), cudaMemcpyHostToDevice, s));
   ASR_CUDA(cudaMemcpyAsync(op->d_pi, pi0.data(), pi0.size(), cudaMemcpyHostToDevice, s));

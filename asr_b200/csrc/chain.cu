@@ -1309,15 +1309,7 @@ int vector_slab(asr_ctx* ctx, size_t bytes, Dev<unsigned char>& own, void** base
   if (ctx->ws_hold) {
     if (ctx->ws_bytes < bytes) {
       ctx->ws_release();
-      cudaError_t rc = cudaMalloc(&ctx->ws, bytes);
-      if (rc != cudaSuccess) {   // what the context holds unused back to the device, then once more
-        cudaGetLastError();
-        cudaStreamSynchronize(ctx->stream);
-        ctx->mem->trim();
-        rc = cudaMalloc(&ctx->ws, bytes);
-      }
-      if (rc != cudaSuccess) {
-        ctx->ws = nullptr;
+      if (!dev_alloc(ctx->mem, ctx->stream, &ctx->ws, bytes)) {
         set_error("chains: device allocation of %zu bytes failed", bytes);
         return ASR_ENOMEM;
       }

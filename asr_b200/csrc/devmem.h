@@ -182,6 +182,22 @@ inline DevStore* dev_store(int device) {
   return st + (device & 63);
 }
 
+// An array that outlives the call (an operator's tables, a supercell's, a context's slab) from the device: where there is
+// no room for it, what the store holds unused goes back first.
+template <typename T>
+bool dev_alloc(DevStore* st, cudaStream_t s, T** p, size_t bytes) {
+  if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  if (st) {
+    cudaStreamSynchronize(s);
+    st->trim();
+    if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+  }
+  *p = nullptr;
+  return false;
+}
+
 // the store, stream and context that the calling thread's temporaries belong to (set for the length of an entry point)
 struct CallMem {
   DevStore* store = nullptr;

@@ -367,10 +367,7 @@ struct DBuf {
   bool get(size_t k, T*& q, DevMem& d) {
     const size_t bytes = std::max<size_t>(k, 1) * sizeof(T);
     if (KEEP) {
-      if (cudaMalloc(&q, bytes) == cudaSuccess) return true;
-      cudaGetLastError();
-      if (call_mem().store) call_mem().store->trim();
-      if (cudaMalloc(&q, bytes) == cudaSuccess) return true;
+      if (dev_alloc(call_mem().store, call_mem().stream, &q, bytes)) return true;
     } else if (d.get(bytes)) {
       q = (T*)d.p;
       return true;
@@ -577,7 +574,10 @@ __global__ void k_count_flips(OpView op, int8_t* nflip) {
   nflip[i] = (int8_t)n;
 }
 int count_flips(asr_ctx* ctx, asr_op* op) {
-  ASR_CUDA(cudaMalloc(&op->d_nflip, op->nn));
+  if (!dev_alloc(ctx->mem, ctx->stream, &op->d_nflip, op->nn)) {
+    set_error("graph build: device allocation of %d bytes failed", op->nn);
+    return ASR_ENOMEM;
+  }
   k_count_flips<<<(op->nn + 255) / 256, 256, 0, ctx->stream>>>(op->view(), op->d_nflip);
   ASR_CUDA(cudaGetLastError());
   ASR_CUDA(cudaStreamSynchronize(ctx->stream));   // the operator may be used next on another stream or context

@@ -622,11 +622,15 @@ int asr_supercell_build(asr_ctx* ctx, int nsite, int nslot, const int* nbr, cons
     }
   std::vector<float> Bf(B.begin(), B.end());
   cudaStream_t s = ctx->stream;
-  bool ok = cudaMalloc(&sc->d_nbr, std::max<size_t>(nb.size(), 1) * sizeof(int)) == cudaSuccess &&
-            cudaMalloc(&sc->d_spc, nsite) == cudaSuccess && cudaMalloc(&sc->d_par, par.size() * sizeof(double)) == cudaSuccess &&
-            cudaMalloc(&sc->d_blocks, B.size() * sizeof(double)) == cudaSuccess &&
-            cudaMalloc(&sc->d_blocks_f, Bf.size() * sizeof(float)) == cudaSuccess;
-  if (!ok) { set_error("asr_supercell_build: device allocation failed"); delete sc; return ASR_ENOMEM; }
+  DevStore* st = ctx->mem;
+  bool ok = dev_alloc(st, s, &sc->d_nbr, std::max<size_t>(nb.size(), 1) * sizeof(int)) && dev_alloc(st, s, &sc->d_spc, nsite) &&
+            dev_alloc(st, s, &sc->d_par, par.size() * sizeof(double)) && dev_alloc(st, s, &sc->d_blocks, B.size() * sizeof(double)) &&
+            dev_alloc(st, s, &sc->d_blocks_f, Bf.size() * sizeof(float));
+  if (!ok) {
+    asr_supercell_free(sc);
+    set_error("asr_supercell_build: device allocation failed");
+    return ASR_ENOMEM;
+  }
   cudaMemcpyAsync(sc->d_nbr, nb.data(), nb.size() * sizeof(int), cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(sc->d_spc, sp.data(), nsite, cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(sc->d_par, par.data(), par.size() * sizeof(double), cudaMemcpyHostToDevice, s);

@@ -100,6 +100,21 @@ static void contexts() {
   CHECK(fake().used == 0 && fake().events == 0);
 }
 
+// an array that outlives the call gets what is held unused; where that is not enough, it fails and gives no pointer
+static void lasting() {
+  DevStore st;
+  st.open(0, fake().total);
+  CHECK(call(st, {4 * GB, MB}));
+  fake().others = fake().total - 5 * GB;
+  char *p = nullptr, *q = p + 1;
+  CHECK(dev_alloc(&st, nullptr, &p, 3 * GB) && p && fake().used == 3 * GB);
+  CHECK(!dev_alloc(&st, nullptr, &q, 3 * GB) && !q && fake().used == 3 * GB);
+  fake().others = 0;
+  cudaFree(p);
+  st.close(nullptr, nullptr);
+  CHECK(fake().used == 0);
+}
+
 int main(int argc, char** argv) {
   for (int k = 1; k < argc; ++k) {
     const std::string s = argv[k];
@@ -108,6 +123,7 @@ int main(int argc, char** argv) {
     else if (s == "scarce") scarce();
     else if (s == "scarce_later") scarce_later();
     else if (s == "contexts") contexts();
+    else if (s == "lasting") lasting();
     else { std::printf("no case %s\n", argv[k]); bad = 1; }
   }
   return bad;
