@@ -1366,7 +1366,7 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
   // projections: per tile nlevmax x 9 nt x 32 complex values
   const size_t proj_tile_bytes = proj ? (size_t)nlevmax * 9 * proj->nt * TL * sizeof(double2) : 0;
   tpb = std::min(tpb, ntile_all);
-  const size_t freeb = ctx->plan_bytes((size_t)tpb * (nvec * vec_bytes + proj_tile_bytes));
+  const size_t freeb = ctx->plan_bytes((size_t)tpb * (nvec * vec_bytes + proj_tile_bytes), proj ? 2 : 1);
   while (tpb > 1 && (size_t)tpb * (nvec * vec_bytes + proj_tile_bytes) > freeb / 2) tpb /= 2;
   int npw = opt.nodes_per_warp > 0 ? opt.nodes_per_warp : op->tuned_npw[prec_ix] > 0 ? op->tuned_npw[prec_ix] : default_npw(nn);
   if (const char* e = getenv("ASR_NODES_PER_WARP")) npw = std::max(1, atoi(e));

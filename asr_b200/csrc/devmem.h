@@ -138,9 +138,10 @@ struct DevStore {
   }
   // Bytes a call may plan with: free device memory and what is held unused.  A call that needs at most `need` bytes for its
   // largest batch plans the same with any figure of twice that or more, so the device (0.1 to 1 ms) is not asked every time
-  // where what is held will do.
-  size_t plan(size_t need) {
-    {
+  // where what is held will do.  That is so for one array; with several, a held block may serve a small one and leave no
+  // room for the others.
+  size_t plan(size_t need, int arrays = 1) {
+    if (arrays == 1) {
       std::lock_guard<std::mutex> g(lock);
       bool fits = pool_unused() / 2 >= need;
       for (int q = 0; q < n; ++q) fits = fits || (blocks[q].bytes >= need && blocks[q].bytes / 2 <= need);

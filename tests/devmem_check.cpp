@@ -115,6 +115,30 @@ static void lasting() {
   CHECK(fake().used == 0);
 }
 
+// batches of two arrays a tile (a chain's vectors and its projections), planned as the chain driver does: what is planned
+// fits, whatever is held
+static void planned() {
+  for (size_t held : {6 * GB, 9 * GB, 11 * GB, 19 * GB})
+    for (size_t free : {0 * GB, 1 * GB, 3 * GB}) {
+      DevStore st;
+      st.open(0, fake().total);
+      CHECK(call(st, {held}));
+      fake().others = fake().total - held - free;
+      const size_t proj = GB / 2, vec = 3 * GB / 4;   // a tile's
+      MemScope scope(&st, nullptr, nullptr);
+      size_t tiles = 8;
+      const size_t freeb = st.plan(tiles * (proj + vec), 2);
+      while (tiles > 1 && tiles * (proj + vec) > freeb / 2) tiles /= 2;
+      DevMem a, b;
+      CHECK(a.get(tiles * vec) && b.get(tiles * proj));
+      b.put();
+      a.put();
+      fake().others = 0;
+      st.close(nullptr, nullptr);
+      CHECK(fake().used == 0);
+    }
+}
+
 int main(int argc, char** argv) {
   for (int k = 1; k < argc; ++k) {
     const std::string s = argv[k];
@@ -124,6 +148,7 @@ int main(int argc, char** argv) {
     else if (s == "scarce_later") scarce_later();
     else if (s == "contexts") contexts();
     else if (s == "lasting") lasting();
+    else if (s == "planned") planned();
     else { std::printf("no case %s\n", argv[k]); bad = 1; }
   }
   return bad;
