@@ -51,11 +51,14 @@ __global__ void k_cf_eval_chain(const double2* a, const double2* b, const int* m
 }
 
 // One eigenvalue problem per chain costs a block per chain, one per (energy, chain) a thread: from 8 energies on the
-// first is less work and fewer dependent steps; below, many chains fill the device better by threads.
+// first is less work and fewer dependent steps; below, many chains fill the device better by threads.  A Beer-Pettifor tail
+// takes the block whatever the number of energies: the threads' form solves its eigenvalue problems another way (cf_tail_dev),
+// and a fraction's bits must not depend on how many energies share the call (20,000 chains of 20 levels at one energy: 14 ms
+// by blocks, 85 by threads).
 void cf_eval(cudaStream_t s, const double2* a, const double2* b, const int* m, int ld, int nchain, const double2* z, int nz, int tail,
              double2* g, double2* edges, int* nfall) {
   const long n = (long)nz * nchain;
-  if (nz >= 8) k_cf_eval_chain<<<nchain, 128, 0, s>>>(a, b, m, ld, z, nz, tail, g, edges, nfall);
+  if (nz >= 8 || tail == ASR_TAIL_BP) k_cf_eval_chain<<<nchain, 128, 0, s>>>(a, b, m, ld, z, nz, tail, g, edges, nfall);
   else k_cf_eval<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(a, b, m, ld, nchain, z, nz, tail, g, edges, nfall);
 }
 
