@@ -1060,16 +1060,16 @@ __global__ void __launch_bounds__(WPB * TL) k_project(OpView op, BatchView bv, t
   int bpt;
   if (!node_iter(bv, npw, it, bpt)) return;
   const int lane = threadIdx.x % TL, w = threadIdx.x / TL;
-  const int L = it.tile * TL + lane;
-  const int grp = bv.lane_group[L];
-  if (grp < 0) return;
-  const unsigned long long chim = bv.ginfo[grp].chimask;
+  const int grp = bv.tile_group[it.tile];
+  const unsigned long long chim = grp >= 0 ? bv.ginfo[grp].chimask : 0ull;
   for (int qn = 0; qn < npw; ++qn) {
     int i = it.first + w + WPB * qn;
     if (i >= bv.nn) break;
+    const int keep = project_mask(op, i, chim);
+    if (bv.lane_group[it.tile * TL + lane] < 0) continue;
     double2 v[9];
     ld9(x + vnode(it.tile, bv.nn, i), lane, v);
-    project_node_sum(op, i, chim, v);
+    project_node(op, i, chim, keep, v);
     st9(x + vnode(it.tile, bv.nn, i), lane, v);
   }
 }
