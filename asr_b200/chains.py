@@ -273,10 +273,9 @@ def edc_green_proj(op: AugclsOp, ed: dict, z, iv: int, nlev: int, tnode, tgop, t
 def autotune(op: AugclsOp, specs, z, precision: str = "fp64", levels: int = 8) -> dict:
     """Choose the batch shape (tiles per batch, nodes per warp) of the chains on this operator by timing the given groups
     (depth capped at ``levels``, at most 64 energies); a candidate must beat the built-in default by 3 %.  Later calls in
-    this precision use the choice; at that shape the fixed-offset link choice is timed against the general one and kept
-    when it is 3 % faster (the step kernels read such links at fixed offsets under either, with the same bits).  Returns dict(tiles_per_batch, nodes_per_warp, ms_tiles (4, 8, 16, 32
-    tiles at 4 nodes per warp), ms_npw (1, 2, 4, 8 nodes per warp), link_gather ("fixed-offset" or "general"),
-    ms_link (general, fixed-offset step at the chosen shape))."""
+    this precision use the choice.  Returns dict(tiles_per_batch, nodes_per_warp, ms_tiles (4, 8, 16, 32 tiles at the default
+    nodes per warp: 1, 2 or 4 by the operator's size), ms_npw (1, 2, 4, 8 nodes per warp), link_gather "general" and
+    ms_link [-1, -1]: one step kernel per precision takes every link, so there is no link choice to time)."""
     z = np.ascontiguousarray(np.atleast_1d(z), dtype=np.complex128)
     arr, keep = _groups(specs)
     tpb, npw = C.c_int(), C.c_int()

@@ -1169,7 +1169,7 @@ int asr_chains_proj(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, int
 
 // Batch-shape autotuner: times (device time of the batches, best of two) the chains of the given groups (depth capped at
 // `levels`, at most 64 of the energies) with
-// 4, 8, 16, 32 tiles per batch at 4 nodes per warp, then 1, 2, 4, 8 nodes per warp at the best batch, and keeps the
+// 4, 8, 16, 32 tiles per batch at the default nodes per warp, then 1, 2, 4, 8 nodes per warp at the best batch, and keeps the
 // fastest pair on the operator for this precision (used whenever a call leaves the shape automatic).  times (8) receives
 // the device times in ms (-1 where a candidate was skipped), or NULL.
 int asr_autotune(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, int ngroup, const double* z, int nz, int precision,
@@ -1220,7 +1220,6 @@ int asr_autotune(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, int ng
       if (!done) { op->tuned_tpb[pix] = tpb; op->tuned_npw[pix] = npw; op->tuned_link[pix] = link; }
     }
   } keep{op, pix, op->tuned_tpb[pix], op->tuned_npw[pix], op->tuned_link[pix]};
-  op->tuned_link[pix] = 0;   // the shapes are timed with the general step kernel
   const int tpbs[4] = {4, 8, 16, 32}, npws[4] = {1, 2, 4, 8};
   double tab[8];
   for (double& t : tab) t = -1.0;
@@ -1244,16 +1243,8 @@ int asr_autotune(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, int ng
     if (tab[4 + c] < margin * best) { best = tab[4 + c]; best_n = npws[c]; }
   op->tuned_tpb[pix] = best_t;
   op->tuned_npw[pix] = best_n;
-  // then the step kernel with fixed-offset link gathers at that shape (the same bits; kept when it is 3 % faster)
-  double t_gen = 0.0, t_link = 0.0;
-  ASR_TRY(timed(best_t, best_n, t_gen));
-  op->tuned_link[pix] = 1;
-  int rc = timed(best_t, best_n, t_link);
-  if (rc != ASR_OK) return rc;
-  op->tuned_link[pix] = t_link < margin * t_gen ? 1 : 0;
+  op->tuned_link[pix] = 0;   // selects nothing: one kernel per precision takes every link
   keep.done = true;
-  op->tuned_link_ms[pix][0] = t_gen;
-  op->tuned_link_ms[pix][1] = t_link;
   if (tpb_out) *tpb_out = best_t;
   if (npw_out) *npw_out = best_n;
   if (times) for (int c = 0; c < 8; ++c) times[c] = tab[c];
@@ -1266,7 +1257,7 @@ int asr_op_tuning(const asr_op* op, int precision, int* tpb, int* npw, int* link
   if (tpb) *tpb = op->tuned_tpb[pix];
   if (npw) *npw = op->tuned_npw[pix];
   if (link) *link = op->tuned_link[pix];
-  if (ms) { ms[0] = op->tuned_link_ms[pix][0]; ms[1] = op->tuned_link_ms[pix][1]; }
+  if (ms) ms[0] = ms[1] = -1.0;
   return ASR_OK;
 }
 

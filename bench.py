@@ -26,13 +26,11 @@ sys.path.insert(0, ROOT)
 
 NZ_SLICE = 192
 # DRAM bytes (read + write) per launch of the step kernel from one ncu capture (4 groups x 128 energies of this operator), the
-# algorithmic bytes of that launch and what was captured, per (precision, link-gather choice; one kernel for both); traffic is
-# scaled to the bench's mean launch
+# algorithmic bytes of that launch and what was captured, per precision; traffic is scaled to the bench's mean launch
 _TAB = 18 * 5 + 3 * 5 + 20
 _FP64 = (3.18e9, 16 * 20969 * (2 * 4608.0 + _TAB), "ncu capture of k_smul_mma<1,1,0> at 16 tiles")
 _FP32 = (0.771e9, 8 * 20969 * (2 * 2304.0 + _TAB), "ncu capture of k_smul<float,1,1,0> at 8 tiles")
-NCU_STEP_TRAFFIC = {("fp64", "fixed-offset"): _FP64, ("fp64", "general"): _FP64,
-                    ("fp32", "fixed-offset"): _FP32, ("fp32", "general"): _FP32}
+NCU_STEP_TRAFFIC = {"fp64": _FP64, "fp32": _FP32}
 
 
 def roof(st, hbm_peak, pipe_peak=None):
@@ -80,7 +78,7 @@ def parse():
     p.add_argument("--adj-energies", type=int, default=48, help="adjoint leg: the first N of the 48 contour energies")
     p.add_argument("--adj-depth", type=int, default=0, help="adjoint leg: every chain this deep (0: the drawn depths)")
     p.add_argument("--link", default="auto", choices=["auto", "general", "fixed"],
-                   help="step-kernel link gathers: the autotuner's choice (auto; general without --autotune), or pinned")
+                   help="link choice of the tuned state (one step kernel per precision takes every link: selects nothing)")
     return p.parse_args()
 
 
@@ -891,8 +889,8 @@ def main():
         tflops = (ks["flops"] / max(ks["launches"], 1)) / (per_launch_ms / 1000.0) / 1e12
         cpu = cpu_baseline(case, fl, groups, z_all) if args.cpu_sample else None
         traffic, traffic_source = None, None
-        if (args.precision, tune["link_gather"]) in NCU_STEP_TRAFFIC:
-            meas, alg, traffic_source = NCU_STEP_TRAFFIC[(args.precision, tune["link_gather"])]
+        if args.precision in NCU_STEP_TRAFFIC:
+            meas, alg, traffic_source = NCU_STEP_TRAFFIC[args.precision]
             traffic = meas * (ks["bytes"] / max(ks["launches"], 1)) / alg
             traffic_source += ", scaled to the mean launch"
         # every timed kernel kind: the chain step and the Lanczos update of the timed region, the KPM Chebyshev step and

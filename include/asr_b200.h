@@ -212,19 +212,18 @@ int asr_epi_blocks(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, cons
  * at 1, 2 or 4 nodes per warp by the operator's size, by 3 %) on the operator for this precision; later calls that leave the shape
  * automatic use it.  The shape does not change results beyond the order of the per-block partial sums (rounding).
  * Each candidate is timed on the device (CUDA events around its batches, allocations excluded, best of two runs).
- * At the chosen shape it then times the run with the fixed-offset link choice against the general one and keeps it when it
- * is 3 % faster; the step kernels of both precisions read such links at fixed offsets under either choice.
  * tpb, npw: the chosen shape; times(8) the device times in ms (-1: skipped) or NULL. */
 int asr_autotune(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups, int ngroup, const double* z, int nz, int precision,
                  int levels, int* tpb, int* npw, double* times);
 
-/* The operator's tuned state for a precision: tpb, npw (0: never tuned, the built-in defaults apply), link = 1 when the
- * fixed-offset link gathers are chosen, ms(2) the device times of the general and the fixed-offset step at the tuned shape
- * (-1: not timed).  Any pointer may be NULL.  No counterpart in the reference. */
+/* The operator's tuned state for a precision: tpb, npw (0: never tuned, the built-in defaults apply), link as set by
+ * asr_op_set_tuning (0 after asr_autotune), ms(2) = -1, -1.  link and ms are of earlier step kernels for links that move no
+ * orbital; one kernel per precision takes every link now, so link selects nothing and nothing is timed for it.  Any pointer
+ * may be NULL.  No counterpart in the reference. */
 int asr_op_tuning(const asr_op* op, int precision, int* tpb, int* npw, int* link, double* ms);
 /* Set the tuned state for a precision (a shape saved from an earlier asr_autotune, or a pinned one): tpb in {4, 8, 16, 32}
- * or 0 (built-in default), npw in {1, 2, 4, 8} or 0, link 0 (general gathers) or 1 (fixed-offset).  Results do not depend
- * on link; the shape changes only the order of the per-block partial sums. */
+ * or 0 (built-in default), npw in {1, 2, 4, 8} or 0, link 0 or 1 (kept and returned by asr_op_tuning, selects nothing).
+ * The shape changes only the order of the per-block partial sums. */
 int asr_op_set_tuning(asr_op* op, int precision, int tpb, int npw, int link);
 
 /* ---- route ed3 (src/asr_ed3.f90): chains on z - K'(z), K' = et - h' + u h' + h' u - h' Qt h', h' = g + d S d ---------- */
