@@ -415,39 +415,10 @@ __host__ __device__ inline double2 cf_species_pv_dev(const double2* a, const dou
 }
 
 // ---- real chains (plain mode)
-__host__ __device__ inline int sturm_count(int n, const double* d, const double* e, double x) {
-  int cnt = 0;
-  double q = d[0] - x;
-  if (q < 0) ++cnt;
-  for (int i = 1; i < n; ++i) {
-    if (q == 0.0) q = DBL_EPSILON * (fabs(e[i - 1]) + DBL_MIN);
-    q = d[i] - x - e[i - 1] * e[i - 1] / q;
-    if (q < 0) ++cnt;
-  }
-  return cnt;
-}
-__host__ __device__ inline double tridiag_extreme(int n, const double* d, const double* e, bool upper) {
-  double lo = d[0], hi = d[0];
-  for (int i = 0; i < n; ++i) {
-    double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < n - 1 ? fabs(e[i]) : 0.0);
-    lo = fmin(lo, d[i] - r);
-    hi = fmax(hi, d[i] + r);
-  }
-  double span = hi - lo;
-  lo -= 1e-12 * (span + 1.0);
-  hi += 1e-12 * (span + 1.0);
-  int target = upper ? n : 1;
-  for (int it = 0; it < 200; ++it) {
-    double mid = 0.5 * (lo + hi);
-    if (mid <= lo || mid >= hi) break;
-    if (sturm_count(n, d, e, mid) >= target) hi = mid; else lo = mid;
-  }
-  return 0.5 * (lo + hi);
-}
 #ifdef __CUDACC__
 // Number of eigenvalues below x of the real tridiagonal (d, e2 = e^2; last diagonal entry dl) from the signs of the leading
 // minors p_j = (d_j - x) p_{j-1} - e2_{j-1} p_{j-2}, rescaled before they leave the double range; a zero minor takes the
-// sign of its predecessor.  No division: the quotients of sturm_count are a chain of dependent divisions.
+// sign of its predecessor.  No division: the quotients of successive minors are a chain of dependent divisions.
 __device__ inline int sturm_minors(int n, const double* d, const double* e2, double dl, double x) {
   int cnt = 0;
   double p0 = 1.0, p1 = (n > 1 ? d[0] : dl) - x;
@@ -499,7 +470,7 @@ __device__ inline void bp_asymptote_warp(const double* a, const double* b, int n
   double B = sqrt(0.5 * (b[n - 1] * b[n - 1] + b[n - 2] * b[n - 2]));
   for (int it = 0; it < 500; ++it) {
     const double dl = upper ? a[n - 1] + B : a[n - 1] - B;
-    double lo = dl, hi = dl;   // Gershgorin bounds, widened as tridiag_extreme's
+    double lo = dl, hi = dl;   // Gershgorin bounds, a little widened
     for (int i = 0; i < n; ++i) {
       const double r = (i > 0 ? fabs(b[i - 1]) : 0.0) + (i < n - 1 ? fabs(b[i]) : 0.0), x = i < n - 1 ? d[i] : dl;
       lo = fmin(lo, x - r);

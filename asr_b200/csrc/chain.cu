@@ -1212,10 +1212,12 @@ __global__ void k_init(BatchView bv, typename St2<ST>::T* u, typename St2<ST>::T
   }
 }
 
+// shared memory of the FP32 step; for FP64 the size that the limit on bond tables is set by (an operation counts eight bytes;
+// the kernel's own is MmaSm)
 size_t smul_smem(const asr_op* op, size_t st_size) {
   size_t b = (size_t)op->ntype * (op->nslot + 1) * 9 * RW * st_size;
   b = (b + 15) & ~(size_t)15;
-  b += (size_t)op->nop * (st_size == sizeof(float) ? OPW * sizeof(uint32_t) : sizeof(unsigned long long));
+  b += (size_t)op->nop * (st_size == sizeof(float) ? OPW * sizeof(uint32_t) : 8);
   return b;
 }
 
@@ -1270,7 +1272,6 @@ int step_apply(asr_ctx* ctx, asr_op* op, const BatchView& bv, bool fused, bool a
   cudaStream_t s = ctx->stream;
   OpView ov = op->view();
   const ST* blk = std::is_same<ST, double>::value ? (const ST*)op->d_blocks : (const ST*)op->d_blocks_f;
-  size_t sm = smul_smem(op, sizeof(ST));
   dim3 B(WPB * TL);
   if (fused) {
     launch_smul<ST, true, true>(op, bv, blk, U, Y, part, npw, grid, s);
@@ -2042,7 +2043,6 @@ void apply_SD(asr_op* op, const BatchView& bv, bool dunif, const typename St2<ST
               typename St2<ST>::T* t2, double2* part, int npw, int grid, cudaStream_t s) {
   OpView ov = op->view();
   const ST* blk = std::is_same<ST, double>::value ? (const ST*)op->d_blocks : (const ST*)op->d_blocks_f;
-  size_t sm = smul_smem(op, sizeof(ST));
   if (dunif) {
     launch_smul<ST, true, false>(op, bv, blk, x, t2, part, npw, grid, s);
   } else {
@@ -2736,8 +2736,6 @@ int run_ed3_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, con
   for (int q = 0; q < nvec; ++q) ASR_TRY(V[q].alloc(vlen));
   T2 *T1 = V[3].p, *T3 = V[4].p, *SA = V[5].p, *TMP = V[6].p, *TV = V[7].p;
   OpView ov = op->view();
-  const ST* blk = std::is_same<ST, double>::value ? (const ST*)op->d_blocks : (const ST*)op->d_blocks_f;
-  const size_t sm = smul_smem(op, sizeof(ST));
   g_out.assign(nlane, make_double2(0, 0));
   f_out.assign(nlane, make_double2(0, 0));
   na_out.assign(nlane, 0.0);
