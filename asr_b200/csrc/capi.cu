@@ -745,6 +745,7 @@ static int chains_common(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups
         for (int q = 0; q < ngroup; ++q)
           ASR_CUDA(cudaMemcpyAsync(d_zz.p + (size_t)q * nz, d_z, nz * sizeof(double2), cudaMemcpyDeviceToDevice, s));
         cf_eval(s, d_ca.p, d_cb.p, d_n.p, NLMAX, ngroup, d_zz.p, nz, tail, d_g, nullptr, d_nf.p);
+        ctx->launches += 1;
         ASR_CUDA(cudaGetLastError());
         ASR_CUDA(cudaStreamSynchronize(s));
       } else {
@@ -752,6 +753,7 @@ static int chains_common(asr_ctx* ctx, asr_op* op, const asr_chain_group* groups
         long nt = (long)nz * ngroup;
         k_real_green<<<(unsigned)((nt + 127) / 128), 128, 0, s>>>(d_a.p, d_b.p, d_n.p, NLMAX, ngroup, d_ai.p, d_bi.p, tail, d_z, nz,
                                                                    d_g);
+        ctx->launches += 2;
         ASR_CUDA(cudaGetLastError());
         ASR_CUDA(cudaStreamSynchronize(s));
       }

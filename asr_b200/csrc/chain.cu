@@ -1264,6 +1264,12 @@ void general_mma(asr_op* op, const BatchView& bv, const double2* U, double2* H1,
   launch_smul<double, true, true, 4>(op, b, op->d_blocks, R1, Y, part, npw, grid, s);
 }
 
+// kernels of one step_apply
+inline int step_launches(bool fp64, bool any_o, bool all_dunif) {
+  if (all_dunif) return !any_o ? 1 : fp64 ? 3 : 6;
+  return any_o ? 7 : 3;
+}
+
 // One chain step of the general operator on the batch; writes y into Y and the a-partials.
 template <typename ST>
 int step_apply(asr_ctx* ctx, asr_op* op, const BatchView& bv, bool fused, bool any_o, bool all_dunif,
@@ -1493,7 +1499,7 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
       k_lanczos_w<ST><<<gridb, WPB * TL, 0, s>>>(op->view(), bvw, Y, U, UP, d_part.p, npw);
       // read y, u, u', write w per (node, lane); about 30 flops per complex element (scaled updates, projection, dot)
       ctx->prof_stop(s, ps, ASR_KERNEL_LANCZOS, (double)nt * nn * 4.0 * 9 * TL * sizeof(T2), (double)nt * nn * TL * 9 * 30.0);
-      ctx->launches += (a_in_step ? 1 : 2) + depth_due + (fused ? 1 : a_in_step ? 3 : any_o ? 7 : all_dunif ? 2 : 3);
+      ctx->launches += (a_in_step ? 1 : 2) + depth_due + step_launches(std::is_same<ST, double>::value, any_o, all_dunif);
     }
     ASR_CUDA(cudaGetLastError());
     if (opt.mode == ASR_MODE_EDC && d_g_out) {
@@ -1506,7 +1512,7 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
       ctx->launches += 2;
     }
     k_scatter_m<<<(nlp + 127) / 128, 128, 0, s>>>(nlp, d_lmap.p, d_m.p, d_m_all.p);
-    ctx->launches += 2;
+    ctx->launches += 1;
     if (a_out) {   // coefficients back to the host (tests): synchronise this batch
       ha.resize((size_t)nlp * NLMAX); hb.resize((size_t)nlp * NLMAX);
       ASR_CUDA(cudaMemcpyAsync(ha.data(), d_a.p, (size_t)nlp * NLMAX * sizeof(double2), cudaMemcpyDeviceToHost, s));
@@ -2459,9 +2465,9 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
     // launches per level: forward (operator, a reduction unless in the step, Lanczos update), recomputation (scalars,
     // operator, update), reverse (fused: 4; else 7 and the operator); the depth test's separate reductions not counted
     const int nsd = dunif ? 1 : 2;                                       // one S application
-    const int nap = gen ? 2 * nsd + 3 : (dunif ? 1 : nsd + 1);           // one operator application
+    const int nap = gen ? (dunif && std::is_same<ST, double>::value ? 3 : 2 * nsd + 3) : (dunif ? 1 : nsd + 1);   // one operator application
     const int fwd = fusedrev ? 2 : nap + 2, rev = fusedrev ? 4 : nap + 7;
-    ctx->launches += 2 + (int64_t)kmax * (fwd + (keep ? 0 : nap + 2) + rev);
+    ctx->launches += 3 + (int64_t)kmax * (fwd + (keep ? 0 : nap + 2) + rev);
   }
   return ASR_OK;
 }
@@ -3055,7 +3061,7 @@ int run_epi_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, con
       k_reduce_b<<<nt, RED_THREADS, 0, s>>>(bv, d_part.p, bpt, k, 1.0e-12);
     }
     ASR_CUDA(cudaGetLastError());
-    ctx->launches += 8 + (int64_t)kmax * (5 + (fused ? 1 : (any_o ? 7 : (dunif ? 2 : 3))));
+    ctx->launches += 8 + (int64_t)kmax * (5 + step_launches(std::is_same<ST, double>::value, any_o, dunif));
     k_ed3_final<<<(nlp + 127) / 128, 128, 0, s>>>(bv, nlp, d_lmap.p, d_c.p, d_closed.p, d_g.p, d_f.p);
     ASR_CUDA(cudaMemcpyAsync(hm.data(), d_m.p, nlp * sizeof(int), cudaMemcpyDeviceToHost, s));
     ASR_CUDA(cudaStreamSynchronize(s));
