@@ -4,12 +4,14 @@
 // (rand_r :88-124, rand_lin_amp :127-165, smul :170-203, hmul :206-215, blk_hamx :219-250, blk_project :284-304), and the
 // plain real chain lanczos (src/reference/asr_recursion.f90:17-58) on augcls_apply (src/asr_augcls.f90:275-297).
 //
-// Layout: a tile holds TL = 32 chains ("lanes", one energy or one start vector each).  Every vector of a tile is stored
-// node-major as x[((tile * nn + node) * 9 + orbital) * 32 + lane], so one warp covers one node of a tile and every
-// load of a node's orbital is one 512-byte (FP64) or 256-byte (FP32) coalesced transaction.  The 9 x 9 bond blocks are
-// kept unrotated in shared memory; the group operation of a link is applied to the gathered neighbour vector
-// (orbital permutation pi(l, g) and signs chi(g) sg(l, g)), so the block table stays (1 + nslot) x 81 per site type
-// instead of the reference's btab(9, 9, nslot, nop, ntype).
+// Layout: a tile holds TL = 32 chains ("lanes", one energy or one start vector each), and one warp covers one node of a tile.
+// Vectors are node-major, 288 values a node.  FP32 (k_smul): orbital-major rows of 32 lanes, x[((tile * nn + node) * 9 +
+// orbital) * 32 + lane], a load of a node's orbital being one 256-byte transaction.  FP64 (k_smul_mma): two quads of orbitals
+// [lane][4 orbitals], then orbital 8 as a row of lanes, the order of the tensor-core fragments (dmma.cuh).  vx() is the place of
+// an element in either.  The 9 x 9 bond blocks are kept unrotated in shared memory, and the group operation of a link
+// (orbital permutation pi(l, g) and signs chi(g) sg(l, g)) is applied to the gathered neighbour vector (FP32) or sits in the
+// block fragment (FP64), so the block table stays (1 + nslot) x 81 per site type instead of the reference's
+// btab(9, 9, nslot, nop, ntype).
 //
 // One chain step (general operator H = E_nu + h - h o h, h = c + d S d, plus X(z) = z pa + pb) is a short sequence of
 // node-parallel kernels; with d uniform and o = 0 (the edc route) it is one fused kernel: y = d S d x + (c + e + X(z)) x
@@ -316,7 +318,7 @@ __device__ __forceinline__ double2 flip_if(double2 x, uint32_t bit) {
   unsigned long long m = (unsigned long long)bit << 63;
   return make_double2(__longlong_as_double(__double_as_longlong(x.x) ^ m), __longlong_as_double(__double_as_longlong(x.y) ^ m));
 }
-constexpr int AHEAD = 148;   // blocks by which the step prefetches the rows of later nodes: half a wave at two per SM
+constexpr int AHEAD = 148;   // blocks by which the step prefetches the rows of later nodes: half a wave at two per SM of a B200
 // a node's lines of 128 bytes into L2, one or two per lane t
 __device__ __forceinline__ void prefetch_node(const void* v, int t) {
   const char* p = (const char*)v;
@@ -531,10 +533,10 @@ __global__ void __launch_bounds__(WPB * TL, 3) k_smul(OpView op, BatchView bv, c
 // octets of lanes that hold a chain (with bv.by_act: a chain that still runs): the last tile of 48 energies has two of
 // four, a real chain one.  The epilogue's arithmetic has every rounding written out (zmul, zfma), so that the forward, the
 // adjoint's recomputation and every tile shape give a lane the same bits.
-// Bound by the FP64 tensor pipe and the latency of the row gathers together (62 % of the pipe's cycles, L1 data pipe 60 %,
-// 16 warps per SM at 128 registers).  fcc ternary, 20,969 nodes, 18 slots, 16 tiles: 2.44 ms per launch (27 TFLOP/s by
-// 6,156 flops per node and lane) with the loads one product step ahead, 2.60 ms without; plain FP64 FMAs (one lane per
-// thread, broadcast block reads) 4.06 ms, with fixed-offset link gathers 3.4 ms.
+// Bound by the FP64 tensor pipe and the latency of the row gathers together (53 % of the pipe's cycles, L1 data pipe 62 %,
+// 16 warps per SM at 128 registers).  fcc ternary, 20,969 nodes, 18 slots, 16 tiles: 2.53 ms per launch (26 TFLOP/s by
+// 6,156 flops per node and lane); plain FP64 FMAs (one lane per thread, broadcast block reads) 4.06 ms, with fixed-offset link
+// gathers 3.4 ms.  The loads one product step ahead gained 6 %, the prefetch into L2 3 %.
 // The diagonal weights of an operator with many classes do not fit beside the bond blocks: the RARE instantiations read them
 // from global memory.
 struct MmaSm {   // shared memory of k_smul_mma: byte offsets; tables: with the diagonal weights
@@ -1364,8 +1366,8 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
   const bool gen2 = std::is_same<ST, double>::value && all_dunif && any_o;
   const int nvec = 3 + (fused ? 0 : gen2 ? 2 : any_o ? 4 : 2);
   // 32-lane tiles per batch: larger batches amortise the per-level reductions and launch gaps; the caller's shape, else
-  // the operator's autotuned one, else the measured defaults of the fcc ternary workload (FP64 16 tiles, FP32 8, 4 nodes
-  // per warp)
+  // the operator's autotuned one, else the measured defaults of the fcc ternary workload (FP64 16 tiles, FP32 8) and the nodes
+  // per warp of the operator's size (default_npw)
   const int prec_ix = std::is_same<ST, double>::value ? 0 : 1;
   int tpb = opt.tiles_per_batch > 0 ? opt.tiles_per_batch
           : op->tuned_tpb[prec_ix] > 0 ? op->tuned_tpb[prec_ix] : (std::is_same<ST, double>::value ? 16 : 8);

@@ -87,7 +87,8 @@ struct BatchView {
 
 // nodes per warp of the node kernels where the caller leaves it open: 4 amortise a block's tables; an operator too small to
 // give every SM two blocks of 32 nodes takes fewer (395 nodes: the step of one tile takes 48 us with 4, 21 us with 1; 994 and
-// 2,536 nodes are fastest with 2).  By the operator alone, so that a lane's sums do not depend on what else runs.
+// 2,536 nodes are fastest with 2).  By the operator alone, so that a lane's sums do not depend on what else runs; the 148 SMs
+// are a B200's and not asked of the device, for the same reason.
 inline int default_npw(int nn) { return nn < 148 * 4 ? 1 : nn < 148 * 64 ? 2 : 4; }
 
 struct RunOptions {
@@ -97,7 +98,7 @@ struct RunOptions {
   int precision = ASR_FP64;
   int project = 1;
   int tiles_per_batch = 0;   // 0: automatic (the operator's tuned value, else 16 in FP64 and 8 in FP32)
-  int nodes_per_warp = 0;    // 0: automatic (the operator's tuned value, else 4)
+  int nodes_per_warp = 0;    // 0: automatic (the operator's tuned value, else default_npw)
 };
 
 // owning device buffer of a call (freed on scope exit)

@@ -18,7 +18,7 @@
 // Layout.  A node's 9 x 32 values are stored as two quads of orbitals, [quad][lane][4 orbitals], then orbital 8, [lane].
 // The fragment load of a quad then reads 128 contiguous bytes per eight threads (4 L1 wavefronts per 512-byte load);
 // orbital-major rows would put the four columns of every eight threads on four lines (16 wavefronts: the L1 data pipe 91 %
-// busy, 3.9 ms per launch of the fcc ternary workload against 2.4 ms in this layout).
+// busy, 3.9 ms per launch of the fcc ternary workload; the first form in this layout took 2.6).
 #pragma once
 #include "common.cuh"
 

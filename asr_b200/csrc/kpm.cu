@@ -1,9 +1,10 @@
 // Kernel polynomial method on an explicit supercell: kpm_moments / kpm_dos (src/reference/asr_kpm.f90:39-87) on the
 // realisation operator lmto_real_op (src/reference/asr_lmto_realization.f90:120-191), generalised to n species.
 //
-// Layout: the nvec random vectors are the innermost index, x[(site * 9 + l) * V + v] with V = 64, so one block row of
-// 64 threads covers one site of every vector and each orbital load is coalesced.  The bond blocks sit in shared
-// memory; d and c per species are tiny tables there too.  One Chebyshev step is one kernel:
+// Layout: the nvec random vectors are the innermost index, x[(site * 9 + l) * V + v] with V = 64, so that each orbital
+// load of a site is coalesced; the FP64 step of the scaled recurrence (k_cheb_d) keeps pairs of vectors in the order of the
+// tensor-core fragments instead (dmma.cuh, cheb_at()).  The bond blocks sit in shared memory; d and c per species are tiny
+// tables there too.  One Chebyshev step is one kernel:
 //     t_{n+1} = 2 (H t_n - cen t_n) / sc - t_{n-1}   (n = 0: t_1 = (H t_0 - cen t_0) / sc),  H = e + c + d S d  (o = 0)
 // with the FP64 partial dots r . t_{n+1}, t_{n+1} . t_{n+1} and t_{n+1} . t_n per vector.  The Rademacher vectors r are
 // regenerated from a counter-based hash (splitmix64) instead of being read.  Two moment sets come out of one matvec
@@ -191,8 +192,8 @@ __device__ __forceinline__ void cheb_reduce(double2 rt, double2 tt, double2 tp, 
 
 // FP32: thread = pair.  The neighbour indices of a site are read once, one per thread.  Per output the FMAs run over the
 // on-site block, then the slots, nine source orbitals each; the rows of the next slot are in flight while a slot is
-// multiplied.  Bound by the shared-memory block reads (25 broadcasts per slot and site) and the gathers' latency.  256,000
-// sites x 64 vectors: 1.73 ms per step (29 TFLOP/s) at two blocks per SM; 2.11 ms without the prefetch, 1.90 / 2.24 ms at three
+// multiplied.  Bound by the shared-memory block reads (25 broadcasts per slot and site; L1 data pipe 73 %, FMA pipe 46 %,
+// issue 0.51 a cycle) and the gathers' latency.  256,000 sites x 64 vectors: 1.73 ms per step (29 TFLOP/s) at two blocks per SM; 2.11 ms without the prefetch, 1.90 / 2.24 ms at three
 // blocks (80 registers) without / with it; one vector per thread and scalar FMAs 2.49 ms.
 template <bool WANT_R>
 __global__ void __launch_bounds__(KW * 32, 2) k_cheb_f(ScView S, const float* __restrict__ blocks, const double* __restrict__ coef,
@@ -251,8 +252,8 @@ __global__ void __launch_bounds__(KW * 32, 2) k_cheb_f(ScView S, const float* __
   cheb_reduce(D.rt, D.tt, D.tp, t, part);
 }
 
-// FP64: NJ octets of pairs (16 vectors each).  Bound by the FP64 tensor pipe and the gathers' latency, as the chain step.
-// 48,668 sites x 64 vectors: 0.40 ms per step (24 TFLOP/s); plain FP64 FMAs, one vector per thread, 1.31 ms.
+// FP64: NJ octets of pairs (16 vectors each).  Bound by the FP64 tensor pipe (60 % of its cycles, and the largest stall) and the
+// gathers' latency, as the chain step.  48,668 sites x 64 vectors: 0.41 ms per step (23.4 TFLOP/s); plain FP64 FMAs, one vector per thread, 1.31 ms.
 template <bool WANT_R, int NJ>
 __global__ void __launch_bounds__(KW * 32, 2) k_cheb_d(ScView S, const double* __restrict__ blocks, const double* __restrict__ coef,
                                                        const double2* __restrict__ u, const double2* __restrict__ uold,
