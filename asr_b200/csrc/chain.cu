@@ -1375,8 +1375,9 @@ int run_lanes_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, c
   // projections: per tile nlevmax x 9 nt x 32 complex values
   const size_t proj_tile_bytes = proj ? (size_t)nlevmax * 9 * proj->nt * TL * sizeof(double2) : 0;
   tpb = std::min(tpb, ntile_all);
-  const size_t freeb = ctx->plan_bytes((size_t)tpb * (nvec * vec_bytes + proj_tile_bytes), proj ? 2 : 1);
+  const size_t freeb = ctx->plan_bytes({(size_t)tpb * nvec * vec_bytes, (size_t)tpb * proj_tile_bytes});
   while (tpb > 1 && (size_t)tpb * (nvec * vec_bytes + proj_tile_bytes) > freeb / 2) tpb /= 2;
+  ctx->mem->room((size_t)tpb * (nvec * vec_bytes + proj_tile_bytes), freeb);
   int npw = opt.nodes_per_warp > 0 ? opt.nodes_per_warp : op->tuned_npw[prec_ix] > 0 ? op->tuned_npw[prec_ix] : default_npw(nn);
   if (const char* e = getenv("ASR_NODES_PER_WARP")) npw = std::max(1, atoi(e));
   const int npb = WPB * npw;
@@ -2143,6 +2144,7 @@ int run_adjoint_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo,
     tpb = (int)std::min<size_t>(tpb, ctx->mem->keep / ((size_t)nvec * vec_bytes));
   if ((size_t)nvec * vec_bytes > freeb) { set_error("adjoint: %d vectors of %zu bytes do not fit", nvec, vec_bytes); return ASR_ENOMEM; }
   tpb = std::min(tpb, ntile_all);
+  ctx->mem->room((size_t)tpb * nvec * vec_bytes, freeb);
   const int npw = default_npw(nn), npb = WPB * npw, bpt = (nn + npb - 1) / npb;
   int gnpb = 64;   // nodes per block of the gradient kernel (16 on the 994-node operator: 155 us a level for 116, the block sums)
   if (const char* e = getenv("ASR_ADJ_GRAD_NODES")) gnpb = std::max(1, atoi(e));
@@ -2720,6 +2722,7 @@ int run_ed3_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, con
   while (tpb > 1 && (size_t)tpb * nvec * vec_bytes > freeb / 2) tpb /= 2;
   if ((size_t)nvec * vec_bytes > freeb) { set_error("ed3: %d vectors of %zu bytes do not fit", nvec, vec_bytes); return ASR_ENOMEM; }
   tpb = std::min(tpb, ntile_all);
+  ctx->mem->room((size_t)tpb * nvec * vec_bytes, freeb);
   const int npw = default_npw(nn), npb = WPB * npw, bpt = (nn + npb - 1) / npb;
   const int nlp = tpb * TL;
   Dev<double> d_gblob, d_oc, d_na, d_nv, d_tn;
@@ -2962,6 +2965,7 @@ int run_epi_t(asr_ctx* ctx, asr_op* op, const std::vector<GroupInfo>& ginfo, con
   while (tpb > 1 && (size_t)tpb * nvec * vec_bytes > freeb / 2) tpb /= 2;
   if ((size_t)nvec * vec_bytes > freeb) { set_error("epi_blocks: %d vectors of %zu bytes do not fit", nvec, vec_bytes); return ASR_ENOMEM; }
   tpb = std::min(tpb, ntile_all);
+  ctx->mem->room((size_t)tpb * nvec * vec_bytes, freeb);
   const int npw = default_npw(nn), npb = WPB * npw, bpt = (nn + npb - 1) / npb;
   const int nlp = tpb * TL;
   Dev<double> d_gblob, d_v9, d_nv;

@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cstddef>
 #include <cstdint>
+#include <initializer_list>
 #include <mutex>
 
 namespace asrb {
@@ -73,9 +74,8 @@ struct DevStore {
   bool get(size_t bytes, cudaStream_t s, Block& b) {
     {
       std::lock_guard<std::mutex> g(lock);
-      int at = -1;
-      for (int q = 0; q < n; ++q)
-        if (blocks[q].bytes >= bytes && blocks[q].bytes / 2 <= bytes && (at < 0 || blocks[q].bytes < blocks[at].bytes)) at = q;
+      const bool taken[MOST] = {};
+      const int at = fit(bytes, taken);
       if (at >= 0) {
         if (cudaStreamWaitEvent(s, blocks[at].done, 0) != cudaSuccess) {
           cudaGetLastError();
@@ -136,18 +136,30 @@ struct DevStore {
     plans = 0;
     return freeb;
   }
-  // Bytes a call may plan with: free device memory and what is held unused.  A call that needs at most `need` bytes for its
-  // largest batch plans the same with any figure of twice that or more, so the device (0.1 to 1 ms) is not asked every time
-  // where what is held will do.  That is so for one array; with several, a held block may serve a small one and leave no
-  // room for the others.
-  size_t plan(size_t need, int arrays = 1) {
-    if (arrays == 1) {
+  // Bytes a call may plan with: free device memory and what is held unused.  need: the arrays of its largest batch, in the order
+  // in which it will take them.  The call plans the same with any figure of twice their sum or more, so the device (0.1 to 1 ms)
+  // is not asked every time where what is held will serve every one of them (a block that serves a small array may leave no
+  // room for the others).
+  size_t plan(std::initializer_list<size_t> need) {
+    {
       std::lock_guard<std::mutex> g(lock);
-      bool fits = pool_unused() / 2 >= need;
-      for (int q = 0; q < n; ++q) fits = fits || (blocks[q].bytes >= need && blocks[q].bytes / 2 <= need);
-      if (fits && ++plans < LOOK) return 2 * need;
+      bool taken[MOST] = {}, ok = true;
+      size_t sum = 0, small = 0;
+      for (size_t bytes : need) {
+        sum += bytes;
+        if (bytes < BIG) { small += bytes; continue; }
+        const int at = fit(bytes, taken);
+        if (at >= 0) taken[at] = true;
+        else ok = false;
+      }
+      if (ok && pool_unused() / 2 >= small && ++plans < LOOK) return 2 * sum;
     }
     return look();
+  }
+  // before a call takes `need` of the freeb bytes that it may plan with: where that is most of them, what is held goes back,
+  // so that no array sits in a block of up to twice its size and leaves too little for the others
+  void room(size_t need, size_t freeb) {
+    if (need > freeb / 2) trim();
   }
 
  private:
@@ -157,6 +169,13 @@ struct DevStore {
         cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess || held <= used)
       return 0;
     return (size_t)(held - used);
+  }
+  // the held block that serves an array (-1: none), of those not taken
+  int fit(size_t bytes, const bool* taken) const {
+    int at = -1;
+    for (int q = 0; q < n; ++q)
+      if (!taken[q] && blocks[q].bytes >= bytes && blocks[q].bytes / 2 <= bytes && (at < 0 || blocks[q].bytes < blocks[at].bytes)) at = q;
+    return at;
   }
   // held blocks down to `most` bytes and `count` (under the lock)
   void drop(size_t most, int count) {

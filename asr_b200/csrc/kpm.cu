@@ -476,7 +476,8 @@ int kpm_run(asr_ctx* ctx, asr_supercell* sc, double cen, double scl, int nmom, i
   const size_t smem = 4 * 9 * sc->nsp * sizeof(double) + (size_t)(sc->ns + 1) * 81 * sizeof(ST);
   const bool general = !sc->o_zero;
   const int grid = ctx->num_sms * 4;
-  ctx->plan_bytes(nel * sizeof(ST));   // whether memory is scarce, where the arrays are not held
+  const size_t one = nel * sizeof(ST);
+  ctx->mem->room((general ? 6 : 3) * one, general ? ctx->plan_bytes({one, one, one, one, one, one}) : ctx->plan_bytes({one, one, one}));
   DevBuf<ST> T0, T1, T2, W1, W2, W3;
   ASR_TRY(T0.alloc(nel)); ASR_TRY(T1.alloc(nel)); ASR_TRY(T2.alloc(nel));
   if (general) { ASR_TRY(W1.alloc(nel)); ASR_TRY(W2.alloc(nel)); ASR_TRY(W3.alloc(nel)); }

@@ -56,7 +56,7 @@ struct asr_ctx {
   size_t ws_bytes = 0;
   asrb::DevStore* mem = nullptr;   // the device's, of the calls' temporaries
   // bytes a call may plan with (DevStore::plan), the held slab with it
-  size_t plan_bytes(size_t need = SIZE_MAX / 2, int arrays = 1) { return mem->plan(need, arrays) + ws_bytes; }
+  size_t plan_bytes(std::initializer_list<size_t> need = {SIZE_MAX / 2}) { return mem->plan(need) + ws_bytes; }
   void ws_release() {
     if (ws) cudaFree(ws);
     ws = nullptr;

@@ -16,7 +16,7 @@ static bool call(DevStore& st, std::initializer_list<size_t> sizes, const void* 
   MemScope scope(&st, nullptr, ctx);
   size_t most = 0;
   for (size_t s : sizes) most = s > most ? s : most;
-  st.plan(most);
+  st.plan({most});
   DevMem m[8];
   int k = 0;
   bool ok = true;
@@ -89,7 +89,7 @@ static void contexts() {
   st.close(nullptr, &c);
   CHECK(call(st, {8 * GB}, &a) && call(st, {33 * MB, MB}, &b));
   fake().others = fake().total - 60 * GB;
-  CHECK(st.plan(SIZE_MAX / 2) == 60 * GB);
+  CHECK(st.plan({SIZE_MAX / 2}) == 60 * GB);
   CHECK(call(st, {59 * GB}, &b));
   fake().others = 0;
   st.trim();
@@ -127,7 +127,7 @@ static void planned() {
       const size_t proj = GB / 2, vec = 3 * GB / 4;   // a tile's
       MemScope scope(&st, nullptr, nullptr);
       size_t tiles = 8;
-      const size_t freeb = st.plan(tiles * (proj + vec), 2);
+      const size_t freeb = st.plan({tiles * vec, tiles * proj});
       while (tiles > 1 && tiles * (proj + vec) > freeb / 2) tiles /= 2;
       DevMem a, b;
       CHECK(a.get(tiles * vec) && b.get(tiles * proj));
@@ -137,6 +137,24 @@ static void planned() {
       st.close(nullptr, nullptr);
       CHECK(fake().used == 0);
     }
+}
+
+// several arrays that together need nearly all there is: a held block of up to twice an array's size is not taken for it
+static void limit() {
+  DevStore st;
+  st.open(0, fake().total);
+  CHECK(call(st, {20 * GB}));
+  fake().others = fake().total - 46 * GB;
+  {
+    MemScope scope(&st, nullptr, nullptr);
+    st.room(44 * GB, st.plan({SIZE_MAX / 2}));
+    DevMem m[4];
+    for (DevMem& x : m) CHECK(x.get(11 * GB));
+    for (DevMem& x : m) x.put();
+  }
+  fake().others = 0;
+  st.close(nullptr, nullptr);
+  CHECK(fake().used == 0);
 }
 
 int main(int argc, char** argv) {
@@ -149,6 +167,7 @@ int main(int argc, char** argv) {
     else if (s == "contexts") contexts();
     else if (s == "lasting") lasting();
     else if (s == "planned") planned();
+    else if (s == "limit") limit();
     else { std::printf("no case %s\n", argv[k]); bad = 1; }
   }
   return bad;

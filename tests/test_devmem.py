@@ -16,7 +16,7 @@ def check(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("case", ["reuse", "many", "scarce", "scarce_later", "contexts", "lasting", "planned"])
+@pytest.mark.parametrize("case", ["reuse", "many", "scarce", "scarce_later", "contexts", "lasting", "planned", "limit"])
 def test_devmem(check, case):
     r = subprocess.run([check, case], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout
